@@ -92,13 +92,13 @@ __device__ __forceinline__ V3 vmf4SampleRef(const float4* L, Pcg& rng) {
     const float u = rng.randf();
     const float v = rng.randf();
     const float r = sqrtf(u);
-    const float theta = (float)((double)(2.0f * kPi * v) - kPiD);
+    const float theta = crMinusPi(2.0f * kPi * v);
     float st, ct;
     crSinCosf(theta, &st, &ct);
     const float vx = r * ct, vy = r * st;
     const float u2 = rng.randf();
     const float W =
-        kappa > 0.0f ? 1.0f + crPowf(kappa, -1.0f) * crLogf(u2 + (1.0f - u2) * crExpf(-2.0f * kappa)) : 1.0f;
+        kappa > 0.0f ? 1.0f + __frcp_rn(kappa) * crLogf(u2 + (1.0f - u2) * crExpf(-2.0f * kappa)) : 1.0f;
     const float sq = safeSqrt(1.0f - W * W);  // powf(W, 2) rounds W^2 once, as the product does
     Basis basis(normalize(mu));
     return normalize(basis.toGlobal(W, sq * vx, sq * vy));
@@ -182,11 +182,11 @@ struct MetalD {  // Material.h:275-384
         V3 Vh = normalize(V3(Ve.x, alpha * Ve.y, alpha * Ve.z));
         float lensq = Vh.y * Vh.y + Vh.z * Vh.z;
         V3 T1 = lensq > 0 ? V3(0, -Vh.z, Vh.y) / safeSqrt(lensq) : V3(0, 0, 1);
-        V3 T2 = cross(Vh, T1);
+        V3 T2 = crossZeroX(Vh, T1);
         float U1 = rng.randf();
         float U2 = rng.randf();
         float r = sqrtf(U1);
-        float phi = (float)(2.0 * kPiD * (double)U2);  // 2.0f * M_PI * U2 in double, as the reference
+        float phi = crTwoPi(U2);  // 2.0f * M_PI * U2 as the reference's double rounds
         float sp, cp;
         crSinCosf(phi, &sp, &cp);
         float t1 = r * cp;
@@ -245,7 +245,7 @@ struct GlossyD {  // Material.h:88-132; clamped: Main.cpp:34-84
         Basis basis(s.sn);
         float sq = safeSqrt(1 - crPowf(r2, 2 / (sh + 1.0f)));
         float sp, cp;
-        crSinCosf((float)(2.0 * kPiD * (double)r1), &sp, &cp);  // cosf(2 * M_PI * r1): the argument in double
+        crSinCosf(crTwoPi(r1), &sp, &cp);  // cosf(2 * M_PI * r1): the argument as the double rounds
         V3 h = normalize(basis.toGlobal(crPowf(r2, 1 / (sh + 1.0f)), cp * sq, sp * sq));
         *wi = -normalize(s.wo - (2.0f * dot(s.wo, h)) * h);
         *p = pdf(s, *wi);
@@ -557,7 +557,7 @@ __device__ __forceinline__ V3 bsdfCosT(const SceneDev& sc, const Material& m, co
 template <int NESTED>
 __device__ __forceinline__ float getPDFT(const SceneDev& sc, const Material& m, const Surface& s, V3 wi) {
     if ((NESTED & 2) && m.kind == MAT_MULTILOBE_SVBRDF)  // Main.cpp:497-499, divided by the double M_PI
-        return (float)((double)clampPositive(dot(s.sn, wi)) / kPiD);
+        return crOverPi(clampPositive(dot(s.sn, wi)));
     if ((NESTED & 1) && m.kind == MAT_MF_NORMALMAP) return getPDFMfnm(sc, m, s, wi);
     return pdfBasic<NESTED>(sc, m, s, wi);
 }

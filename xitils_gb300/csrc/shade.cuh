@@ -189,8 +189,12 @@ __device__ __forceinline__ void loadMixture(const float4* m, VmfMixture& mx) {
 // Mpaths/s -- while the Lambert-only variant stays at three (the Cornell box
 // 9.5 against 9.9 ms of shading over five renders at four, the room 40.8
 // against 42.2). Without emitters (no emission, no NEE code) and with the
-// standard integrator only, the metal variant shades the terrain in 9.2 ms per
+// standard integrator only, the metal variant shaded the terrain in 9.2 ms per
 // render at four blocks (1878 Mpaths/s) and 9.1 ms at five (51 registers, 1884).
+// All of these were bound by the FP64 pipe (61 % busy in the terrain, 68 % in the
+// shell-mapped cloth): the frames' cross products and the glossy pow now round through
+// float pairs (crmath.cuh), 38.4 -> 36.7 ms for the whole terrain render, 44.9 -> 41.1
+// for the cloth, 7.1 -> 6.65 for normal mapping.
 template <class J, int NESTED, bool EXTRAS>
 __global__ void __launch_bounds__(kShadeBlock, (NESTED & 3) ? 2 : (NESTED & kNoEmitters) ? 5 : (NESTED & kOnlyMetal) ? 4 : 3) k_shade(J jobs, PathQueue in, HitQueue hq, PathQueue out,
                                                        ShadowQueue sq, Ctrl* ctrl) {

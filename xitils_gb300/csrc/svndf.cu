@@ -83,7 +83,7 @@ __global__ void __launch_bounds__(32 * kSvWarps) k_svndfFit(TextureDev src, floa
             const float u = rng.randf();
             const float v = rng.randf();
             const float theta = crAsinf(u);
-            const float phi = (float)((double)(2.0f * kPi * v) - kPiD);
+            const float phi = crMinusPi(2.0f * kPi * v);
             float st, ct, sp, cp;
             crSinCosf(theta, &st, &ct);
             crSinCosf(phi, &sp, &cp);
@@ -124,7 +124,7 @@ __global__ void __launch_bounds__(32 * kSvWarps) k_svndfFit(TextureDev src, floa
             r = r / a;
             a /= (float)n;
             const float len = length(r);
-            float kappa = (3 * len - crPowf(len, 3.0f)) / (1.0f - dot(r, r));
+            float kappa = (3 * len - crCubef(len)) / (1.0f - dot(r, r));
             const V3 mu = normalize(r);
             if (kappa > kSvKappaLimit) kappa = kSvKappaLimit;
             if (kappa < 0.0f) kappa = 0.0f;

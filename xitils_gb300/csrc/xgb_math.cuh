@@ -5,7 +5,7 @@
 //   dot(a, b)   = (a.x*b.x + a.y*b.y) + (a.z*b.z + 0)   (libsimdpp SSE3 horizontal adds)
 //   v / s       = v * (1 / s)                            (Vector.h:356-361)
 //   normalize   = v / length(v)                          (Vector.h:615)
-//   cross       = FP64 products rounded once to float    (Vector.h:637-654)
+//   cross       = FP64 products rounded once to float    (Vector.h:637-654), here by exact float sums
 // Translation units that include this header for shading are compiled with
 // -fmad=false so that no multiply-add is contracted, matching the reference's
 // unfused float arithmetic; transcendental functions are CUDA's own.
@@ -14,11 +14,9 @@
 #include <math.h>
 #include <stdint.h>
 
-namespace xgb {
+#include "crmath.cuh"
 
-#ifndef XGB_CROSS64
-#define XGB_CROSS64 1
-#endif
+namespace xgb {
 
 constexpr float kPi = 3.14159265358979323846f;  // (float)M_PI, Utils.h:32
 constexpr double kPiD = 3.14159265358979323846;
@@ -52,12 +50,12 @@ __device__ __forceinline__ float safeSqrt(float x) { return sqrtf(clampPositive(
 __device__ __forceinline__ float minf_ref(float a, float b) { return a < b ? a : b; }
 
 __device__ __forceinline__ V3 cross(V3 a, V3 b) {
-#if XGB_CROSS64
-    double ax = a.x, ay = a.y, az = a.z, bx = b.x, by = b.y, bz = b.z;
-    return V3((float)(ay * bz - az * by), (float)(az * bx - ax * bz), (float)(ax * by - ay * bx));
-#else
-    return V3(a.y * b.z - a.z * b.y, a.z * b.x - a.x * b.z, a.x * b.y - a.y * b.x);
-#endif
+    return V3(cr::diffProd(a.y, b.z, a.z, b.y), cr::diffProd(a.z, b.x, a.x, b.z), cr::diffProd(a.x, b.y, a.y, b.x));
+}
+// cross(a, b) with b.x exactly zero: two components are single products, which one
+// float multiplication rounds as the FP64 expression does.
+__device__ __forceinline__ V3 crossZeroX(V3 a, V3 b) {
+    return V3(cr::diffProd(a.y, b.z, a.z, b.y), -__fmul_rn(a.x, b.z), __fmul_rn(a.x, b.y));
 }
 
 // Utils.h:81-83
@@ -71,17 +69,21 @@ __device__ __forceinline__ float2 lerp3(float2 a, float2 b, float2 c, float t1, 
 
 __device__ __forceinline__ V3 v3(float4 a) { return V3(a.x, a.y, a.z); }
 
-// Vector.h:781-795. cross(v, axis) with a unit axis is exact in float.
+// Vector.h:781-795. cross(v, axis) with a unit axis is exact in float, and leaves that
+// axis' component zero, so of cross(e1, e2) only that component is a difference of
+// two products: the frame is computed with the axis rotated to x and rotated back.
 struct Basis {
     V3 e1, e2, e3;
     __device__ explicit Basis(V3 v) {
         e1 = normalize(v);
-        V3 c;
-        if (fabsf(v.x) < 0.5f) c = V3(v.y * 0.0f - v.z * 0.0f, v.z * 1.0f - v.x * 0.0f, v.x * 0.0f - v.y * 1.0f);
-        else if (fabsf(v.y) < 0.5f) c = V3(v.y * 0.0f - v.z * 1.0f, v.z * 0.0f - v.x * 0.0f, v.x * 1.0f - v.y * 0.0f);
-        else c = V3(v.y * 1.0f - v.z * 0.0f, v.z * 0.0f - v.x * 1.0f, v.x * 0.0f - v.y * 0.0f);
-        e2 = normalize(c);
-        e3 = normalize(cross(e1, e2));
+        const bool ax = fabsf(v.x) < 0.5f, ay = !ax && fabsf(v.y) < 0.5f;
+        // (axis, next, next but one) of v and e1
+        const float vj = ax ? v.y : ay ? v.z : v.x, vk = ax ? v.z : ay ? v.x : v.y;
+        const V3 r1(ax ? e1.x : ay ? e1.y : e1.z, ax ? e1.y : ay ? e1.z : e1.x, ax ? e1.z : ay ? e1.x : e1.y);
+        const V3 r2 = normalize(V3(0.0f, vk, -vj));
+        const V3 r3 = crossZeroX(r1, r2);
+        e2 = ax ? r2 : ay ? V3(r2.z, r2.x, r2.y) : V3(r2.y, r2.z, r2.x);
+        e3 = normalize(ax ? r3 : ay ? V3(r3.z, r3.x, r3.y) : V3(r3.y, r3.z, r3.x));
     }
     __device__ V3 fromGlobal(V3 v) const { return V3(dot(v, e1), dot(v, e2), dot(v, e3)); }
     __device__ V3 toGlobal(float x, float y, float z) const { return e1 * x + e2 * y + e3 * z; }
