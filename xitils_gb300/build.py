@@ -4,7 +4,7 @@ Each CUDA translation unit is compiled by nvcc in parallel with
 ``-gencode arch=compute_103a,code=sm_103a`` and linked into the in-tree shared
 library ``xitils_gb300/libxgb.so`` (CUDA runtime linked statically; no PyTorch
 dependency). Per-unit flags:
-  * integrator.cu, shade_*.cu, svndf.cu: ``-fmad=false``
+  * integrator.cu, shade_*.cu, tail*.cu, svndf.cu: ``-fmad=false``
     -- shading and fitting arithmetic stays unfused, as in the reference's float code;
   * api.cu: host code compiled with ``-ffp-contract=off`` for the same reason.
 """
@@ -31,6 +31,7 @@ UNITS = {
     "guide.cu": [], "guide_tc.cu": [], "image.cu": [], "batch.cu": [],
     "svndf.cu": ["-fmad=false"],
     "shade_layered.cu": ["-fmad=false"], "shade_nested.cu": ["-fmad=false"], "shade_batch_nested.cu": ["-fmad=false"],
+    "tail.cu": ["-fmad=false"], "tail_layered.cu": ["-fmad=false"], "tail_nested.cu": ["-fmad=false"],
 }
 
 

@@ -1345,8 +1345,24 @@ xgb_status xgb_render(xgb_scene* s, const xgb_integrator_params* params, xgb_fil
     double stageMs[5] = {0, 0, 0, 0, 0};
     double inferMs = 0.0, trainMs = 0.0;
     uint64_t launches = 0;
+    // Tail launches (tail.cuh) instead of wavefront iterations once at most tailMax paths are
+    // left: not with a learned proposal, whose inference is a launch of its own per vertex,
+    // nor while profiling, which attributes every stage; traversal limits other than the
+    // defaults count the steps of the wavefront's kernels.
+    const bool tail = !gd && !prof && s->maxSteps == kDefaultMaxSteps && s->stackLimit == kMaxStackLimit;
+    const unsigned int tailMax = tailMaxPaths(s->sd);
+    // Once every camera path has started the counters are read every two iterations, so
+    // that the tail starts in time; a call not much larger than a tail begins that way.
+    bool ending = total <= cap && total <= 16ull * tailMax;
     for (int guard = 0;; ++guard) {
-        for (int k = 0; k < kIterPerCheck; ++k) {
+        const bool direct = tail && guard == 0 && total <= tailMax && total <= cap;
+        if (direct) {
+            launchPlan(s->ctrl, cap, st, kPlanTail);
+            launchGenerate(s->sd, rp, s->rb.q[parity], s->ctrl, gShade, st);
+            launches += 2;
+        }
+        const int nIter = direct ? 0 : tail && ending ? 2 : kIterPerCheck;
+        for (int k = 0; k < nIter; ++k) {
             PathQueue& X = s->rb.q[parity];
             PathQueue& Y = s->rb.q[parity ^ 1];
             cudaEvent_t* ev = prof ? &s->events[kEv * k] : nullptr;
@@ -1369,9 +1385,16 @@ xgb_status xgb_render(xgb_scene* s, const xgb_integrator_params* params, xgb_fil
             launches += 5;
             parity ^= 1;
         }
+        if (tail) {
+            if (!direct) { launchPlan(s->ctrl, cap, st, kPlanTailIfFew, tailMax); ++launches; }
+            launchTail(s->sd, rp, s->rb.q[parity], s->rb.q[parity ^ 1], s->ctrl, ctx->numSMs, st);
+            ++launches;
+        }
         XGB_CUDA(ctx, cudaGetLastError());
         XGB_CUDA(ctx, cudaMemcpyAsync(s->ctrlHost, s->ctrl, sizeof(Ctrl), cudaMemcpyDeviceToHost, st));
         XGB_CUDA(ctx, cudaStreamSynchronize(st));
+        if (tail && s->ctrlHost->nTail) parity ^= 1;
+        ending = s->ctrlHost->nextPath >= s->ctrlHost->totalPaths;
         if (prof) {
             // stages: plan, generate, extend, [guide inference], shade, shadow
             for (int k = 0; k < kIterPerCheck; ++k) {

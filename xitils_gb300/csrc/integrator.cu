@@ -16,9 +16,11 @@
 
 namespace xgb {
 
-__global__ void k_plan(Ctrl* c, unsigned int capacity) {
+__global__ void k_plan(Ctrl* c, unsigned int capacity, int mode, unsigned int tailMax) {
     unsigned int nCont = c->nOut;
     unsigned long long remain = c->totalPaths - c->nextPath;
+    c->nTail = 0;
+    if (mode == kPlanTailIfFew && (remain != 0 || nCont == 0 || nCont > tailMax)) return;
     unsigned long long room = capacity - nCont;
     unsigned int nNew = (unsigned int)(remain < room ? remain : room);
     c->firstNew = c->nextPath;
@@ -30,6 +32,7 @@ __global__ void k_plan(Ctrl* c, unsigned int capacity) {
     c->extendHead = 0;
     c->shadowHead = 0;
     if (c->nActive) c->iterations += 1;
+    if (mode != kPlanWave) c->nTail = c->nActive;
 }
 
 // Camera paths: RenderTargetTile::GenerateFilmPosition (RenderTarget.h:68-80)
@@ -130,7 +133,9 @@ __global__ void __launch_bounds__(kShadeBlock) k_generate(J jobs, PathQueue q, c
     }
 }
 
-void launchPlan(Ctrl* ctrl, unsigned int capacity, cudaStream_t s) { k_plan<<<1, 1, 0, s>>>(ctrl, capacity); }
+void launchPlan(Ctrl* ctrl, unsigned int capacity, cudaStream_t s, int mode, unsigned int tailMax) {
+    k_plan<<<1, 1, 0, s>>>(ctrl, capacity, mode, tailMax);
+}
 
 void launchGenerate(const SceneDev& sc, const RenderParams& rp, PathQueue q, Ctrl* ctrl, int grid, cudaStream_t s) {
     k_generate<OneJob><<<grid, kShadeBlock, 0, s>>>(OneJob{sc, rp}, q, ctrl);

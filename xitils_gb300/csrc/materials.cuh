@@ -265,6 +265,16 @@ __device__ __forceinline__ float fresnelDielectric(V3 wo, V3 n, float eta_o, flo
     return 0.5f * (a * a) * (1.0f + b * b);
 }
 
+// The glossy materials' base lobe (clamped for GlossyClamped) and GlossyWithHighLight's
+// second one: the family shares one copy of the code below, so that a kernel which
+// carries every material stays small (shading stalls on instruction fetches first).
+__device__ __forceinline__ GlossyD glossyBase(const Material& m) {
+    return GlossyD{V3(m.albedo.x, m.albedo.y, m.albedo.z), m.sharpness, m.kind == MAT_GLOSSY_CLAMPED};
+}
+__device__ __forceinline__ GlossyD glossyHighlight(const Material& m) {
+    return GlossyD{V3(m.highlight.x, m.highlight.y, m.highlight.z), m.sharpnessHL, false};
+}
+
 // ------------------------------------------------------- material dispatch --
 __device__ __forceinline__ float metalRoughness(const SceneDev& sc, const Material& m, const Surface& s) {
     if (m.tex < 0) return m.roughness;
@@ -306,11 +316,13 @@ __device__ __forceinline__ V3 bsdfCosBasic(const SceneDev& sc, const Material& m
         float r = metalRoughness(sc, m, s);
         return MetalD{r * r, V3(m.albedo.x, m.albedo.y, m.albedo.z), (m.flags & 1) != 0}.bsdfCos(s, wi);
     }
-    case MAT_GLOSSY: return GlossyD{V3(m.albedo.x, m.albedo.y, m.albedo.z), m.sharpness, false}.bsdfCos(s, wi);
-    case MAT_GLOSSY_CLAMPED: return GlossyD{V3(m.albedo.x, m.albedo.y, m.albedo.z), m.sharpness, true}.bsdfCos(s, wi);
-    case MAT_GLOSSY_HIGHLIGHT:
-        return (1.0f - m.rate) * GlossyD{V3(m.albedo.x, m.albedo.y, m.albedo.z), m.sharpness, false}.bsdfCos(s, wi) +
-               m.rate * GlossyD{V3(m.highlight.x, m.highlight.y, m.highlight.z), m.sharpnessHL, false}.bsdfCos(s, wi);
+    case MAT_GLOSSY:
+    case MAT_GLOSSY_CLAMPED:
+    case MAT_GLOSSY_HIGHLIGHT: {
+        const V3 base = glossyBase(m).bsdfCos(s, wi);
+        if (m.kind != MAT_GLOSSY_HIGHLIGHT) return base;
+        return (1.0f - m.rate) * base + m.rate * glossyHighlight(m).bsdfCos(s, wi);
+    }
     default: return V3();  // emission and delta BSDFs
     }
 }
@@ -329,11 +341,13 @@ __device__ __forceinline__ float pdfBasic(const SceneDev& sc, const Material& m,
         float r = metalRoughness(sc, m, s);
         return MetalD{r * r, V3(m.albedo.x, m.albedo.y, m.albedo.z), (m.flags & 1) != 0}.pdf(s, wi);
     }
-    case MAT_GLOSSY: return GlossyD{V3(), m.sharpness, false}.pdf(s, wi);
-    case MAT_GLOSSY_CLAMPED: return GlossyD{V3(), m.sharpness, true}.pdf(s, wi);
-    case MAT_GLOSSY_HIGHLIGHT:
-        return (1.0f - m.rate) * GlossyD{V3(), m.sharpness, false}.pdf(s, wi) +
-               m.rate * GlossyD{V3(), m.sharpnessHL, false}.pdf(s, wi);
+    case MAT_GLOSSY:
+    case MAT_GLOSSY_CLAMPED:
+    case MAT_GLOSSY_HIGHLIGHT: {
+        const float base = glossyBase(m).pdf(s, wi);
+        if (m.kind != MAT_GLOSSY_HIGHLIGHT) return base;
+        return (1.0f - m.rate) * base + m.rate * glossyHighlight(m).pdf(s, wi);
+    }
     default: return 0.0f;
     }
 }
@@ -365,24 +379,22 @@ __device__ __forceinline__ V3 sampleBasic(const SceneDev& sc, const Material& m,
         return MetalD{r * r, V3(m.albedo.x, m.albedo.y, m.albedo.z), (m.flags & 1) != 0}.evalAndSample(s, rng, wi, pdf);
     }
     case MAT_GLOSSY:
-        return GlossyD{V3(m.albedo.x, m.albedo.y, m.albedo.z), m.sharpness, false}.evalAndSample(s, rng, wi, pdf);
     case MAT_GLOSSY_CLAMPED:
-        return GlossyD{V3(m.albedo.x, m.albedo.y, m.albedo.z), m.sharpness, true}.evalAndSample(s, rng, wi, pdf);
-    case MAT_GLOSSY_HIGHLIGHT: {  // Material.h:148-162
-        GlossyD base{V3(m.albedo.x, m.albedo.y, m.albedo.z), m.sharpness, false};
-        GlossyD hl{V3(m.highlight.x, m.highlight.y, m.highlight.z), m.sharpnessHL, false};
-        V3 eval;
-        float tmp;
-        if (rng.randf() <= m.rate) {
-            V3 te = hl.evalAndSample(s, rng, wi, &tmp);
-            eval = (1.0f - m.rate) * base.bsdfCos(s, *wi) + m.rate * te;
-            *pdf = (1.0f - m.rate) * base.pdf(s, *wi) + m.rate * tmp;
-        } else {
-            V3 te = base.evalAndSample(s, rng, wi, &tmp);
-            eval = (1.0f - m.rate) * te + m.rate * hl.bsdfCos(s, *wi);
-            *pdf = (1.0f - m.rate) * tmp + m.rate * hl.pdf(s, *wi);
+    case MAT_GLOSSY_HIGHLIGHT: {  // Material.h:111-131, :148-162
+        const bool both = m.kind == MAT_GLOSSY_HIGHLIGHT;
+        const bool highlight = both && rng.randf() <= m.rate;  // which of the two is sampled
+        const GlossyD base = glossyBase(m), hl = glossyHighlight(m);
+        float ps;
+        const V3 es = (highlight ? hl : base).evalAndSample(s, rng, wi, &ps);
+        if (!both) {
+            *pdf = ps;
+            return es;
         }
-        return eval;
+        const GlossyD other = highlight ? base : hl;
+        const V3 eo = other.bsdfCos(s, *wi);
+        const float po = other.pdf(s, *wi);
+        *pdf = (1.0f - m.rate) * (highlight ? po : ps) + m.rate * (highlight ? ps : po);
+        return (1.0f - m.rate) * (highlight ? eo : es) + m.rate * (highlight ? es : eo);
     }
     case MAT_SPECULAR_REFLECTION:  // Material.h:180-187
         *wi = -normalize(s.wo - (2.0f * dot(s.sn, s.wo)) * s.sn);
@@ -407,6 +419,23 @@ __device__ __forceinline__ V3 sampleBasic(const SceneDev& sc, const Material& m,
     }
     default: return V3();  // Emission: zero, pdf untouched (Material.h:400-402)
     }
+}
+
+// The basic materials as calls, for the materials that evaluate another one: their code
+// asks for the base's sampler, value and density at up to seven places, and inlined
+// there the kernels outgrew the instruction cache.
+#ifndef XGB_NESTED_CALL
+#define XGB_NESTED_CALL __noinline__
+#endif
+static __device__ XGB_NESTED_CALL V3 bsdfCosCall(const SceneDev& sc, const Material& m, const Surface& s, V3 wi) {
+    return bsdfCosBasic(sc, m, s, wi);
+}
+static __device__ XGB_NESTED_CALL float pdfCall(const SceneDev& sc, const Material& m, const Surface& s, V3 wi) {
+    return pdfBasic(sc, m, s, wi);
+}
+static __device__ XGB_NESTED_CALL V3 sampleCall(const SceneDev& sc, const Material& m, const Surface& s, Pcg& rng, V3* wi,
+                                                float* pdf) {
+    return sampleBasic(sc, m, s, rng, wi, pdf);
 }
 
 // ---- MicrofacetNormalMapping, TangentFacetMode = SameMaterialExplicit ------
@@ -451,7 +480,7 @@ __device__ __forceinline__ Surface svbrdfPerturb(const SceneDev& sc, const Mater
 __device__ __forceinline__ V3 bsdfCosMfnm(const SceneDev& sc, const Material& m, const Surface& s, Pcg& rng, V3 wi) {
     const Material& b = sc.materials[m.base];
     MfnmFrame f = mfnmFrame(s);  // Main.cpp:94-171
-    if (f.kind == 0) return bsdfCosBasic(sc, b, s, wi);
+    if (f.kind == 0) return bsdfCosCall(sc, b, s, wi);
     if (f.kind == 1) return V3(0.0f);
     V3 result(0.0f), weight(1.0f);
     bool d = rng.randf() < lambda_p(s.wo, f.wp, f.wt, f.wg);
@@ -462,8 +491,8 @@ __device__ __forceinline__ V3 bsdfCosMfnm(const SceneDev& sc, const Material& m,
     while (true) {
         V3 wm = d ? f.wp : f.wt;
         facet.n = wm; facet.sn = wm; facet.wo = -wr;
-        result = result + weight * G1m(wi, wm, f.wp, f.wt, f.wg) * bsdfCosBasic(sc, b, facet, wi);
-        weight = weight * sampleBasic(sc, b, facet, rng, &wr, &pdf);
+        result = result + weight * G1m(wi, wm, f.wp, f.wt, f.wg) * bsdfCosCall(sc, b, facet, wi);
+        weight = weight * sampleCall(sc, b, facet, rng, &wr, &pdf);
         float g = G1m(wr, wm, f.wp, f.wt, f.wg);
         if (rng.randf() < g) break;
         d = !d;
@@ -477,7 +506,7 @@ __device__ __forceinline__ V3 bsdfCosMfnm(const SceneDev& sc, const Material& m,
 __device__ __forceinline__ float getPDFMfnm(const SceneDev& sc, const Material& m, const Surface& s, V3 wi) {
     const Material& b = sc.materials[m.base];
     MfnmFrame f = mfnmFrame(s);  // Main.cpp:254-321
-    if (f.kind == 0) return pdfBasic(sc, b, s, wi);
+    if (f.kind == 0) return pdfCall(sc, b, s, wi);
     if (f.kind == 1) return 1.0f;
     float prob = lambda_p(s.wo, f.wp, f.wt, f.wg);
     Surface facet = s;
@@ -485,13 +514,13 @@ __device__ __forceinline__ float getPDFMfnm(const SceneDev& sc, const Material& 
     float g_wi_wp = G1m(wi, f.wp, f.wp, f.wt, f.wg);
     if (prob > 0.0f) {
         facet.n = f.wp; facet.sn = f.wp;
-        pdf += prob * g_wi_wp * pdfBasic(sc, b, facet, wi);
+        pdf += prob * g_wi_wp * pdfCall(sc, b, facet, wi);
         diff += prob * (1.0f - g_wi_wp);
     }
     if (prob < 1.0f) {
         facet.n = f.wt; facet.sn = f.wt;
         float g_wi_wt = G1m(wi, f.wt, f.wp, f.wt, f.wg);
-        pdf += prob * g_wi_wt * pdfBasic(sc, b, facet, wi);
+        pdf += prob * g_wi_wt * pdfCall(sc, b, facet, wi);
         diff += prob * g_wi_wt;
     }
     return pdf + diff * clampPositive(dot(wi, f.wg)) / kPi;
@@ -501,7 +530,7 @@ __device__ __forceinline__ V3 evalAndSampleMfnm(const SceneDev& sc, const Materi
                                                 V3* wi, float* pdf) {
     const Material& b = sc.materials[m.base];
     MfnmFrame f = mfnmFrame(s);  // Main.cpp:173-252
-    if (f.kind == 0) return sampleBasic(sc, b, s, rng, wi, pdf);
+    if (f.kind == 0) return sampleCall(sc, b, s, rng, wi, pdf);
     if (f.kind == 1) return V3(0.0f);
     V3 weight(1.0f);
     bool d = rng.randf() < lambda_p(s.wo, f.wp, f.wt, f.wg);
@@ -514,7 +543,7 @@ __device__ __forceinline__ V3 evalAndSampleMfnm(const SceneDev& sc, const Materi
         ++i;
         V3 wm = d ? f.wp : f.wt;
         facet.n = wm; facet.sn = wm; facet.wo = -wr;
-        weight = weight * sampleBasic(sc, b, facet, rng, &wr, &tmppdf);
+        weight = weight * sampleCall(sc, b, facet, rng, &wr, &tmppdf);
         if (tmppdf >= 0.0f) specular = false;
         float g = G1m(wr, wm, f.wp, f.wt, f.wg);
         if (rng.randf() < g) break;
@@ -550,8 +579,9 @@ __device__ __forceinline__ V3 albedoOf(const SceneDev& sc, const Material& m, co
 template <int NESTED>
 __device__ __forceinline__ V3 bsdfCosT(const SceneDev& sc, const Material& m, const Surface& s, Pcg& rng, V3 wi) {
     if ((NESTED & 2) && m.kind == MAT_MULTILOBE_SVBRDF)  // Main.cpp:489-491
-        return bsdfCosBasic(sc, sc.materials[m.base], svbrdfPerturb(sc, m, s, rng), wi);
+        return bsdfCosCall(sc, sc.materials[m.base], svbrdfPerturb(sc, m, s, rng), wi);
     if ((NESTED & 1) && m.kind == MAT_MF_NORMALMAP) return bsdfCosMfnm(sc, m, s, rng, wi);
+    if (NESTED & 3) return bsdfCosCall(sc, m, s, wi);
     return bsdfCosBasic<NESTED>(sc, m, s, wi);
 }
 template <int NESTED>
@@ -559,6 +589,7 @@ __device__ __forceinline__ float getPDFT(const SceneDev& sc, const Material& m, 
     if ((NESTED & 2) && m.kind == MAT_MULTILOBE_SVBRDF)  // Main.cpp:497-499, divided by the double M_PI
         return crOverPi(clampPositive(dot(s.sn, wi)));
     if ((NESTED & 1) && m.kind == MAT_MF_NORMALMAP) return getPDFMfnm(sc, m, s, wi);
+    if (NESTED & 3) return pdfCall(sc, m, s, wi);
     return pdfBasic<NESTED>(sc, m, s, wi);
 }
 // Returns material_eval = f * cos / pdf and samples wi (Material.h:22-28).
@@ -567,8 +598,9 @@ template <int NESTED>
 __device__ __forceinline__ V3 evalAndSampleT(const SceneDev& sc, const Material& m, const Surface& s, Pcg& rng, V3* wi,
                                              float* pdf) {
     if ((NESTED & 2) && m.kind == MAT_MULTILOBE_SVBRDF)  // Main.cpp:493-495
-        return sampleBasic(sc, sc.materials[m.base], svbrdfPerturb(sc, m, s, rng), rng, wi, pdf);
+        return sampleCall(sc, sc.materials[m.base], svbrdfPerturb(sc, m, s, rng), rng, wi, pdf);
     if ((NESTED & 1) && m.kind == MAT_MF_NORMALMAP) return evalAndSampleMfnm(sc, m, s, rng, wi, pdf);
+    if (NESTED & 3) return sampleCall(sc, m, s, rng, wi, pdf);
     return sampleBasic<NESTED>(sc, m, s, rng, wi, pdf);
 }
 

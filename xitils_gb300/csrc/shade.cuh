@@ -176,6 +176,218 @@ __device__ __forceinline__ void loadMixture(const float4* m, VmfMixture& mx) {
     mx.lobe[4].alpha = a1.x; mx.lobe[5].alpha = a1.y; mx.lobe[6].alpha = a1.z; mx.lobe[7].alpha = a1.w;
 }
 
+// What a shade step is compiled for besides the plain radiance: first-hit planes, the
+// learned proposal (guided sampling and training records).
+constexpr int kAov = 1, kProposal = 2;
+
+// One vertex of one path: the state of a queue record (o4, d4, t4, rs; its slot i in `in`
+// for the training fields), the hit of its ray, and what follows: a continuing path, a
+// shadow ray, or neither.
+template <class J, int NESTED, int EXTRAS>
+__device__ __forceinline__ void shadeVertex(const J& jobs, const PathQueue& in, unsigned int i, float4 o4, float4 d4,
+                                            float4 t4, uint2 rs, float4 h, int instId, ShadeOut& r, bool& cont,
+                                            bool& shadow, bool& done) {
+    constexpr bool kGuide = (EXTRAS & kProposal) != 0;
+    const int prim = __float_as_int(h.w);
+    const int meta = __float_as_int(d4.w);
+    int len = meta & 0xFFFF;
+    const int flags = meta >> 16;
+    const int packed = __float_as_int(t4.w);
+    int job, pix;
+    jobs.decode(packed, job, pix);
+    const SceneDev& sc = jobs.scene(job);
+    const RenderParams& rp = jobs.params(job);
+    // the one-kind variants run the standard integrator only
+    const bool naive = !(NESTED & (kOnlyMetal | kOnlyDiffuse)) && rp.integrator == 1;
+    const float pdfPrev = o4.w;
+    V3 dir(d4.x, d4.y, d4.z);
+    V3 thr(t4.x, t4.y, t4.z);
+    // guide training: the record of the vertex this ray left takes the
+    // path's accumulated contribution now, before this vertex adds any
+    const unsigned int pid = (kGuide && rp.train) ? in.pid[i] : 0u;
+    if (kGuide && rp.train) {
+        const int prevRec = in.grec[i];
+        if (prevRec >= 0) {
+            float4 a = rp.pathAcc[pid];
+            rp.arena[prevRec].snap = make_float3(a.x, a.y, a.z);
+        }
+    }
+    V3 acc(0.0f);  // this vertex's contributions (training accumulator)
+    auto contribute = [&](V3 c) {
+        filmAddS(rp, pix, c);
+        if (kGuide && rp.train) acc = acc + c;
+    };
+    Pcg rng;
+    rng.state = ((uint64_t)rs.y << 32) | rs.x;
+    rng.inc = ((uint64_t)(unsigned int)pix << 1) | 1u;
+    if (prim < 0) {
+        // Miss: the sky, with no MIS (PathTracer.h:133-136, 192-197).
+        if (sc.skyKind != SKY_NONE) {
+            V3 Ls = skyRadiance(sc, dir);
+            V3 L = thr * Ls;
+            if (naive) L = clampPositive(L);  // PathTracer.h:96
+            contribute(L);
+        }
+        done = true;
+    } else {
+        const Instance& inst = sc.instances[instId];
+        const Material& mat = sc.materials[inst.material];
+        Surface s = makeSurface(sc, inst, prim, h.y, h.z, dir);
+        // a scene without emitters (kNoEmitters) carries no emission or NEE code
+        const bool emissive = !(NESTED & kNoEmitters) && mat.kind == MAT_EMISSION;
+        if ((EXTRAS & kAov) && rp.aov && (flags & FLAG_PRIMARY)) aovAdd(rp, pix, albedoOf(sc, mat, s), s.n);
+        // Emission, the depth limit and Russian roulette; `go`: the path samples this
+        // vertex. An emitter's evalAndSample is zero: a standard path ends there (its NEE
+        // contribution is multiplied by Emission::bsdfCos() == 0).
+        bool go = naive;
+        if (naive) {  // NaivePathTracer::eval (PathTracer.h:75-100)
+            if (emissive) filmAddS(rp, pix, thr * emission(mat, -dir, s.n));
+        } else if (emissive) {
+            if (flags & FLAG_PRIMARY) {
+                contribute(thr * emission(mat, -dir, s.n));  // PathTracer.h:143-145
+            } else {
+                // BSDF-sampled hit on an emitter (PathTracer.h:171-190).
+                float mis;
+                if (pdfPrev >= 0.0f && sc.nLights > 0) {
+                    float pl = sc.lightPdf[sc.lights[inst.lightIndex].triOffset + prim];
+                    float cosLight = fabsf(dot(dir, s.sn));
+                    float distSq = h.x * h.x;
+                    pl *= distSq / cosLight;
+                    mis = (pdfPrev * pdfPrev) / ((pdfPrev * pdfPrev) + (pl * pl));
+                } else {
+                    mis = 1.0f;
+                }
+                if (mis > 0.0f) contribute(thr * mis * emission(mat, -dir, s.n));
+            }
+        } else if (!(rp.maxDepth > 0 && len > rp.maxDepth)) {
+            go = true;
+            if (len > rp.rrStart) {  // PathTracer.h:149-155
+                if (rng.randf() >= rp.rrProb) go = false;
+                else thr = thr / rp.rrProb;
+            }
+        }
+        if (!go) {
+            done = true;
+        } else {
+            V3 wi;
+            float pdf = pdfPrev;  // left untouched by materials that do not set it
+            V3 f;
+            const bool guidedHere = kGuide && !naive && rp.guided && guidable(sc, mat);
+            VmfMixture mx;
+            float fcos = 0.0f;  // luminance of bsdfCos(wi) at a guided vertex
+            bool sampleBsdf = true;
+            if (guidedHere) {
+                // One-sample MIS of the BSDF and the learned vMF mixture (balance
+                // heuristic): pdf = frac p_bsdf + (1 - frac) p_vmf; unbiased at any
+                // network state because the BSDF keeps support everywhere.
+                loadMixture(rp.mix + (size_t)i * 10, mx);
+                sampleBsdf = rng.randf() < rp.bsdfFrac;
+                pdf = 0.0f;
+            }
+            // the one place that samples the BSDF, for every integrator and technique (the
+            // code of all materials is the kernel's largest part)
+            if (sampleBsdf) f = evalAndSampleT<NESTED>(sc, mat, s, rng, &wi, &pdf);
+            if (guidedHere) {
+                const float frac = rp.bsdfFrac;
+                if (sampleBsdf) {
+                    const V3 e = f;
+                    const float pb = pdf;
+                    float pm = frac * pb + (1.0f - frac) * mixturePdf(mx, wi);
+                    f = (pb > 0.0f && pm > 0.0f) ? e * (pb / pm) : V3(0.0f);
+                    fcos = luminance(e) * pb;
+                    pdf = pm;
+                } else {
+                    wi = mixtureSample(mx, rng);
+                    float pb = getPDFT<NESTED>(sc, mat, s, wi);
+                    float pm = frac * pb + (1.0f - frac) * mixturePdf(mx, wi);
+                    V3 bc = bsdfCosT<NESTED>(sc, mat, s, rng, wi);
+                    f = pm > 0.0f ? bc / pm : V3(0.0f);
+                    fcos = luminance(bc);
+                    pdf = pm;
+                }
+            }
+            V3 thrNext = thr * f;
+            bool alive = (naive || !isZero(f)) && !isZero(thrNext);
+            if (naive) {
+                // the next loop top (depth limit, Russian roulette) before tracing
+                if (alive && rp.maxDepth > 0 && len + 1 > rp.maxDepth) alive = false;
+                if (alive && len + 1 > rp.rrStart) {
+                    if (rng.randf() >= rp.rrProb) alive = false;
+                    else thrNext = thrNext / rp.rrProb;
+                }
+            }
+            if (!(NESTED & kNoEmitters) && !naive && sc.nLights > 0) {  // PathTracer.h:202-233
+                LightSampleD ls = sampleLight(sc, rng);
+                V3 toL = ls.p - s.p;
+                float dist = length(toL);
+                V3 sd = toL / dist;
+                V3 so = s.p + kRayOffset * sd;
+                float stMax = dist - kShadowMargin;
+                if (dot(sd, ls.n) < 0) {
+                    float distSq = dist * dist;
+                    float mis;
+                    if (pdf >= 0.0f) {
+                        float pb = getPDFT<NESTED>(sc, mat, s, sd);
+                        if (guidedHere) pb = rp.bsdfFrac * pb + (1.0f - rp.bsdfFrac) * mixturePdf(mx, sd);
+                        float cosLight = fabsf(dot(-sd, ls.sn));
+                        pb *= cosLight / distSq;
+                        mis = (ls.pdf * ls.pdf) / ((pb * pb) + (ls.pdf * ls.pdf));
+                    } else {
+                        mis = 0.0f;
+                    }
+                    if (mis > 0.0f) {
+                        float G = fabsf(dot(-sd, ls.sn)) / distSq;
+                        Pcg spec = rng;  // bsdfCos draws only if the light is visible
+                        V3 bc = bsdfCosT<NESTED>(sc, mat, s, spec, sd);
+                        V3 Le = emission(sc.materials[ls.material], -sd, ls.n);
+                        V3 c = thr * mis * bc * Le * G / ls.pdf;
+                        r.so = make_float4(so.x, so.y, so.z, stMax);
+                        r.sd = make_float4(sd.x, sd.y, sd.z, __int_as_float(packed));
+                        r.sc = make_float4(c.x, c.y, c.z, 0.0f);
+                        r.stochastic = spec.state != rng.state;
+                        r.srng = make_uint2((unsigned int)spec.state, (unsigned int)(spec.state >> 32));
+                        shadow = true;
+                    }
+                }
+            }
+            if (alive) {
+                V3 no = s.p + kRayOffset * wi;
+                r.o = make_float4(no.x, no.y, no.z, pdf);
+                r.d = make_float4(wi.x, wi.y, wi.z, __int_as_float(len + 1));
+                r.thr = make_float4(thrNext.x, thrNext.y, thrNext.z, __int_as_float(packed));
+                r.rng = make_uint2((unsigned int)rng.state, (unsigned int)(rng.state >> 32));
+                cont = true;
+                if (kGuide && rp.train && guidedHere && pdf > 0.0f && keepRecord(pid, len, rp.recordProb)) {
+                    unsigned int slot = atomicAdd(rp.arenaCount, 1u);
+                    if (slot < (unsigned int)rp.arenaCap) {
+                        GuideRecord g;
+                        g.p = make_float3(s.p.x, s.p.y, s.p.z);
+                        g.pdf = pdf;
+                        g.n = make_float3(s.sn.x, s.sn.y, s.sn.z);
+                        g.fcos = fcos;
+                        g.wo = make_float3(s.wo.x, s.wo.y, s.wo.z);
+                        g.pid = pid;
+                        g.wi = make_float3(wi.x, wi.y, wi.z);
+                        g.radiance = 0.0f;
+                        g.snap = make_float3(__int_as_float(0x7fc00000), 0.0f, 0.0f);
+                        g.pad0 = 0.0f;
+                        g.thr = make_float3(thrNext.x, thrNext.y, thrNext.z);
+                        g.pad1 = 0.0f;
+                        rp.arena[slot] = g;
+                        r.grec = (int)slot;
+                    }
+                }
+            } else {
+                done = true;
+            }
+        }
+    }
+    if (kGuide && rp.train && !isZero(acc)) {
+        float4 a = rp.pathAcc[pid];
+        rp.pathAcc[pid] = make_float4(a.x + acc.x, a.y + acc.y, a.z + acc.z, a.w);
+    }
+}
+
 // EXTRAS: the learned proposal (guided sampling, training records), AOV planes;
 // plain renders run the variant without that code (fewer registers, a smaller
 // instruction footprint). Occupancy bounds, measured on GB300: without nested
@@ -217,214 +429,8 @@ __global__ void __launch_bounds__(kShadeBlock, (NESTED & 3) ? 2 : (NESTED & kNoE
             uint2 rs = __ldcs(&in.rng[i]);
             float4 h = __ldcs(&hq.h[i]);
             const int instId = __ldcs(&hq.inst[i]);
-            const int prim = __float_as_int(h.w);
-            const int meta = __float_as_int(d4.w);
-            int len = meta & 0xFFFF;
-            const int flags = meta >> 16;
-            const int packed = __float_as_int(t4.w);
-            int job, pix;
-            jobs.decode(packed, job, pix);
-            const SceneDev& sc = jobs.scene(job);
-            const RenderParams& rp = jobs.params(job);
-            // the one-kind variants run the standard integrator only
-            const bool naive = !(NESTED & (kOnlyMetal | kOnlyDiffuse)) && rp.integrator == 1;
-            const float pdfPrev = o4.w;
-            V3 dir(d4.x, d4.y, d4.z);
-            V3 thr(t4.x, t4.y, t4.z);
-            // guide training: the record of the vertex this ray left takes the
-            // path's accumulated contribution now, before this vertex adds any
-            const unsigned int pid = (EXTRAS && rp.train) ? in.pid[i] : 0u;
-            if (EXTRAS && rp.train) {
-                const int prevRec = in.grec[i];
-                if (prevRec >= 0) {
-                    float4 a = rp.pathAcc[pid];
-                    rp.arena[prevRec].snap = make_float3(a.x, a.y, a.z);
-                }
-            }
-            V3 acc(0.0f);  // this vertex's contributions (training accumulator)
-            auto contribute = [&](V3 c) {
-                filmAddS(rp, pix, c);
-                if (EXTRAS && rp.train) acc = acc + c;
-            };
-            Pcg rng;
-            rng.state = ((uint64_t)rs.y << 32) | rs.x;
-            rng.inc = ((uint64_t)(unsigned int)pix << 1) | 1u;
-            if (prim < 0) {
-                // Miss: the sky, with no MIS (PathTracer.h:133-136, 192-197).
-                if (sc.skyKind != SKY_NONE) {
-                    V3 Ls = skyRadiance(sc, dir);
-                    V3 L = thr * Ls;
-                    if (naive) L = clampPositive(L);  // PathTracer.h:96
-                    contribute(L);
-                }
-                done = true;
-            } else {
-                const Instance& inst = sc.instances[instId];
-                const Material& mat = sc.materials[inst.material];
-                Surface s = makeSurface(sc, inst, prim, h.y, h.z, dir);
-                // a scene without emitters (kNoEmitters) carries no emission or NEE code
-                const bool emissive = !(NESTED & kNoEmitters) && mat.kind == MAT_EMISSION;
-                if (EXTRAS && rp.aov && (flags & FLAG_PRIMARY)) aovAdd(rp, pix, albedoOf(sc, mat, s), s.n);
-                if (naive) {
-                    // NaivePathTracer::eval (PathTracer.h:75-100): emission, BSDF sample,
-                    // then the next loop top (depth limit, Russian roulette) before tracing.
-                    if (emissive) filmAddS(rp, pix, thr * emission(mat, -dir, s.n));
-                    V3 wi;
-                    float pdf = pdfPrev;
-                    thr = thr * evalAndSampleT<NESTED>(sc, mat, s, rng, &wi, &pdf);
-                    bool alive = !isZero(thr);
-                    len += 1;
-                    if (alive && rp.maxDepth > 0 && len > rp.maxDepth) alive = false;
-                    if (alive && len > rp.rrStart) {
-                        if (rng.randf() >= rp.rrProb) alive = false;
-                        else thr = thr / rp.rrProb;
-                    }
-                    if (alive) {
-                        V3 no = s.p + kRayOffset * wi;
-                        r.o = make_float4(no.x, no.y, no.z, pdf);
-                        r.d = make_float4(wi.x, wi.y, wi.z, __int_as_float(len));
-                        r.thr = make_float4(thr.x, thr.y, thr.z, __int_as_float(packed));
-                        r.rng = make_uint2((unsigned int)rng.state, (unsigned int)(rng.state >> 32));
-                        cont = true;
-                    } else {
-                        done = true;
-                    }
-                } else if (flags & FLAG_PRIMARY) {
-                    if (emissive) contribute(thr * emission(mat, -dir, s.n));  // PathTracer.h:143-145
-                } else if (emissive) {
-                    // BSDF-sampled hit on an emitter (PathTracer.h:171-190).
-                    float mis;
-                    if (pdfPrev >= 0.0f && sc.nLights > 0) {
-                        float pl = sc.lightPdf[sc.lights[inst.lightIndex].triOffset + prim];
-                        float cosLight = fabsf(dot(dir, s.sn));
-                        float distSq = h.x * h.x;
-                        pl *= distSq / cosLight;
-                        mis = (pdfPrev * pdfPrev) / ((pdfPrev * pdfPrev) + (pl * pl));
-                    } else {
-                        mis = 1.0f;
-                    }
-                    if (mis > 0.0f) contribute(thr * mis * emission(mat, -dir, s.n));
-                }
-                // An emitter's evalAndSample is zero: the path ends there (its NEE
-                // contribution is multiplied by Emission::bsdfCos() == 0).
-                if (naive) {
-                    // handled above
-                } else if (emissive) {
-                    done = true;
-                } else if (rp.maxDepth > 0 && len > rp.maxDepth) {
-                    done = true;
-                } else {
-                    bool alive = true;
-                    if (len > rp.rrStart) {  // PathTracer.h:149-155
-                        if (rng.randf() >= rp.rrProb) alive = false;
-                        else thr = thr / rp.rrProb;
-                    }
-                    if (!alive) {
-                        done = true;
-                    } else {
-                        V3 wi;
-                        float pdf = pdfPrev;  // left untouched by materials that do not set it
-                        V3 f;
-                        const bool guidedHere = EXTRAS && rp.guided && guidable(sc, mat);
-                        VmfMixture mx;
-                        float fcos = 0.0f;  // luminance of bsdfCos(wi) at a guided vertex
-                        if (!guidedHere) {
-                            f = evalAndSampleT<NESTED>(sc, mat, s, rng, &wi, &pdf);
-                        } else {
-                            // One-sample MIS of the BSDF and the learned vMF mixture (balance
-                            // heuristic): pdf = frac p_bsdf + (1 - frac) p_vmf; unbiased at any
-                            // network state because the BSDF keeps support everywhere.
-                            loadMixture(rp.mix + (size_t)i * 10, mx);
-                            const float frac = rp.bsdfFrac;
-                            if (rng.randf() < frac) {
-                                float pb = 0.0f;
-                                V3 e = evalAndSampleT<NESTED>(sc, mat, s, rng, &wi, &pb);
-                                float pm = frac * pb + (1.0f - frac) * mixturePdf(mx, wi);
-                                f = (pb > 0.0f && pm > 0.0f) ? e * (pb / pm) : V3(0.0f);
-                                fcos = luminance(e) * pb;
-                                pdf = pm;
-                            } else {
-                                wi = mixtureSample(mx, rng);
-                                float pb = getPDFT<NESTED>(sc, mat, s, wi);
-                                float pm = frac * pb + (1.0f - frac) * mixturePdf(mx, wi);
-                                V3 bc = bsdfCosT<NESTED>(sc, mat, s, rng, wi);
-                                f = pm > 0.0f ? bc / pm : V3(0.0f);
-                                fcos = luminance(bc);
-                                pdf = pm;
-                            }
-                        }
-                        if (!(NESTED & kNoEmitters) && !naive && sc.nLights > 0) {  // PathTracer.h:202-233
-                            LightSampleD ls = sampleLight(sc, rng);
-                            V3 toL = ls.p - s.p;
-                            float dist = length(toL);
-                            V3 sd = toL / dist;
-                            V3 so = s.p + kRayOffset * sd;
-                            float stMax = dist - kShadowMargin;
-                            if (dot(sd, ls.n) < 0) {
-                                float distSq = dist * dist;
-                                float mis;
-                                if (pdf >= 0.0f) {
-                                    float pb = getPDFT<NESTED>(sc, mat, s, sd);
-                                    if (guidedHere) pb = rp.bsdfFrac * pb + (1.0f - rp.bsdfFrac) * mixturePdf(mx, sd);
-                                    float cosLight = fabsf(dot(-sd, ls.sn));
-                                    pb *= cosLight / distSq;
-                                    mis = (ls.pdf * ls.pdf) / ((pb * pb) + (ls.pdf * ls.pdf));
-                                } else {
-                                    mis = 0.0f;
-                                }
-                                if (mis > 0.0f) {
-                                    float G = fabsf(dot(-sd, ls.sn)) / distSq;
-                                    Pcg spec = rng;  // bsdfCos draws only if the light is visible
-                                    V3 bc = bsdfCosT<NESTED>(sc, mat, s, spec, sd);
-                                    V3 Le = emission(sc.materials[ls.material], -sd, ls.n);
-                                    V3 c = thr * mis * bc * Le * G / ls.pdf;
-                                    r.so = make_float4(so.x, so.y, so.z, stMax);
-                                    r.sd = make_float4(sd.x, sd.y, sd.z, __int_as_float(packed));
-                                    r.sc = make_float4(c.x, c.y, c.z, 0.0f);
-                                    r.stochastic = spec.state != rng.state;
-                                    r.srng = make_uint2((unsigned int)spec.state, (unsigned int)(spec.state >> 32));
-                                    shadow = true;
-                                }
-                            }
-                        }
-                        V3 thrNext = thr * f;
-                        if (!isZero(f) && !isZero(thrNext)) {
-                            V3 no = s.p + kRayOffset * wi;
-                            r.o = make_float4(no.x, no.y, no.z, pdf);
-                            r.d = make_float4(wi.x, wi.y, wi.z, __int_as_float(len + 1));
-                            r.thr = make_float4(thrNext.x, thrNext.y, thrNext.z, __int_as_float(packed));
-                            r.rng = make_uint2((unsigned int)rng.state, (unsigned int)(rng.state >> 32));
-                            cont = true;
-                            if (EXTRAS && rp.train && guidedHere && pdf > 0.0f && keepRecord(pid, len, rp.recordProb)) {
-                                unsigned int slot = atomicAdd(rp.arenaCount, 1u);
-                                if (slot < (unsigned int)rp.arenaCap) {
-                                    GuideRecord g;
-                                    g.p = make_float3(s.p.x, s.p.y, s.p.z);
-                                    g.pdf = pdf;
-                                    g.n = make_float3(s.sn.x, s.sn.y, s.sn.z);
-                                    g.fcos = fcos;
-                                    g.wo = make_float3(s.wo.x, s.wo.y, s.wo.z);
-                                    g.pid = pid;
-                                    g.wi = make_float3(wi.x, wi.y, wi.z);
-                                    g.radiance = 0.0f;
-                                    g.snap = make_float3(__int_as_float(0x7fc00000), 0.0f, 0.0f);
-                                    g.pad0 = 0.0f;
-                                    g.thr = make_float3(thrNext.x, thrNext.y, thrNext.z);
-                                    g.pad1 = 0.0f;
-                                    rp.arena[slot] = g;
-                                    r.grec = (int)slot;
-                                }
-                            }
-                        } else {
-                            done = true;
-                        }
-                    }
-                }
-            }
-            if (EXTRAS && rp.train && !isZero(acc)) {
-                float4 a = rp.pathAcc[pid];
-                rp.pathAcc[pid] = make_float4(a.x + acc.x, a.y + acc.y, a.z + acc.z, a.w);
-            }
+            shadeVertex<J, NESTED, EXTRAS ? (kAov | kProposal) : 0>(jobs, in, i, o4, d4, t4, rs, h, instId, r, cont,
+                                                                    shadow, done);
         }
         // compacted writes: continuing paths, then shadow rays (which may point at them)
         unsigned int mc = __ballot_sync(kFull, cont);

@@ -34,21 +34,6 @@ __device__ __forceinline__ void creditPath(const RenderParams& rp, unsigned int 
 
 constexpr int kTraceBlock = 128;
 
-// World-space ray for the instance-box tests of the flat kernels: origin and
-// 1/d only (no watertight constants), computed once per ray.
-struct BoxRay {
-    float ox, oy, oz, ix, iy, iz;
-};
-__device__ __forceinline__ bool instBoxHit(const BoxRay& b, const float4* boxes, int inst, float tMax) {
-    const float4 lo = __ldg(&boxes[2 * inst]), hi = __ldg(&boxes[2 * inst + 1]);
-    float tx0 = (lo.x - b.ox) * b.ix, tx1 = (hi.x - b.ox) * b.ix;
-    float ty0 = (lo.y - b.oy) * b.iy, ty1 = (hi.y - b.oy) * b.iy;
-    float tz0 = (lo.z - b.oz) * b.iz, tz1 = (hi.z - b.oz) * b.iz;
-    float tn = fmaxf(fmaxf(fminf(tx0, tx1), fminf(ty0, ty1)), fmaxf(fminf(tz0, tz1), 0.0f));
-    float tf = fminf(fminf(fmaxf(tx0, tx1), fmaxf(ty0, ty1)), fminf(fmaxf(tz0, tz1), tMax));
-    return tn <= tf * 1.00000095367431640625f;
-}
-
 template <bool COUNT>
 __global__ void __launch_bounds__(kTraceBlock) k_extend(SceneDev sc, PathQueue q, HitQueue h, Ctrl* ctrl) {
     const unsigned int n = ctrl->nActive;
@@ -142,7 +127,6 @@ struct BatchScenes {
 // next one at once (one atomicAdd per group of lanes), so the warp never waits
 // for its slowest ray. Results are those of traceScene: the same watertight
 // tests and the same closest-hit acceptance (tMax shrinks across instances).
-constexpr int kFlatInstances = 16;
 
 template <bool ANY, bool COUNT>
 __global__ void __launch_bounds__(kTraceBlock) k_trace_wide(SceneDev sc, RenderParams rp, PathQueue q, HitQueue h,
@@ -290,7 +274,7 @@ __global__ void __launch_bounds__(kTraceBlock) k_trace_wide(SceneDev sc, RenderP
         // leaf phase: the postponed leaf children's triangles, together
         if (leafCnt) {
             if (COUNT) wc.tris += leafCnt;
-            if (testTris<ANY>(tris, leafFirst, leafCnt, r, tMax, hit, inst) && ANY) {
+            if (testTris(tris, leafFirst, leafCnt, r, tMax, hit, inst, ANY) && ANY) {
                 occluded = true;
                 inMesh = false;
             }

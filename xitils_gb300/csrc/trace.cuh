@@ -242,7 +242,7 @@ __device__ __forceinline__ float shellRed(const MeshDev& m, float u, float v) {
 // asked by TriangleIndexed::intersect once the hit is inside [0, tMax]
 // (:132-141): the texcoord lerp(uv0, uv1, uv2, b0, b1) (Utils.h:81-83), then
 // red < height with height = layer / (layers - 1) (TriangleMesh.h:305-318).
-__device__ __noinline__ bool shellDiscard(const MeshDev& m, int prim, float b0, float b1) {
+static __device__ __noinline__ bool shellDiscard(const MeshDev& m, int prim, float b0, float b1) {
     const int i0 = __ldg(&m.idx[3 * prim]), i1 = __ldg(&m.idx[3 * prim + 1]), i2 = __ldg(&m.idx[3 * prim + 2]);
     const float2 a = __ldg(&m.uv[i0]), b = __ldg(&m.uv[i1]), c = __ldg(&m.uv[i2]);
     const float w = __fsub_rn(__fsub_rn(1.0f, b0), b1);
@@ -252,10 +252,10 @@ __device__ __noinline__ bool shellDiscard(const MeshDev& m, int prim, float b0, 
     return shellRed(m, u, v) < height;
 }
 
-// Watertight tests of `cnt` triangles from `first`; ANY: stops at the first hit.
-template <bool ANY>
+// Watertight tests of `cnt` triangles from `first`; any: stops at the first hit (a
+// constant in the kernels of one ray type, a variable where one copy serves both).
 __device__ __forceinline__ bool testTris(const TriV* tris, int first, int cnt, const WRay& r, float& tMax, TraceHit& hit,
-                                         int inst) {
+                                         int inst, bool any) {
     bool found = false;
     for (int k = 0; k < cnt; ++k) {
         const TriV* tv = tris + first + k;
@@ -264,7 +264,7 @@ __device__ __forceinline__ bool testTris(const TriV* tris, int first, int cnt, c
         if (watertight(r, p0, p1, p2, tMax, t, b0, b1)) {
             tMax = t;
             found = true;
-            if (ANY) return true;
+            if (any) return true;
             hit.t = t; hit.b0 = b0; hit.b1 = b1;
             hit.prim = __float_as_int(p0.w);
             hit.inst = inst;
@@ -274,10 +274,9 @@ __device__ __forceinline__ bool testTris(const TriV* tris, int first, int cnt, c
 }
 
 // testTris for a mesh that may be shell-mapped (generic traversal path).
-template <bool ANY>
 __device__ __forceinline__ bool testTrisMesh(const MeshDev& m, int first, int cnt, const WRay& r, float& tMax,
-                                             TraceHit& hit, int inst) {
-    if (!m.shellLayers) return testTris<ANY>(m.tris, first, cnt, r, tMax, hit, inst);
+                                             TraceHit& hit, int inst, bool any) {
+    if (!m.shellLayers) return testTris(m.tris, first, cnt, r, tMax, hit, inst, any);
     bool found = false;
     for (int k = 0; k < cnt; ++k) {
         const TriV* tv = m.tris + first + k;
@@ -286,7 +285,7 @@ __device__ __forceinline__ bool testTrisMesh(const MeshDev& m, int first, int cn
         if (watertight(r, p0, p1, p2, tMax, t, b0, b1) && !shellDiscard(m, __float_as_int(p0.w), b0, b1)) {
             tMax = t;
             found = true;
-            if (ANY) return true;
+            if (any) return true;
             hit.t = t; hit.b0 = b0; hit.b1 = b1;
             hit.prim = __float_as_int(p0.w);
             hit.inst = inst;
@@ -295,10 +294,10 @@ __device__ __forceinline__ bool testTrisMesh(const MeshDev& m, int first, int cn
     return found;
 }
 
-// Traverses one binary mesh BVH (Node2). ANY: returns at the first accepted hit.
-template <bool ANY, bool COUNT>
+// Traverses one binary mesh BVH (Node2). any: returns at the first accepted hit.
+template <bool COUNT>
 __device__ __forceinline__ bool traverseBlas2(const MeshDev& m, const WRay& r, float& tMax, TraceHit& hit, int inst,
-                                             unsigned int* errors, WorkCount& wc, Limits lim) {
+                                             unsigned int* errors, WorkCount& wc, Limits lim, bool any) {
     int stack[kStackDepth];
     int sp = 0;
     int node = m.rootIsLeaf ? m.rootLeaf : 0;
@@ -338,7 +337,7 @@ __device__ __forceinline__ bool traverseBlas2(const MeshDev& m, const WRay& r, f
                     if (m.shellLayers && shellDiscard(m, __float_as_int(p0.w), b0, b1)) continue;
                     tMax = t;
                     found = true;
-                    if (ANY) return true;
+                    if (any) return true;
                     hit.t = t; hit.b0 = b0; hit.b1 = b1;
                     hit.prim = __float_as_int(p0.w);
                     hit.inst = inst;
@@ -351,13 +350,13 @@ __device__ __forceinline__ bool traverseBlas2(const MeshDev& m, const WRay& r, f
     return found;
 }
 
-// Traverses one 8-wide mesh BVH (WNode). ANY: returns at the first accepted hit.
-template <bool ANY, bool COUNT>
+// Traverses one 8-wide mesh BVH (WNode). any: returns at the first accepted hit.
+template <bool COUNT>
 __device__ __forceinline__ bool traverseBlasWide(const MeshDev& m, const WRay& r, float& tMax, TraceHit& hit, int inst,
-                                                 unsigned int* errors, WorkCount& wc, Limits lim) {
+                                                 unsigned int* errors, WorkCount& wc, Limits lim, bool any) {
     if (m.rootIsLeaf) {
         if (COUNT) wc.tris += m.nTris;
-        return testTrisMesh<ANY>(m, 0, m.nTris, r, tMax, hit, inst);
+        return testTrisMesh(m, 0, m.nTris, r, tMax, hit, inst, any);
     }
     const int oct = rayOctant(r);
     unsigned int stack[kWideStack];
@@ -392,9 +391,9 @@ __device__ __forceinline__ bool traverseBlasWide(const MeshDev& m, const WRay& r
         } else {
             const int cnt = (int)(mb >> 5);
             if (COUNT) wc.tris += cnt;
-            if (testTrisMesh<ANY>(m, h.triBase + (int)(mb & 31u), cnt, r, tMax, hit, inst)) {
+            if (testTrisMesh(m, h.triBase + (int)(mb & 31u), cnt, r, tMax, hit, inst, any)) {
                 found = true;
-                if (ANY) return true;
+                if (any) return true;
             }
         }
     }
@@ -404,8 +403,96 @@ __device__ __forceinline__ bool traverseBlasWide(const MeshDev& m, const WRay& r
 template <bool ANY, bool COUNT>
 __device__ __forceinline__ bool traverseBlas(const MeshDev& m, const WRay& r, float& tMax, TraceHit& hit, int inst,
                                              unsigned int* errors, WorkCount& wc, Limits lim) {
-    return m.wide ? traverseBlasWide<ANY, COUNT>(m, r, tMax, hit, inst, errors, wc, lim)
-                  : traverseBlas2<ANY, COUNT>(m, r, tMax, hit, inst, errors, wc, lim);
+    return m.wide ? traverseBlasWide<COUNT>(m, r, tMax, hit, inst, errors, wc, lim, ANY)
+                  : traverseBlas2<COUNT>(m, r, tMax, hit, inst, errors, wc, lim, ANY);
+}
+
+// World-space ray for the instance-box tests of the flat kernels: origin and
+// 1/d only (no watertight constants), computed once per ray.
+struct BoxRay {
+    float ox, oy, oz, ix, iy, iz;
+};
+__device__ __forceinline__ bool instBoxHit(const BoxRay& b, const float4* boxes, int inst, float tMax) {
+    const float4 lo = __ldg(&boxes[2 * inst]), hi = __ldg(&boxes[2 * inst + 1]);
+    float tx0 = (lo.x - b.ox) * b.ix, tx1 = (hi.x - b.ox) * b.ix;
+    float ty0 = (lo.y - b.oy) * b.iy, ty1 = (hi.y - b.oy) * b.iy;
+    float tz0 = (lo.z - b.oz) * b.iz, tz1 = (hi.z - b.oz) * b.iz;
+    float tn = fmaxf(fmaxf(fminf(tx0, tx1), fminf(ty0, ty1)), fmaxf(fminf(tz0, tz1), 0.0f));
+    float tf = fminf(fminf(fmaxf(tx0, tx1), fmaxf(ty0, ty1)), fminf(fmaxf(tz0, tz1), tMax));
+    return tn <= tf * 1.00000095367431640625f;
+}
+
+// Most instances that the flat kernels and traceFlat walk as a list.
+constexpr int kFlatInstances = 16;
+
+// Scene::intersect (any = false) or Scene::intersectAny as one function, for a kernel that
+// traces both kinds of rays next to other code: one copy of the traversal keeps the
+// kernel inside the instruction cache. A scene of at most kFlatInstances instances is
+// walked as a list, as the flat kernels of trace.cu do, any other over its top-level
+// BVH, as traceScene does, so that equal distances go to the same triangle as there.
+static __device__ __noinline__ bool traverseWideCall(const MeshDev& m, const WRay& r, float& tMax, TraceHit& hit, int inst,
+                                                     unsigned int* errors, Limits lim, bool any) {
+    WorkCount wc;
+    return traverseBlasWide<false>(m, r, tMax, hit, inst, errors, wc, lim, any);
+}
+static __device__ __noinline__ bool traceCall(const SceneDev& sc, V3 o, V3 d, float tMax, bool any, TraceHit& hit,
+                                              unsigned int* errors) {
+    hit.prim = -1;
+    hit.inst = -1;
+    hit.t = tMax;
+    const Limits lim = limitsOf(sc);
+    const bool flat = sc.nInstances <= kFlatInstances && sc.blasLayout != 2;
+    const BoxRay br{o.x, o.y, o.z, 1.0f / d.x, 1.0f / d.y, 1.0f / d.z};
+    const WRay wr = makeWRay(o, d);
+    const int stackCap = lim.stack < kTlasStack ? lim.stack : kTlasStack;
+    int stack[kTlasStack];
+    int sp = 0;
+    int next = flat ? 0 : sc.tlasRootIsLeaf ? leafEncode(0, 1) : 0;  // instance of the list, or top-level node
+    bool found = false;
+    for (int guard = 0;; ++guard) {
+        if (guard > lim.steps) { atomicOr(errors, 4u); return found; }
+        int inst;
+        if (flat) {
+            while (next < sc.nInstances && !instBoxHit(br, sc.instBox, next, tMax)) ++next;
+            if (next >= sc.nInstances) return found;
+            inst = next++;
+        } else if (next >= 0) {
+            const Node2* nd = sc.tlas + next;
+            const float4 a = __ldg(&nd->a), b = __ldg(&nd->b), c = __ldg(&nd->c);
+            const int4 dd = __ldg(&nd->d);
+            float t0, t1;
+            const bool h0 = slab(wr, a.x, a.y, a.z, a.w, b.x, b.y, tMax, t0);
+            const bool h1 = slab(wr, b.z, b.w, c.x, c.y, c.z, c.w, tMax, t1);
+            if (h0 && h1) {
+                if (sp >= stackCap) { atomicOr(errors, 1u); return found; }
+                stack[sp++] = t1 < t0 ? dd.x : dd.y;
+                next = t1 < t0 ? dd.y : dd.x;
+            } else if (h0 || h1) {
+                next = h0 ? dd.x : dd.y;
+            } else {
+                if (sp == 0) return found;
+                next = stack[--sp];
+            }
+            continue;
+        } else {
+            inst = leafFirst(next);
+        }
+        const Instance& in = sc.instances[inst];
+        const MeshDev& m = sc.meshes[in.mesh];
+        WRay r = wr;
+        if (!in.identity) r = makeWRay(xformPointRn(in.matInv, o), xformVectorRn(in.matInv, d));
+        WorkCount wc;
+        const bool h = m.wide ? traverseWideCall(m, r, tMax, hit, inst, errors, lim, any)
+                              : traverseBlas2<false>(m, r, tMax, hit, inst, errors, wc, lim, any);
+        if (h) {
+            found = true;
+            if (any) return true;
+        }
+        if (!flat) {
+            if (sp == 0) return found;
+            next = stack[--sp];
+        }
+    }
 }
 
 // Scene::intersect (ANY = false) / Scene::intersectAny (ANY = true).

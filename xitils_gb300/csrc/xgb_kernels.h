@@ -54,7 +54,7 @@ struct Ctrl {
     unsigned int extendHead;       // persistent work counters
     unsigned int shadowHead;
     unsigned int errors;           // bit 0: traversal stack overflow
-    unsigned int pad;
+    unsigned int nTail;            // paths the next tail launch finishes (0: it does nothing)
     unsigned long long extensionRays;
     unsigned long long shadowRays;
     unsigned long long iterations;
@@ -160,7 +160,22 @@ void launchShadeBatch(const BatchView& b, PathQueue in, HitQueue h, PathQueue ou
 void launchExtendBatch(const BatchView& b, PathQueue q, HitQueue h, Ctrl* ctrl, int numSMs, cudaStream_t s);
 void launchShadowBatch(const BatchView& b, ShadowQueue sq, PathQueue out, Ctrl* ctrl, int numSMs, cudaStream_t s);
 
-void launchPlan(Ctrl* ctrl, unsigned int capacity, cudaStream_t s);
+// Queue bookkeeping of an iteration. mode kPlanWave: a wavefront iteration; kPlanTail: the
+// new camera paths go to a tail launch; kPlanTailIfFew: nothing happens (and the tail launch
+// that follows does nothing) unless every camera path has started and at most tailMax paths
+// are left, which then go to the tail launch.
+enum PlanMode : int { kPlanWave = 0, kPlanTail = 1, kPlanTailIfFew = 2 };
+void launchPlan(Ctrl* ctrl, unsigned int capacity, cudaStream_t s, int mode = kPlanWave, unsigned int tailMax = 0);
+// Paths up to which a tail launch beats the remaining wavefront iterations. Measured with
+// 4,096 / 16,384 / 65,536 / 131,072 paths (none: no tail launches), ms per call: occluded
+// room 384^2 x 8 55.6 / 51.1 / 46.6 / 45.9 (73.8), shell-mapped cloth 320^2 x 4 27.3 / 23.8 /
+// 21.5 / 22.6 (40.9), its SVBRDF variant 26.7 / 24.4 / 23.0 / 25.7 (33.4); microfacet normal
+// mapping, whose walks of up to 100 facets per BSDF call make a warp's lanes wait for one
+// another and its code overflow the instruction cache, 400^2 x 4 6.4 / 7.3 / 10.3 / 10.3 (6.5).
+inline unsigned int tailMaxPaths(const SceneDev& sc) { return (sc.nested & 1) ? 4096u : 65536u; }
+// Finishes the ctrl->nTail paths of `in`; those that outlive the launch's bound go to `out` (tail.cuh).
+void launchTail(const SceneDev& sc, const RenderParams& rp, PathQueue in, PathQueue out, Ctrl* ctrl, int numSMs,
+                cudaStream_t s);
 void launchGenerate(const SceneDev& sc, const RenderParams& rp, PathQueue q, Ctrl* ctrl, int grid, cudaStream_t s);
 // Extension / shadow rays and shading of the wavefront; grids sized from the
 // launched kernel's occupancy on numSMs SMs (one full wave).
