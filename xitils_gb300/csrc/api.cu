@@ -898,6 +898,50 @@ static int buildTlas(std::vector<Node2>& nodes, std::vector<int>& items, const s
     return me;
 }
 
+// Top level of a world BVH over up to 65,536 boxes, node 0 its root; leaves carry codes[i].
+// A few boxes are merged two by two, the pair with the smallest common box first (the
+// walls, lights and meshes of a room); many take buildTlas' median splits, whose depth
+// the traversal's stack has room for.
+static void buildWorldTop(std::vector<Node2>& nodes, const std::vector<Box>& boxes, const std::vector<int>& codes) {
+    const int n = (int)boxes.size();
+    if (n > 16) {
+        std::vector<int> items(n);
+        for (int i = 0; i < n; ++i) items[i] = i;
+        Box root;
+        buildTlas(nodes, items, boxes, 0, n, &root);
+        for (Node2& nd : nodes) {
+            if (nd.d.x < 0) nd.d.x = codes[leafFirst(nd.d.x)];
+            if (nd.d.y < 0) nd.d.y = codes[leafFirst(nd.d.y)];
+        }
+        return;
+    }
+    std::vector<Box> box(boxes);
+    std::vector<int> code(codes);
+    nodes.resize(n - 1);
+    for (int next = n - 2; next >= 0; --next) {
+        int bi = 0, bj = 1;
+        float best = INFINITY;
+        for (int i = 0; i < (int)box.size(); ++i)
+            for (int j = i + 1; j < (int)box.size(); ++j) {
+                Box u = box[i];
+                u.add(box[j]);
+                const float x = u.hi[0] - u.lo[0], y = u.hi[1] - u.lo[1], z = u.hi[2] - u.lo[2];
+                const float area = x * y + y * z + z * x;
+                if (area < best) { best = area; bi = i; bj = j; }
+            }
+        const Box l = box[bi], r = box[bj];
+        Node2& nd = nodes[next];
+        nd.a = make_float4(l.lo[0], l.lo[1], l.lo[2], l.hi[0]);
+        nd.b = make_float4(l.hi[1], l.hi[2], r.lo[0], r.lo[1]);
+        nd.c = make_float4(r.lo[2], r.hi[0], r.hi[1], r.hi[2]);
+        nd.d = make_int4(code[bi], code[bj], 0, 0);
+        box[bi].add(r);
+        code[bi] = next;
+        box.erase(box.begin() + bj);
+        code.erase(code.begin() + bj);
+    }
+}
+
 xgb_status xgb_scene_build(xgb_scene* s, void* stream) {
     if (!s) return XGB_INVALID_ARG;
     xgb_ctx* ctx = s->ctx;
@@ -1082,6 +1126,60 @@ xgb_status xgb_scene_build(xgb_scene* s, void* stream) {
         sd.kinds |= 1 << m.kind;
     }
     sd.instBox = dBox;
+    sd.world = WorldDev{};
+    long long totalTris = 0;
+    for (const SceneObject& o : s->objects) totalTris += o.mesh->nTris;
+    constexpr long long kWorldMinTris = 4096;  // of few instances, only large scenes gain (trace.cu::useWorld)
+    if (blasLayout == 0 && inst.size() == 1) {
+        const xgb_mesh* m = s->objects[0].mesh;
+        sd.world = WorldDev{m->dNodes2, m->dTris, m->rootIsLeaf ? m->rootLeaf : 0, 0, 1.0f, 0.0f};
+    } else if (blasLayout == 0 && inst.size() <= 65536 &&
+               (inst.size() > 16 || (!anyShell && totalTris >= kWorldMinTris))) {
+        // triangle and node numbers: leaf codes hold 27 bits, the traversal's hit marker 30
+        std::vector<int> codes(inst.size());
+        std::vector<int> nodeBase(inst.size(), 0), triBase(inst.size(), 0);
+        long long nodes = (long long)inst.size() - 1, tris = 0;
+        int enters = 0;
+        for (size_t i = 0; i < inst.size(); ++i) {
+            const xgb_mesh* m = s->objects[i].mesh;
+            if (!inst[i].identity) {
+                codes[i] = leafEncode((int)i, kEnterCount);
+                enters = 1;
+                continue;
+            }
+            nodeBase[i] = (int)std::min<long long>(nodes, INT32_MAX);
+            triBase[i] = (int)std::min<long long>(tris, INT32_MAX);
+            tris += m->nTris;
+            if (!m->rootIsLeaf) nodes += m->nTris - 1;
+            if (tris >= (1ll << 27)) break;
+            codes[i] = m->rootIsLeaf ? leafEncode(triBase[i], m->nTris) : nodeBase[i];
+        }
+        Node2* wn = nullptr;
+        TriV* wt = nullptr;
+        // without room for the copies the scene keeps the kernels that walk its instances
+        if (tris < (1ll << 27) && cudaMalloc((void**)&wn, sizeof(Node2) * (size_t)nodes) == cudaSuccess &&
+            cudaMalloc((void**)&wt, sizeof(TriV) * (size_t)std::max<long long>(tris, 1)) == cudaSuccess) {
+            s->allocations.push_back(wn);
+            s->allocations.push_back(wt);
+            std::vector<Node2> top;
+            buildWorldTop(top, boxes, codes);
+            XGB_CUDA(ctx, cudaMemcpyAsync(wn, top.data(), sizeof(Node2) * top.size(), cudaMemcpyHostToDevice, st));
+            for (size_t i = 0; i < inst.size(); ++i) {
+                const xgb_mesh* m = s->objects[i].mesh;
+                if (inst[i].identity)
+                    worldCopy(m->dNodes2, m->dTris, m->nTris, m->rootIsLeaf != 0, (int)i, nodeBase[i], triBase[i], wn, wt, st);
+            }
+            XGB_CUDA(ctx, cudaGetLastError());
+            XGB_CUDA(ctx, cudaStreamSynchronize(st));  // `top` is read by the copy
+            const float diag = (sceneBox.hi[0] - sceneBox.lo[0]) + (sceneBox.hi[1] - sceneBox.lo[1]) +
+                               (sceneBox.hi[2] - sceneBox.lo[2]);
+            sd.world = WorldDev{wn, wt, 0, enters, 1.0f + 0x1p-19f, std::isfinite(diag) ? diag * 0x1p-22f : 0.0f};
+        } else {
+            dfree(wn);
+            dfree(wt);
+            cudaGetLastError();
+        }
+    }
     sd.materials = dMat;
     sd.textures = dTex;
     sd.svndfs = dSv;
@@ -1371,7 +1469,7 @@ xgb_status xgb_render(xgb_scene* s, const xgb_integrator_params* params, xgb_fil
             if (prof) cudaEventRecord(ev[1], st);
             launchGenerate(s->sd, rp, X, s->ctrl, gShade, st);
             if (prof) cudaEventRecord(ev[2], st);
-            launchExtend(s->sd, X, s->rb.hits, s->ctrl, ctx->numSMs, prof, st);
+            launchExtend(s->sd, X, s->rb.hits, (unsigned int*)s->rb.shadow.o, s->ctrl, ctx->numSMs, prof, st);
             if (prof) cudaEventRecord(ev[3], st);
             if (gd) {
                 guideInferPaths(s->sd, gd->g, gb, X, s->rb.hits, s->ctrl, s->mix, gShade, st);

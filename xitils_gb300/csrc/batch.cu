@@ -62,7 +62,7 @@ struct BatchState {
     unsigned int graphCap = 0;
     int graphIters = 0;
     int graphJobs = 0;
-    int graphFlat = -1;
+    int graphKernels = -1;
     std::map<std::string, xgb_batch_options> tuned;
     xgb_render_stats last{};
 };
@@ -149,7 +149,7 @@ void enqueueBlock(BatchState* b, const BatchView& v, unsigned int cap, int iters
         PathQueue& Y = b->q[(k & 1) ^ 1];
         launchPlan(b->ctrl, cap, st);
         launchGenerateBatch(v, X, b->ctrl, numSMs * 8, st);
-        launchExtendBatch(v, X, b->hits, b->ctrl, numSMs, st);
+        launchExtendBatch(v, X, b->hits, (unsigned int*)b->shadow.o, b->ctrl, numSMs, st);
         launchShadeBatch(v, X, b->hits, Y, b->shadow, b->ctrl, numSMs, st);
         launchShadowBatch(v, b->shadow, Y, b->ctrl, numSMs, st);
     }
@@ -170,12 +170,10 @@ std::string shapeKey(const xgb_batch_job* jobs, int n) {
 xgb_status runBatch(xgb_ctx* ctx, BatchState* b, const xgb_batch_job* jobs, int n, const xgb_batch_options& o,
                     cudaStream_t st, int device, int numSMs, double* seconds) {
     unsigned long long total = 0;
-    int flat = 1, single = 1, nested = 0;
+    int nested = 0;
     for (int i = 0; i < n; ++i) {
         SceneDev sd; int dev, sms, built; cudaStream_t cs;
         sceneView(jobs[i].scene, &sd, &dev, &sms, &cs, &built);
-        if (sd.nInstances > 16 || sd.blasLayout != 0 || sd.shell) flat = 0;
-        if (sd.nInstances != 1 || sd.blasLayout != 0 || sd.shell) single = 0;
         nested |= sd.nested ? 1 : 0;
         void* fd; int w, h, f64, fdev; cudaStream_t fcs;
         filmPlane(jobs[i].film, &fd, &w, &h, &f64, &fdev, &fcs);
@@ -215,16 +213,15 @@ xgb_status runBatch(xgb_ctx* ctx, BatchState* b, const xgb_batch_job* jobs, int 
     if (e == cudaSuccess) e = cudaMemcpyAsync(b->dStart, b->hStart, sizeof(unsigned long long) * (n + 1), cudaMemcpyHostToDevice, st);
     if (e == cudaSuccess) e = cudaMemcpyAsync(b->ctrl, b->ctrlHost, sizeof(Ctrl), cudaMemcpyHostToDevice, st);
     if (e != cudaSuccess) return contextFail(ctx, XGB_CUDA_ERROR, std::string("xgb_render_batch: ") + cudaGetErrorString(e));
-    const int layout = single ? kBatchSingle : flat ? kBatchFlat : 0;
-    const BatchView v{b->dScenes, b->dParams, b->dStart, n, layout, nested};
-    const int kernels = layout | (nested << 2);  // which kernels a captured graph holds
+    const BatchView v{b->dScenes, b->dParams, b->dStart, n, batchKernels(b->hScenes, n), nested};
+    const int kernels = v.kernels | (nested << 4);  // which kernels a captured graph holds
     const int iters = std::max(2, (o.iterations_per_sync + 1) & ~1);
     const auto t0 = std::chrono::steady_clock::now();
     uint64_t launches = 0;
     for (int block = 0;; ++block) {
         const bool replay = o.use_graph && block > 0;  // the first block runs direct (and primes the occupancy cache)
         if (replay && !(b->graph && b->graphCap == capR && b->graphIters == iters && b->graphJobs == n &&
-                        b->graphFlat == kernels)) {
+                        b->graphKernels == kernels)) {
             if (b->graph) { cudaGraphExecDestroy(b->graph); b->graph = nullptr; }
             cudaGraph_t g = nullptr;
             e = cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal);
@@ -238,7 +235,7 @@ xgb_status runBatch(xgb_ctx* ctx, BatchState* b, const xgb_batch_job* jobs, int 
                 b->graph = nullptr;
                 return contextFail(ctx, XGB_CUDA_ERROR, std::string("xgb_render_batch: graph capture: ") + cudaGetErrorString(e));
             }
-            b->graphCap = capR; b->graphIters = iters; b->graphJobs = n; b->graphFlat = kernels;
+            b->graphCap = capR; b->graphIters = iters; b->graphJobs = n; b->graphKernels = kernels;
         }
         if (replay) e = cudaGraphLaunch(b->graph, st);
         else { enqueueBlock(b, v, capR, iters, numSMs, st); e = cudaGetLastError(); }

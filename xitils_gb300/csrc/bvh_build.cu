@@ -695,4 +695,29 @@ cudaError_t buildBlas(const BlasBuildInput& in, BlasBuildOutput* out, cudaStream
     return cudaSuccess;
 }
 
+namespace {
+__global__ void k_worldNodes(const Node2* __restrict__ src, int n, int nodeBase, int triBase, Node2* dst) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    Node2 nd = src[i];
+    auto moved = [&](int c) { return c >= 0 ? c + nodeBase : leafEncode(leafFirst(c) + triBase, leafCount(c)); };
+    nd.d.x = moved(nd.d.x);
+    nd.d.y = moved(nd.d.y);
+    dst[nodeBase + i] = nd;
+}
+__global__ void k_worldTris(const TriV* __restrict__ src, int n, int inst, int triBase, TriV* dst) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    TriV t = src[i];
+    t.p1.w = __int_as_float(inst);
+    dst[triBase + i] = t;
+}
+}  // namespace
+
+void worldCopy(const Node2* nodes, const TriV* tris, int n, bool rootIsLeaf, int inst, int nodeBase, int triBase,
+               Node2* worldNodes, TriV* worldTris, cudaStream_t s) {
+    if (!rootIsLeaf) k_worldNodes<<<(n - 1 + 255) / 256, 256, 0, s>>>(nodes, n - 1, nodeBase, triBase, worldNodes);
+    k_worldTris<<<(n + 255) / 256, 256, 0, s>>>(tris, n, inst, triBase, worldTris);
+}
+
 }  // namespace xgb

@@ -31,6 +31,7 @@ __global__ void k_plan(Ctrl* c, unsigned int capacity, int mode, unsigned int ta
     c->nShadow = 0;
     c->extendHead = 0;
     c->shadowHead = 0;
+    c->nRetrace = 0;
     if (c->nActive) c->iterations += 1;
     if (mode != kPlanWave) c->nTail = c->nActive;
 }

@@ -297,6 +297,56 @@ __global__ void __launch_bounds__(kTraceBlock) k_trace_wide(SceneDev sc, RenderP
         atomicAdd(ANY ? &ctrl->shadowRays : &ctrl->extensionRays, (unsigned long long)n);
 }
 
+// The warp goes on to test triangles when fewer lanes than this are still looking for a
+// leaf. Measured in the flat kernel with 1 / 4 / 8 / 16 lanes: occluded room 47.1 / 42.7 /
+// 42.2 / 44.1 ms per call, Cornell box 4.57 / 4.50 / 4.58 / 4.82, batch 11.8 / 11.5 / 11.7 /
+// 12.8; with discarded hits (shell-mapped cloth) 21.4 / 22.2 / 22.8 / 24.3.
+template <bool SHELL>
+constexpr int kLookingLanes = SHELL ? 1 : 4;
+
+// ---- ray fetch of the persistent per-lane kernels ---------------------------------
+constexpr unsigned int kWarp = 0xFFFFFFFFu;
+// A warp takes new rays when this many of its lanes are without one (or all are). Taking
+// each as soon as a lane is free stalls the other lanes for an atomic and two loads from
+// DRAM each time, and mixes rays that started together: with 1 / 8 / 16 / 24 lanes the
+// terrain's render took 38.7 / 37.5 / 35.0 / 34.7 ms (a pixel's samples stay in one warp),
+// the Cornell box's 4.51 / 4.48 / 4.45 / 4.28, the batch's 11.28 / 11.03 / 11.08 / 11.22, the
+// occluded room's, whose rays are the least alike, 44.5 / 44.0 / 44.1 / 45.9.
+constexpr unsigned int kFetchLanes = 16;
+// Rays of the queue for the lanes of a warp, in order, one atomicAdd for all that want one.
+// Every lane of the warp makes the same calls. (Claiming chunks of 32 / 64 / 128 rays ahead,
+// to save atomics, left some warps with work when the others had none: the batch took
+// 12.1 / 13.2 / 16.6 ms instead of 11.3.)
+struct RayClaims {
+    unsigned int* head;
+    unsigned int n, lanes, next;
+    // few rays: a warp works with its share of lanes only, so that they wait for fewer others
+    __device__ __forceinline__ RayClaims(unsigned int* h, unsigned int count) : head(h), n(count), next(0) {
+        const unsigned int warps = gridDim.x * (kTraceBlock / 32);
+        lanes = min(32u, (n + warps - 1u) / warps);
+    }
+    // The lanes that want a ray (0: none, or not yet worth the trip).
+    __device__ __forceinline__ unsigned int wanted(bool idle) const {
+        const unsigned int m = __ballot_sync(kWarp, idle && (threadIdx.x & 31) < lanes && next < n);
+        return (unsigned int)__popc(m) >= min(kFetchLanes, lanes) ? m : 0u;
+    }
+    // The next rays for the lanes of `want`; returns whether this lane got one.
+    __device__ __forceinline__ bool take(unsigned int want, unsigned int* ray) {
+        const unsigned int lane = threadIdx.x & 31;
+        const unsigned int rank = __popc(want & ((1u << lane) - 1u)), count = __popc(want);
+        unsigned int base = 0;
+        if (lane == 0) base = atomicAdd(head, count);
+        base = __shfl_sync(kWarp, base, 0);
+        const unsigned int i = base + rank;
+        next = base + count;
+        if (((want >> lane) & 1u) && i < n) {
+            *ray = i;
+            return true;
+        }
+        return false;
+    }
+};
+
 // ---- scenes of a few instances: binary mesh BVHs ------------------------------------------------
 // With at most kFlatInstances instances the top level is a short list: a lane
 // walks the instances in order (those whose world box the ray still reaches
@@ -322,7 +372,8 @@ __global__ void __launch_bounds__(kTraceBlock) k_trace_flat2(S scenes, PathQueue
     int job = 0;
     int nInst = 0;
     const int lane = threadIdx.x & 31;
-    const unsigned int ltMask = (1u << lane) - 1u;
+    RayClaims claims(head, n);
+    const int looking = claims.lanes == 32u ? kLookingLanes<SHELL> : 1;
     int stack[kStackDepth];
     int sp = 0;
     int nodeAddr = kSentinel, leafAddr = 0;
@@ -344,15 +395,9 @@ __global__ void __launch_bounds__(kTraceBlock) k_trace_flat2(S scenes, PathQueue
     bool fetch = true;
     WorkCount wc;
     for (int guard = 0;; ++guard) {
-        if (fetch) {
-            // lanes without a ray fetch the next ones together
-            const unsigned int act = __activemask();
-            const int leader = __ffs(act) - 1;
-            unsigned int base = 0;
-            if (lane == leader) base = atomicAdd(head, (unsigned int)__popc(act));
-            base = __shfl_sync(act, base, leader);
-            ray = base + __popc(act & ltMask);
-            if (ray >= n) break;
+        // every lane of the warp comes here; those without a ray take the next ones together
+        const unsigned int want = claims.wanted(fetch);
+        if (want && claims.take(want, &ray)) {
             float4 o4, d4;
             if (ANY) { o4 = __ldcs(&s.o[ray]); d4 = __ldcs(&s.d[ray]); tMax = o4.w; }
             else { o4 = __ldcs(&q.o[ray]); d4 = __ldcs(&q.d[ray]); tMax = __int_as_float(0x7f800000); }
@@ -375,6 +420,8 @@ __global__ void __launch_bounds__(kTraceBlock) k_trace_flat2(S scenes, PathQueue
             leafAddr = 0;
             fetch = false;
         }
+        if (!__any_sync(kWarp, !fetch)) break;
+        if (fetch) continue;
         if (nodeAddr == kSentinel && leafAddr >= 0) {
             // next instance whose world box the ray still reaches
             for (++inst; inst < nInst; ++inst)
@@ -447,7 +494,7 @@ __global__ void __launch_bounds__(kTraceBlock) k_trace_flat2(S scenes, PathQueue
                 leafAddr = nodeAddr;
                 nodeAddr = sp > 0 ? stack[--sp] : kSentinel;
             }
-            if (!__any_sync(__activemask(), searching)) break;
+            if (__popc(__ballot_sync(__activemask(), searching)) < looking) break;
         }
         while (leafAddr < 0) {
             int first = leafFirst(leafAddr), cnt = leafCount(leafAddr);
@@ -471,7 +518,6 @@ __global__ void __launch_bounds__(kTraceBlock) k_trace_flat2(S scenes, PathQueue
         }
     }
     if (COUNT) {
-        __syncwarp();  // every lane of the warp has left the loop
         unsigned long long nv = wc.nodes, nt = wc.tris;
         for (int off = 16; off > 0; off >>= 1) {
             nv += __shfl_down_sync(0xFFFFFFFFu, nv, off);
@@ -486,124 +532,124 @@ __global__ void __launch_bounds__(kTraceBlock) k_trace_flat2(S scenes, PathQueue
         atomicAdd(ANY ? &ctrl->shadowRays : &ctrl->extensionRays, (unsigned long long)n);
 }
 
-// ---- single-mesh scenes ------------------------------------------------------
-// When the scene is one instance, traversal runs as a persistent per-lane state
-// machine in the style of Aila & Laine ("Understanding the Efficiency of Ray
-// Traversal on GPUs", HPG 2009): a lane whose ray is finished fetches the next
-// one at once (one atomicAdd per group of lanes), inner nodes and leaves are
-// processed in separate inner loops, and the first leaf a lane reaches is
-// postponed until every lane of the warp holds one, so that the warp tests
-// triangles together. Results are identical to traceScene: the same slab and
-// watertight tests, the same closest-hit acceptance.
-
+// ---- one BVH per scene -------------------------------------------------------------
+// The traversal of every scene with binary meshes: the scene's world BVH (WorldDev) as a
+// persistent per-lane state machine in the style of Aila & Laine ("Understanding the
+// Efficiency of Ray Traversal on GPUs", HPG 2009): a lane whose ray is finished fetches
+// the next one at once (one atomicAdd per group of lanes), inner nodes and leaves are
+// processed in separate inner loops, and the first leaf a lane reaches is postponed until
+// few lanes of the warp are still looking for one, so that the warp tests triangles
+// together.
+//
+// ENTER: some leaves are instances with a transform. A lane that takes one pushes what it
+// has left, then kReturn, moves its ray into object space and goes on in that mesh; when
+// kReturn comes back it reads its ray again from the queue.
+//
+// The order of the instances: the flat and general kernels visit instances in the scene's
+// order (or top-level order) and a hit is accepted while t <= tMax, so where two
+// instances are hit at distances within rounding of each other, the order decides. Here
+// the nearer box goes first, whatever its instance. So boxes and triangles are visited
+// up to a little beyond the best hit (cullMul, cullAbs), a triangle of another instance
+// accepted or refused within that margin marks the ray, and a marked ray is traced again in the
+// instance order (k_retrace).
+//
 // Ten blocks per SM (48 registers, no spills) rather than the nine that 55 registers
 // allow: the terrain's traversal ran 2.5 % faster; twelve (40 registers) spill and
-// ran 7 % slower.
-//
-// S = OneScene: the mesh, its instance transform and the bounds are the kernel's
-// constants. S = BatchScenes: every job of the batch is a one-instance scene with
-// a binary mesh BVH; a lane loads its ray's mesh when it fetches the ray (the job
-// in the high bits of the pixel field), at eight blocks per SM for the registers
-// that takes.
-template <class S>
-struct SingleTraits {
-    static constexpr int kMinBlocks = 10;
-};
-template <>
-struct SingleTraits<BatchScenes> {
-    static constexpr int kMinBlocks = 8;
+// ran 7 % slower. A batch (S = BatchScenes) reads its ray's BVH when it fetches the ray.
+constexpr int kReturn = kSentinel - 1;
+constexpr int kWorldDepth = kStackDepth + kTlasStack;  // a mesh's entries and the top level's
+constexpr int kWorldStack = kWorldDepth + 2;           // and a return
+constexpr int kMarked = 0x40000000;  // in the hit triangle's index: traced again in instance order
+// A scene of one instance keeps the mesh's own bound (xgb_scene_set_traversal_limits).
+__device__ __forceinline__ int worldStackCap(const SceneDev& sc) {
+    return sc.nInstances == 1 ? sc.stackLimit : kWorldDepth;
+}
+
+template <class S, bool ENTER>
+struct WorldTraits {
+    static constexpr int kMinBlocks = std::is_same<S, OneScene>::value && !ENTER ? 10 : 8;
 };
 
-template <bool ANY, bool COUNT, class S>
-__global__ void __launch_bounds__(kTraceBlock, SingleTraits<S>::kMinBlocks)
-    k_trace_single(S scenes, PathQueue q, HitQueue h, ShadowQueue s, PathQueue out, Ctrl* ctrl) {
+template <bool ANY, bool COUNT, class S, bool ENTER, bool SHELL>
+__global__ void __launch_bounds__(kTraceBlock, (WorldTraits<S, ENTER>::kMinBlocks))
+    k_trace_world(S scenes, PathQueue q, HitQueue h, unsigned int* retrace, ShadowQueue s, PathQueue out, Ctrl* ctrl) {
     constexpr bool kBatch = !std::is_same<S, OneScene>::value;
     const unsigned int n = ANY ? ctrl->nShadow : ctrl->nActive;
     unsigned int* head = ANY ? &ctrl->shadowHead : &ctrl->extendHead;
-    // one scene: its only mesh for every ray; a batch: the current ray's
-    const Instance* in0 = kBatch ? nullptr : &scenes.scene(0).instances[0];
-    const bool identity0 = kBatch ? true : in0->identity != 0;
-    const MeshDev m0 = kBatch ? MeshDev{} : scenes.scene(0).meshes[in0->mesh];
-    const Node2* nodes = m0.nodes2;
-    const TriV* tris = m0.tris;
-    int job = 0;
-    int rayMaxSteps = 0, rayStack = 0;  // a batch: the current ray's job's bounds
     const int lane = threadIdx.x & 31;
-    const unsigned int ltMask = (1u << lane) - 1u;
-    int stack[kStackDepth];
+    RayClaims claims(head, n);
+    const int looking = claims.lanes == 32u ? kLookingLanes<SHELL> : 1;
+    bool holds = false;  // the lane has a ray
+    // one scene: its BVH for every ray; a batch: the current ray's
+    const Node2* nodes = kBatch ? nullptr : scenes.scene(0).world.nodes;
+    const TriV* tris = kBatch ? nullptr : scenes.scene(0).world.tris;
+    int job = 0;
+    int rayStack = 0;   // a batch: the current ray's job's bound
+    int inst = -1;      // ENTER: the instance the ray is in (-1: world space)
+    int hitInst = -1;   // ENTER: the instance of a hit found inside one
+    int stack[kWorldStack];
     int sp = 0;
     int nodeAddr = kSentinel, leafAddr = 0;
     unsigned int ray = 0;
     WRay r;
-    float tMax = 0.0f;
-    TraceHit hit;
-    hit.prim = -1;
-    hit.t = 0.0f;
-    hit.b0 = hit.b1 = 0.0f;
+    float tMax = 0.0f, tCull = 0.0f, b0 = 0.0f, b1 = 0.0f;
+    int hitTri = -1;  // index in the triangle array, ENTER: the original triangle index
     bool occluded = false;
     WorkCount wc;
     for (int guard = 0;; ++guard) {
-        if (nodeAddr == kSentinel) {
-            // lanes without a ray fetch the next ones together
-            const unsigned int act = __activemask();
-            const int leader = __ffs(act) - 1;
-            unsigned int base = 0;
-            if (lane == leader) base = atomicAdd(head, (unsigned int)__popc(act));
-            base = __shfl_sync(act, base, leader);
-            ray = base + __popc(act & ltMask);
-            if (ray >= n) break;
+        // every lane of the warp comes here; those without a ray take the next ones together
+        const unsigned int want = claims.wanted(!holds);
+        if (want && claims.take(want, &ray)) {
+            holds = true;
             float4 o4, d4;
             if (ANY) { o4 = __ldcs(&s.o[ray]); d4 = __ldcs(&s.d[ray]); tMax = o4.w; }
             else { o4 = __ldcs(&q.o[ray]); d4 = __ldcs(&q.d[ray]); tMax = __int_as_float(0x7f800000); }
             V3 o(o4.x, o4.y, o4.z), d(d4.x, d4.y, d4.z);
-            const Instance* in = in0;
-            bool identity = identity0;
-            if (kBatch) {
-                job = scenes.jobOf(ANY ? __float_as_uint(d4.w) : __float_as_uint(__ldg(&q.thr[ray].w)));
-                in = &scenes.scene(job).instances[0];
-                identity = in->identity != 0;
-                rayMaxSteps = scenes.scene(job).maxSteps;
-                rayStack = scenes.scene(job).stackLimit;
+            if (kBatch) job = scenes.jobOf(ANY ? __float_as_uint(d4.w) : __float_as_uint(__ldg(&q.thr[ray].w)));
+            const SceneDev& sc = scenes.scene(job);
+            if (kBatch || ENTER) {  // a shadow ray may have ended inside an instance
+                nodes = sc.world.nodes;
+                tris = sc.world.tris;
             }
-            if (!identity) {
-                o = xformPointRn(in->matInv, o);
-                d = xformVectorRn(in->matInv, d);
+            if (kBatch) rayStack = worldStackCap(sc);
+            if (sc.nInstances == 1) {  // the mesh's own arrays: its transform applies to every ray
+                const Instance& in = sc.instances[0];
+                if (!in.identity) {
+                    o = xformPointRn(in.matInv, o);
+                    d = xformVectorRn(in.matInv, d);
+                }
             }
             r = makeWRay(o, d);
-            hit.prim = -1;
-            hit.t = tMax;
+            hitTri = -1;
+            tCull = tMax;
             occluded = false;
             sp = 0;
             guard = 0;
-            int rootIsLeaf = m0.rootIsLeaf, rootLeaf = m0.rootLeaf;
-            if (kBatch) {
-                const MeshDev& m = scenes.scene(job).meshes[in->mesh];
-                nodes = m.nodes2;
-                tris = m.tris;
-                rootIsLeaf = m.rootIsLeaf;
-                rootLeaf = m.rootLeaf;
-            }
-            if (rootIsLeaf) { leafAddr = rootLeaf; nodeAddr = kSentinel; }
-            else { leafAddr = 0; nodeAddr = 0; }
+            if (ENTER) inst = hitInst = -1;
+            const int root = sc.world.root;
+            if (root < 0) { leafAddr = root; nodeAddr = kSentinel; }
+            else { leafAddr = 0; nodeAddr = root; }
         }
-        if (guard > (kBatch ? rayMaxSteps : scenes.scene(0).maxSteps)) {
+        if (!__any_sync(kWarp, holds)) break;
+        if (!holds) continue;
+        if (guard > scenes.scene(job).maxSteps) {
             atomicOr(&ctrl->errors, 4u);
             nodeAddr = kSentinel;
             leafAddr = 0;
         }
         bool searching = true;
-        while ((unsigned int)nodeAddr < (unsigned int)kSentinel) {
+        while ((unsigned int)nodeAddr < (unsigned int)kReturn) {
             if (COUNT) wc.nodes++;
             const Node2* nd = nodes + nodeAddr;
             float4 a = __ldg(&nd->a), b = __ldg(&nd->b), c = __ldg(&nd->c);
             int4 dd = __ldg(&nd->d);
             float t0, t1;
-            bool h0 = slab(r, a.x, a.y, a.z, a.w, b.x, b.y, tMax, t0);
-            bool h1 = slab(r, b.z, b.w, c.x, c.y, c.z, c.w, tMax, t1);
+            bool h0 = slab(r, a.x, a.y, a.z, a.w, b.x, b.y, tCull, t0);
+            bool h1 = slab(r, b.z, b.w, c.x, c.y, c.z, c.w, tCull, t1);
             if (h0 && h1) {
                 int near = dd.x, far = dd.y;
                 if (t1 < t0) { near = dd.y; far = dd.x; }
-                if (sp >= (kBatch ? rayStack : scenes.scene(0).stackLimit)) {
+                if (sp >= (kBatch ? rayStack : worldStackCap(scenes.scene(0)))) {
                     atomicOr(&ctrl->errors, 1u);
                     sp = 0;
                     nodeAddr = kSentinel;
@@ -623,27 +669,83 @@ __global__ void __launch_bounds__(kTraceBlock, SingleTraits<S>::kMinBlocks)
                 leafAddr = nodeAddr;
                 nodeAddr = sp > 0 ? stack[--sp] : kSentinel;
             }
-            if (!__any_sync(__activemask(), searching)) break;
+            if (__popc(__ballot_sync(__activemask(), searching)) < looking) break;
+        }
+        if (ENTER && nodeAddr < 0 && leafAddr >= 0) {  // a leaf waited below kReturn
+            leafAddr = nodeAddr;
+            nodeAddr = sp > 0 ? stack[--sp] : kSentinel;
         }
         while (leafAddr < 0) {
-            int first = leafFirst(leafAddr), cnt = leafCount(leafAddr);
+            const int first = leafFirst(leafAddr), cnt = leafCount(leafAddr);
+            if (ENTER && cnt == kEnterCount) {
+                // into the instance: what is left of the world waits below kReturn
+                if (nodeAddr != kSentinel) stack[sp++] = nodeAddr;
+                stack[sp++] = kReturn;
+                const SceneDev& sc = scenes.scene(job);
+                const Instance& in = sc.instances[first];
+                const MeshDev& m = sc.meshes[in.mesh];
+                const float4 o4 = ANY ? s.o[ray] : q.o[ray], d4 = ANY ? s.d[ray] : q.d[ray];
+                r = makeWRay(xformPointRn(in.matInv, V3(o4.x, o4.y, o4.z)), xformVectorRn(in.matInv, V3(d4.x, d4.y, d4.z)));
+                inst = first;
+                nodes = m.nodes2;
+                tris = m.tris;
+                leafAddr = m.rootIsLeaf ? m.rootLeaf : 0;
+                nodeAddr = m.rootIsLeaf ? stack[--sp] : 0;
+                if (!m.rootIsLeaf) break;
+                continue;
+            }
             if (COUNT) wc.tris += cnt;
             for (int k = 0; k < cnt; ++k) {
                 const TriV* tv = tris + first + k;
-                float4 p0 = __ldg(&tv->p0), p1 = __ldg(&tv->p1), p2 = __ldg(&tv->p2);
-                float t, b0, b1;
-                if (watertight(r, p0, p1, p2, tMax, t, b0, b1)) {
-                    tMax = t;
+                const float4 p0 = __ldg(&tv->p0), p1 = __ldg(&tv->p1), p2 = __ldg(&tv->p2);
+                float t, c0, c1;
+                if (watertight(r, p0, p1, p2, ANY ? tMax : tCull, t, c0, c1)) {
+                    if (SHELL) {
+                        const int of = ENTER && inst >= 0 ? inst : __float_as_int(p1.w);
+                        const SceneDev& sc = scenes.scene(job);
+                        const MeshDev& m = sc.meshes[sc.instances[of].mesh];
+                        if (m.shellLayers && shellDiscard(m, __float_as_int(p0.w), c0, c1)) continue;
+                    }
                     if (ANY) { occluded = true; break; }
-                    hit.t = t; hit.b0 = b0; hit.b1 = b1;
-                    hit.prim = __float_as_int(p0.w);
+                    const WorldDev& w = scenes.scene(job).world;
+                    const float beyond = fmaf(t, w.cullMul, w.cullAbs);
+                    int marked = hitTri >= 0 ? hitTri & kMarked : 0;
+                    if (hitTri >= 0 && !(beyond < tMax)) {  // refused, or hardly nearer
+                        const int now = ENTER && inst >= 0 ? inst : __float_as_int(p1.w);
+                        const int before = ENTER ? hitInst : __float_as_int(__ldg(&tris[hitTri & ~kMarked].p1.w));
+                        if (now != before) {
+                            marked = kMarked;
+                            hitTri |= kMarked;
+                            if (!(t <= tMax)) continue;
+                        } else if (!watertight(r, p0, p1, p2, tMax, t, c0, c1)) {
+                            continue;  // within a mesh the order is its own, and so is the rule
+                        }
+                    }
+                    tMax = t;
+                    tCull = beyond;
+                    b0 = c0;
+                    b1 = c1;
+                    hitTri = marked | (ENTER ? __float_as_int(p0.w) : first + k);
+                    if (ENTER) hitInst = inst >= 0 ? inst : __float_as_int(p1.w);
                 }
             }
             if (ANY && occluded) { leafAddr = 0; nodeAddr = kSentinel; break; }
             leafAddr = nodeAddr;  // another leaf was postponed: take it next
             if (nodeAddr < 0) nodeAddr = sp > 0 ? stack[--sp] : kSentinel;
         }
+        if (ENTER && nodeAddr == kReturn && leafAddr >= 0) {  // back to world space
+            const SceneDev& sc = scenes.scene(job);
+            const float4 o4 = ANY ? s.o[ray] : q.o[ray], d4 = ANY ? s.d[ray] : q.d[ray];
+            r = makeWRay(V3(o4.x, o4.y, o4.z), V3(d4.x, d4.y, d4.z));
+            inst = -1;
+            nodes = sc.world.nodes;
+            tris = sc.world.tris;
+            nodeAddr = sp > 0 ? stack[--sp] : kSentinel;
+            leafAddr = 0;
+        }
         if (nodeAddr == kSentinel && leafAddr >= 0) {  // ray finished
+            holds = false;
+            const SceneDev& sc = scenes.scene(job);
             if (ANY) {
                 if (!occluded) {
                     float4 cc = s.c[ray];
@@ -654,13 +756,24 @@ __global__ void __launch_bounds__(kTraceBlock, SingleTraits<S>::kMinBlocks)
                     if (rp.train) creditPath(rp, s.pid[ray], cc);
                 }
             } else {
-                __stcs(&h.h[ray], make_float4(hit.prim >= 0 ? hit.t : tMax, hit.b0, hit.b1, __int_as_float(hit.prim)));
-                __stcs(&h.inst[ray], hit.prim >= 0 ? 0 : -1);
+                int prim = -1, of = -1;
+                if (hitTri >= 0) {
+                    if ((hitTri & kMarked) && sc.nInstances > 1) retrace[atomicAdd(&ctrl->nRetrace, 1u)] = ray;
+                    if (ENTER) {
+                        prim = hitTri & ~kMarked;
+                        of = hitInst;
+                    } else {
+                        const TriV* tv = tris + (hitTri & ~kMarked);
+                        prim = __float_as_int(__ldg(&tv->p0.w));
+                        of = __float_as_int(__ldg(&tv->p1.w));
+                    }
+                }
+                __stcs(&h.h[ray], make_float4(tMax, b0, b1, __int_as_float(prim)));
+                __stcs(&h.inst[ray], of);
             }
         }
     }
     if (COUNT) {
-        __syncwarp();  // every lane of the warp has left the loop
         unsigned long long nv = wc.nodes, nt = wc.tris;
         for (int off = 16; off > 0; off >>= 1) {
             nv += __shfl_down_sync(0xFFFFFFFFu, nv, off);
@@ -673,6 +786,22 @@ __global__ void __launch_bounds__(kTraceBlock, SingleTraits<S>::kMinBlocks)
     }
     if (blockIdx.x == 0 && threadIdx.x == 0)
         atomicAdd(ANY ? &ctrl->shadowRays : &ctrl->extensionRays, (unsigned long long)n);
+}
+
+// The marked rays of a k_trace_world launch, in the instance order.
+template <class S>
+__global__ void __launch_bounds__(kTraceBlock) k_retrace(S scenes, PathQueue q, HitQueue h, const unsigned int* retrace,
+                                                         Ctrl* ctrl) {
+    const unsigned int n = ctrl->nRetrace;
+    for (unsigned int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
+        const unsigned int ray = retrace[k];
+        const float4 o = q.o[ray], d = q.d[ray];
+        TraceHit hit;
+        traceCall(scenes.scene(scenes.jobOf(__float_as_uint(q.thr[ray].w))), V3(o.x, o.y, o.z), V3(d.x, d.y, d.z),
+                  __int_as_float(0x7f800000), false, hit, &ctrl->errors);
+        h.h[ray] = make_float4(hit.t, hit.b0, hit.b1, __int_as_float(hit.prim));
+        h.inst[ray] = hit.inst;
+    }
 }
 
 // ---- batches of scenes (xgb_render_batch) -----------------------------------------
@@ -766,13 +895,45 @@ static int persistentGrid(K kernel, int numSMs) {
     return numSMs * it->second;
 }
 
-// Of the specialised kernels only the flat binary one carries the shell-mapping
-// discard (its SHELL variant, which also takes one-instance shell scenes); a scene
-// with a shell-mapped mesh otherwise takes the generic pair.
-void launchExtend(const SceneDev& sc, PathQueue q, HitQueue h, Ctrl* ctrl, int numSMs, bool count, cudaStream_t s) {
+// The world BVH's kernel takes scenes of one instance, scenes of more than kFlatInstances,
+// and the shadow rays of those between that have a world BVH (large ones, see
+// xgb_scene_build), unless several instances come with traversal limits other than the
+// defaults, which count the steps of the kernels that walk the instances. Against the
+// flat kernel on scenes of few instances: any hit 17.0 -> 13.9 ms per call in the occluded
+// room (200,000 triangles and a light), 3.5 -> 2.9 with the proposal, 0.73 -> 0.79 in the
+// Cornell box (36 triangles, ten instances), the shell-mapped cloth 7.6 -> 7.8; closest hit
+// 42.6 -> 44.6, 8.1 -> 8.7, 1.85 -> 2.14, 21.6 -> 22.1. Against the generic pair (67 instances,
+// normal mapping): 3.15 -> 2.34 and 1.40 -> 1.03. 8-wide meshes keep the wide kernel (at most
+// kFlatInstances instances) and the generic pair (any other, and shell-mapped ones).
+static bool useWorld(const SceneDev& sc, bool any) {
+    if (!sc.world.tris) return false;
+    if (sc.nInstances == 1) return true;
+    return (any || sc.nInstances > kFlatInstances) && sc.maxSteps == kDefaultMaxSteps && sc.stackLimit == kMaxStackLimit;
+}
+#define XGB_LAUNCH(K) K<<<persistentGrid(K, numSMs), kTraceBlock, 0, s>>>
+constexpr int kRetraceBlocks = 152;  // a launch that usually finds a handful of rays
+template <bool ANY, bool COUNT>
+static void launchWorld(const SceneDev& sc, const RenderParams& rp, PathQueue q, HitQueue h, unsigned int* retrace,
+                        ShadowQueue sq, PathQueue out, Ctrl* ctrl, int numSMs, cudaStream_t s) {
+    const OneScene one{sc, rp};
+    if (sc.shell) {
+        if (sc.world.enters) XGB_LAUNCH((k_trace_world<ANY, COUNT, OneScene, true, true>))(one, q, h, retrace, sq, out, ctrl);
+        else XGB_LAUNCH((k_trace_world<ANY, COUNT, OneScene, false, true>))(one, q, h, retrace, sq, out, ctrl);
+    } else {
+        if (sc.world.enters) XGB_LAUNCH((k_trace_world<ANY, COUNT, OneScene, true, false>))(one, q, h, retrace, sq, out, ctrl);
+        else XGB_LAUNCH((k_trace_world<ANY, COUNT, OneScene, false, false>))(one, q, h, retrace, sq, out, ctrl);
+    }
+    if (!ANY && sc.nInstances > 1) k_retrace<OneScene><<<kRetraceBlocks, kTraceBlock, 0, s>>>(one, q, h, retrace, ctrl);
+}
+void launchExtend(const SceneDev& sc, PathQueue q, HitQueue h, unsigned int* retrace, Ctrl* ctrl, int numSMs, bool count,
+                  cudaStream_t s) {
     RenderParams none{};
     const bool flat = sc.nInstances <= kFlatInstances;
-#define XGB_LAUNCH(K) K<<<persistentGrid(K, numSMs), kTraceBlock, 0, s>>>
+    if (useWorld(sc, false)) {
+        if (count) launchWorld<false, true>(sc, none, q, h, retrace, ShadowQueue{}, PathQueue{}, ctrl, numSMs, s);
+        else launchWorld<false, false>(sc, none, q, h, retrace, ShadowQueue{}, PathQueue{}, ctrl, numSMs, s);
+        return;
+    }
     if (sc.shell) {
         if (flat && sc.blasLayout == 0) {
             if (count) XGB_LAUNCH((k_trace_flat2<false, true, OneScene, true>))(OneScene{sc, none}, q, h, ShadowQueue{}, PathQueue{}, ctrl);
@@ -787,9 +948,6 @@ void launchExtend(const SceneDev& sc, PathQueue q, HitQueue h, Ctrl* ctrl, int n
     if (flat && sc.blasLayout == 1) {
         if (count) XGB_LAUNCH((k_trace_wide<false, true>))(sc, none, q, h, ShadowQueue{}, PathQueue{}, ctrl);
         else XGB_LAUNCH((k_trace_wide<false, false>))(sc, none, q, h, ShadowQueue{}, PathQueue{}, ctrl);
-    } else if (sc.nInstances == 1 && sc.blasLayout == 0) {
-        if (count) XGB_LAUNCH((k_trace_single<false, true, OneScene>))(OneScene{sc, none}, q, h, ShadowQueue{}, PathQueue{}, ctrl);
-        else XGB_LAUNCH((k_trace_single<false, false, OneScene>))(OneScene{sc, none}, q, h, ShadowQueue{}, PathQueue{}, ctrl);
     } else if (flat && sc.blasLayout == 0) {
         if (count) XGB_LAUNCH((k_trace_flat2<false, true, OneScene>))(OneScene{sc, none}, q, h, ShadowQueue{}, PathQueue{}, ctrl);
         else XGB_LAUNCH((k_trace_flat2<false, false, OneScene>))(OneScene{sc, none}, q, h, ShadowQueue{}, PathQueue{}, ctrl);
@@ -799,22 +957,13 @@ void launchExtend(const SceneDev& sc, PathQueue q, HitQueue h, Ctrl* ctrl, int n
         XGB_LAUNCH((k_extend<false>))(sc, q, h, ctrl);
     }
 }
-void launchExtendBatch(const BatchView& b, PathQueue q, HitQueue h, Ctrl* ctrl, int numSMs, cudaStream_t s) {
-    if (b.flat == kBatchSingle)
-        XGB_LAUNCH((k_trace_single<false, false, BatchScenes>))(BatchScenes{b}, q, h, ShadowQueue{}, PathQueue{}, ctrl);
-    else if (b.flat) XGB_LAUNCH((k_trace_flat2<false, false, BatchScenes>))(BatchScenes{b}, q, h, ShadowQueue{}, PathQueue{}, ctrl);
-    else XGB_LAUNCH(k_extend_batch)(b, q, h, ctrl);
-}
-void launchShadowBatch(const BatchView& b, ShadowQueue sq, PathQueue out, Ctrl* ctrl, int numSMs, cudaStream_t s) {
-    if (b.flat == kBatchSingle)
-        XGB_LAUNCH((k_trace_single<true, false, BatchScenes>))(BatchScenes{b}, PathQueue{}, HitQueue{}, sq, out, ctrl);
-    else if (b.flat) XGB_LAUNCH((k_trace_flat2<true, false, BatchScenes>))(BatchScenes{b}, PathQueue{}, HitQueue{}, sq, out, ctrl);
-    else XGB_LAUNCH(k_shadow_batch)(b, sq, out, ctrl);
-}
-
 void launchShadow(const SceneDev& sc, const RenderParams& rp, ShadowQueue sq, PathQueue out, Ctrl* ctrl, int numSMs,
                   cudaStream_t s) {
     const bool flat = sc.nInstances <= kFlatInstances;
+    if (useWorld(sc, true)) {
+        launchWorld<true, false>(sc, rp, PathQueue{}, HitQueue{}, nullptr, sq, out, ctrl, numSMs, s);
+        return;
+    }
     if (sc.shell) {
         if (flat && sc.blasLayout == 0)
             XGB_LAUNCH((k_trace_flat2<true, false, OneScene, true>))(OneScene{sc, rp}, PathQueue{}, HitQueue{}, sq, out, ctrl);
@@ -822,12 +971,53 @@ void launchShadow(const SceneDev& sc, const RenderParams& rp, ShadowQueue sq, Pa
         return;
     }
     if (flat && sc.blasLayout == 1) XGB_LAUNCH((k_trace_wide<true, false>))(sc, rp, PathQueue{}, HitQueue{}, sq, out, ctrl);
-    else if (sc.nInstances == 1 && sc.blasLayout == 0)
-        XGB_LAUNCH((k_trace_single<true, false, OneScene>))(OneScene{sc, rp}, PathQueue{}, HitQueue{}, sq, out, ctrl);
     else if (flat && sc.blasLayout == 0)
         XGB_LAUNCH((k_trace_flat2<true, false, OneScene>))(OneScene{sc, rp}, PathQueue{}, HitQueue{}, sq, out, ctrl);
     else XGB_LAUNCH(k_shadow)(sc, rp, sq, out, ctrl);
-#undef XGB_LAUNCH
 }
+
+int batchKernels(const SceneDev* scenes, int n) {
+    bool world = true, worldShadow = true, enters = false, flat = true;
+    for (int j = 0; j < n; ++j) {
+        const SceneDev& sc = scenes[j];
+        const bool all = !sc.shell && useWorld(sc, true);
+        worldShadow = worldShadow && all;
+        // scenes of few instances take it only where others in the batch need it
+        world = world && all;
+        enters = enters || sc.world.enters;
+        flat = flat && sc.nInstances <= kFlatInstances && sc.blasLayout == 0 && !sc.shell;
+    }
+    bool single = true;
+    for (int j = 0; j < n; ++j) single = single && scenes[j].nInstances == 1;
+    if (flat && !(single && world)) return worldShadow && !enters ? kBatchFlatWorldShadow : kBatchFlat;
+    return world ? (enters ? kBatchWorldEnter : kBatchWorld) : kBatchGeneral;
+}
+void launchExtendBatch(const BatchView& b, PathQueue q, HitQueue h, unsigned int* retrace, Ctrl* ctrl, int numSMs,
+                       cudaStream_t s) {
+    const BatchScenes sc{b};
+    switch (b.kernels) {
+    case kBatchWorld:
+    case kBatchWorldEnter:
+        if (b.kernels == kBatchWorld)
+            XGB_LAUNCH((k_trace_world<false, false, BatchScenes, false, false>))(sc, q, h, retrace, ShadowQueue{}, PathQueue{}, ctrl);
+        else XGB_LAUNCH((k_trace_world<false, false, BatchScenes, true, false>))(sc, q, h, retrace, ShadowQueue{}, PathQueue{}, ctrl);
+        k_retrace<BatchScenes><<<kRetraceBlocks, kTraceBlock, 0, s>>>(sc, q, h, retrace, ctrl);
+        break;
+    case kBatchFlat:
+    case kBatchFlatWorldShadow: XGB_LAUNCH((k_trace_flat2<false, false, BatchScenes>))(sc, q, h, ShadowQueue{}, PathQueue{}, ctrl); break;
+    default: XGB_LAUNCH(k_extend_batch)(b, q, h, ctrl);
+    }
+}
+void launchShadowBatch(const BatchView& b, ShadowQueue sq, PathQueue out, Ctrl* ctrl, int numSMs, cudaStream_t s) {
+    const BatchScenes sc{b};
+    switch (b.kernels) {
+    case kBatchWorld:
+    case kBatchFlatWorldShadow: XGB_LAUNCH((k_trace_world<true, false, BatchScenes, false, false>))(sc, PathQueue{}, HitQueue{}, nullptr, sq, out, ctrl); break;
+    case kBatchWorldEnter: XGB_LAUNCH((k_trace_world<true, false, BatchScenes, true, false>))(sc, PathQueue{}, HitQueue{}, nullptr, sq, out, ctrl); break;
+    case kBatchFlat: XGB_LAUNCH((k_trace_flat2<true, false, BatchScenes>))(sc, PathQueue{}, HitQueue{}, sq, out, ctrl); break;
+    default: XGB_LAUNCH(k_shadow_batch)(b, sq, out, ctrl);
+    }
+}
+#undef XGB_LAUNCH
 
 }  // namespace xgb

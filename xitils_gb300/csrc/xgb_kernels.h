@@ -37,6 +37,11 @@ struct BlasBuildOutput {
 // Returns a CUDA error code (cudaSuccess on success).
 cudaError_t buildBlas(const BlasBuildInput& in, BlasBuildOutput* out, cudaStream_t stream);
 
+// An instance's share of a world BVH (WorldDev): the mesh's n - 1 nodes renumbered to start
+// at nodeBase, its n triangles at triBase with the instance's number.
+void worldCopy(const Node2* nodes, const TriV* tris, int n, bool rootIsLeaf, int inst, int nodeBase, int triBase,
+               Node2* worldNodes, TriV* worldTris, cudaStream_t s);
+
 // SVNDF fit of a displacement map (svndf.cu): lobes [resV][resU][5] float4, low
 // heights [resV][resU] float4 (red channel). rate in [1, 16].
 cudaError_t svndfFit(const TextureDev& src, float scale, int rate, uint32_t seed, int resU, int resV, float4* lobes,
@@ -54,6 +59,8 @@ struct Ctrl {
     unsigned int extendHead;       // persistent work counters
     unsigned int shadowHead;
     unsigned int errors;           // bit 0: traversal stack overflow
+    unsigned int nRetrace;         // rays whose hits the instance order decides (k_trace_world)
+    unsigned int pad;
     unsigned int nTail;            // paths the next tail launch finishes (0: it does nothing)
     unsigned long long extensionRays;
     unsigned long long shadowRays;
@@ -144,20 +151,23 @@ struct RenderParams {
 
 // Device arrays of a batch of render jobs sharing one wavefront (xgb_render_batch):
 // a path of job j carries j << 24 | pixel in its pixel field.
-constexpr int kBatchFlat = 1, kBatchSingle = 2;
+// Which traversal kernels a batch takes: every scene has a world BVH (without / with
+// instances to enter); every scene has <= 16 instances and binary mesh BVHs; any other.
+enum BatchKernels : int { kBatchGeneral = 0, kBatchFlat = 1, kBatchWorld = 2, kBatchWorldEnter = 3, kBatchFlatWorldShadow = 4 };
 struct BatchView {
     const SceneDev* scenes;
     const RenderParams* params;
     const unsigned long long* start;  // nJobs + 1 prefix sums of the jobs' path counts
     int nJobs;
-    int flat;    // kBatchFlat: every scene has <= 16 instances and binary mesh BVHs (the persistent per-lane
-                 // kernels); kBatchSingle: every scene is one instance of a binary mesh BVH; 0: general
+    int kernels; // BatchKernels
     int nested;  // some scene has a material that evaluates another (the shade kernel with that code)
 };
+int batchKernels(const SceneDev* scenes, int n);
 void launchGenerateBatch(const BatchView& b, PathQueue q, Ctrl* ctrl, int grid, cudaStream_t s);
 void launchShadeBatch(const BatchView& b, PathQueue in, HitQueue h, PathQueue out, ShadowQueue sq, Ctrl* ctrl,
                       int numSMs, cudaStream_t s);
-void launchExtendBatch(const BatchView& b, PathQueue q, HitQueue h, Ctrl* ctrl, int numSMs, cudaStream_t s);
+void launchExtendBatch(const BatchView& b, PathQueue q, HitQueue h, unsigned int* retrace, Ctrl* ctrl, int numSMs,
+                       cudaStream_t s);
 void launchShadowBatch(const BatchView& b, ShadowQueue sq, PathQueue out, Ctrl* ctrl, int numSMs, cudaStream_t s);
 
 // Queue bookkeeping of an iteration. mode kPlanWave: a wavefront iteration; kPlanTail: the
@@ -179,7 +189,9 @@ void launchTail(const SceneDev& sc, const RenderParams& rp, PathQueue in, PathQu
 void launchGenerate(const SceneDev& sc, const RenderParams& rp, PathQueue q, Ctrl* ctrl, int grid, cudaStream_t s);
 // Extension / shadow rays and shading of the wavefront; grids sized from the
 // launched kernel's occupancy on numSMs SMs (one full wave).
-void launchExtend(const SceneDev& sc, PathQueue q, HitQueue h, Ctrl* ctrl, int numSMs, bool count, cudaStream_t s);
+// retrace: room for one number per path in the queue (the shadow queue, which is empty then).
+void launchExtend(const SceneDev& sc, PathQueue q, HitQueue h, unsigned int* retrace, Ctrl* ctrl, int numSMs, bool count,
+                  cudaStream_t s);
 void launchShade(const SceneDev& sc, const RenderParams& rp, PathQueue in, HitQueue h, PathQueue out, ShadowQueue sq,
                  Ctrl* ctrl, int numSMs, cudaStream_t s);
 void launchShadow(const SceneDev& sc, const RenderParams& rp, ShadowQueue sq, PathQueue out, Ctrl* ctrl, int numSMs,

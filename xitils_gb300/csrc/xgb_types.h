@@ -50,11 +50,15 @@ constexpr int kWideLeafMax = 3;  // triangles per leaf child of a WNode
 __host__ __device__ inline int leafEncode(int first, int count) { return ~((first << 4) | (count - 1)); }
 __host__ __device__ inline int leafFirst(int code) { return (~code) >> 4; }
 __host__ __device__ inline int leafCount(int code) { return ((~code) & 15) + 1; }
+// Leaf of a world BVH that is an instance with a transform: a triangle leaf's code with a
+// count that no triangle leaf has.
+constexpr int kEnterCount = 16;
+static_assert(kLeafMax < kEnterCount, "leaf codes of triangles and of instances are distinct");
 
 // Triangle vertices gathered in BVH leaf order: p0.xyz + original triangle index, p1, p2.
 struct __align__(16) TriV {
     float4 p0;  // w = __int_as_float(original triangle index)
-    float4 p1;
+    float4 p1;  // w = __int_as_float(instance) (0 in a mesh's own array)
     float4 p2;
 };
 
@@ -149,6 +153,20 @@ struct LightDev {
     int triOffset;
 };
 
+// One binary BVH over every instance of a scene (all meshes binary): the nodes and
+// triangles of the instances with an identity transform, copied and renumbered, under a
+// top level whose other leaves are instances to enter with their own ray. A scene of one
+// instance uses its mesh's arrays as they are.
+struct WorldDev {
+    const Node2* nodes;  // nullptr: no such BVH (8-wide meshes)
+    const TriV* tris;
+    int root;      // node, or a leaf code
+    int enters;    // 1 when some leaf is an instance with a transform
+    // Boxes and triangles up to hit * cullMul + cullAbs are still visited (see trace.cu: rays
+    // whose nearest hits of two instances are that close are decided by the instance order).
+    float cullMul, cullAbs;
+};
+
 constexpr int kDefaultMaxSteps = 1 << 22;
 constexpr int kMaxStackLimit = 64;
 
@@ -170,6 +188,7 @@ struct SceneDev {
     int maxSteps;
     int stackLimit;
     const float4* instBox;  // per instance: world box lo (xyz), hi (xyz) as 2 float4
+    WorldDev world;
     const Material* materials;
     const TextureDev* textures;
     const SvndfDev* svndfs;
