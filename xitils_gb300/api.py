@@ -227,9 +227,8 @@ def _release(obj, destroy: str) -> None:
     """Destroys obj's handle while its context is alive. Every wrapper keeps Python
     references to the handles its handle points at (a scene to its meshes, materials,
     textures and guide; a material to its textures, base and SVNDF; a shell-mapped
-    mesh to its displacement map), so nothing the library still reads is freed; the
-    library's destroy calls free device memory with cudaFree, which waits for the
-    device's work in flight."""
+    mesh to its displacement map), so nothing the library still reads is freed; every
+    call that uses device memory has waited for its work when it returns."""
     h = getattr(obj, "h", None)
     ctx = getattr(obj, "ctx", None)
     if h and ctx is not None and getattr(ctx, "h", None):

@@ -24,7 +24,7 @@
 // to 8 bits against its own box (rounded outwards), and gathers the leaf
 // children's triangles next to each other (48 B per triangle).
 #include <cub/device/device_radix_sort.cuh>
-#include <cub/device/device_select.cuh>
+#include <algorithm>
 
 #include "xgb_kernels.h"
 
@@ -237,59 +237,242 @@ __global__ void k_plocInit(const unsigned int* __restrict__ vals, int n, const f
     parent[k] = -1;
 }
 
-__global__ void __launch_bounds__(kPlocBlock) k_plocNearest(const int* __restrict__ clusters, int nc,
-                                                            const float4* __restrict__ nodeLo,
-                                                            const float4* __restrict__ nodeHi, int* nn) {
-    __shared__ float4 sLo[kPlocBlock + 2 * kPlocRadius], sHi[kPlocBlock + 2 * kPlocRadius];
-    const int b0 = blockIdx.x * kPlocBlock;
-    for (int t = threadIdx.x; t < kPlocBlock + 2 * kPlocRadius; t += kPlocBlock) {
-        int j = b0 - kPlocRadius + t;
-        if (j >= 0 && j < nc) {
-            int id = clusters[j];
-            sLo[t] = nodeLo[id];
-            sHi[t] = nodeHi[id];
-        }
-    }
-    __syncthreads();
-    const int i = b0 + threadIdx.x;
-    if (i >= nc) return;
-    const int si = threadIdx.x + kPlocRadius;
-    const float4 lo = sLo[si], hi = sHi[si];
+// A round is two launches without a host round trip in between or after it: the cluster
+// counts stay on the device (state.count[round parity]), the grids are fixed and walk
+// tiles of kPlocBlock clusters. (With separate nearest-neighbour, merge, select and scan
+// launches, a copy of the count and a synchronisation, a round took 45 us, of which the
+// kernels 18, and a mesh of 180,000 triangles 47 rounds: 2.1 ms. Now 18 rounds of 15 us
+// and 131 us in one block.)
+struct PlocState {
+    int count[2];  // clusters in the input of even / odd rounds
+    int nodes;     // inner nodes created
+    int error;     // the single-block rounds ran out of their bound
+};
+constexpr int kPlocHalo = 2 * kPlocRadius;
+// Up to this many clusters one block finishes the tree on its own (k_plocFinish).
+constexpr int kPlocFinish = 2048;
+constexpr int kPlocMaxRounds = 4096;
+constexpr int kPlocGroup = 6;        // rounds between reads of the count
+constexpr int kPlocGrid = 152 * 4;  // blocks of a round
+
+struct PlocTree {
+    float4* lo;
+    float4* hi;
+    int* left;    // [id - n]
+    int* right;
+    int* parent;
+    int* count;
+    int n;
+};
+
+// The cluster within kPlocRadius positions of position i whose common box with it is
+// smallest; boxes of positions [first, ...) in sLo / sHi; -1 for a single cluster.
+__device__ __forceinline__ int plocNearest(const float4* sLo, const float4* sHi, int first, int i, int nc) {
+    const float4 lo = sLo[i - first], hi = sHi[i - first];
     float best = __int_as_float(0x7f800000);
     int bestJ = -1;
     const int jLo = max(0, i - kPlocRadius), jHi = min(nc - 1, i + kPlocRadius);
     for (int j = jLo; j <= jHi; ++j) {
         if (j == i) continue;
-        const float4 l2 = sLo[j - b0 + kPlocRadius], h2 = sHi[j - b0 + kPlocRadius];
-        float a = halfArea(make_float4(fminf(lo.x, l2.x), fminf(lo.y, l2.y), fminf(lo.z, l2.z), 0.f),
-                           make_float4(fmaxf(hi.x, h2.x), fmaxf(hi.y, h2.y), fmaxf(hi.z, h2.z), 0.f));
+        const float4 l2 = sLo[j - first], h2 = sHi[j - first];
+        const float a = halfArea(make_float4(fminf(lo.x, l2.x), fminf(lo.y, l2.y), fminf(lo.z, l2.z), 0.f),
+                                 make_float4(fmaxf(hi.x, h2.x), fmaxf(hi.y, h2.y), fmaxf(hi.z, h2.z), 0.f));
         if (a < best || bestJ < 0) { best = a; bestJ = j; }  // ascending j: ties go to the lower index
     }
-    nn[i] = bestJ;
+    return bestJ;
 }
 
-__global__ void k_plocMerge(int* clusters, int nc, const int* __restrict__ nn, int n, float4* nodeLo, float4* nodeHi,
-                            int* left, int* right, int* parent, int* count, int* counter, int* keep) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= nc) return;
-    const int j = nn[i];
-    const bool mutual = j >= 0 && nn[j] == i;
-    if (mutual && i < j) {
-        const int a = clusters[i], b = clusters[j];
-        const int id = n + atomicAdd(counter, 1);
-        const float4 al = nodeLo[a], ah = nodeHi[a], bl = nodeLo[b], bh = nodeHi[b];
-        nodeLo[id] = make_float4(fminf(al.x, bl.x), fminf(al.y, bl.y), fminf(al.z, bl.z), 0.f);
-        nodeHi[id] = make_float4(fmaxf(ah.x, bh.x), fmaxf(ah.y, bh.y), fmaxf(ah.z, bh.z), 0.f);
-        left[id - n] = a;
-        right[id - n] = b;
-        parent[a] = id;
-        parent[b] = id;
-        parent[id] = -1;
-        count[id] = count[a] + count[b];
-        clusters[i] = id;  // only this thread touches slot i; slot j is dropped by its own thread
-        keep[i] = 1;
-    } else {
-        keep[i] = mutual ? 0 : 1;
+// A new inner node over clusters a (the lower position) and b.
+__device__ __forceinline__ void plocJoin(const PlocTree& t, int id, int a, int b, float4 lo, float4 hi) {
+    t.lo[id] = lo;
+    t.hi[id] = hi;
+    t.left[id - t.n] = a;
+    t.right[id - t.n] = b;
+    t.parent[a] = id;
+    t.parent[b] = id;
+    t.parent[id] = -1;
+    t.count[id] = t.count[a] + t.count[b];
+}
+
+// Nearest neighbours and merges of one round; a tile's surviving clusters, in order, at
+// out[tile * kPlocBlock ...] and their number in tileCount. The neighbours of the
+// kPlocRadius positions on either side of a tile are computed again here, so that a tile
+// needs no other's results.
+__global__ void __launch_bounds__(kPlocBlock) k_plocMerge(const int* __restrict__ clusters, PlocTree t, PlocState* state,
+                                                          int parity, int* out, int* tileCount) {
+    __shared__ float4 sLo[kPlocBlock + 2 * kPlocHalo], sHi[kPlocBlock + 2 * kPlocHalo];
+    __shared__ int sId[kPlocBlock + 2 * kPlocHalo];
+    __shared__ int sNN[kPlocBlock + kPlocHalo];
+    __shared__ int sWarp[kPlocBlock / 32], sWarpNew[kPlocBlock / 32], sBase;
+    const int nc = state->count[parity];
+    if (nc <= kPlocFinish) return;  // k_plocCompact passes the clusters on as they are
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (int tile = blockIdx.x; tile * kPlocBlock < nc; tile += gridDim.x) {
+        const int b0 = tile * kPlocBlock, first = b0 - kPlocHalo;
+        for (int k = threadIdx.x; k < kPlocBlock + 2 * kPlocHalo; k += kPlocBlock) {
+            const int j = first + k;
+            if (j >= 0 && j < nc) {
+                const int id = clusters[j];
+                sId[k] = id;
+                sLo[k] = t.lo[id];
+                sHi[k] = t.hi[id];
+            }
+        }
+        __syncthreads();
+        for (int k = threadIdx.x; k < kPlocBlock + kPlocHalo; k += kPlocBlock) {
+            const int i = b0 - kPlocRadius + k;
+            if (i >= 0 && i < nc) sNN[k] = plocNearest(sLo, sHi, first, i, nc);
+        }
+        __syncthreads();
+        const int i = b0 + threadIdx.x;
+        const bool valid = i < nc;
+        const int j = valid ? sNN[threadIdx.x + kPlocRadius] : -1;
+        const bool mutual = j >= 0 && sNN[j - b0 + kPlocRadius] == i;
+        const bool joins = mutual && i < j, keep = valid && (!mutual || joins);
+        const unsigned int mk = __ballot_sync(0xFFFFFFFFu, keep), mj = __ballot_sync(0xFFFFFFFFu, joins);
+        if (lane == 0) {
+            sWarp[warp] = __popc(mk);
+            sWarpNew[warp] = __popc(mj);
+        }
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            int kept = 0, made = 0;
+            for (int w = 0; w < kPlocBlock / 32; ++w) {
+                const int k = sWarp[w], m = sWarpNew[w];
+                sWarp[w] = kept;
+                sWarpNew[w] = made;
+                kept += k;
+                made += m;
+            }
+            tileCount[tile] = kept;
+            sBase = made ? atomicAdd(&state->nodes, made) : 0;
+        }
+        __syncthreads();
+        if (keep) {
+            int id = sId[i - first];
+            if (joins) {
+                const int a = id, b = sId[j - first];
+                const float4 al = sLo[i - first], ah = sHi[i - first], bl = sLo[j - first], bh = sHi[j - first];
+                id = t.n + sBase + sWarpNew[warp] + __popc(mj & ((1u << lane) - 1u));
+                plocJoin(t, id, a, b, make_float4(fminf(al.x, bl.x), fminf(al.y, bl.y), fminf(al.z, bl.z), 0.f),
+                         make_float4(fmaxf(ah.x, bh.x), fmaxf(ah.y, bh.y), fmaxf(ah.z, bh.z), 0.f));
+            }
+            out[b0 + sWarp[warp] + __popc(mk & ((1u << lane) - 1u))] = id;
+        }
+        __syncthreads();  // the shared arrays are reused by the next tile
+    }
+}
+
+// The tiles' survivors next to each other; the next round's count.
+__global__ void __launch_bounds__(kPlocBlock) k_plocCompact(const int* __restrict__ clusters, const int* __restrict__ in,
+                                                            const int* __restrict__ tileCount, PlocState* state, int parity,
+                                                            int* out) {
+    __shared__ int sSum[kPlocBlock / 32];
+    const int nc = state->count[parity];
+    const int tiles = (nc + kPlocBlock - 1) / kPlocBlock;
+    if (nc <= kPlocFinish) {
+        for (int i = blockIdx.x * kPlocBlock + threadIdx.x; i < nc; i += gridDim.x * kPlocBlock) out[i] = clusters[i];
+        if (blockIdx.x == 0 && threadIdx.x == 0) state->count[parity ^ 1] = nc;
+        return;
+    }
+    int offset = 0, summed = 0;  // survivors of the tiles before `summed`
+    for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+        int part = 0;
+        for (int k = summed + threadIdx.x; k < tile; k += kPlocBlock) part += tileCount[k];
+        for (int o = 16; o > 0; o >>= 1) part += __shfl_down_sync(0xFFFFFFFFu, part, o);
+        if ((threadIdx.x & 31) == 0) sSum[threadIdx.x >> 5] = part;
+        __syncthreads();
+        for (int w = 0; w < kPlocBlock / 32; ++w) offset += sSum[w];
+        summed = tile;
+        const int cnt = tileCount[tile];
+        if ((int)threadIdx.x < cnt) out[offset + threadIdx.x] = in[tile * kPlocBlock + threadIdx.x];
+        if (tile == tiles - 1 && threadIdx.x == 0) state->count[parity ^ 1] = offset + cnt;
+        __syncthreads();
+    }
+}
+
+// The rounds from kPlocFinish clusters to one, in one block, boxes and ids in shared memory.
+constexpr int kPlocFinishThreads = 1024;
+constexpr int kPlocFinishSmem = kPlocFinish * (2 * (int)sizeof(float4) + 2 * (int)sizeof(int));
+__global__ void __launch_bounds__(kPlocFinishThreads) k_plocFinish(const int* __restrict__ clusters, PlocTree t,
+                                                                   PlocState* state, int parity) {
+    extern __shared__ __align__(16) unsigned char plocRaw[];
+    float4* sLo = reinterpret_cast<float4*>(plocRaw);
+    float4* sHi = sLo + kPlocFinish;
+    int* sId = reinterpret_cast<int*>(sHi + kPlocFinish);
+    int* sNN = sId + kPlocFinish;
+    __shared__ int sWarp[kPlocFinishThreads / 32], sNew[kPlocFinishThreads / 32];
+    int nc = state->count[parity];
+    int nodes = state->nodes;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    if (nc > kPlocFinish) return;
+    for (int i = tid; i < nc; i += kPlocFinishThreads) {
+        const int id = clusters[i];
+        sId[i] = id;
+        sLo[i] = t.lo[id];
+        sHi[i] = t.hi[id];
+    }
+    __syncthreads();
+    for (int round = 0; nc > 1; ++round) {
+        if (round >= kPlocMaxRounds) {  // cannot happen: every round joins at least one pair
+            if (tid == 0) state->error = 1;
+            return;
+        }
+        for (int i = tid; i < nc; i += kPlocFinishThreads) sNN[i] = plocNearest(sLo, sHi, 0, i, nc);
+        __syncthreads();
+        constexpr int kPer = kPlocFinish / kPlocFinishThreads;
+        int id[kPer], rank[kPer];  // this thread's survivors and their new positions (-1: none)
+        float4 lo[kPer], hi[kPer];
+        int kept = 0;
+#pragma unroll
+        for (int h = 0; h < kPer; ++h) {
+            const int i = tid + h * kPlocFinishThreads;
+            const bool valid = i < nc;
+            const int j = valid ? sNN[i] : -1;
+            const bool mutual = j >= 0 && sNN[j] == i;
+            const bool joins = mutual && i < j, keep = valid && (!mutual || joins);
+            const unsigned int mk = __ballot_sync(0xFFFFFFFFu, keep), mj = __ballot_sync(0xFFFFFFFFu, joins);
+            if (lane == 0) {
+                sWarp[warp] = __popc(mk);
+                sNew[warp] = __popc(mj);
+            }
+            __syncthreads();
+            // every warp sums the counts of the warps before it and of all
+            int wk = sWarp[lane], wj = sNew[lane];
+            int pk = wk, pj = wj;
+            for (int o = 1; o < 32; o <<= 1) {
+                const int uk = __shfl_up_sync(0xFFFFFFFFu, pk, o), uj = __shfl_up_sync(0xFFFFFFFFu, pj, o);
+                if (lane >= o) { pk += uk; pj += uj; }
+            }
+            const int allK = __shfl_sync(0xFFFFFFFFu, pk, 31), allJ = __shfl_sync(0xFFFFFFFFu, pj, 31);
+            const int beforeK = __shfl_sync(0xFFFFFFFFu, pk - wk, warp), beforeJ = __shfl_sync(0xFFFFFFFFu, pj - wj, warp);
+            rank[h] = keep ? kept + beforeK + __popc(mk & ((1u << lane) - 1u)) : -1;
+            if (keep) {
+                id[h] = sId[i];
+                lo[h] = sLo[i];
+                hi[h] = sHi[i];
+                if (joins) {
+                    const int a = id[h], b = sId[j];
+                    const float4 bl = sLo[j], bh = sHi[j];
+                    lo[h] = make_float4(fminf(lo[h].x, bl.x), fminf(lo[h].y, bl.y), fminf(lo[h].z, bl.z), 0.f);
+                    hi[h] = make_float4(fmaxf(hi[h].x, bh.x), fmaxf(hi[h].y, bh.y), fmaxf(hi[h].z, bh.z), 0.f);
+                    id[h] = t.n + nodes + beforeJ + __popc(mj & ((1u << lane) - 1u));
+                    plocJoin(t, id[h], a, b, lo[h], hi[h]);
+                }
+            }
+            kept += allK;
+            nodes += allJ;
+            __syncthreads();
+        }
+#pragma unroll
+        for (int h = 0; h < kPer; ++h)
+            if (rank[h] >= 0) {
+                sId[rank[h]] = id[h];
+                sLo[rank[h]] = lo[h];
+                sHi[rank[h]] = hi[h];
+            }
+        nc = kept;
+        __syncthreads();  // also: this round's node counts are visible to the next's joins
     }
 }
 
@@ -512,7 +695,8 @@ __global__ void k_wideRound(WideBuild wb, const WideItem* in, int nIn, WideItem*
 
 struct DeviceScratch {
     void* p = nullptr;
-    ~DeviceScratch() { if (p) cudaFree(p); }
+    cudaStream_t stream = nullptr;
+    ~DeviceScratch() { if (p) cudaFreeAsync(p, stream); }
 };
 
 }  // namespace
@@ -522,7 +706,6 @@ cudaError_t buildBlas(const BlasBuildInput& in, BlasBuildOutput* out, cudaStream
     if (n <= 0) return cudaErrorInvalidValue;
     if (n >= (1 << 24)) return cudaErrorInvalidValue;  // node indices travel in 24 bits on the traversal stack
     out->nodes = nullptr;
-    out->nodes2 = nullptr;
     out->nWide = 0;
     const bool wide = in.layout == kLayoutWide;
     out->wide = wide ? 1 : 0;
@@ -534,8 +717,6 @@ cudaError_t buildBlas(const BlasBuildInput& in, BlasBuildOutput* out, cudaStream
     size_t sortTemp = 0;
     cub::DeviceRadixSort::SortPairs(nullptr, sortTemp, (unsigned int*)nullptr, (unsigned int*)nullptr,
                                     (unsigned int*)nullptr, (unsigned int*)nullptr, n, 0, 30, stream);
-    size_t selTemp = 0;
-    cub::DeviceSelect::Flagged(nullptr, selTemp, (int*)nullptr, (int*)nullptr, (int*)nullptr, (int*)nullptr, n, stream);
     size_t off = 0;
     auto take = [&](size_t bytes) { size_t o = off; off += (bytes + 255) & ~(size_t)255; return o; };
     const size_t oTriLo = take(sizeof(float4) * n), oTriHi = take(sizeof(float4) * n), oCent = take(sizeof(float4) * n);
@@ -548,16 +729,20 @@ cudaError_t buildBlas(const BlasBuildInput& in, BlasBuildOutput* out, cudaStream
     const size_t oNLo = take(sizeof(float4) * nNodes), oNHi = take(sizeof(float4) * nNodes);
     const size_t oSort = take(sortTemp);
     const size_t oClB = take(4 * (size_t)n), oNN = take(4 * (size_t)n), oKeep = take(4 * (size_t)n);
-    const size_t oCount = take(4 * nNodes), oStart = take(4 * nNodes), oCounters = take(16), oSel = take(selTemp);
+    const size_t oCount = take(4 * nNodes), oStart = take(4 * nNodes), oCounters = take(16);
     // unified (PLOC-numbered) tree for the wide conversion: LBVH writes its own copy
-    const size_t oULeft = take(4 * (size_t)n), oURight = take(4 * (size_t)n);
-    const size_t oULo = take(sizeof(float4) * nNodes), oUHi = take(sizeof(float4) * nNodes);
-    const size_t oTrisBin = take(sizeof(TriV) * n);
-    const size_t oItemsA = take(sizeof(WideItem) * n), oItemsB = take(sizeof(WideItem) * n);
-    const size_t oWide = take(sizeof(WNode) * n);  // upper bound: a wide node has >= 2 children
+    const size_t nU = in.builder == kBuilderPloc ? 0 : (size_t)n, nW = wide ? (size_t)n : 0;
+    const size_t oULeft = take(4 * nU), oURight = take(4 * nU);
+    const size_t oULo = take(2 * sizeof(float4) * nU), oUHi = take(2 * sizeof(float4) * nU);
+    const size_t oTrisBin = take(sizeof(TriV) * nW);
+    const size_t oItemsA = take(sizeof(WideItem) * nW), oItemsB = take(sizeof(WideItem) * nW);
+    const size_t oWide = take(sizeof(WNode) * nW);  // upper bound: a wide node has >= 2 children
     const size_t oWCounters = take(16);
-    DeviceScratch scratch;
-    if ((e = cudaMalloc(&scratch.p, off)) != cudaSuccess) return e;
+    DeviceScratch scratch{nullptr, stream};
+    if ((e = cudaMallocFromPoolAsync(&scratch.p, off, in.pool, stream)) != cudaSuccess) {
+        scratch.p = nullptr;
+        return e;
+    }
     char* base = (char*)scratch.p;
     float4* triLo = (float4*)(base + oTriLo);
     float4* triHi = (float4*)(base + oTriHi);
@@ -572,17 +757,8 @@ cudaError_t buildBlas(const BlasBuildInput& in, BlasBuildOutput* out, cudaStream
     int* count = (int*)(base + oCount);
     int* start = (int*)(base + oStart);
     TriV* trisBin = wide ? (TriV*)(base + oTrisBin) : out->tris;  // the binary layout gathers in place
-    Node2* nodes2 = nullptr;
-    if (!wide && n >= 2) {
-        if ((e = cudaMalloc((void**)&nodes2, sizeof(Node2) * (size_t)(n - 1))) != cudaSuccess) return e;
-        out->nodes2 = nodes2;  // the caller frees it, also on failure
-    }
-    int* hostCount = nullptr;
-    if ((e = cudaMallocHost((void**)&hostCount, 16)) != cudaSuccess) return e;
-    struct HostFree {
-        int* p;
-        ~HostFree() { cudaFreeHost(p); }
-    } hostFree{hostCount};
+    Node2* nodes2 = out->nodes2;
+    int hostCount[4] = {0, 0, 0, 0}, plocFailed = 0;
 
     unsigned int initBounds[12];
     for (int k = 0; k < 12; ++k) initBounds[k] = (k % 6) < 3 ? 0xFFFFFFFFu : 0u;
@@ -600,26 +776,32 @@ cudaError_t buildBlas(const BlasBuildInput& in, BlasBuildOutput* out, cudaStream
     if (in.builder == kBuilderPloc) {
         int* clA = (int*)(base + oKeys);  // the unsorted keys are free once sorted
         int* clB = (int*)(base + oClB);
-        int* nn = (int*)(base + oNN);
-        int* keep = (int*)(base + oKeep);
-        int* counters = (int*)(base + oCounters);  // [0] nodes created, [1] clusters selected
-        if ((e = cudaMemsetAsync(counters, 0, 16, stream)) != cudaSuccess) return e;
+        int* survivors = (int*)(base + oNN);
+        int* tileCount = (int*)(base + oKeep);
+        PlocState* state = (PlocState*)(base + oCounters);
+        const PlocTree tree{nodeLo, nodeHi, left, right, parent, count, n};
+        const PlocState init{{n, n}, 0, 0};
+        if ((e = cudaMemcpyAsync(state, &init, sizeof(init), cudaMemcpyHostToDevice, stream)) != cudaSuccess) return e;
         k_plocInit<<<G, B, 0, stream>>>(vals2, n, triLo, triHi, nodeLo, nodeHi, clA, count, parent);
-        int nc = n;
-        for (int round = 0; nc > 1; ++round) {
-            if (round > 4 * 1024) return cudaErrorUnknown;  // cannot happen: every round merges at least one pair
-            const int Gc = (nc + kPlocBlock - 1) / kPlocBlock;
-            k_plocNearest<<<Gc, kPlocBlock, 0, stream>>>(clA, nc, nodeLo, nodeHi, nn);
-            k_plocMerge<<<Gc, kPlocBlock, 0, stream>>>(clA, nc, nn, n, nodeLo, nodeHi, left, right, parent, count,
-                                                        counters, keep);
-            size_t tb = selTemp;
-            if ((e = cub::DeviceSelect::Flagged(base + oSel, tb, clA, keep, clB, counters + 1, nc, stream)) != cudaSuccess)
-                return e;
-            if ((e = cudaMemcpyAsync(hostCount, counters + 1, 4, cudaMemcpyDeviceToHost, stream)) != cudaSuccess) return e;
+        if ((e = cudaFuncSetAttribute(k_plocFinish, cudaFuncAttributeMaxDynamicSharedMemorySize, kPlocFinishSmem)) != cudaSuccess)
+            return e;
+        // rounds in groups until few clusters are left, then one block makes the rest
+        const int grid = std::min((n + kPlocBlock - 1) / kPlocBlock, kPlocGrid);
+        int parity = 0, rounds = 0;
+        for (int nc = n; nc > kPlocFinish; rounds += kPlocGroup) {
+            if (rounds > kPlocMaxRounds) return cudaErrorUnknown;  // cannot happen: every round merges at least one pair
+            for (int k = 0; k < kPlocGroup; ++k) {
+                k_plocMerge<<<grid, kPlocBlock, 0, stream>>>(clA, tree, state, parity, survivors, tileCount);
+                k_plocCompact<<<grid, kPlocBlock, 0, stream>>>(clA, survivors, tileCount, state, parity, clB);
+                std::swap(clA, clB);
+                parity ^= 1;
+            }
+            if ((e = cudaMemcpyAsync(hostCount, &state->count[parity], 4, cudaMemcpyDeviceToHost, stream)) != cudaSuccess) return e;
             if ((e = cudaStreamSynchronize(stream)) != cudaSuccess) return e;
             nc = *hostCount;
-            std::swap(clA, clB);
         }
+        k_plocFinish<<<1, kPlocFinishThreads, kPlocFinishSmem, stream>>>(clA, tree, state, parity);
+        if ((e = cudaMemcpyAsync(&plocFailed, &state->error, 4, cudaMemcpyDeviceToHost, stream)) != cudaSuccess) return e;
         const int nAll = 2 * n - 1;
         k_dfsOffset<<<(nAll + B - 1) / B, B, 0, stream>>>(nAll, n, parent, left, right, count, start);
         if (!wide && n >= 2)
@@ -673,9 +855,9 @@ cudaError_t buildBlas(const BlasBuildInput& in, BlasBuildOutput* out, cudaStream
         const int nWide = hostCount[0];
         if (hostCount[1] != n) return cudaErrorUnknown;  // every triangle lands in exactly one leaf child
         WNode* nodes = nullptr;
-        if ((e = cudaMalloc((void**)&nodes, sizeof(WNode) * nWide)) != cudaSuccess) return e;
+        if ((e = cudaMallocFromPoolAsync((void**)&nodes, sizeof(WNode) * nWide, in.pool, stream)) != cudaSuccess) return e;
         if ((e = cudaMemcpyAsync(nodes, base + oWide, sizeof(WNode) * nWide, cudaMemcpyDeviceToDevice, stream)) != cudaSuccess) {
-            cudaFree(nodes);
+            cudaFreeAsync(nodes, stream);
             return e;
         }
         out->nodes = nodes;
@@ -685,6 +867,7 @@ cudaError_t buildBlas(const BlasBuildInput& in, BlasBuildOutput* out, cudaStream
     if ((e = cudaMemcpyAsync(hb, bounds, sizeof(hb), cudaMemcpyDeviceToHost, stream)) != cudaSuccess) return e;
     if ((e = cudaStreamSynchronize(stream)) != cudaSuccess) return e;
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    if (plocFailed) return cudaErrorUnknown;
     for (int k = 0; k < 3; ++k) {
         out->boundsLo[k] = orderedFloat(hb[6 + k]);
         out->boundsHi[k] = orderedFloat(hb[9 + k]);
@@ -693,6 +876,28 @@ cudaError_t buildBlas(const BlasBuildInput& in, BlasBuildOutput* out, cudaStream
     out->rootIsLeaf = n <= rootMax ? 1 : 0;
     out->rootLeaf = leafEncode(0, n <= rootMax ? n : 1);
     return cudaSuccess;
+}
+
+namespace {
+__global__ void k_expandVec3(const float* __restrict__ src, int stride, size_t n, float4* dst) {
+    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
+        const float* p = src + (size_t)stride * i;
+        dst[i] = make_float4(p[0], p[1], p[2], 0.0f);
+    }
+}
+__global__ void k_expandUv(const float* __restrict__ src, int stride, size_t n, float2* dst) {
+    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
+        const float* p = src + (size_t)stride * i;
+        dst[i] = make_float2(p[0], p[1]);
+    }
+}
+int rowGrid(size_t n) { return (int)std::min<size_t>((n + 255) / 256, 152 * 8); }
+}  // namespace
+void expandVec3(const float* src, int stride, size_t n, float4* dst, cudaStream_t s) {
+    k_expandVec3<<<rowGrid(n), 256, 0, s>>>(src, stride, n, dst);
+}
+void expandUv(const float* src, int stride, size_t n, float2* dst, cudaStream_t s) {
+    k_expandUv<<<rowGrid(n), 256, 0, s>>>(src, stride, n, dst);
 }
 
 namespace {

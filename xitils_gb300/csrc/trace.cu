@@ -857,27 +857,36 @@ __global__ void __launch_bounds__(kTraceBlock) k_shadow_batch(BatchView b, Shado
 }
 
 // ---- ray queries (xgb_scene_intersect / xgb_scene_occluded) -------------------
-__global__ void __launch_bounds__(kTraceBlock) k_query(SceneDev sc, const float4* o, const float4* d, int n, int any,
-                                                       float4* hits, int* occluded, unsigned int* errors) {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        float4 oo = o[i], dd = d[i];
-        TraceHit hit;
-        WorkCount wc;
-        if (any) {
-            occluded[i] = traceScene<true>(sc, V3(oo.x, oo.y, oo.z), V3(dd.x, dd.y, dd.z), oo.w, hit, errors, wc) ? 1 : 0;
-        } else {
-            traceScene<false>(sc, V3(oo.x, oo.y, oo.z), V3(dd.x, dd.y, dd.z), oo.w, hit, errors, wc);
-            hits[2 * i] = make_float4(hit.t, __int_as_float(hit.inst), __int_as_float(hit.prim), 0.0f);
-            hits[2 * i + 1] = make_float4(hit.b0, hit.b1, 0.0f, 0.0f);
+// A warp takes 32 rays at a time; traceScene is the instance order of queries.
+template <bool ANY>
+__global__ void __launch_bounds__(kTraceBlock) k_query(SceneDev sc, const float* __restrict__ rays, int n, float* hits,
+                                                       int* occluded, QueryState* state) {
+    const int lane = threadIdx.x & 31;
+    for (;;) {
+        unsigned int base = 0;
+        if (lane == 0) base = atomicAdd(&state->head, 32u);
+        base = __shfl_sync(0xFFFFFFFFu, base, 0);
+        if (base >= (unsigned int)n) break;
+        const unsigned int i = base + lane;
+        if (i < (unsigned int)n) {
+            const float* r = rays + 7 * (size_t)i;
+            TraceHit hit;
+            hit.b0 = hit.b1 = 0.0f;
+            WorkCount wc;
+            const bool found = traceScene<ANY>(sc, V3(r[0], r[1], r[2]), V3(r[3], r[4], r[5]), r[6], hit, &state->errors, wc);
+            if (ANY) {
+                occluded[i] = found ? 1 : 0;
+            } else {
+                float* h = hits + 5 * (size_t)i;
+                h[0] = hit.t;
+                h[1] = (float)hit.inst;
+                h[2] = (float)hit.prim;
+                h[3] = hit.b0;
+                h[4] = hit.b1;
+            }
         }
     }
 }
-
-void launchQuery(const SceneDev& sc, const float4* o, const float4* d, int n, int any, float4* hits, int* occluded,
-                 unsigned int* errors, int grid, cudaStream_t s) {
-    k_query<<<grid, kTraceBlock, 0, s>>>(sc, o, d, n, any, hits, occluded, errors);
-}
-
 
 // Persistent grids: SMs x resident blocks of the kernel actually launched
 // (looked up once per kernel; all kernels here use kTraceBlock threads).
@@ -1017,6 +1026,12 @@ void launchShadowBatch(const BatchView& b, ShadowQueue sq, PathQueue out, Ctrl* 
     case kBatchFlat: XGB_LAUNCH((k_trace_flat2<true, false, BatchScenes>))(sc, PathQueue{}, HitQueue{}, sq, out, ctrl); break;
     default: XGB_LAUNCH(k_shadow_batch)(b, sq, out, ctrl);
     }
+}
+
+void launchQuery(const SceneDev& sc, const float* rays, int n, int any, float* hits, int* occluded, QueryState* state,
+                 int numSMs, cudaStream_t s) {
+    if (any) XGB_LAUNCH((k_query<true>))(sc, rays, n, hits, occluded, state);
+    else XGB_LAUNCH((k_query<false>))(sc, rays, n, hits, occluded, state);
 }
 #undef XGB_LAUNCH
 

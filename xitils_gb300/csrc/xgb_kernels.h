@@ -19,11 +19,12 @@ struct BlasBuildInput {
     int nTris;
     int builder;        // kBuilderPloc or kBuilderLbvh
     int layout;         // kLayoutBinary or kLayoutWide
+    cudaMemPool_t pool; // scratch memory and the wide nodes come from it
 };
 struct BlasBuildOutput {
-    WNode* nodes;       // wide layout: device, allocated by buildBlas (cudaMalloc, nWide entries; the caller frees it)
+    WNode* nodes;       // wide layout: device, allocated by buildBlas (nWide entries; the caller frees it)
     int nWide;
-    Node2* nodes2;      // binary layout: device, allocated by buildBlas (nTris - 1 entries; the caller frees it)
+    Node2* nodes2;      // binary layout: device, nTris - 1 entries, allocated by the caller
     int wide;
     TriV* tris;         // device, nTris entries (leaf order), allocated by the caller
     float4* gnrm;       // device, nTris entries (original order)
@@ -36,6 +37,10 @@ struct BlasBuildOutput {
 // converted into an 8-wide compressed BVH, on `stream`, and synchronises it.
 // Returns a CUDA error code (cudaSuccess on success).
 cudaError_t buildBlas(const BlasBuildInput& in, BlasBuildOutput* out, cudaStream_t stream);
+
+// Rows of `stride` floats (3 or 4) -> float4 with w = 0; of 2 or 4 floats -> float2.
+void expandVec3(const float* src, int stride, size_t n, float4* dst, cudaStream_t s);
+void expandUv(const float* src, int stride, size_t n, float2* dst, cudaStream_t s);
 
 // An instance's share of a world BVH (WorldDev): the mesh's n - 1 nodes renumbered to start
 // at nodeBase, its n triangles at triBase with the instance's number.
@@ -198,9 +203,13 @@ void launchShadow(const SceneDev& sc, const RenderParams& rp, ShadowQueue sq, Pa
                   cudaStream_t s);
 // Film plane (float4 or double4 per pixel) -> packed float RGB, strideFloats 3 or 4 (image.cu).
 void launchPackFilm(const void* film, int fp64, size_t n, int strideFloats, float* out, int grid, cudaStream_t s);
-// Ray queries on a built scene: rays o (xyz, w = tMax) and d; closest hits as 2 float4
-// per ray (t, bits(instance), bits(triangle), -; b0, b1, -, -) or any-hit flags.
-void launchQuery(const SceneDev& sc, const float4* o, const float4* d, int n, int any, float4* hits, int* occluded,
-                 unsigned int* errors, int grid, cudaStream_t s);
+// Ray queries on a built scene: rays of 7 floats (o, d, tMax); closest hits as 5 floats per ray
+// (t, instance, triangle, b0, b1; -1 for none) or any-hit flags.
+struct QueryState {
+    unsigned int head;    // rays handed out
+    unsigned int errors;
+};
+void launchQuery(const SceneDev& sc, const float* rays, int n, int any, float* hits, int* occluded, QueryState* state,
+                 int numSMs, cudaStream_t s);
 
 }  // namespace xgb
