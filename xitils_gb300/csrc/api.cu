@@ -1637,25 +1637,27 @@ static xgb_status sceneQuery(xgb_scene* s, int n, const float* rays, int any, fl
     // two thirds of a call of 300,000 rays)
     char* dev = nullptr;
     const size_t rayBytes = (28 * (size_t)n + 255) & ~(size_t)255, outBytes = ((any ? 4 : 20) * (size_t)n + 255) & ~(size_t)255;
-    if (poolAlloc(ctx, (void**)&dev, rayBytes + outBytes + 256, st) != cudaSuccess)
+    if (poolAlloc(ctx, (void**)&dev, rayBytes + outBytes + sizeof(Ctrl), st) != cudaSuccess)
         return fail(ctx, XGB_OOM, "xgb_scene_intersect: out of device memory");
     char* dOut = dev + rayBytes;
-    QueryState* dState = (QueryState*)(dev + rayBytes + outBytes);
+    Ctrl* dCtrl = (Ctrl*)(dev + rayBytes + outBytes);
+    Ctrl ctrl;
+    std::memset(&ctrl, 0, sizeof(ctrl));
+    ctrl.nActive = ctrl.nShadow = (unsigned int)n;
     cudaError_t e = cudaMemcpyAsync(dev, rays, 28 * (size_t)n, cudaMemcpyHostToDevice, st);
-    if (e == cudaSuccess) e = cudaMemsetAsync(dState, 0, sizeof(QueryState), st);
-    QueryState state{};
+    if (e == cudaSuccess) e = cudaMemcpyAsync(dCtrl, &ctrl, sizeof(Ctrl), cudaMemcpyHostToDevice, st);
     if (e == cudaSuccess) {
-        launchQuery(s->sd, (const float*)dev, n, any, (float*)dOut, (int*)dOut, dState, ctx->numSMs, st);
+        launchQuery(s->sd, (const float*)dev, n, any, (float*)dOut, (int*)dOut, dCtrl, ctx->numSMs, st);
         e = cudaGetLastError();
     }
     if (e == cudaSuccess) e = any ? cudaMemcpyAsync(occ, dOut, 4 * (size_t)n, cudaMemcpyDeviceToHost, st)
                                   : cudaMemcpyAsync(hits, dOut, 20 * (size_t)n, cudaMemcpyDeviceToHost, st);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(&state, dState, sizeof(state), cudaMemcpyDeviceToHost, st);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(&ctrl, dCtrl, sizeof(Ctrl), cudaMemcpyDeviceToHost, st);
     cudaFreeAsync(dev, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) return cudaFail(ctx, e, "xgb_scene_intersect");
-    if (state.errors & ERR_STACK) return fail(ctx, XGB_QUEUE_OVERFLOW, "xgb_scene_intersect: traversal stack overflow");
-    if (state.errors & ERR_LOOP) return fail(ctx, XGB_DEVICE_TIMEOUT, "xgb_scene_intersect: traversal iteration bound exceeded");
+    if (ctrl.errors & ERR_STACK) return fail(ctx, XGB_QUEUE_OVERFLOW, "xgb_scene_intersect: traversal stack overflow");
+    if (ctrl.errors & ERR_LOOP) return fail(ctx, XGB_DEVICE_TIMEOUT, "xgb_scene_intersect: traversal iteration bound exceeded");
     return XGB_OK;
 }
 
@@ -1757,14 +1759,14 @@ float initUniform(uint64_t& state) {
 
 extern "C" {
 
-// Reads and clears the error word of the tensor-memory row inference (after the
-// stream has been synchronised); XGB_DEVICE_TIMEOUT when one of its waits gave up.
-static xgb_status guideRowErrors(xgb_guide* gd, const char* what) {
-    unsigned int e = 0;
-    unsigned int* word = reinterpret_cast<unsigned int*>(gd->g.scratch.scalars + 2);
-    if (cudaMemcpy(&e, word, 4, cudaMemcpyDeviceToHost) != cudaSuccess) return fail(gd->ctx, XGB_CUDA_ERROR, what);
+// The error word of the tensor-memory row inference, copied with the results: cleared and
+// XGB_DEVICE_TIMEOUT when one of its waits gave up.
+static unsigned int* guideRowErrorWord(xgb_guide* gd) {
+    return reinterpret_cast<unsigned int*>(gd->g.scratch.scalars + 2);
+}
+static xgb_status guideRowErrors(xgb_guide* gd, unsigned int e, const char* what) {
     if (e & ERR_WAIT) {
-        cudaMemset(word, 0, 4);
+        cudaMemset(guideRowErrorWord(gd), 0, 4);
         return fail(gd->ctx, XGB_DEVICE_TIMEOUT, std::string(what) + ": network inference wait timed out");
     }
     return XGB_OK;
@@ -1910,28 +1912,32 @@ xgb_status xgb_guide_infer(xgb_guide* gd, int n, const float* pos, const float* 
     if (!gd->hasBounds) return fail(gd->ctx, XGB_INVALID_ARG, "xgb_guide_infer: call xgb_guide_set_bounds first");
     xgb_ctx* ctx = gd->ctx;
     cudaStream_t st = ctx->stream;
-    const int R = gd->g.maxRows;
+    if (n == 0) return XGB_OK;
+    // the rows of the caller's array come straight from the device (a cudaMalloc and cudaFree
+    // per call, padded rows and a host loop that dropped the padding took 0.4 of 0.68 ms for
+    // 20,000 points)
+    const int R = std::min(gd->g.maxRows, (n + 63) / 64 * 64);
     float* dIn = nullptr;
-    XGB_CUDA(ctx, cudaMalloc((void**)&dIn, 4 * 9 * (size_t)R));
-    std::vector<float> y((size_t)R * kGuideOutPad);
-    for (int b = 0; b < n; b += R) {
+    XGB_CUDA(ctx, poolAlloc(ctx, (void**)&dIn, 4 * 9 * (size_t)R, st));
+    unsigned int errors = 0;
+    cudaError_t e = cudaSuccess;
+    for (int b = 0; b < n && e == cudaSuccess; b += R) {
         int cnt = std::min(R, n - b);
         int rows = ((cnt + 63) / 64) * 64;
         cudaMemcpyAsync(dIn, pos + 3 * (size_t)b, 12 * (size_t)cnt, cudaMemcpyHostToDevice, st);
-        cudaMemcpyAsync(dIn + 3 * R, nrm + 3 * (size_t)b, 12 * (size_t)cnt, cudaMemcpyHostToDevice, st);
-        cudaMemcpyAsync(dIn + 6 * R, wo + 3 * (size_t)b, 12 * (size_t)cnt, cudaMemcpyHostToDevice, st);
-        guideFeaturesFromPoints(dIn, dIn + 3 * R, dIn + 6 * R, cnt, rows, gd->bounds, gd->g.scratch.X0, st);
-        guideInferRows(gd->g, gd->g.scratch.X0, rows, gd->g.scratch.Y, st);
-        cudaMemcpyAsync(y.data(), gd->g.scratch.Y, 4 * (size_t)rows * kGuideOutPad, cudaMemcpyDeviceToHost, st);
-        if (cudaStreamSynchronize(st) != cudaSuccess) {
-            cudaFree(dIn);
-            return fail(ctx, XGB_CUDA_ERROR, "xgb_guide_infer failed");
-        }
-        for (int r = 0; r < cnt; ++r)
-            std::memcpy(out + (size_t)(b + r) * kGuideOut, y.data() + (size_t)r * kGuideOutPad, 4 * kGuideOut);
+        cudaMemcpyAsync(dIn + 3 * (size_t)R, nrm + 3 * (size_t)b, 12 * (size_t)cnt, cudaMemcpyHostToDevice, st);
+        cudaMemcpyAsync(dIn + 6 * (size_t)R, wo + 3 * (size_t)b, 12 * (size_t)cnt, cudaMemcpyHostToDevice, st);
+        guideFeaturesFromPoints(dIn, dIn + 3 * (size_t)R, dIn + 6 * (size_t)R, cnt, rows, gd->bounds, gd->g.scratch.X0, st);
+        guideInferRows(gd->g, gd->g.scratch.X0, rows, gd->g.scratch.Y, kGuideOut, st);
+        cudaMemcpyAsync(out + (size_t)b * kGuideOut, gd->g.scratch.Y, 4 * (size_t)cnt * kGuideOut, cudaMemcpyDeviceToHost, st);
+        unsigned int word = 0;
+        cudaMemcpyAsync(&word, guideRowErrorWord(gd), 4, cudaMemcpyDeviceToHost, st);
+        e = cudaStreamSynchronize(st);
+        errors |= word;
     }
-    cudaFree(dIn);
-    return guideRowErrors(gd, "xgb_guide_infer");
+    cudaFreeAsync(dIn, st);
+    if (e != cudaSuccess) return fail(ctx, XGB_CUDA_ERROR, "xgb_guide_infer failed");
+    return guideRowErrors(gd, errors, "xgb_guide_infer");
 }
 
 xgb_status xgb_guide_sample(xgb_guide* gd, int n, const float* pos, const float* nrm, const float* wo, uint32_t seed,
@@ -1942,22 +1948,24 @@ xgb_status xgb_guide_sample(xgb_guide* gd, int n, const float* pos, const float*
     if (n == 0) return XGB_OK;
     xgb_ctx* ctx = gd->ctx;
     cudaStream_t st = ctx->stream;
-    const int R = gd->g.maxRows;
+    const int R = (n + 63) / 64 * 64;
     float* dIn = nullptr;
-    XGB_CUDA(ctx, cudaMalloc((void**)&dIn, 4 * 13 * (size_t)R));
+    XGB_CUDA(ctx, poolAlloc(ctx, (void**)&dIn, 4 * 13 * (size_t)R, st));
     int rows = ((n + 63) / 64) * 64;
     cudaMemcpyAsync(dIn, pos, 12 * (size_t)n, cudaMemcpyHostToDevice, st);
     cudaMemcpyAsync(dIn + 3 * R, nrm, 12 * (size_t)n, cudaMemcpyHostToDevice, st);
     cudaMemcpyAsync(dIn + 6 * R, wo, 12 * (size_t)n, cudaMemcpyHostToDevice, st);
     guideFeaturesFromPoints(dIn, dIn + 3 * R, dIn + 6 * R, n, rows, gd->bounds, gd->g.scratch.X0, st);
-    guideInferRows(gd->g, gd->g.scratch.X0, rows, gd->g.scratch.Y, st);
+    guideInferRows(gd->g, gd->g.scratch.X0, rows, gd->g.scratch.Y, kGuideOutPad, st);
     guideSampleRows(gd->g.scratch.Y, n, seed, dIn + 9 * R, dIn + 12 * R, st);
     cudaMemcpyAsync(dirs, dIn + 9 * R, 12 * (size_t)n, cudaMemcpyDeviceToHost, st);
     cudaMemcpyAsync(pdf, dIn + 12 * R, 4 * (size_t)n, cudaMemcpyDeviceToHost, st);
+    unsigned int errors = 0;
+    cudaMemcpyAsync(&errors, guideRowErrorWord(gd), 4, cudaMemcpyDeviceToHost, st);
+    cudaFreeAsync(dIn, st);
     cudaError_t e = cudaStreamSynchronize(st);
-    cudaFree(dIn);
     if (e != cudaSuccess) return cudaFail(ctx, e, "xgb_guide_sample");
-    return guideRowErrors(gd, "xgb_guide_sample");
+    return guideRowErrors(gd, errors, "xgb_guide_sample");
 }
 
 xgb_status xgb_guide_train_batch(xgb_guide* gd, int n, const float* pos, const float* nrm, const float* wo,

@@ -46,9 +46,9 @@ struct GuideDevice {
 __device__ void guideStoreBf16(const GuideWeights& w, int i, float p);
 
 void guideRefresh(const GuideDevice& g, cudaStream_t s);
-// Network outputs Y [rowsPad][48] of feature rows X0 [rowsPad][64] (tcgen05 kernel of
-// guide_tc.cu); a timed-out wait sets ERR_WAIT in the word at g.scratch.scalars + 2.
-void guideInferRows(const GuideDevice& g, const __nv_bfloat16* X0, int rowsPad, float* Y, cudaStream_t s);
+// Network outputs Y [rowsPad][ldY] (ldY 40 or 48 columns) of feature rows X0 [rowsPad][64]
+// (tcgen05 kernel of guide_tc.cu); a timed-out wait sets ERR_WAIT in the word at g.scratch.scalars + 2.
+void guideInferRows(const GuideDevice& g, const __nv_bfloat16* X0, int rowsPad, float* Y, int ldY, cudaStream_t s);
 // Bytes of GuideScratch::partial.
 size_t guidePartialBytes();
 // One Adam step (lr > 0) or gradients only (lr == 0) on records [0, n) (at most maxRows).

@@ -272,9 +272,9 @@ __device__ __forceinline__ void tcAbort(TcSmem& S, int group, uint32_t parity, u
 }
 
 // Rows of feature vectors (xgb_guide_infer / xgb_guide_sample): X0 [rows][64]
-// BF16, Y [rows][48] FP32.
+// BF16, the first ldY (48, or the 40 outputs) columns as rows of Y, FP32.
 __global__ void __launch_bounds__(kTcThreads, kTcCtasPerSm) k_inferRowsTc(const __nv_bfloat16* X0, int rows, GuideWeights w,
-                                                            float* Y, unsigned int* errors, int waitLimit) {
+                                                            float* Y, int ldY, unsigned int* errors, int waitLimit) {
     extern __shared__ unsigned char tcRaw[];
     TcSmem& S = *reinterpret_cast<TcSmem*>(tcRaw);
     tcSetup(S, w);
@@ -294,9 +294,12 @@ __global__ void __launch_bounds__(kTcThreads, kTcCtasPerSm) k_inferRowsTc(const 
             tcAbort(S, group, parity, errors);
             break;
         }
-        if (i < rows)
+        if (i < rows) {
+            float4* o = reinterpret_cast<float4*>(Y + (size_t)i * ldY);  // ldY is a multiple of 4
 #pragma unroll
-            for (int k = 0; k < kGuideOutPad; ++k) Y[(size_t)i * kGuideOutPad + k] = y[k];
+            for (int k = 0; k < kGuideOutPad / 4; ++k)
+                if (4 * k < ldY) o[k] = make_float4(y[4 * k], y[4 * k + 1], y[4 * k + 2], y[4 * k + 3]);
+        }
     }
     tcTeardown(S);
 }
@@ -370,12 +373,12 @@ cudaError_t guideTcPrepare() {
     return e;
 }
 
-void guideInferRows(const GuideDevice& g, const __nv_bfloat16* X0, int rowsPad, float* Y, cudaStream_t s) {
+void guideInferRows(const GuideDevice& g, const __nv_bfloat16* X0, int rowsPad, float* Y, int ldY, cudaStream_t s) {
     const int groups = (rowsPad + kTcRows - 1) / kTcRows;
     int grid = (groups + kTcGroups - 1) / kTcGroups;
     if (gLaunchCtas > 0 && grid > gLaunchCtas) grid = gLaunchCtas;
     k_inferRowsTc<<<grid > 0 ? grid : 1, kTcThreads, sizeof(TcSmem), s>>>(
-        X0, rowsPad, g.w, Y, reinterpret_cast<unsigned int*>(g.scratch.scalars + 2), g.waitLimit);
+        X0, rowsPad, g.w, Y, ldY, reinterpret_cast<unsigned int*>(g.scratch.scalars + 2), g.waitLimit);
 }
 
 void guideInferPaths(const SceneDev& sc, const GuideDevice& g, GuideBounds gb, PathQueue q, HitQueue h, Ctrl* ctrl,

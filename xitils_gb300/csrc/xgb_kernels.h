@@ -204,12 +204,9 @@ void launchShadow(const SceneDev& sc, const RenderParams& rp, ShadowQueue sq, Pa
 // Film plane (float4 or double4 per pixel) -> packed float RGB, strideFloats 3 or 4 (image.cu).
 void launchPackFilm(const void* film, int fp64, size_t n, int strideFloats, float* out, int grid, cudaStream_t s);
 // Ray queries on a built scene: rays of 7 floats (o, d, tMax); closest hits as 5 floats per ray
-// (t, instance, triangle, b0, b1; -1 for none) or any-hit flags.
-struct QueryState {
-    unsigned int head;    // rays handed out
-    unsigned int errors;
-};
-void launchQuery(const SceneDev& sc, const float* rays, int n, int any, float* hits, int* occluded, QueryState* state,
-                 int numSMs, cudaStream_t s);
+// (t, instance, triangle, b0, b1; -1 for none) or any-hit flags. ctrl: zero but for nActive
+// and nShadow = n.
+void launchQuery(const SceneDev& sc, const float* rays, int n, int any, float* hits, int* occluded, Ctrl* ctrl, int numSMs,
+                 cudaStream_t s);
 
 }  // namespace xgb
