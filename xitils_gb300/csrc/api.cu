@@ -1517,9 +1517,10 @@ xgb_status xgb_render(xgb_scene* s, const xgb_integrator_params* params, xgb_fil
     // defaults count the steps of the wavefront's kernels.
     const bool tail = !gd && !prof && s->maxSteps == kDefaultMaxSteps && s->stackLimit == kMaxStackLimit;
     const unsigned int tailMax = tailMaxPaths(s->sd);
-    // Once every camera path has started the counters are read every two iterations, so
-    // that the tail starts in time; a call not much larger than a tail begins that way.
-    bool ending = total <= cap && total <= 16ull * tailMax;
+    // Once every camera path has started, the fewer paths are left the sooner the counters
+    // are read again, so that the tail starts in time (a read costs 20 us).
+    bool ending = total <= cap;
+    unsigned long long left = total;
     for (int guard = 0;; ++guard) {
         const bool direct = tail && guard == 0 && total <= tailMax && total <= cap;
         if (direct) {
@@ -1527,7 +1528,7 @@ xgb_status xgb_render(xgb_scene* s, const xgb_integrator_params* params, xgb_fil
             launchGenerate(s->sd, rp, s->rb.q[parity], s->ctrl, gShade, st);
             launches += 2;
         }
-        const int nIter = direct ? 0 : tail && ending ? 2 : kIterPerCheck;
+        const int nIter = direct ? 0 : !tail || !ending || left > 4ull * tailMax ? kIterPerCheck : left > 2ull * tailMax ? 4 : 2;
         for (int k = 0; k < nIter; ++k) {
             PathQueue& X = s->rb.q[parity];
             PathQueue& Y = s->rb.q[parity ^ 1];
@@ -1561,6 +1562,7 @@ xgb_status xgb_render(xgb_scene* s, const xgb_integrator_params* params, xgb_fil
         XGB_CUDA(ctx, cudaStreamSynchronize(st));
         if (tail && s->ctrlHost->nTail) parity ^= 1;
         ending = s->ctrlHost->nextPath >= s->ctrlHost->totalPaths;
+        left = s->ctrlHost->nOut;
         if (prof) {
             // stages: plan, generate, extend, [guide inference], shade, shadow
             for (int k = 0; k < kIterPerCheck; ++k) {

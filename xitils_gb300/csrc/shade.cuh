@@ -408,14 +408,23 @@ __device__ __forceinline__ void shadeVertex(const J& jobs, const PathQueue& in, 
 // float pairs (crmath.cuh), 38.4 -> 36.7 ms for the whole terrain render, 44.9 -> 41.1
 // for the cloth, 7.1 -> 6.65 for normal mapping.
 template <class J, int NESTED, bool EXTRAS>
-__global__ void __launch_bounds__(kShadeBlock, (NESTED & 3) ? 2 : (NESTED & kNoEmitters) ? 5 : (NESTED & kOnlyMetal) ? 4 : 3) k_shade(J jobs, PathQueue in, HitQueue hq, PathQueue out,
+__global__ void __launch_bounds__(kShadeBlock, (NESTED & 3) ? 2 : (NESTED & kNoEmitters) ? 5 : (NESTED & (kOnlyMetal | kOnlyDiffuse)) ? 4 : 3) k_shade(J jobs, PathQueue in, HitQueue hq, PathQueue out,
                                                        ShadowQueue sq, Ctrl* ctrl) {
+    // The two output counts are taken by one 64-bit atomic; plain materials take it once per
+    // block. All of a launch's atomics go to one address, which serves about one per
+    // nanosecond: with one per warp for each count and one for the finished paths, a
+    // shade launch lasted as long as its atomics (Cornell box: 1.7 million in 1.85 ms).
+    // Nested materials' warps take too different times to wait for one another.
+    constexpr bool kBlockwise = !(NESTED & 3);
+    constexpr unsigned int kWarps = kShadeBlock / 32;
+    __shared__ unsigned int sCont[kWarps], sShadow[kWarps], sOutAt[kWarps], sShadowAt[kWarps];
     const unsigned int n = ctrl->nActive;
-    const int lane = threadIdx.x & 31;
-    const unsigned int warpId = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const unsigned int nWarps = (gridDim.x * blockDim.x) >> 5;
-    for (unsigned int base = warpId * 32u; base < n; base += nWarps * 32u) {
-        const unsigned int i = base + lane;
+    const unsigned int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    unsigned int ended = 0;
+    // a block's threads together, or each warp on its own, step through the queue
+    const unsigned int first = blockIdx.x * kShadeBlock + (kBlockwise ? 0u : warp * 32u);
+    for (unsigned int base = first; base < n; base += gridDim.x * kShadeBlock) {
+        const unsigned int i = base + (kBlockwise ? threadIdx.x : lane);
         bool cont = false, shadow = false, done = false;
         ShadeOut r;
         r.stochastic = false;
@@ -432,12 +441,48 @@ __global__ void __launch_bounds__(kShadeBlock, (NESTED & 3) ? 2 : (NESTED & kNoE
             shadeVertex<J, NESTED, EXTRAS ? (kAov | kProposal) : 0>(jobs, in, i, o4, d4, t4, rs, h, instId, r, cont,
                                                                     shadow, done);
         }
+        ended += done ? 1u : 0u;
         // compacted writes: continuing paths, then shadow rays (which may point at them)
-        unsigned int mc = __ballot_sync(kFull, cont);
-        unsigned int oc = 0;
-        if (lane == 0 && mc) oc = atomicAdd(&ctrl->nOut, (unsigned int)__popc(mc));
-        oc = __shfl_sync(kFull, oc, 0);
-        unsigned int slot = oc + __popc(mc & ((1u << lane) - 1u));
+        const unsigned int mc = __ballot_sync(kFull, cont), ms = __ballot_sync(kFull, shadow);
+        unsigned int oc, os;
+        unsigned long long* counts = reinterpret_cast<unsigned long long*>(&ctrl->nOut);
+        if (kBlockwise) {
+            if (lane == 0) {
+                sCont[warp] = __popc(mc);
+                sShadow[warp] = __popc(ms);
+            }
+            __syncthreads();
+            if (warp == 0) {
+                // both counts in one word each way: at most 256 per block
+                const unsigned int mine = lane < kWarps ? sCont[lane] | sShadow[lane] << 16 : 0u;
+                unsigned int upTo = mine;
+#pragma unroll
+                for (unsigned int o = 1; o < kWarps; o <<= 1) {
+                    const unsigned int v = __shfl_up_sync(kFull, upTo, o);
+                    if (lane >= o) upTo += v;
+                }
+                const unsigned int all = __shfl_sync(kFull, upTo, kWarps - 1);
+                unsigned long long at = 0;
+                if (lane == 0 && all)
+                    at = atomicAdd(counts, (unsigned long long)(all & 0xFFFFu) | (unsigned long long)(all >> 16) << 32);
+                at = __shfl_sync(kFull, at, 0);
+                if (lane < kWarps) {
+                    sOutAt[lane] = (unsigned int)at + ((upTo - mine) & 0xFFFFu);
+                    sShadowAt[lane] = (unsigned int)(at >> 32) + ((upTo - mine) >> 16);
+                }
+            }
+            __syncthreads();
+            oc = sOutAt[warp];
+            os = sShadowAt[warp];
+        } else {
+            unsigned long long at = 0;
+            if (lane == 0 && (mc | ms))
+                at = atomicAdd(counts, (unsigned long long)__popc(mc) | (unsigned long long)__popc(ms) << 32);
+            at = __shfl_sync(kFull, at, 0);
+            oc = (unsigned int)at;
+            os = (unsigned int)(at >> 32);
+        }
+        const unsigned int slot = oc + __popc(mc & ((1u << lane) - 1u));
         const bool train = EXTRAS && jobs.params(0).train;  // guide training runs with one job only
         if (cont) {
             __stcs(&out.o[slot], r.o);
@@ -449,12 +494,8 @@ __global__ void __launch_bounds__(kShadeBlock, (NESTED & 3) ? 2 : (NESTED & kNoE
                 out.pid[slot] = in.pid[i];
             }
         }
-        unsigned int ms = __ballot_sync(kFull, shadow);
-        unsigned int os = 0;
-        if (lane == 0 && ms) os = atomicAdd(&ctrl->nShadow, (unsigned int)__popc(ms));
-        os = __shfl_sync(kFull, os, 0);
         if (shadow) {
-            unsigned int ss = os + __popc(ms & ((1u << lane) - 1u));
+            const unsigned int ss = os + __popc(ms & ((1u << lane) - 1u));
             __stcs(&sq.o[ss], r.so);
             __stcs(&sq.d[ss], r.sd);
             r.sc.w = __int_as_float((r.stochastic && cont) ? (int)slot : -1);
@@ -462,9 +503,9 @@ __global__ void __launch_bounds__(kShadeBlock, (NESTED & 3) ? 2 : (NESTED & kNoE
             __stcs(&sq.rng[ss], r.srng);
             if (train) sq.pid[ss] = in.pid[i];
         }
-        unsigned int md = __ballot_sync(kFull, done);
-        if (lane == 0 && md) atomicAdd(&ctrl->pathsDone, (unsigned long long)__popc(md));
     }
+    ended = __reduce_add_sync(kFull, ended);
+    if (lane == 0 && ended) atomicAdd(&ctrl->pathsDone, (unsigned long long)ended);
 }
 
 // Grid of a shade launch: kShadeWaves full waves of the variant's resident

@@ -2,6 +2,7 @@
 // translation units. No CUDA types beyond cudaStream_t cross this boundary.
 #pragma once
 #include <cuda_runtime.h>
+#include <stddef.h>
 #include <stdint.h>
 
 #include "xgb_types.h"
@@ -60,7 +61,7 @@ struct Ctrl {
     unsigned int nCont;            // paths carried over into this iteration's input queue
     unsigned int nActive;          // paths in this iteration's input queue
     unsigned int nOut;             // paths written to the output queue by shade
-    unsigned int nShadow;          // shadow rays written by shade
+    unsigned int nShadow;          // shadow rays written by shade (counted with nOut as one 64-bit word)
     unsigned int extendHead;       // persistent work counters
     unsigned int shadowHead;
     unsigned int errors;           // bit 0: traversal stack overflow
@@ -74,6 +75,8 @@ struct Ctrl {
     unsigned long long nodeVisits;  // profiling counters (extension rays)
     unsigned long long triTests;
 };
+
+static_assert(offsetof(Ctrl, nOut) % 8 == 0 && offsetof(Ctrl, nShadow) == offsetof(Ctrl, nOut) + 4, "one 64-bit counter");
 
 // ERR_WAIT: a bounded mbarrier wait of the tensor-memory inference kernels gave up.
 enum ErrorBits : unsigned int { ERR_STACK = 1u, ERR_QUEUE = 2u, ERR_LOOP = 4u, ERR_WAIT = 8u };
