@@ -388,6 +388,18 @@ __device__ __forceinline__ void shadeVertex(const J& jobs, const PathQueue& in, 
     }
 }
 
+// Grid of a shade launch: kShadeWaves full waves of the variant's resident
+// blocks (SMs x blocks per SM at its register bound). Whole waves leave no
+// partial last wave idling SMs (eight blocks per SM at three resident ran as
+// 2.67 waves); many small blocks let SMs whose blocks finish early take more,
+// which the uneven per-path cost of nested materials needs. Measured on GB300,
+// shading time per render against the earlier eight blocks per SM: one wave --
+// terrain 12.1 instead of 12.6 ms, normal mapping 5.96 instead of 4.4; four
+// waves -- 12.7 / 4.4; eight waves -- terrain 12.6, shell mapping 7.6 instead
+// of 8.6, normal mapping 3.6.
+constexpr int kShadeWaves = 8;
+constexpr unsigned int kShadeBins = 4;
+
 // EXTRAS: the learned proposal (guided sampling, training records), AOV planes;
 // plain renders run the variant without that code (fewer registers, a smaller
 // instruction footprint). Occupancy bounds, measured on GB300: without nested
@@ -398,9 +410,8 @@ __device__ __forceinline__ void shadeVertex(const J& jobs, const PathQueue& in, 
 // normal-mapping scene 101 instead of 88 Mpaths/s at one block (140 registers);
 // the GGX-metal-only variant four blocks (64 registers, ~200 bytes of spills) --
 // terrain shading 10.1 instead of 11.6 ms per render at three, 1834 instead of 1762
-// Mpaths/s -- while the Lambert-only variant stays at three (the Cornell box
-// 9.5 against 9.9 ms of shading over five renders at four, the room 40.8
-// against 42.2). Without emitters (no emission, no NEE code) and with the
+// Mpaths/s -- and the Lambert-only variant four too (the Cornell box 1.13 against
+// 1.27 ms of shading per render at three; before the block-wise counts below four lost). Without emitters (no emission, no NEE code) and with the
 // standard integrator only, the metal variant shaded the terrain in 9.2 ms per
 // render at four blocks (1878 Mpaths/s) and 9.1 ms at five (51 registers, 1884).
 // All of these were bound by the FP64 pipe (61 % busy in the terrain, 68 % in the
@@ -421,103 +432,140 @@ __global__ void __launch_bounds__(kShadeBlock, (NESTED & 3) ? 2 : (NESTED & kNoE
     const unsigned int n = ctrl->nActive;
     const unsigned int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     unsigned int ended = 0;
-    // a block's threads together, or each warp on its own, step through the queue
-    const unsigned int first = blockIdx.x * kShadeBlock + (kBlockwise ? 0u : warp * 32u);
-    for (unsigned int base = first; base < n; base += gridDim.x * kShadeBlock) {
-        const unsigned int i = base + (kBlockwise ? threadIdx.x : lane);
-        bool cont = false, shadow = false, done = false;
-        ShadeOut r;
-        r.stochastic = false;
-        r.grec = -1;
-        if (i < n) {
-            // Queue records are read once and written once per iteration and far
-            // exceed L2 at 2^23 paths in flight: streaming (evict-first) loads and
-            // stores keep L2 for BVH nodes, triangles and textures (terrain shading
-            // 12.7 -> 11.6 ms per render, 1495 -> 1533 Mpaths/s on GB300).
-            float4 o4 = __ldcs(&in.o[i]), d4 = __ldcs(&in.d[i]), t4 = __ldcs(&in.thr[i]);
-            uint2 rs = __ldcs(&in.rng[i]);
-            float4 h = __ldcs(&hq.h[i]);
-            const int instId = __ldcs(&hq.inst[i]);
-            shadeVertex<J, NESTED, EXTRAS ? (kAov | kProposal) : 0>(jobs, in, i, o4, d4, t4, rs, h, instId, r, cont,
-                                                                    shadow, done);
-        }
-        ended += done ? 1u : 0u;
-        // compacted writes: continuing paths, then shadow rays (which may point at them)
-        const unsigned int mc = __ballot_sync(kFull, cont), ms = __ballot_sync(kFull, shadow);
-        unsigned int oc, os;
-        unsigned long long* counts = reinterpret_cast<unsigned long long*>(&ctrl->nOut);
-        if (kBlockwise) {
-            if (lane == 0) {
-                sCont[warp] = __popc(mc);
-                sShadow[warp] = __popc(ms);
-            }
-            __syncthreads();
-            if (warp == 0) {
-                // both counts in one word each way: at most 256 per block
-                const unsigned int mine = lane < kWarps ? sCont[lane] | sShadow[lane] << 16 : 0u;
-                unsigned int upTo = mine;
+    // A block's threads together, or each warp on its own, step through the queue.
+    //
+    // A scene without emitters is lit by its sky: after the first vertex half of the rays
+    // miss, and a warp that holds both kinds runs both codes (12 of 32 threads active). So
+    // a block takes kShadeBins slots per thread and shades the hits first, then the misses,
+    // each in the queue's order: terrain 1024^2 x 64 shading 6.7 -> 5.4 ms. Not with fewer
+    // than two waves of such chunks (512^2 x 4: 1.17 -> 1.20 ms per call, x 16: 2.38 ->
+    // 2.32), nor where few rays miss (Cornell box 1.13 -> 1.19 ms of shading) or few paths
+    // are left at most vertices (guided room 1.23 -> 2.34).
+    constexpr bool kSorted = (NESTED & kNoEmitters) != 0;
+    __shared__ unsigned short sOrder[kSorted ? kShadeBlock * kShadeBins : 1];
+    __shared__ unsigned int sHits[kSorted ? kWarps * kShadeBins : 1];
+    static_assert(!kSorted || kWarps * kShadeBins == 32, "one warp scans the counts");
+    const bool sorted = kSorted && n >= 2u * (gridDim.x / kShadeWaves) * kShadeBlock * kShadeBins;
+    const unsigned int chunk = sorted ? kShadeBlock * kShadeBins : kBlockwise ? kShadeBlock : 32u;
+    const unsigned int begin = kBlockwise ? blockIdx.x * chunk : (blockIdx.x * kWarps + warp) * chunk;
+    for (unsigned int start = begin; start < n; start += gridDim.x * (kBlockwise ? 1u : kWarps) * chunk) {
+        const unsigned int count = min(chunk, n - start);
+        unsigned int hits = count;  // the first so many of the chunk may have paths that go on
+        if (kSorted && sorted) {
+            unsigned int m[kShadeBins];
 #pragma unroll
-                for (unsigned int o = 1; o < kWarps; o <<= 1) {
-                    const unsigned int v = __shfl_up_sync(kFull, upTo, o);
-                    if (lane >= o) upTo += v;
-                }
-                const unsigned int all = __shfl_sync(kFull, upTo, kWarps - 1);
-                unsigned long long at = 0;
-                if (lane == 0 && all)
-                    at = atomicAdd(counts, (unsigned long long)(all & 0xFFFFu) | (unsigned long long)(all >> 16) << 32);
-                at = __shfl_sync(kFull, at, 0);
-                if (lane < kWarps) {
-                    sOutAt[lane] = (unsigned int)at + ((upTo - mine) & 0xFFFFu);
-                    sShadowAt[lane] = (unsigned int)(at >> 32) + ((upTo - mine) >> 16);
-                }
+            for (unsigned int k = 0; k < kShadeBins; ++k) {
+                const unsigned int j = k * kShadeBlock + threadIdx.x;
+                m[k] = __ballot_sync(kFull, j < count && __float_as_int(hq.h[start + j].w) >= 0);
+                if (lane == 0) sHits[k * kWarps + warp] = __popc(m[k]);
             }
             __syncthreads();
-            oc = sOutAt[warp];
-            os = sShadowAt[warp];
-        } else {
-            unsigned long long at = 0;
-            if (lane == 0 && (mc | ms))
-                at = atomicAdd(counts, (unsigned long long)__popc(mc) | (unsigned long long)__popc(ms) << 32);
-            at = __shfl_sync(kFull, at, 0);
-            oc = (unsigned int)at;
-            os = (unsigned int)(at >> 32);
+            const unsigned int mine = sHits[lane];
+            unsigned int upTo = mine;
+#pragma unroll
+            for (unsigned int o = 1; o < 32; o <<= 1) {
+                const unsigned int v = __shfl_up_sync(kFull, upTo, o);
+                if (lane >= o) upTo += v;
+            }
+            hits = __shfl_sync(kFull, upTo, 31);
+#pragma unroll
+            for (unsigned int k = 0; k < kShadeBins; ++k) {
+                const unsigned int j = k * kShadeBlock + threadIdx.x;
+                const unsigned int before =
+                    __shfl_sync(kFull, upTo - mine, k * kWarps + warp) + __popc(m[k] & ((1u << lane) - 1u));
+                if (j < count) sOrder[(m[k] >> lane) & 1u ? before : hits + j - before] = (unsigned short)j;
+            }
+            __syncthreads();
         }
-        const unsigned int slot = oc + __popc(mc & ((1u << lane) - 1u));
-        const bool train = EXTRAS && jobs.params(0).train;  // guide training runs with one job only
-        if (cont) {
-            __stcs(&out.o[slot], r.o);
-            __stcs(&out.d[slot], r.d);
-            __stcs(&out.thr[slot], r.thr);
-            __stcs(&out.rng[slot], r.rng);
-            if (train) {
-                out.grec[slot] = r.grec;
-                out.pid[slot] = in.pid[i];
+        for (unsigned int step = 0; step < count; step += kBlockwise ? kShadeBlock : 32u) {
+            const unsigned int j = step + (kBlockwise ? threadIdx.x : lane);
+            const unsigned int i = start + (kSorted && sorted && j < count ? sOrder[j] : j);
+            bool cont = false, shadow = false, done = false;
+            ShadeOut r;
+            r.stochastic = false;
+            r.grec = -1;
+            if (j < count) {
+                // Queue records are read once and written once per iteration and far
+                // exceed L2 at 2^23 paths in flight: streaming (evict-first) loads and
+                // stores keep L2 for BVH nodes, triangles and textures (terrain shading
+                // 12.7 -> 11.6 ms per render, 1495 -> 1533 Mpaths/s on GB300).
+                float4 o4 = __ldcs(&in.o[i]), d4 = __ldcs(&in.d[i]), t4 = __ldcs(&in.thr[i]);
+                uint2 rs = __ldcs(&in.rng[i]);
+                float4 h = __ldcs(&hq.h[i]);
+                const int instId = __ldcs(&hq.inst[i]);
+                shadeVertex<J, NESTED, EXTRAS ? (kAov | kProposal) : 0>(jobs, in, i, o4, d4, t4, rs, h, instId, r, cont,
+                                                                        shadow, done);
+            }
+            ended += done ? 1u : 0u;
+            if (kSorted && step >= hits) continue;  // misses only
+            // compacted writes: continuing paths, then shadow rays (which may point at them)
+            const unsigned int mc = __ballot_sync(kFull, cont), ms = __ballot_sync(kFull, shadow);
+            unsigned int oc, os;
+            unsigned long long* counts = reinterpret_cast<unsigned long long*>(&ctrl->nOut);
+            if (kBlockwise) {
+                if (lane == 0) {
+                    sCont[warp] = __popc(mc);
+                    sShadow[warp] = __popc(ms);
+                }
+                __syncthreads();
+                if (warp == 0) {
+                    // both counts in one word each way: at most 256 per block
+                    const unsigned int mine = lane < kWarps ? sCont[lane] | sShadow[lane] << 16 : 0u;
+                    unsigned int upTo = mine;
+#pragma unroll
+                    for (unsigned int o = 1; o < kWarps; o <<= 1) {
+                        const unsigned int v = __shfl_up_sync(kFull, upTo, o);
+                        if (lane >= o) upTo += v;
+                    }
+                    const unsigned int all = __shfl_sync(kFull, upTo, kWarps - 1);
+                    unsigned long long at = 0;
+                    if (lane == 0 && all)
+                        at = atomicAdd(counts, (unsigned long long)(all & 0xFFFFu) | (unsigned long long)(all >> 16) << 32);
+                    at = __shfl_sync(kFull, at, 0);
+                    if (lane < kWarps) {
+                        sOutAt[lane] = (unsigned int)at + ((upTo - mine) & 0xFFFFu);
+                        sShadowAt[lane] = (unsigned int)(at >> 32) + ((upTo - mine) >> 16);
+                    }
+                }
+                __syncthreads();
+                oc = sOutAt[warp];
+                os = sShadowAt[warp];
+            } else {
+                unsigned long long at = 0;
+                if (lane == 0 && (mc | ms))
+                    at = atomicAdd(counts, (unsigned long long)__popc(mc) | (unsigned long long)__popc(ms) << 32);
+                at = __shfl_sync(kFull, at, 0);
+                oc = (unsigned int)at;
+                os = (unsigned int)(at >> 32);
+            }
+            const unsigned int slot = oc + __popc(mc & ((1u << lane) - 1u));
+            const bool train = EXTRAS && jobs.params(0).train;  // guide training runs with one job only
+            if (cont) {
+                __stcs(&out.o[slot], r.o);
+                __stcs(&out.d[slot], r.d);
+                __stcs(&out.thr[slot], r.thr);
+                __stcs(&out.rng[slot], r.rng);
+                if (train) {
+                    out.grec[slot] = r.grec;
+                    out.pid[slot] = in.pid[i];
+                }
+            }
+            if (shadow) {
+                const unsigned int ss = os + __popc(ms & ((1u << lane) - 1u));
+                __stcs(&sq.o[ss], r.so);
+                __stcs(&sq.d[ss], r.sd);
+                r.sc.w = __int_as_float((r.stochastic && cont) ? (int)slot : -1);
+                __stcs(&sq.c[ss], r.sc);
+                __stcs(&sq.rng[ss], r.srng);
+                if (train) sq.pid[ss] = in.pid[i];
             }
         }
-        if (shadow) {
-            const unsigned int ss = os + __popc(ms & ((1u << lane) - 1u));
-            __stcs(&sq.o[ss], r.so);
-            __stcs(&sq.d[ss], r.sd);
-            r.sc.w = __int_as_float((r.stochastic && cont) ? (int)slot : -1);
-            __stcs(&sq.c[ss], r.sc);
-            __stcs(&sq.rng[ss], r.srng);
-            if (train) sq.pid[ss] = in.pid[i];
-        }
+        if (kSorted && sorted) __syncthreads();
     }
     ended = __reduce_add_sync(kFull, ended);
     if (lane == 0 && ended) atomicAdd(&ctrl->pathsDone, (unsigned long long)ended);
 }
 
-// Grid of a shade launch: kShadeWaves full waves of the variant's resident
-// blocks (SMs x blocks per SM at its register bound). Whole waves leave no
-// partial last wave idling SMs (eight blocks per SM at three resident ran as
-// 2.67 waves); many small blocks let SMs whose blocks finish early take more,
-// which the uneven per-path cost of nested materials needs. Measured on GB300,
-// shading time per render against the earlier eight blocks per SM: one wave --
-// terrain 12.1 instead of 12.6 ms, normal mapping 5.96 instead of 4.4; four
-// waves -- 12.7 / 4.4; eight waves -- terrain 12.6, shell mapping 7.6 instead
-// of 8.6, normal mapping 3.6.
-constexpr int kShadeWaves = 8;
 template <class J, int NESTED, bool EXTRAS>
 inline int shadeGrid(int numSMs) {
     // looked up once per variant (a thread-safe static initialisation)
