@@ -821,17 +821,25 @@ __global__ void __launch_bounds__(kTraceBlock, (WorldTraits<S, ENTER>::kMinBlock
         atomicAdd(ANY ? &ctrl->shadowRays : &ctrl->extensionRays, (unsigned long long)n);
 }
 
-// The marked rays of a k_trace_world launch, in the instance order.
+// The marked rays of a k_trace_world launch, in the instance order. The hit that was found
+// bounds them: what is no more than the margin of cullMul and cullAbs beyond it has been
+// seen to be hit, so boxes further off need no visit, and where several hits within the
+// margin follow one another the order alone decides, as from an unbounded start. Few rays
+// are marked, so each warp takes one first: together in a warp they would wait for one
+// another (microfacet normal mapping 400^2 x 4: 5.31 -> 5.18 ms per call).
 template <class S>
 __global__ void __launch_bounds__(kTraceBlock) k_retrace(S scenes, PathQueue q, HitQueue h, const unsigned int* retrace,
                                                          Ctrl* ctrl) {
     const unsigned int n = ctrl->nRetrace;
-    for (unsigned int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
+    const unsigned int warps = gridDim.x * (kTraceBlock / 32);
+    const unsigned int warp = (threadIdx.x >> 5) * gridDim.x + blockIdx.x;
+    for (unsigned int k = (threadIdx.x & 31) * warps + warp; k < n; k += 32u * warps) {
         const unsigned int ray = retrace[k];
         const float4 o = q.o[ray], d = q.d[ray];
+        const SceneDev& sc = scenes.scene(scenes.jobOf(__float_as_uint(q.thr[ray].w)));
         TraceHit hit;
-        traceCall(scenes.scene(scenes.jobOf(__float_as_uint(q.thr[ray].w))), V3(o.x, o.y, o.z), V3(d.x, d.y, d.z),
-                  __int_as_float(0x7f800000), false, hit, &ctrl->errors);
+        traceCall(sc, V3(o.x, o.y, o.z), V3(d.x, d.y, d.z), fmaf(h.h[ray].x, sc.world.cullMul, sc.world.cullAbs), false,
+                  hit, &ctrl->errors);
         h.h[ray] = make_float4(hit.t, hit.b0, hit.b1, __int_as_float(hit.prim));
         h.inst[ray] = hit.inst;
     }
