@@ -597,7 +597,7 @@ __global__ void __launch_bounds__(kTraceBlock, (WorldTraits<S, ENTER>::kMinBlock
     int rayStack = 0;   // a batch: the current ray's job's bound
     int inst = -1;      // ENTER: the instance the ray is in (-1: world space)
     int hitInst = -1;   // ENTER: the instance of a hit found inside one
-    int stack[kWorldStack];
+    int stack[kWorldStack + 1];
     int sp = 0;
     int nodeAddr = kSentinel, leafAddr = 0;
     unsigned int ray = 0;
@@ -668,23 +668,20 @@ __global__ void __launch_bounds__(kTraceBlock, (WorldTraits<S, ENTER>::kMinBlock
             float t0, t1;
             bool h0 = slab(r, a.x, a.y, a.z, a.w, b.x, b.y, tCull, t0);
             bool h1 = slab(r, b.z, b.w, c.x, c.y, c.z, c.w, tCull, t1);
-            if (h0 && h1) {
-                int near = dd.x, far = dd.y;
-                if (t1 < t0) { near = dd.y; far = dd.x; }
-                if (sp >= (kBatch ? rayStack : worldStackCap(scenes.scene(0)))) {
-                    atomicOr(&ctrl->errors, 1u);
-                    sp = 0;
-                    nodeAddr = kSentinel;
-                    break;
-                }
-                stack[sp++] = far;
-                nodeAddr = near;
-            } else if (h0) {
-                nodeAddr = dd.x;
-            } else if (h1) {
-                nodeAddr = dd.y;
+            // one branch for a hit or a pop, selects within: 31.8 -> 31.5 ms for the terrain
+            // against a branch per combination, 32.4 with the bound checked before the push
+            if (h0 || h1) {
+                const bool second = !h0 || (h1 && t1 < t0);
+                nodeAddr = second ? dd.y : dd.x;
+                if (h0 && h1) stack[sp++] = second ? dd.x : dd.y;
             } else {
                 nodeAddr = sp > 0 ? stack[--sp] : kSentinel;
+            }
+            if (sp > (kBatch ? rayStack : worldStackCap(scenes.scene(0)))) {
+                atomicOr(&ctrl->errors, 1u);
+                sp = 0;
+                nodeAddr = kSentinel;
+                break;
             }
             if (nodeAddr < 0 && leafAddr >= 0) {  // first leaf: postpone it, keep descending
                 searching = false;
