@@ -901,6 +901,8 @@ static Box transformBox(const float* m, const Box& b) {
     return r;
 }
 
+static float3 corner(const float* p) { return make_float3(p[0], p[1], p[2]); }
+
 // Top-level BVH over instance boxes: median split on the longest centroid axis.
 static int buildTlas(std::vector<Node2>& nodes, std::vector<int>& items, const std::vector<Box>& boxes, int begin,
                      int end, Box* outBox) {
@@ -927,9 +929,7 @@ static int buildTlas(std::vector<Node2>& nodes, std::vector<int>& items, const s
     int cl = buildTlas(nodes, items, boxes, begin, mid, &l);
     int cr = buildTlas(nodes, items, boxes, mid, end, &r);
     Node2& nd = nodes[me];
-    nd.a = make_float4(l.lo[0], l.lo[1], l.lo[2], l.hi[0]);
-    nd.b = make_float4(l.hi[1], l.hi[2], r.lo[0], r.lo[1]);
-    nd.c = make_float4(r.lo[2], r.hi[0], r.hi[1], r.hi[2]);
+    setBoxes(nd, corner(l.lo), corner(l.hi), corner(r.lo), corner(r.hi));
     nd.d = make_int4(cl, cr, 0, 0);
     return me;
 }
@@ -994,9 +994,7 @@ static void buildWorldTop(std::vector<Node2>& nodes, const std::vector<Box>& box
             }
         const Box l = box[bi], r = box[bj];
         Node2& nd = nodes[next];
-        nd.a = make_float4(l.lo[0], l.lo[1], l.lo[2], l.hi[0]);
-        nd.b = make_float4(l.hi[1], l.hi[2], r.lo[0], r.lo[1]);
-        nd.c = make_float4(r.lo[2], r.hi[0], r.hi[1], r.hi[2]);
+        setBoxes(nd, corner(l.lo), corner(l.hi), corner(r.lo), corner(r.hi));
         nd.d = make_int4(code[bi], code[bj], 0, 0);
         box[bi].add(r);
         code[bi] = next;

@@ -192,9 +192,7 @@ __global__ void k_emit(int n, const int* __restrict__ left, const int* __restric
     int a = left[i], b = right[i];
     float4 al = nodeLo[a], ah = nodeHi[a], bl = nodeLo[b], bh = nodeHi[b];
     Node2 nd;
-    nd.a = make_float4(al.x, al.y, al.z, ah.x);
-    nd.b = make_float4(ah.y, ah.z, bl.x, bl.y);
-    nd.c = make_float4(bl.z, bh.x, bh.y, bh.z);
+    setBoxes(nd, al, ah, bl, bh);
     nd.d = make_int4(childCode(a, n, first, last), childCode(b, n, first, last), 0, 0);
     nodes[i] = nd;
 }
@@ -502,9 +500,7 @@ __global__ void k_plocEmit(int n, const int* __restrict__ left, const int* __res
     const int a = left[k], b = right[k];
     const float4 al = nodeLo[a], ah = nodeHi[a], bl = nodeLo[b], bh = nodeHi[b];
     Node2 nd;
-    nd.a = make_float4(al.x, al.y, al.z, ah.x);
-    nd.b = make_float4(ah.y, ah.z, bl.x, bl.y);
-    nd.c = make_float4(bl.z, bh.x, bh.y, bh.z);
+    setBoxes(nd, al, ah, bl, bh);
     nd.d = make_int4(plocChild(a, n, count, dfs), plocChild(b, n, count, dfs), 0, 0);
     nodes[(2 * n - 2) - id] = nd;
 }

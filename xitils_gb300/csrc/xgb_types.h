@@ -17,11 +17,18 @@ namespace xgb {
 // Binary BVH node holding both children's boxes (one 64-byte line per visit).
 // child >= 0: inner node index; child < 0: leaf, ~child = (first << 4) | (count - 1).
 struct __align__(16) Node2 {
-    float4 a;  // c0.lo.x c0.lo.y c0.lo.z c0.hi.x
-    float4 b;  // c0.hi.y c0.hi.z c1.lo.x c1.lo.y
-    float4 c;  // c1.lo.z c1.hi.x c1.hi.y c1.hi.z
+    float4 a;  // c0.lo.x c0.lo.y c0.hi.x c0.hi.y
+    float4 b;  // c1.lo.x c1.lo.y c1.hi.x c1.hi.y
+    float4 c;  // c0.lo.z c0.hi.z c1.lo.z c1.hi.z
     int4 d;    // child0 child1 - -
 };
+// Planes in pairs that the slab test takes two at a time (trace.cuh::slabs).
+template <class P0, class P1, class P2, class P3>
+__host__ __device__ inline void setBoxes(Node2& nd, const P0& lo0, const P1& hi0, const P2& lo1, const P3& hi1) {
+    nd.a = make_float4(lo0.x, lo0.y, hi0.x, hi0.y);
+    nd.b = make_float4(lo1.x, lo1.y, hi1.x, hi1.y);
+    nd.c = make_float4(lo0.z, hi0.z, lo1.z, hi1.z);
+}
 static_assert(sizeof(Node2) == 64, "Node2 size");
 
 // Triangles per leaf of a binary mesh BVH. Measured on GB300 (leaf limit 2 / 3 / 4 / 6 / 8):
