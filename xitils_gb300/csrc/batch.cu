@@ -63,6 +63,7 @@ struct BatchState {
     int graphIters = 0;
     int graphJobs = 0;
     int graphKernels = -1;
+    SideLane side;  // without one the shadow rays take the same stream
     std::map<std::string, xgb_batch_options> tuned;
     xgb_render_stats last{};
 };
@@ -72,6 +73,7 @@ std::map<xgb_ctx*, BatchState*> g_states;
 
 void freeState(BatchState* b) {
     if (b->graph) cudaGraphExecDestroy(b->graph);
+    b->side.destroy();
     for (void* p : {(void*)b->block, (void*)b->ctrl, (void*)b->dScenes, (void*)b->dParams, (void*)b->dStart})
         if (p) cudaFree(p);
     for (void* p : {(void*)b->ctrlHost, (void*)b->hScenes, (void*)b->hParams, (void*)b->hStart})
@@ -123,6 +125,7 @@ cudaError_t ensureJobs(BatchState* b, int n) {
         cudaError_t e = cudaMalloc((void**)&b->ctrl, sizeof(Ctrl));
         if (e == cudaSuccess) e = cudaMallocHost((void**)&b->ctrlHost, sizeof(Ctrl));
         if (e != cudaSuccess) return e;
+        b->side.create();
     }
     if (b->jobCap >= n) return cudaSuccess;
     if (b->graph) { cudaGraphExecDestroy(b->graph); b->graph = nullptr; }
@@ -149,10 +152,18 @@ void enqueueBlock(BatchState* b, const BatchView& v, unsigned int cap, int iters
         PathQueue& Y = b->q[(k & 1) ^ 1];
         launchPlan(b->ctrl, cap, st);
         launchGenerateBatch(v, X, b->ctrl, numSMs * 8, st);
-        launchExtendBatch(v, X, b->hits, (unsigned int*)b->shadow.o, b->ctrl, numSMs, st);
+        // the last vertex's shadow rays beside the rays to the next (see xgb_render)
+        if (k > 0) {
+            if (b->side.stream) b->side.begin(st);
+            launchShadowBatch(v, b->shadow, X, b->ctrl, numSMs, b->side.stream ? b->side.stream : st);
+            if (b->side.stream) b->side.end();
+        }
+        launchExtendBatch(v, X, b->hits, (unsigned int*)Y.o, b->ctrl, numSMs, st);
+        if (k > 0 && b->side.stream) b->side.wait(st);
         launchShadeBatch(v, X, b->hits, Y, b->shadow, b->ctrl, numSMs, st);
-        launchShadowBatch(v, b->shadow, Y, b->ctrl, numSMs, st);
     }
+    launchPlan(b->ctrl, cap, st, kPlanShadow);
+    launchShadowBatch(v, b->shadow, b->q[0], b->ctrl, numSMs, st);
 }
 
 std::string shapeKey(const xgb_batch_job* jobs, int n) {

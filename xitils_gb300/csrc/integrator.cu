@@ -17,6 +17,12 @@
 namespace xgb {
 
 __global__ void k_plan(Ctrl* c, unsigned int capacity, int mode, unsigned int tailMax) {
+    if (mode == kPlanShadow || mode == kPlanWave) {
+        c->nShadowDue = c->nShadow;
+        c->nShadow = 0;
+        c->shadowHead = 0;
+    }
+    if (mode == kPlanShadow) return;
     unsigned int nCont = c->nOut;
     unsigned long long remain = c->totalPaths - c->nextPath;
     c->nTail = 0;
@@ -28,12 +34,10 @@ __global__ void k_plan(Ctrl* c, unsigned int capacity, int mode, unsigned int ta
     c->nCont = nCont;
     c->nActive = nCont + nNew;
     c->nOut = 0;
-    c->nShadow = 0;
     c->extendHead = 0;
-    c->shadowHead = 0;
     c->nRetrace = 0;
     if (c->nActive) c->iterations += 1;
-    if (mode != kPlanWave) c->nTail = c->nActive;
+    if (mode == kPlanTail || mode == kPlanTailIfFew) c->nTail = c->nActive;
 }
 
 // Camera paths: RenderTargetTile::GenerateFilmPosition (RenderTarget.h:68-80)
@@ -132,6 +136,22 @@ __global__ void __launch_bounds__(kShadeBlock) k_generate(J jobs, PathQueue q, c
             rp.pathAcc[g] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         }
     }
+}
+
+bool SideLane::create() {
+    if (cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking) == cudaSuccess &&
+        cudaEventCreateWithFlags(&fork, cudaEventDisableTiming) == cudaSuccess &&
+        cudaEventCreateWithFlags(&join, cudaEventDisableTiming) == cudaSuccess)
+        return true;
+    destroy();
+    cudaGetLastError();
+    return false;
+}
+void SideLane::destroy() {
+    if (fork) cudaEventDestroy(fork);
+    if (join) cudaEventDestroy(join);
+    if (stream) cudaStreamDestroy(stream);
+    *this = SideLane{};
 }
 
 void launchPlan(Ctrl* ctrl, unsigned int capacity, cudaStream_t s, int mode, unsigned int tailMax) {

@@ -70,7 +70,7 @@ __global__ void __launch_bounds__(kTraceBlock) k_extend(SceneDev sc, PathQueue q
 
 __global__ void __launch_bounds__(kTraceBlock) k_shadow(SceneDev sc, RenderParams rp, ShadowQueue s, PathQueue out,
                                                         Ctrl* ctrl) {
-    const unsigned int n = ctrl->nShadow;
+    const unsigned int n = ctrl->nShadowDue;
     const int lane = threadIdx.x & 31;
     for (;;) {
         unsigned int base = 0;
@@ -142,7 +142,7 @@ struct QueryRays {
 template <bool ANY, bool COUNT>
 __global__ void __launch_bounds__(kTraceBlock) k_trace_wide(SceneDev sc, RenderParams rp, PathQueue q, HitQueue h,
                                                             ShadowQueue s, PathQueue out, Ctrl* ctrl) {
-    const unsigned int n = ANY ? ctrl->nShadow : ctrl->nActive;
+    const unsigned int n = ANY ? ctrl->nShadowDue : ctrl->nActive;
     unsigned int* head = ANY ? &ctrl->shadowHead : &ctrl->extendHead;
     const int nInst = sc.nInstances;
     const int lane = threadIdx.x & 31;
@@ -376,7 +376,7 @@ constexpr int kSentinel = 0x7FFFFFFF;
 template <bool ANY, bool COUNT, class S, bool SHELL = false>
 __global__ void __launch_bounds__(kTraceBlock) k_trace_flat2(S scenes, PathQueue q, HitQueue h, ShadowQueue s,
                                                             PathQueue out, Ctrl* ctrl) {
-    const unsigned int n = ANY ? ctrl->nShadow : ctrl->nActive;
+    const unsigned int n = ANY ? ctrl->nShadowDue : ctrl->nActive;
     unsigned int* head = ANY ? &ctrl->shadowHead : &ctrl->extendHead;
     constexpr bool kBatch = !std::is_same<S, OneScene>::value;
     int rayMaxSteps = 0, rayStack = 0;  // a batch: the current ray's job's bounds
@@ -584,7 +584,7 @@ template <bool ANY, bool COUNT, class S, bool ENTER, bool SHELL>
 __global__ void __launch_bounds__(kTraceBlock, (WorldTraits<S, ENTER>::kMinBlocks))
     k_trace_world(S scenes, PathQueue q, HitQueue h, unsigned int* retrace, ShadowQueue s, PathQueue out, Ctrl* ctrl) {
     constexpr bool kBatch = std::is_same<S, BatchScenes>::value, kQuery = std::is_same<S, QueryRays>::value;
-    const unsigned int n = ANY ? ctrl->nShadow : ctrl->nActive;
+    const unsigned int n = ANY ? ctrl->nShadowDue : ctrl->nActive;
     unsigned int* head = ANY ? &ctrl->shadowHead : &ctrl->extendHead;
     RayClaims claims(head, n);
     const int looking = claims.lanes == 32u ? kLookingLanes<SHELL> : 1;
@@ -867,7 +867,7 @@ __global__ void __launch_bounds__(kTraceBlock) k_extend_batch(BatchView b, PathQ
 }
 
 __global__ void __launch_bounds__(kTraceBlock) k_shadow_batch(BatchView b, ShadowQueue s, PathQueue out, Ctrl* ctrl) {
-    const unsigned int n = ctrl->nShadow;
+    const unsigned int n = ctrl->nShadowDue;
     const int lane = threadIdx.x & 31;
     WorkCount wc;
     for (;;) {

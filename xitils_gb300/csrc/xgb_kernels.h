@@ -66,7 +66,7 @@ struct Ctrl {
     unsigned int shadowHead;
     unsigned int errors;           // bit 0: traversal stack overflow
     unsigned int nRetrace;         // rays whose hits the instance order decides (k_trace_world)
-    unsigned int pad;
+    unsigned int nShadowDue;       // shadow rays of the previous shade launch, traced beside the next rays
     unsigned int nTail;            // paths the next tail launch finishes (0: it does nothing)
     unsigned long long extensionRays;
     unsigned long long shadowRays;
@@ -182,7 +182,20 @@ void launchShadowBatch(const BatchView& b, ShadowQueue sq, PathQueue out, Ctrl* 
 // new camera paths go to a tail launch; kPlanTailIfFew: nothing happens (and the tail launch
 // that follows does nothing) unless every camera path has started and at most tailMax paths
 // are left, which then go to the tail launch.
-enum PlanMode : int { kPlanWave = 0, kPlanTail = 1, kPlanTailIfFew = 2 };
+// A wavefront iteration also hands the shadow rays of the last shade launch to launchShadow;
+// kPlanShadow does only that.
+enum PlanMode : int { kPlanWave = 0, kPlanTail = 1, kPlanTailIfFew = 2, kPlanShadow = 3 };
+// A second stream for the launches that run beside others, with its two events.
+struct SideLane {
+    cudaStream_t stream = nullptr;
+    cudaEvent_t fork = nullptr, join = nullptr;
+    bool create();
+    void destroy();
+    // Work of `stream` starts after what `s` has enqueued; and `s` goes on after it.
+    void begin(cudaStream_t s) const { cudaEventRecord(fork, s); cudaStreamWaitEvent(stream, fork, 0); }
+    void end() const { cudaEventRecord(join, stream); }
+    void wait(cudaStream_t s) const { cudaStreamWaitEvent(s, join, 0); }
+};
 void launchPlan(Ctrl* ctrl, unsigned int capacity, cudaStream_t s, int mode = kPlanWave, unsigned int tailMax = 0);
 // Paths up to which a tail launch beats the remaining wavefront iterations. Measured with
 // 4,096 / 16,384 / 65,536 / 131,072 paths (none: no tail launches), ms per call: occluded
@@ -197,7 +210,7 @@ void launchTail(const SceneDev& sc, const RenderParams& rp, PathQueue in, PathQu
 void launchGenerate(const SceneDev& sc, const RenderParams& rp, PathQueue q, Ctrl* ctrl, int grid, cudaStream_t s);
 // Extension / shadow rays and shading of the wavefront; grids sized from the
 // launched kernel's occupancy on numSMs SMs (one full wave).
-// retrace: room for one number per path in the queue (the shadow queue, which is empty then).
+// retrace: room for one number per path in the queue (the output queue, which is empty then).
 void launchExtend(const SceneDev& sc, PathQueue q, HitQueue h, unsigned int* retrace, Ctrl* ctrl, int numSMs, bool count,
                   cudaStream_t s);
 void launchShade(const SceneDev& sc, const RenderParams& rp, PathQueue in, HitQueue h, PathQueue out, ShadowQueue sq,
@@ -208,7 +221,7 @@ void launchShadow(const SceneDev& sc, const RenderParams& rp, ShadowQueue sq, Pa
 void launchPackFilm(const void* film, int fp64, size_t n, int strideFloats, float* out, int grid, cudaStream_t s);
 // Ray queries on a built scene: rays of 7 floats (o, d, tMax); closest hits as 5 floats per ray
 // (t, instance, triangle, b0, b1; -1 for none) or any-hit flags. ctrl: zero but for nActive
-// and nShadow = n.
+// and nShadowDue = n.
 void launchQuery(const SceneDev& sc, const float* rays, int n, int any, float* hits, int* occluded, Ctrl* ctrl, int numSMs,
                  cudaStream_t s);
 
