@@ -1227,9 +1227,12 @@ xgb_status xgb_scene_build(xgb_scene* s, void* stream) {
         sd.kinds |= 1 << m.kind;
     }
     sd.instBox = dBox;
-    sd.world = WorldDev{};
     long long totalTris = 0;
     for (const SceneObject& o : s->objects) totalTris += o.mesh->nTris;
+    const float diag = (sceneBox.hi[0] - sceneBox.lo[0]) + (sceneBox.hi[1] - sceneBox.lo[1]) + (sceneBox.hi[2] - sceneBox.lo[2]);
+    sd.tieAbs = std::isfinite(diag) ? diag * 0x1p-22f : 0.0f;
+    sd.teams = blasLayout == 0 && std::isfinite(diag) && totalTris >= kTeamMinTris;
+    sd.world = WorldDev{};
     constexpr long long kWorldMinTris = 4096;  // of few instances, only large scenes gain (trace.cu::useWorld)
     if (blasLayout == 0 && inst.size() == 1) {
         const xgb_mesh* m = s->objects[0].mesh;
@@ -1270,9 +1273,7 @@ xgb_status xgb_scene_build(xgb_scene* s, void* stream) {
             }
             XGB_CUDA(ctx, cudaGetLastError());
             XGB_CUDA(ctx, cudaStreamSynchronize(st));  // `top` is read by the copy
-            const float diag = (sceneBox.hi[0] - sceneBox.lo[0]) + (sceneBox.hi[1] - sceneBox.lo[1]) +
-                               (sceneBox.hi[2] - sceneBox.lo[2]);
-            sd.world = WorldDev{wn, wt, 0, enters, 1.0f + 0x1p-19f, std::isfinite(diag) ? diag * 0x1p-22f : 0.0f};
+            sd.world = WorldDev{wn, wt, 0, enters, 1.0f + 0x1p-19f, sd.tieAbs};
         } else {
             cudaGetLastError();
         }
@@ -1578,10 +1579,10 @@ xgb_status xgb_render(xgb_scene* s, const xgb_integrator_params* params, xgb_fil
             const bool beside = side.lane.stream && k > 0;
             if (beside) {
                 side.lane.begin(st);
-                launchShadow(s->sd, rp, s->rb.shadow, X, s->ctrl, ctx->numSMs, side.lane.stream);
+                launchShadow(s->sd, rp, s->rb.shadow, X, s->ctrl, ctx->numSMs, !tail && !prof, side.lane.stream);
                 side.lane.end();
             }
-            launchExtend(s->sd, X, s->rb.hits, (unsigned int*)Y.o, s->ctrl, ctx->numSMs, prof, st);
+            launchExtend(s->sd, X, s->rb.hits, (unsigned int*)Y.o, s->ctrl, ctx->numSMs, prof, !tail && !prof, st);
             if (prof) cudaEventRecord(ev[3], st);
             if (gd) {
                 guideInferPaths(s->sd, gd->g, gb, X, s->rb.hits, s->ctrl, s->mix, gShade, st);
@@ -1593,7 +1594,7 @@ xgb_status xgb_render(xgb_scene* s, const xgb_integrator_params* params, xgb_fil
             if (prof) cudaEventRecord(ev[5], st);
             if (shadows && (!side.lane.stream || k + 1 == nIter)) {
                 launchPlan(s->ctrl, cap, st, kPlanShadow);
-                launchShadow(s->sd, rp, s->rb.shadow, Y, s->ctrl, ctx->numSMs, st);
+                launchShadow(s->sd, rp, s->rb.shadow, Y, s->ctrl, ctx->numSMs, !tail && !prof, st);
                 ++launches;
             }
             if (prof) cudaEventRecord(ev[6], st);

@@ -155,13 +155,13 @@ extern "C" xgb_status xgb_render_noalloc(xgb_scene* scene, const xgb_integrator_
             PathQueue& Y = q[parity ^ 1];
             launchPlan(ctrl, cap, st);
             launchGenerate(sd, rp, X, ctrl, gShade, st);
-            if (k > 0) launchShadow(sd, rp, sq, X, ctrl, numSMs, st);  // of the last vertex
-            launchExtend(sd, X, hits, (unsigned int*)Y.o, ctrl, numSMs, false, st);
+            if (k > 0) launchShadow(sd, rp, sq, X, ctrl, numSMs, true, st);  // of the last vertex
+            launchExtend(sd, X, hits, (unsigned int*)Y.o, ctrl, numSMs, false, true, st);
             launchShade(sd, rp, X, hits, Y, sq, ctrl, numSMs, st);
             parity ^= 1;
         }
         launchPlan(ctrl, cap, st, kPlanShadow);
-        launchShadow(sd, rp, sq, q[parity], ctrl, numSMs, st);
+        launchShadow(sd, rp, sq, q[parity], ctrl, numSMs, true, st);
         if (cudaGetLastError() != cudaSuccess) return XGB_CUDA_ERROR;
         if (cudaMemcpyAsync(&host, ctrl, sizeof(Ctrl), cudaMemcpyDeviceToHost, st) != cudaSuccess) return XGB_CUDA_ERROR;
         if (cudaStreamSynchronize(st) != cudaSuccess) return XGB_CUDA_ERROR;

@@ -105,6 +105,7 @@ struct OneScene {
     RenderParams rp;
     __device__ __forceinline__ int jobOf(unsigned int) const { return 0; }
     __device__ __forceinline__ int pixelOf(unsigned int packed) const { return (int)packed; }
+    __device__ __forceinline__ bool teams() const { return sc.teams != 0; }
     __device__ __forceinline__ const SceneDev& scene(int) const { return sc; }
     __device__ __forceinline__ const RenderParams& params(int) const { return rp; }
 };
@@ -112,9 +113,20 @@ struct BatchScenes {
     BatchView b;
     __device__ __forceinline__ int jobOf(unsigned int packed) const { return (int)(packed >> 24); }
     __device__ __forceinline__ int pixelOf(unsigned int packed) const { return (int)(packed & 0xFFFFFFu); }
+    __device__ __forceinline__ bool teams() const { return b.teams != 0; }
     __device__ __forceinline__ const SceneDev& scene(int j) const { return b.scenes[j]; }
     __device__ __forceinline__ const RenderParams& params(int j) const { return b.params[j]; }
 };
+// What an unoccluded shadow ray does.
+template <class S>
+__device__ __forceinline__ void shadowLit(const S& scenes, int job, ShadowQueue s, PathQueue out, unsigned int ray) {
+    const float4 cc = s.c[ray];
+    const RenderParams& rp = scenes.params(job);
+    filmAdd(rp, scenes.pixelOf(__float_as_uint(s.d[ray].w)), V3(cc.x, cc.y, cc.z));
+    const int target = __float_as_int(cc.w);
+    if (target >= 0) out.rng[target] = s.rng[ray];
+    if (rp.train) creditPath(rp, s.pid[ray], cc);
+}
 // Ray queries on a scene of one instance (xgb_scene_intersect / xgb_scene_occluded): the rays
 // and results are the caller's rows, 7 floats (o, d, tMax) and 5 (t, instance, triangle, b0,
 // b1; -1 for none) or a flag.
@@ -124,6 +136,7 @@ struct QueryRays {
     float* hits;
     int* occluded;
     __device__ __forceinline__ int jobOf(unsigned int) const { return 0; }
+    __device__ __forceinline__ bool teams() const { return false; }
     __device__ __forceinline__ const SceneDev& scene(int) const { return sc; }
 };
 
@@ -377,6 +390,7 @@ template <bool ANY, bool COUNT, class S, bool SHELL = false>
 __global__ void __launch_bounds__(kTraceBlock) k_trace_flat2(S scenes, PathQueue q, HitQueue h, ShadowQueue s,
                                                             PathQueue out, Ctrl* ctrl) {
     const unsigned int n = ANY ? ctrl->nShadowDue : ctrl->nActive;
+    if (n <= kTeamQueue && scenes.teams()) return;  // k_trace_team's
     unsigned int* head = ANY ? &ctrl->shadowHead : &ctrl->extendHead;
     constexpr bool kBatch = !std::is_same<S, OneScene>::value;
     int rayMaxSteps = 0, rayStack = 0;  // a batch: the current ray's job's bounds
@@ -440,14 +454,7 @@ __global__ void __launch_bounds__(kTraceBlock) k_trace_flat2(S scenes, PathQueue
             if (ANY && occluded) inst = nInst;
             if (inst >= nInst) {  // ray finished
                 if (ANY) {
-                    if (!occluded) {
-                        float4 cc = s.c[ray];
-                        const RenderParams& rp = scenes.params(job);
-                        filmAdd(rp, scenes.pixelOf(__float_as_uint(s.d[ray].w)), V3(cc.x, cc.y, cc.z));
-                        int target = __float_as_int(cc.w);
-                        if (target >= 0) out.rng[target] = s.rng[ray];
-                        if (rp.train) creditPath(rp, s.pid[ray], cc);
-                    }
+                    if (!occluded) shadowLit(scenes, job, s, out, ray);
                 } else {
                     __stcs(&h.h[ray], make_float4(hit.prim >= 0 ? hit.t : tMax, hit.b0, hit.b1, __int_as_float(hit.prim)));
                     __stcs(&h.inst[ray], hit.inst);
@@ -585,6 +592,7 @@ __global__ void __launch_bounds__(kTraceBlock, (WorldTraits<S, ENTER>::kMinBlock
     k_trace_world(S scenes, PathQueue q, HitQueue h, unsigned int* retrace, ShadowQueue s, PathQueue out, Ctrl* ctrl) {
     constexpr bool kBatch = std::is_same<S, BatchScenes>::value, kQuery = std::is_same<S, QueryRays>::value;
     const unsigned int n = ANY ? ctrl->nShadowDue : ctrl->nActive;
+    if (n <= kTeamQueue && scenes.teams()) return;  // k_trace_team's
     unsigned int* head = ANY ? &ctrl->shadowHead : &ctrl->extendHead;
     RayClaims claims(head, n);
     const int looking = claims.lanes == 32u ? kLookingLanes<SHELL> : 1;
@@ -766,14 +774,7 @@ __global__ void __launch_bounds__(kTraceBlock, (WorldTraits<S, ENTER>::kMinBlock
             if constexpr (kQuery && ANY) {
                 scenes.occluded[ray] = occluded ? 1 : 0;
             } else if constexpr (ANY) {
-                if (!occluded) {
-                    float4 cc = s.c[ray];
-                    const RenderParams& rp = scenes.params(job);
-                    filmAdd(rp, scenes.pixelOf(__float_as_uint(s.d[ray].w)), V3(cc.x, cc.y, cc.z));
-                    int target = __float_as_int(cc.w);
-                    if (target >= 0) out.rng[target] = s.rng[ray];
-                    if (rp.train) creditPath(rp, s.pid[ray], cc);
-                }
+                if (!occluded) shadowLit(scenes, job, s, out, ray);
             } else {
                 int prim = -1, of = -1;
                 if (hitTri >= 0) {
@@ -838,6 +839,46 @@ __global__ void __launch_bounds__(kTraceBlock) k_retrace(S scenes, PathQueue q, 
         h.h[ray] = make_float4(hit.t, hit.b0, hit.b1, __int_as_float(hit.prim));
         h.inst[ray] = hit.inst;
     }
+}
+
+// Launches of at most kTeamQueue rays: a ray for each team of lanes, up to kTeamRays per warp.
+// Such a launch is bound by the chain of node fetches of its longest ray, which 32 lanes
+// shorten: the occluded room with the proposal (256^2 x 8, whose last thirty iterations are such
+// launches) 10.9 -> 9.15 ms per call, a batch of 8 9.93 -> 9.87.
+template <bool ANY, class S>
+__global__ void __launch_bounds__(kTraceBlock, 6) k_trace_team(const __grid_constant__ S scenes, PathQueue q, HitQueue h,
+                                                               ShadowQueue s, PathQueue out, Ctrl* ctrl) {
+    __shared__ uint2 sStacks[kTraceBlock / 32][kTeamEntries];
+    const unsigned int n = ANY ? ctrl->nShadowDue : ctrl->nActive;
+    if (n == 0 || n > kTeamQueue || !scenes.teams()) return;
+    const unsigned int warps = gridDim.x * (kTraceBlock / 32), lane = threadIdx.x & 31;
+    const unsigned int teams = n <= warps ? 1u : n <= 2u * warps ? 2u : kTeamRays;
+    for (;;) {
+        unsigned int base = 0;
+        if (lane == 0) base = atomicAdd(ANY ? &ctrl->shadowHead : &ctrl->extendHead, teams);
+        base = __shfl_sync(kWarp, base, 0);
+        if (base >= n) break;
+        const unsigned int k = base + lane / (32u / teams);
+        const bool has = k < n;
+        const unsigned int ray = has ? k : base;
+        const float4 o = ANY ? s.o[ray] : q.o[ray], d = ANY ? s.d[ray] : q.d[ray];
+        const int job = scenes.jobOf(ANY ? __float_as_uint(d.w) : __float_as_uint(q.thr[ray].w));
+        TraceHit hit;
+        const bool mine = traceTeam(scenes.scene(job), has, V3(o.x, o.y, o.z), V3(d.x, d.y, d.z),
+                                    ANY ? o.w : __int_as_float(0x7f800000), ANY, 32u / teams, sStacks[threadIdx.x >> 5], hit,
+                                    &ctrl->errors);
+        if (mine) {
+            if constexpr (ANY) {
+                if (hit.prim < 0) shadowLit(scenes, job, s, out, ray);
+            } else {
+                h.h[ray] = make_float4(hit.t, hit.b0, hit.b1, __int_as_float(hit.prim));
+                h.inst[ray] = hit.inst;
+            }
+        }
+        __syncwarp();
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0)
+        atomicAdd(ANY ? &ctrl->shadowRays : &ctrl->extensionRays, (unsigned long long)n);
 }
 
 // ---- batches of scenes (xgb_render_batch) -----------------------------------------
@@ -957,6 +998,18 @@ static bool useWorld(const SceneDev& sc, bool any) {
     return (any || sc.nInstances > kFlatInstances) && sc.maxSteps == kDefaultMaxSteps && sc.stackLimit == kMaxStackLimit;
 }
 #define XGB_LAUNCH(K) K<<<persistentGrid(K, numSMs), kTraceBlock, 0, s>>>
+// Traversal limits other than the defaults count the steps of the kernels below.
+static SceneDev withTeams(const SceneDev& sc, bool any, bool teams) {
+    SceneDev r = sc;
+    r.teams = sc.teams && teams && sc.maxSteps == kDefaultMaxSteps && sc.stackLimit == kMaxStackLimit &&
+              (sc.nInstances <= kFlatInstances || useWorld(sc, any));
+    return r;
+}
+int batchTeams(const SceneDev* scenes, int n) {
+    bool teams = true;
+    for (int j = 0; j < n; ++j) teams = teams && withTeams(scenes[j], false, true).teams;
+    return teams && batchKernels(scenes, n) != kBatchGeneral;
+}
 constexpr int kRetraceBlocks = 152;  // a launch that usually finds a handful of rays
 template <bool ANY, bool COUNT>
 static void launchWorld(const SceneDev& sc, const RenderParams& rp, PathQueue q, HitQueue h, unsigned int* retrace,
@@ -971,8 +1024,10 @@ static void launchWorld(const SceneDev& sc, const RenderParams& rp, PathQueue q,
     }
     if (!ANY && sc.nInstances > 1) k_retrace<OneScene><<<kRetraceBlocks, kTraceBlock, 0, s>>>(one, q, h, retrace, ctrl);
 }
-void launchExtend(const SceneDev& sc, PathQueue q, HitQueue h, unsigned int* retrace, Ctrl* ctrl, int numSMs, bool count,
-                  cudaStream_t s) {
+void launchExtend(const SceneDev& scene, PathQueue q, HitQueue h, unsigned int* retrace, Ctrl* ctrl, int numSMs, bool count,
+                  bool teams, cudaStream_t s) {
+    const SceneDev sc = withTeams(scene, false, teams && !count);
+    if (sc.teams) XGB_LAUNCH((k_trace_team<false, OneScene>))(OneScene{sc, RenderParams{}}, q, h, ShadowQueue{}, PathQueue{}, ctrl);
     RenderParams none{};
     const bool flat = sc.nInstances <= kFlatInstances;
     if (useWorld(sc, false)) {
@@ -1003,8 +1058,10 @@ void launchExtend(const SceneDev& sc, PathQueue q, HitQueue h, unsigned int* ret
         XGB_LAUNCH((k_extend<false>))(sc, q, h, ctrl);
     }
 }
-void launchShadow(const SceneDev& sc, const RenderParams& rp, ShadowQueue sq, PathQueue out, Ctrl* ctrl, int numSMs,
-                  cudaStream_t s) {
+void launchShadow(const SceneDev& scene, const RenderParams& rp, ShadowQueue sq, PathQueue out, Ctrl* ctrl, int numSMs,
+                  bool teams, cudaStream_t s) {
+    const SceneDev sc = withTeams(scene, true, teams);
+    if (sc.teams) XGB_LAUNCH((k_trace_team<true, OneScene>))(OneScene{sc, rp}, PathQueue{}, HitQueue{}, sq, out, ctrl);
     const bool flat = sc.nInstances <= kFlatInstances;
     if (useWorld(sc, true)) {
         launchWorld<true, false>(sc, rp, PathQueue{}, HitQueue{}, nullptr, sq, out, ctrl, numSMs, s);
@@ -1041,6 +1098,7 @@ int batchKernels(const SceneDev* scenes, int n) {
 void launchExtendBatch(const BatchView& b, PathQueue q, HitQueue h, unsigned int* retrace, Ctrl* ctrl, int numSMs,
                        cudaStream_t s) {
     const BatchScenes sc{b};
+    if (b.teams) XGB_LAUNCH((k_trace_team<false, BatchScenes>))(sc, q, h, ShadowQueue{}, PathQueue{}, ctrl);
     switch (b.kernels) {
     case kBatchWorld:
     case kBatchWorldEnter:
@@ -1056,6 +1114,7 @@ void launchExtendBatch(const BatchView& b, PathQueue q, HitQueue h, unsigned int
 }
 void launchShadowBatch(const BatchView& b, ShadowQueue sq, PathQueue out, Ctrl* ctrl, int numSMs, cudaStream_t s) {
     const BatchScenes sc{b};
+    if (b.teams) XGB_LAUNCH((k_trace_team<true, BatchScenes>))(sc, PathQueue{}, HitQueue{}, sq, out, ctrl);
     switch (b.kernels) {
     case kBatchWorld:
     case kBatchFlatWorldShadow: XGB_LAUNCH((k_trace_world<true, false, BatchScenes, false, false>))(sc, PathQueue{}, HitQueue{}, nullptr, sq, out, ctrl); break;

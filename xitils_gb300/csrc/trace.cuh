@@ -508,6 +508,172 @@ static __device__ __noinline__ bool traceCall(const SceneDev& sc, V3 o, V3 d, fl
     }
 }
 
+// ---- a ray for several lanes -------------------------------------------------------
+// Some rays take twenty times as long as the average one (grazing rays through the occluded
+// room: 0.3 ms next to 31 others in a warp), and a launch lasts as long as its slowest. In
+// launches of few rays the lanes of a team share one ray's traversal.
+constexpr unsigned int kLanes = 0xFFFFFFFFu;
+constexpr unsigned int kTeamRays = 4;  // teams per warp, at most
+// Entries of a warp's shared stacks, 512 / teams each: a node or leaf code and the instance
+// it is in (-1: a node or leaf of the top level).
+constexpr unsigned int kTeamEntries = 512;
+// Room that a depth-first descent needs: the stacks of the sequential traversal.
+constexpr unsigned int kTeamReserve = kStackDepth + kTlasStack;
+static_assert(kTeamEntries / kTeamRays > kTeamReserve + (unsigned int)kFlatInstances, "a team's stack");
+
+// One ray per team of `size` lanes (a power of two, at least 32 / kTeamRays; every lane of the
+// warp calls with its team's ray, or with has = false). The team's lanes take up to `size`
+// entries off its stack at a time, the nearest first, test them side by side, and push
+// the children that the ray reaches. Near its capacity the stack is taken one entry at a
+// time, depth first. One lane of each team with a ray returns true, with the result (any:
+// prim 0, or -1 for no hit).
+//
+// The nearest of all accepted hits is the sequential traversal's, unless another one lies
+// within rounding of it, where the order decides: then the ray is traced again in
+// order (traceCall), from that distance. Boxes are visited up to that margin beyond the
+// nearest hit.
+static __device__ __noinline__ bool traceTeam(const SceneDev& sc, bool has, V3 o, V3 d, float reach, bool any, unsigned int size,
+                                              uint2* stacks, TraceHit& out, unsigned int* errors) {
+    const unsigned int lane = threadIdx.x & 31, rank = lane & (size - 1u), team = lane / size;
+    const unsigned int mates = (size == 32u ? kLanes : (1u << size) - 1u) << (lane - rank);
+    const unsigned int below = mates & ~((2u << lane) - 1u);  // ranks after this lane's
+    const unsigned int cap = kTeamEntries / (32u / size);
+    uint2* const stack = stacks + team * cap;
+    const BoxRay br{o.x, o.y, o.z, 1.0f / d.x, 1.0f / d.y, 1.0f / d.z};
+    const WRay wr = makeWRay(o, d);
+    WRay r = wr;
+    float best = INFINITY, other = INFINITY;  // this lane's nearest hit, and its next one
+    float b0 = 0.0f, b1 = 0.0f;
+    int prim = -1, hitInst = -1;
+    const float start = reach;
+    int inst = -1;
+    const Node2* nodes = nullptr;
+    const TriV* tris = nullptr;
+    const MeshDev* mesh = nullptr;
+    unsigned int count = 0;
+    if (has) {
+        if (sc.nInstances <= kFlatInstances) {
+            count = (unsigned int)sc.nInstances;
+            for (unsigned int k = rank; k < count; k += size) stack[count - 1u - k] = make_uint2((unsigned int)leafEncode((int)k, 1), ~0u);
+        } else {
+            count = 1;
+            if (rank == 0) stack[0] = make_uint2(0u, ~0u);
+        }
+    }
+    __syncwarp();
+    for (int guard = 0; __any_sync(kLanes, count > 0); ++guard) {
+        if (guard > sc.maxSteps) {
+            if (lane == 0) atomicOr(errors, 4u);
+            break;
+        }
+        // a full stack: one entry at a time
+        unsigned int take = min(count, size);
+        if (count + take + kTeamReserve > cap) take = min(count, 1u);
+        const bool work = rank < take;
+        uint2 e = make_uint2(0u, 0u);
+        if (work) e = stack[count - 1u - rank];
+        count -= take;
+        __syncwarp();
+        unsigned int pushes = 0;
+        uint2 near = make_uint2(0u, 0u), far = near;
+        bool found = false;
+        if (work) {
+            const int code = (int)e.x;
+            if ((int)e.y < 0 && code < 0) {  // an instance
+                const int k = leafFirst(code);
+                if (instBoxHit(br, sc.instBox, k, reach)) {
+                    const MeshDev& m = sc.meshes[sc.instances[k].mesh];
+                    near = make_uint2(m.rootIsLeaf ? (unsigned int)m.rootLeaf : 0u, (unsigned int)k);
+                    pushes = 1;
+                }
+            } else {
+                const bool top = (int)e.y < 0;
+                if (!top && (int)e.y != inst) {
+                    inst = (int)e.y;
+                    const Instance& in = sc.instances[inst];
+                    mesh = &sc.meshes[in.mesh];
+                    nodes = mesh->nodes2;
+                    tris = mesh->tris;
+                    if (in.identity) r = wr;
+                    else r = makeWRay(xformPointRn(in.matInv, o), xformVectorRn(in.matInv, d));
+                }
+                if (code >= 0) {
+                    const NodeHits h = slabs((top ? sc.tlas : nodes) + code, top ? wr : r, reach);
+                    const bool second = !h.h0 || (h.h1 && h.t1 < h.t0);
+                    pushes = (h.h0 ? 1u : 0u) + (h.h1 ? 1u : 0u);
+                    near = make_uint2((unsigned int)(second ? h.child.y : h.child.x), e.y);
+                    far = make_uint2((unsigned int)(second ? h.child.x : h.child.y), e.y);
+                } else {
+                    const int first = leafFirst(code), cnt = leafCount(code);
+                    for (int k = 0; k < cnt; ++k) {
+                        const TriV* tv = tris + first + k;
+                        const float4 p0 = __ldg(&tv->p0), p1 = __ldg(&tv->p1), p2 = __ldg(&tv->p2);
+                        float t, c0, c1;
+                        if (!watertight(r, p0, p1, p2, reach, t, c0, c1)) continue;
+                        if (mesh->shellLayers && shellDiscard(*mesh, __float_as_int(p0.w), c0, c1)) continue;
+                        found = true;
+                        if (any) {
+                            best = 0.0f;
+                            prim = 0;
+                            break;
+                        }
+                        if (!(t < INFINITY)) other = -1.0f;  // left to the sequential traversal
+                        if (t < best) {
+                            other = fminf(other, best);
+                            best = t;
+                            b0 = c0;
+                            b1 = c1;
+                            prim = __float_as_int(p0.w);
+                            hitInst = inst;
+                        } else {
+                            other = fminf(other, t);
+                        }
+                    }
+                }
+            }
+        }
+        const unsigned int m1 = __ballot_sync(kLanes, pushes >= 1u), m2 = __ballot_sync(kLanes, pushes == 2u);
+        unsigned int at = count + __popc(m1 & below) + __popc(m2 & below);
+        count += __popc(m1 & mates) + __popc(m2 & mates);
+        if (count > cap) {  // a descent deeper than the sequential traversal's stacks
+            if (pushes) atomicOr(errors, 1u);
+            count = 0;
+        } else {
+            if (pushes == 2u) stack[at++] = far;
+            if (pushes >= 1u) stack[at] = near;
+        }
+        const unsigned int hits = __ballot_sync(kLanes, found);
+        if (hits) {
+            float t = best;
+            for (unsigned int k = size >> 1; k; k >>= 1) t = fminf(t, __shfl_xor_sync(kLanes, t, k));
+            if (!any) reach = fminf(reach, fmaf(t, 1.0f + 0x1p-19f, sc.tieAbs));
+            else if (hits & mates) count = 0;
+        }
+        __syncwarp();
+    }
+    // the team's nearest hit
+    float t = best;
+    for (unsigned int k = size >> 1; k; k >>= 1) t = fminf(t, __shfl_xor_sync(kLanes, t, k));
+    const bool hit = t < INFINITY;
+    const unsigned int owners = __ballot_sync(kLanes, hit && best == t) & mates;
+    const bool owner = owners && lane == (unsigned int)__ffs(owners) - 1u;
+    const float margin = fmaf(t, 1.0f + 0x1p-19f, sc.tieAbs);
+    const bool close = (hit && !owner && best <= margin) || (other < INFINITY && other <= margin);
+    const bool tie = (__ballot_sync(kLanes, !any && close) & mates) != 0u;
+    if (!has || !(hit ? owner : rank == 0)) return false;
+    out.t = hit ? t : start;
+    out.b0 = b0;
+    out.b1 = b1;
+    out.prim = prim;
+    out.inst = hitInst;
+    if (tie) {
+        out.b0 = out.b1 = 0.0f;
+        traceCall(sc, o, d, fminf(start, margin), false, out, errors);
+        if (out.prim < 0) out.t = start;
+    }
+    return true;
+}
+
 // Scene::intersect (ANY = false) / Scene::intersectAny (ANY = true).
 template <bool ANY, bool COUNT = false>
 __device__ __forceinline__ bool traceScene(const SceneDev& sc, V3 o, V3 d, float tMax, TraceHit& hit,

@@ -168,8 +168,10 @@ struct BatchView {
     const unsigned long long* start;  // nJobs + 1 prefix sums of the jobs' path counts
     int nJobs;
     int kernels; // BatchKernels
-    int nested;  // some scene has a material that evaluates another (the shade kernel with that code)
+    int nested;
+    int teams;  // small queues go to teams of lanes  // some scene has a material that evaluates another (the shade kernel with that code)
 };
+int batchTeams(const SceneDev* scenes, int n);
 int batchKernels(const SceneDev* scenes, int n);
 void launchGenerateBatch(const BatchView& b, PathQueue q, Ctrl* ctrl, int grid, cudaStream_t s);
 void launchShadeBatch(const BatchView& b, PathQueue in, HitQueue h, PathQueue out, ShadowQueue sq, Ctrl* ctrl,
@@ -210,13 +212,15 @@ void launchTail(const SceneDev& sc, const RenderParams& rp, PathQueue in, PathQu
 void launchGenerate(const SceneDev& sc, const RenderParams& rp, PathQueue q, Ctrl* ctrl, int grid, cudaStream_t s);
 // Extension / shadow rays and shading of the wavefront; grids sized from the
 // launched kernel's occupancy on numSMs SMs (one full wave).
+// teams: whether small queues go to teams of lanes, where the scene allows it (not where a tail
+// launch takes over before a queue gets that small).
 // retrace: room for one number per path in the queue (the output queue, which is empty then).
-void launchExtend(const SceneDev& sc, PathQueue q, HitQueue h, unsigned int* retrace, Ctrl* ctrl, int numSMs, bool count,
+void launchExtend(const SceneDev& sc, PathQueue q, HitQueue h, unsigned int* retrace, Ctrl* ctrl, int numSMs, bool count, bool teams,
                   cudaStream_t s);
 void launchShade(const SceneDev& sc, const RenderParams& rp, PathQueue in, HitQueue h, PathQueue out, ShadowQueue sq,
                  Ctrl* ctrl, int numSMs, cudaStream_t s);
 void launchShadow(const SceneDev& sc, const RenderParams& rp, ShadowQueue sq, PathQueue out, Ctrl* ctrl, int numSMs,
-                  cudaStream_t s);
+                  bool teams, cudaStream_t s);
 // Film plane (float4 or double4 per pixel) -> packed float RGB, strideFloats 3 or 4 (image.cu).
 void launchPackFilm(const void* film, int fp64, size_t n, int strideFloats, float* out, int grid, cudaStream_t s);
 // Ray queries on a built scene: rays of 7 floats (o, d, tMax); closest hits as 5 floats per ray

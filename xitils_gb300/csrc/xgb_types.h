@@ -174,6 +174,13 @@ struct WorldDev {
     float cullMul, cullAbs;
 };
 
+// Launches of at most kTeamQueue rays, in scenes whose rays can take long, go to teams: with
+// 6,000 / 16,384 / 40,000 the occluded room with the proposal took 9.41 / 9.15 / 9.05 ms per call;
+// 19,000 rays of a full launch took 0.29 ms, what the per-lane kernels need for 200,000.
+constexpr unsigned int kTeamQueue = 16384;
+// Rays of a small scene take few steps: rooms of 742 / 3,022 / 6,022 / 18,022 triangles with the
+// proposal, 120 x 100 x 4, per-lane kernels 2.53 / 2.46 / 2.85 / 3.45 ms, teams 2.83 / 2.60 / 2.82 / 3.10.
+constexpr long long kTeamMinTris = 6000;
 constexpr int kDefaultMaxSteps = 1 << 22;
 constexpr int kMaxStackLimit = 64;
 
@@ -195,6 +202,10 @@ struct SceneDev {
     int maxSteps;
     int stackLimit;
     const float4* instBox;  // per instance: world box lo (xyz), hi (xyz) as 2 float4
+    // 1: the rays of a small queue may be traced by teams of lanes (trace.cuh::traceTeam). Two hits
+    // of a ray within tieAbs (plus 2^-19 of the distance) of each other may be decided by their order.
+    int teams;
+    float tieAbs;
     WorldDev world;
     const Material* materials;
     const TextureDev* textures;
