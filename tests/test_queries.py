@@ -46,3 +46,22 @@ def test_one_instance_equals_two(scenes_of, n, moved):
     occ = one.scene.occluded(rays)
     np.testing.assert_array_equal(occ, two.scene.occluded(rays))
     np.testing.assert_array_equal(occ != 0, a[:, 2] >= 0)
+
+
+def test_limits_count_every_step(scenes_of):
+    """With a limit on the steps a one-instance scene refuses what a two-instance scene
+    refuses: a tree of 18,000 triangles cannot be descended in ten nodes and leaves."""
+    from xitils_gb300 import api
+
+    rng = np.random.default_rng(0)
+    o = rng.uniform((0.2, 1.0, 0.2), (0.8, 1.0, 0.8), (64, 3))
+    rays = np.concatenate([o, np.tile([0.0, -1.0, 0.0], (64, 1)), np.full((64, 1), np.inf)], axis=1).astype(np.float32)
+    for b in scenes_of[False]:
+        want = b.scene.intersect(rays)
+        try:
+            b.scene.set_traversal_limits(max_steps=10)
+            with pytest.raises(api.XgbError):
+                b.scene.intersect(rays)
+        finally:
+            b.scene.set_traversal_limits(0, 0)
+        np.testing.assert_array_equal(b.scene.intersect(rays), want)

@@ -1125,10 +1125,12 @@ void launchShadowBatch(const BatchView& b, ShadowQueue sq, PathQueue out, Ctrl* 
 }
 
 // One instance takes the persistent per-lane kernel: 300,000 closest hits on a terrain of
-// 520,000 triangles 0.63 -> 0.57 ms for the whole call, most of it copies.
+// 520,000 triangles 0.63 -> 0.57 ms for the whole call, most of it copies. Traversal limits
+// other than the defaults count traceScene's steps, one per node and leaf.
 void launchQuery(const SceneDev& sc, const float* rays, int n, int any, float* hits, int* occluded, Ctrl* ctrl, int numSMs,
                  cudaStream_t s) {
-    if (sc.nInstances == 1 && sc.world.tris && !sc.shell) {
+    const bool limits = sc.maxSteps != kDefaultMaxSteps || sc.stackLimit != kMaxStackLimit;
+    if (sc.nInstances == 1 && sc.world.tris && !sc.shell && !limits) {
         const QueryRays in{sc, rays, hits, occluded};
         if (any)
             XGB_LAUNCH((k_trace_world<true, false, QueryRays, false, false>))(in, PathQueue{}, HitQueue{}, nullptr, ShadowQueue{}, PathQueue{}, ctrl);
