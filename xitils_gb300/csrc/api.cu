@@ -1231,7 +1231,8 @@ xgb_status xgb_scene_build(xgb_scene* s, void* stream) {
     for (const SceneObject& o : s->objects) totalTris += o.mesh->nTris;
     const float diag = (sceneBox.hi[0] - sceneBox.lo[0]) + (sceneBox.hi[1] - sceneBox.lo[1]) + (sceneBox.hi[2] - sceneBox.lo[2]);
     sd.tieAbs = std::isfinite(diag) ? diag * 0x1p-22f : 0.0f;
-    sd.teams = blasLayout == 0 && std::isfinite(diag) && totalTris >= kTeamMinTris;
+    sd.large = totalTris >= kTeamMinTris;
+    sd.teams = blasLayout == 0 && std::isfinite(diag) && sd.large;
     sd.world = WorldDev{};
     constexpr long long kWorldMinTris = 4096;  // of few instances, only large scenes gain (trace.cu::useWorld)
     if (blasLayout == 0 && inst.size() == 1) {

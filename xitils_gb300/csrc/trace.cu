@@ -332,27 +332,29 @@ constexpr int kLookingLanes = SHELL ? 1 : 4;
 constexpr unsigned int kWarp = 0xFFFFFFFFu;
 // A warp takes new rays when this many of its lanes are without one (or all are). Taking
 // each as soon as a lane is free stalls the other lanes for an atomic and two loads from
-// DRAM each time, and mixes rays that started together: with 1 / 8 / 16 / 24 lanes the
-// terrain's render took 38.7 / 37.5 / 35.0 / 34.7 ms (a pixel's samples stay in one warp),
-// the Cornell box's 4.51 / 4.48 / 4.45 / 4.28, the batch's 11.28 / 11.03 / 11.08 / 11.22, the
-// occluded room's, whose rays are the least alike, 44.5 / 44.0 / 44.1 / 45.9.
-constexpr unsigned int kFetchLanes = 16;
+// DRAM each time, and mixes rays that started together: with 1 / 8 lanes the terrain's
+// render took 38.7 / 37.5 ms, the Cornell box's 4.51 / 4.48. Rays that are alike (closest hits on one
+// BVH) or short (scenes of few triangles) wait for more lanes, 16 / 20 / 24 / 28: terrain
+// 30.9 / 30.6 / 30.5 / 30.8 ms, Cornell box 3.59 / 3.52 / 3.43 / 3.41. Elsewhere 8 / 16 / 22: occluded room
+// 37.4 / 37.8 / 38.8, shell-mapped cloth 19.3 / 19.2 / 19.2, batch 10.04 / 10.04 / 10.06.
+constexpr unsigned int kFetchLanes = 16, kFetchLanesMore = 24;
 // Rays of the queue for the lanes of a warp, in order, one atomicAdd for all that want one.
 // Every lane of the warp makes the same calls. (Claiming chunks of 32 / 64 / 128 rays ahead,
 // to save atomics, left some warps with work when the others had none: the batch took
 // 12.1 / 13.2 / 16.6 ms instead of 11.3.)
 struct RayClaims {
     unsigned int* head;
-    unsigned int n, lanes, next;
+    unsigned int n, lanes, next, fetch;
     // few rays: a warp works with its share of lanes only, so that they wait for fewer others
-    __device__ __forceinline__ RayClaims(unsigned int* h, unsigned int count) : head(h), n(count), next(0) {
+    __device__ __forceinline__ RayClaims(unsigned int* h, unsigned int count, unsigned int fetchLanes)
+        : head(h), n(count), next(0), fetch(fetchLanes) {
         const unsigned int warps = gridDim.x * (kTraceBlock / 32);
         lanes = min(32u, (n + warps - 1u) / warps);
     }
     // The lanes that want a ray (0: none, or not yet worth the trip).
     __device__ __forceinline__ unsigned int wanted(bool idle) const {
         const unsigned int m = __ballot_sync(kWarp, idle && (threadIdx.x & 31) < lanes && next < n);
-        return (unsigned int)__popc(m) >= min(kFetchLanes, lanes) ? m : 0u;
+        return (unsigned int)__popc(m) >= min(fetch, lanes) ? m : 0u;
     }
     // The next rays for the lanes of `want`; returns whether this lane got one.
     __device__ __forceinline__ bool take(unsigned int want, unsigned int* ray) {
@@ -397,7 +399,7 @@ __global__ void __launch_bounds__(kTraceBlock) k_trace_flat2(S scenes, PathQueue
     int job = 0;
     int nInst = 0;
     const int lane = threadIdx.x & 31;
-    RayClaims claims(head, n);
+    RayClaims claims(head, n, kBatch || scenes.scene(0).large ? kFetchLanes : kFetchLanesMore);
     const int looking = claims.lanes == 32u ? kLookingLanes<SHELL> : 1;
     int stack[kStackDepth];
     int sp = 0;
@@ -594,7 +596,7 @@ __global__ void __launch_bounds__(kTraceBlock, (WorldTraits<S, ENTER>::kMinBlock
     const unsigned int n = ANY ? ctrl->nShadowDue : ctrl->nActive;
     if (n <= kTeamQueue && scenes.teams()) return;  // k_trace_team's
     unsigned int* head = ANY ? &ctrl->shadowHead : &ctrl->extendHead;
-    RayClaims claims(head, n);
+    RayClaims claims(head, n, ANY ? kFetchLanes : kFetchLanesMore);
     const int looking = claims.lanes == 32u ? kLookingLanes<SHELL> : 1;
     bool holds = false;  // the lane has a ray
     // one scene: its BVH for every ray; a batch: the current ray's

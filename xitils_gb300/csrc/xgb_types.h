@@ -206,6 +206,7 @@ struct SceneDev {
     // of a ray within tieAbs (plus 2^-19 of the distance) of each other may be decided by their order.
     int teams;
     float tieAbs;
+    int large;  // 1: at least kTeamMinTris triangles over all instances
     WorldDev world;
     const Material* materials;
     const TextureDev* textures;
