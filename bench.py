@@ -52,12 +52,12 @@ L2_BYTES = 129 * 1024 * 1024
 EXTEND_BYTES_PER_RAY = 52
 # BVH traffic per visit (reported against L2, not HBM): 64 B node, 48 B triangle.
 NODE_BYTES, TRI_BYTES = 64, 48
-# DRAM bytes per extension ray of k_trace_single: dram__bytes_read.sum +
-# dram__bytes_write.sum summed over the 24 closest-hit launches of one terrain
-# render (6.98 GB for 119,571,102 rays, camera paths in runs of 64 samples of a
+# DRAM bytes per extension ray of k_trace_world: dram__bytes_read.sum +
+# dram__bytes_write.sum summed over the 18 closest-hit launches of one terrain
+# render (7.31 GB for 122,302,959 rays, camera paths in runs of 64 samples of a
 # pixel), from a one-pass ncu capture; scaled to the average launch for
 # roofline.traffic.
-EXTEND_DRAM_BYTES_PER_RAY = 58.4
+EXTEND_DRAM_BYTES_PER_RAY = 59.7
 
 
 def wavefront_bytes(paths: int, ext: int, shadow: int) -> int:
@@ -100,7 +100,7 @@ def parse():
     return p.parse_args()
 
 
-SINGLE_KERNEL = "k_trace_single (closest-hit traversal of a one-instance scene, binary BVH, persistent)"
+SINGLE_KERNEL = "k_trace_world (closest-hit traversal of a one-instance scene, binary BVH, persistent)"
 FLAT_KERNEL = "k_trace_flat2 (closest-hit traversal of a scene of <= 16 instances, binary BVHs, persistent)"
 
 

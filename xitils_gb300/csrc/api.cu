@@ -1541,7 +1541,7 @@ xgb_status xgb_render(xgb_scene* s, const xgb_integrator_params* params, xgb_fil
     }
     double stageMs[5] = {0, 0, 0, 0, 0};
     double inferMs = 0.0, trainMs = 0.0;
-    uint64_t launches = 0;
+    uint64_t launches = 0, waves = 0;
     // Tail launches (tail.cuh) instead of wavefront iterations once at most tailMax paths are
     // left: not with a learned proposal, whose inference is a launch of its own per vertex,
     // nor while profiling, which attributes every stage; traversal limits other than the
@@ -1580,10 +1580,10 @@ xgb_status xgb_render(xgb_scene* s, const xgb_integrator_params* params, xgb_fil
             const bool beside = side.lane.stream && k > 0;
             if (beside) {
                 side.lane.begin(st);
-                launchShadow(s->sd, rp, s->rb.shadow, X, s->ctrl, ctx->numSMs, !tail && !prof, side.lane.stream);
+                launches += launchShadow(s->sd, rp, s->rb.shadow, X, s->ctrl, ctx->numSMs, !tail && !prof, side.lane.stream);
                 side.lane.end();
             }
-            launchExtend(s->sd, X, s->rb.hits, (unsigned int*)Y.o, s->ctrl, ctx->numSMs, prof, !tail && !prof, st);
+            launches += launchExtend(s->sd, X, s->rb.hits, (unsigned int*)Y.o, s->ctrl, ctx->numSMs, prof, !tail && !prof, st);
             if (prof) cudaEventRecord(ev[3], st);
             if (gd) {
                 guideInferPaths(s->sd, gd->g, gb, X, s->rb.hits, s->ctrl, s->mix, gShade, st);
@@ -1595,11 +1595,12 @@ xgb_status xgb_render(xgb_scene* s, const xgb_integrator_params* params, xgb_fil
             if (prof) cudaEventRecord(ev[5], st);
             if (shadows && (!side.lane.stream || k + 1 == nIter)) {
                 launchPlan(s->ctrl, cap, st, kPlanShadow);
-                launchShadow(s->sd, rp, s->rb.shadow, Y, s->ctrl, ctx->numSMs, !tail && !prof, st);
+                launches += launchShadow(s->sd, rp, s->rb.shadow, Y, s->ctrl, ctx->numSMs, !tail && !prof, st);
                 ++launches;
             }
             if (prof) cudaEventRecord(ev[6], st);
-            launches += shadows ? 5 : 4;
+            launches += 3;  // plan, generate, shade
+            ++waves;
             parity ^= 1;
         }
         if (tail) {
@@ -1669,7 +1670,7 @@ xgb_status xgb_render(xgb_scene* s, const xgb_integrator_params* params, xgb_fil
     s->last.profiled = prof ? 1 : 0;
     for (int j = 0; j < 5; ++j) {
         s->last.kernel_ms[j] = stageMs[j];
-        s->last.stage_launches[j] = launches / 5;
+        s->last.stage_launches[j] = j < 4 || shadows ? waves : 0;
     }
     if (c.errors & ERR_STACK) return fail(ctx, XGB_QUEUE_OVERFLOW, "xgb_render: traversal stack overflow");
     if (c.errors & ERR_LOOP) return fail(ctx, XGB_DEVICE_TIMEOUT, "xgb_render: traversal iteration bound exceeded");

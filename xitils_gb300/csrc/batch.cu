@@ -250,7 +250,7 @@ xgb_status runBatch(xgb_ctx* ctx, BatchState* b, const xgb_batch_job* jobs, int 
         }
         if (replay) e = cudaGraphLaunch(b->graph, st);
         else { enqueueBlock(b, v, capR, iters, numSMs, st); e = cudaGetLastError(); }
-        launches += 5 * (uint64_t)iters;
+        launches += (5 + (v.teams ? 2 : 0)) * (uint64_t)iters + 1;  // k_plan once more for the last shadow rays
         if (e == cudaSuccess) e = cudaMemcpyAsync(b->ctrlHost, b->ctrl, sizeof(Ctrl), cudaMemcpyDeviceToHost, st);
         if (e == cudaSuccess) e = cudaStreamSynchronize(st);
         if (e != cudaSuccess) return contextFail(ctx, XGB_CUDA_ERROR, std::string("xgb_render_batch: ") + cudaGetErrorString(e));

@@ -1014,7 +1014,7 @@ int batchTeams(const SceneDev* scenes, int n) {
 }
 constexpr int kRetraceBlocks = 152;  // a launch that usually finds a handful of rays
 template <bool ANY, bool COUNT>
-static void launchWorld(const SceneDev& sc, const RenderParams& rp, PathQueue q, HitQueue h, unsigned int* retrace,
+static int launchWorld(const SceneDev& sc, const RenderParams& rp, PathQueue q, HitQueue h, unsigned int* retrace,
                         ShadowQueue sq, PathQueue out, Ctrl* ctrl, int numSMs, cudaStream_t s) {
     const OneScene one{sc, rp};
     if (sc.shell) {
@@ -1024,18 +1024,21 @@ static void launchWorld(const SceneDev& sc, const RenderParams& rp, PathQueue q,
         if (sc.world.enters) XGB_LAUNCH((k_trace_world<ANY, COUNT, OneScene, true, false>))(one, q, h, retrace, sq, out, ctrl);
         else XGB_LAUNCH((k_trace_world<ANY, COUNT, OneScene, false, false>))(one, q, h, retrace, sq, out, ctrl);
     }
-    if (!ANY && sc.nInstances > 1) k_retrace<OneScene><<<kRetraceBlocks, kTraceBlock, 0, s>>>(one, q, h, retrace, ctrl);
+    if (ANY || sc.nInstances == 1) return 1;
+    k_retrace<OneScene><<<kRetraceBlocks, kTraceBlock, 0, s>>>(one, q, h, retrace, ctrl);
+    return 2;
 }
-void launchExtend(const SceneDev& scene, PathQueue q, HitQueue h, unsigned int* retrace, Ctrl* ctrl, int numSMs, bool count,
-                  bool teams, cudaStream_t s) {
+int launchExtend(const SceneDev& scene, PathQueue q, HitQueue h, unsigned int* retrace, Ctrl* ctrl, int numSMs, bool count,
+                 bool teams, cudaStream_t s) {
     const SceneDev sc = withTeams(scene, false, teams && !count);
     if (sc.teams) XGB_LAUNCH((k_trace_team<false, OneScene>))(OneScene{sc, RenderParams{}}, q, h, ShadowQueue{}, PathQueue{}, ctrl);
+    const int before = sc.teams ? 1 : 0;
     RenderParams none{};
     const bool flat = sc.nInstances <= kFlatInstances;
     if (useWorld(sc, false)) {
-        if (count) launchWorld<false, true>(sc, none, q, h, retrace, ShadowQueue{}, PathQueue{}, ctrl, numSMs, s);
-        else launchWorld<false, false>(sc, none, q, h, retrace, ShadowQueue{}, PathQueue{}, ctrl, numSMs, s);
-        return;
+        const int n = count ? launchWorld<false, true>(sc, none, q, h, retrace, ShadowQueue{}, PathQueue{}, ctrl, numSMs, s)
+                            : launchWorld<false, false>(sc, none, q, h, retrace, ShadowQueue{}, PathQueue{}, ctrl, numSMs, s);
+        return n + before;
     }
     if (sc.shell) {
         if (flat && sc.blasLayout == 0) {
@@ -1046,7 +1049,7 @@ void launchExtend(const SceneDev& scene, PathQueue q, HitQueue h, unsigned int* 
         } else {
             XGB_LAUNCH((k_extend<false>))(sc, q, h, ctrl);
         }
-        return;
+        return 1 + before;
     }
     if (flat && sc.blasLayout == 1) {
         if (count) XGB_LAUNCH((k_trace_wide<false, true>))(sc, none, q, h, ShadowQueue{}, PathQueue{}, ctrl);
@@ -1059,26 +1062,28 @@ void launchExtend(const SceneDev& scene, PathQueue q, HitQueue h, unsigned int* 
     } else {
         XGB_LAUNCH((k_extend<false>))(sc, q, h, ctrl);
     }
+    return 1 + before;
 }
-void launchShadow(const SceneDev& scene, const RenderParams& rp, ShadowQueue sq, PathQueue out, Ctrl* ctrl, int numSMs,
-                  bool teams, cudaStream_t s) {
+int launchShadow(const SceneDev& scene, const RenderParams& rp, ShadowQueue sq, PathQueue out, Ctrl* ctrl, int numSMs,
+                 bool teams, cudaStream_t s) {
     const SceneDev sc = withTeams(scene, true, teams);
     if (sc.teams) XGB_LAUNCH((k_trace_team<true, OneScene>))(OneScene{sc, rp}, PathQueue{}, HitQueue{}, sq, out, ctrl);
+    const int before = sc.teams ? 1 : 0;
     const bool flat = sc.nInstances <= kFlatInstances;
     if (useWorld(sc, true)) {
-        launchWorld<true, false>(sc, rp, PathQueue{}, HitQueue{}, nullptr, sq, out, ctrl, numSMs, s);
-        return;
+        return before + launchWorld<true, false>(sc, rp, PathQueue{}, HitQueue{}, nullptr, sq, out, ctrl, numSMs, s);
     }
     if (sc.shell) {
         if (flat && sc.blasLayout == 0)
             XGB_LAUNCH((k_trace_flat2<true, false, OneScene, true>))(OneScene{sc, rp}, PathQueue{}, HitQueue{}, sq, out, ctrl);
         else XGB_LAUNCH(k_shadow)(sc, rp, sq, out, ctrl);
-        return;
+        return 1 + before;
     }
     if (flat && sc.blasLayout == 1) XGB_LAUNCH((k_trace_wide<true, false>))(sc, rp, PathQueue{}, HitQueue{}, sq, out, ctrl);
     else if (flat && sc.blasLayout == 0)
         XGB_LAUNCH((k_trace_flat2<true, false, OneScene>))(OneScene{sc, rp}, PathQueue{}, HitQueue{}, sq, out, ctrl);
     else XGB_LAUNCH(k_shadow)(sc, rp, sq, out, ctrl);
+    return 1 + before;
 }
 
 int batchKernels(const SceneDev* scenes, int n) {

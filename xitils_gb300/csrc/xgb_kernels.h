@@ -215,11 +215,12 @@ void launchGenerate(const SceneDev& sc, const RenderParams& rp, PathQueue q, Ctr
 // teams: whether small queues go to teams of lanes, where the scene allows it (not where a tail
 // launch takes over before a queue gets that small).
 // retrace: room for one number per path in the queue (the output queue, which is empty then).
-void launchExtend(const SceneDev& sc, PathQueue q, HitQueue h, unsigned int* retrace, Ctrl* ctrl, int numSMs, bool count, bool teams,
+// Both return the number of kernels launched.
+int launchExtend(const SceneDev& sc, PathQueue q, HitQueue h, unsigned int* retrace, Ctrl* ctrl, int numSMs, bool count, bool teams,
                   cudaStream_t s);
 void launchShade(const SceneDev& sc, const RenderParams& rp, PathQueue in, HitQueue h, PathQueue out, ShadowQueue sq,
                  Ctrl* ctrl, int numSMs, cudaStream_t s);
-void launchShadow(const SceneDev& sc, const RenderParams& rp, ShadowQueue sq, PathQueue out, Ctrl* ctrl, int numSMs,
+int launchShadow(const SceneDev& sc, const RenderParams& rp, ShadowQueue sq, PathQueue out, Ctrl* ctrl, int numSMs,
                   bool teams, cudaStream_t s);
 // Film plane (float4 or double4 per pixel) -> packed float RGB, strideFloats 3 or 4 (image.cu).
 void launchPackFilm(const void* film, int fp64, size_t n, int strideFloats, float* out, int grid, cudaStream_t s);
