@@ -1,8 +1,8 @@
 // xgb_render_noalloc: the render call of xgb_render for callers that must not
 // allocate GPU memory.
 //
-// xgb_render sizes its path queues to the work and allocates them with
-// cudaMalloc on first use. Some hosts cannot allow that: an engine that reserves
+// xgb_render sizes its path queues to the work and allocates them from a
+// memory pool on first use. Some hosts cannot allow that: an engine that reserves
 // all device memory through its own pool at start-up, a frame loop where the
 // implicit device synchronisation of cudaMalloc/cudaFree would stall the other
 // streams, or a plug-in host that hands the renderer a stream and nothing else.

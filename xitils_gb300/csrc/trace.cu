@@ -378,7 +378,7 @@ struct RayClaims {
 // walks the instances in order (those whose world box the ray still reaches
 // within tMax) and traverses each mesh BVH as a persistent per-lane state machine
 // in the style of Aila & Laine ("Understanding the Efficiency of Ray Traversal
-// on GPUs", HPG 2009): a lane whose ray is finished fetches the next one at once
+// on GPUs", HPG 2009): lanes whose rays are finished fetch the next ones together
 // (one atomicAdd per group of lanes), inner nodes and leaves are processed in
 // separate inner loops, and the first leaf a lane reaches is postponed until
 // every lane of the warp holds one, so that the warp tests triangles together.
@@ -554,8 +554,8 @@ __global__ void __launch_bounds__(kTraceBlock) k_trace_flat2(S scenes, PathQueue
 // ---- one BVH per scene -------------------------------------------------------------
 // The traversal of every scene with binary meshes: the scene's world BVH (WorldDev) as a
 // persistent per-lane state machine in the style of Aila & Laine ("Understanding the
-// Efficiency of Ray Traversal on GPUs", HPG 2009): a lane whose ray is finished fetches
-// the next one at once (one atomicAdd per group of lanes), inner nodes and leaves are
+// Efficiency of Ray Traversal on GPUs", HPG 2009): lanes whose rays are finished fetch
+// the next ones together (RayClaims), inner nodes and leaves are
 // processed in separate inner loops, and the first leaf a lane reaches is postponed until
 // few lanes of the warp are still looking for one, so that the warp tests triangles
 // together.
