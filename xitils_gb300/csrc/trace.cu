@@ -379,17 +379,23 @@ struct RayClaims {
 // within tMax) and traverses each mesh BVH as a persistent per-lane state machine
 // in the style of Aila & Laine ("Understanding the Efficiency of Ray Traversal
 // on GPUs", HPG 2009): lanes whose rays are finished fetch the next ones together
-// (one atomicAdd per group of lanes), inner nodes and leaves are processed in
-// separate inner loops, and the first leaf a lane reaches is postponed until
-// every lane of the warp holds one, so that the warp tests triangles together.
+// (RayClaims), inner nodes and leaves are processed in separate inner loops, and
+// the first leaf a lane reaches is postponed until few lanes of the warp are
+// still looking for one, so that the warp tests triangles together.
 // Results are those of traceScene: the same slab and watertight tests and the
 // same closest-hit acceptance (tMax shrinks across instances).
 constexpr int kSentinel = 0x7FFFFFFF;
 
+// The instance boxes are tested when the warp fetches, by all lanes that take a ray
+// together; afterwards a lane goes from one reached instance to the next, and tests a box again only
+// where a hit has come closer. Against a search by each lane at its own time: Cornell box
+// (8 instances) 3.43 -> 3.34 ms per call, 3.28 held to eight blocks per SM (64 registers; seven
+// with shell mapping); scenes of two to seven instances the same within 0.3 %.
+//
 // SHELL: the scene has shell-mapped meshes, whose accepted hits go through the
 // discard test (shellDiscard, trace.cuh) before tMax shrinks.
 template <bool ANY, bool COUNT, class S, bool SHELL = false>
-__global__ void __launch_bounds__(kTraceBlock) k_trace_flat2(S scenes, PathQueue q, HitQueue h, ShadowQueue s,
+__global__ void __launch_bounds__(kTraceBlock, SHELL ? 7 : 8) k_trace_flat2(S scenes, PathQueue q, HitQueue h, ShadowQueue s,
                                                             PathQueue out, Ctrl* ctrl) {
     const unsigned int n = ANY ? ctrl->nShadowDue : ctrl->nActive;
     if (n <= kTeamQueue && scenes.teams()) return;  // k_trace_team's
@@ -397,14 +403,14 @@ __global__ void __launch_bounds__(kTraceBlock) k_trace_flat2(S scenes, PathQueue
     constexpr bool kBatch = !std::is_same<S, OneScene>::value;
     int rayMaxSteps = 0, rayStack = 0;  // a batch: the current ray's job's bounds
     int job = 0;
-    int nInst = 0;
     const int lane = threadIdx.x & 31;
     RayClaims claims(head, n, kBatch || scenes.scene(0).large ? kFetchLanes : kFetchLanesMore);
     const int looking = claims.lanes == 32u ? kLookingLanes<SHELL> : 1;
     int stack[kStackDepth];
     int sp = 0;
     int nodeAddr = kSentinel, leafAddr = 0;
-    int inst = nInst;  // instance being traversed; nInst = ray finished
+    int inst = 0;               // instance being traversed
+    unsigned int reached = 0;  // instances after it whose world box the ray reaches
     unsigned int ray = 0;
     V3 wo(0.f, 0.f, 0.f), wd(0.f, 0.f, 1.f);
     BoxRay br{0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
@@ -432,7 +438,6 @@ __global__ void __launch_bounds__(kTraceBlock) k_trace_flat2(S scenes, PathQueue
             wd = V3(d4.x, d4.y, d4.z);
             br = BoxRay{wo.x, wo.y, wo.z, 1.0f / wd.x, 1.0f / wd.y, 1.0f / wd.z};
             job = scenes.jobOf(ANY ? __float_as_uint(d4.w) : __float_as_uint(q.thr[ray].w));
-            nInst = scenes.scene(job).nInstances;
             if (kBatch) {  // the job's traversal bounds, read once per ray
                 rayMaxSteps = scenes.scene(job).maxSteps;
                 rayStack = min(kStackDepth, scenes.scene(job).stackLimit);
@@ -442,7 +447,12 @@ __global__ void __launch_bounds__(kTraceBlock) k_trace_flat2(S scenes, PathQueue
             hit.t = tMax;
             occluded = false;
             guard = 0;
-            inst = -1;
+            {
+                const SceneDev& sc = scenes.scene(job);
+                reached = 0;
+                for (int k = 0; k < sc.nInstances; ++k)
+                    if (instBoxHit(br, sc.instBox, k, tMax)) reached |= 1u << k;
+            }
             nodeAddr = kSentinel;
             leafAddr = 0;
             fetch = false;
@@ -451,10 +461,13 @@ __global__ void __launch_bounds__(kTraceBlock) k_trace_flat2(S scenes, PathQueue
         if (fetch) continue;
         if (nodeAddr == kSentinel && leafAddr >= 0) {
             // next instance whose world box the ray still reaches
-            for (++inst; inst < nInst; ++inst)
-                if (instBoxHit(br, scenes.scene(job).instBox, inst, tMax)) break;
-            if (ANY && occluded) inst = nInst;
-            if (inst >= nInst) {  // ray finished
+            bool more = false;
+            while (reached && !(ANY && occluded) && !more) {
+                inst = __ffs(reached) - 1;
+                reached &= reached - 1;
+                more = ANY || hit.prim < 0 || instBoxHit(br, scenes.scene(job).instBox, inst, tMax);
+            }
+            if (!more) {  // ray finished
                 if (ANY) {
                     if (!occluded) shadowLit(scenes, job, s, out, ray);
                 } else {
@@ -480,7 +493,7 @@ __global__ void __launch_bounds__(kTraceBlock) k_trace_flat2(S scenes, PathQueue
             atomicOr(&ctrl->errors, 4u);
             nodeAddr = kSentinel;
             leafAddr = 0;
-            inst = nInst;
+            reached = 0;
         }
         bool searching = true;
         while ((unsigned int)nodeAddr < (unsigned int)kSentinel) {
