@@ -205,7 +205,14 @@ void launchPlan(Ctrl* ctrl, unsigned int capacity, cudaStream_t s, int mode = kP
 // 21.5 / 22.6 (40.9), its SVBRDF variant 26.7 / 24.4 / 23.0 / 25.7 (33.4); microfacet normal
 // mapping, whose walks of up to 100 facets per BSDF call make a warp's lanes wait for one
 // another and its code overflow the instruction cache, 400^2 x 4 6.4 / 7.3 / 10.3 / 10.3 (6.5).
-inline unsigned int tailMaxPaths(const SceneDev& sc) { return (sc.nested & 1) ? 4096u : 65536u; }
+// Scenes without lights, whose paths leave for the sky after a vertex or two, gain from larger
+// ones: with 65,536 / 262,144 / 524,288 / 1,048,576 paths the terrain took at 134,000 camera paths 0.585 /
+// 0.450 / 0.436 / 0.440, 524,000 1.62 / 1.17 / 1.14 / 1.14, 700,000 1.70 / 1.45 / 1.31 / 1.53, 2.1
+// million 2.35 / 2.36 / 2.06 / 2.00, 67 million 30.5 / 30.4 / 30.4 / 30.4; the Cornell box at 262,000 paths
+// 0.58 / 1.30 / 1.29 with its light, so scenes with lights keep 65,536.
+inline unsigned int tailMaxPaths(const SceneDev& sc) {
+    return (sc.nested & 1) ? 4096u : sc.nLights == 0 && !sc.nested ? 524288u : 65536u;
+}
 // Finishes the ctrl->nTail paths of `in`; those that outlive the launch's bound go to `out` (tail.cuh).
 void launchTail(const SceneDev& sc, const RenderParams& rp, PathQueue in, PathQueue out, Ctrl* ctrl, int numSMs,
                 cudaStream_t s);
