@@ -244,11 +244,14 @@ __global__ void k_plocInit(const unsigned int* __restrict__ vals, int n, const f
 struct PlocState {
     int count[2];  // clusters in the input of even / odd rounds
     int nodes;     // inner nodes created
-    int error;     // the single-block rounds ran out of their bound
+    int pairs;     // the next round joins neighbours two by two (plocStalled)
 };
 constexpr int kPlocHalo = 2 * kPlocRadius;
 // Up to this many clusters one block finishes the tree on its own (k_plocFinish).
 constexpr int kPlocFinish = 2048;
+// A round on the grid (more than kPlocFinish clusters) that is not stalled joins at least one
+// cluster in 288, the one after a stalled round every second: fewer than 2,700 rounds from
+// 2^24 triangles on.
 constexpr int kPlocMaxRounds = 4096;
 constexpr int kPlocGroup = 6;        // rounds between reads of the count
 constexpr int kPlocGrid = 152 * 4;  // blocks of a round
@@ -263,9 +266,20 @@ struct PlocTree {
     int n;
 };
 
+// Nearest clusters need not be mutual: along boxes that grow from one to the next each
+// prefers the one before, and areas that are NaN (vertices that are not finite) can even
+// close a ring. A round that joins hardly any clusters, or none, is followed by one that
+// joins neighbours two by two, so that the rounds end, and soon, for any boxes. Meshes of
+// random, regular and graded triangles join one cluster in 90 or more in every round and
+// keep their trees.
+__device__ __forceinline__ int plocStalled(int before, int joined) {
+    return joined == 0 || joined < before / 256 ? 1 : 0;
+}
+
 // The cluster within kPlocRadius positions of position i whose common box with it is
 // smallest; boxes of positions [first, ...) in sLo / sHi; -1 for a single cluster.
-__device__ __forceinline__ int plocNearest(const float4* sLo, const float4* sHi, int first, int i, int nc) {
+__device__ __forceinline__ int plocNearest(const float4* sLo, const float4* sHi, int first, int i, int nc, int pairs) {
+    if (pairs) return (i ^ 1) < nc ? i ^ 1 : -1;
     const float4 lo = sLo[i - first], hi = sHi[i - first];
     float best = __int_as_float(0x7f800000);
     int bestJ = -1;
@@ -276,6 +290,16 @@ __device__ __forceinline__ int plocNearest(const float4* sLo, const float4* sHi,
         const float a = halfArea(make_float4(fminf(lo.x, l2.x), fminf(lo.y, l2.y), fminf(lo.z, l2.z), 0.f),
                                  make_float4(fmaxf(hi.x, h2.x), fmaxf(hi.y, h2.y), fmaxf(hi.z, h2.z), 0.f));
         if (a < best || bestJ < 0) { best = a; bestJ = j; }  // ascending j: ties go to the lower index
+    }
+    // Inside a run of equal boxes (one triangle many times, triangles collapsed onto a vertex)
+    // all of them would choose the first of their window, of which one pair is mutual: a round
+    // for each triangle, and a chain as deep as the run. They pair up instead.
+    if (bestJ == i - kPlocRadius && (i ^ 1) < nc) {
+        auto same = [&](int j) {
+            const float4 l2 = sLo[j - first], h2 = sHi[j - first];
+            return l2.x == lo.x && l2.y == lo.y && l2.z == lo.z && h2.x == hi.x && h2.y == hi.y && h2.z == hi.z;
+        };
+        if (same(bestJ) && same(i ^ 1)) bestJ = i ^ 1;
     }
     return bestJ;
 }
@@ -304,6 +328,7 @@ __global__ void __launch_bounds__(kPlocBlock) k_plocMerge(const int* __restrict_
     __shared__ int sWarp[kPlocBlock / 32], sWarpNew[kPlocBlock / 32], sBase;
     const int nc = state->count[parity];
     if (nc <= kPlocFinish) return;  // k_plocCompact passes the clusters on as they are
+    const int pairs = state->pairs;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     for (int tile = blockIdx.x; tile * kPlocBlock < nc; tile += gridDim.x) {
         const int b0 = tile * kPlocBlock, first = b0 - kPlocHalo;
@@ -319,7 +344,7 @@ __global__ void __launch_bounds__(kPlocBlock) k_plocMerge(const int* __restrict_
         __syncthreads();
         for (int k = threadIdx.x; k < kPlocBlock + kPlocHalo; k += kPlocBlock) {
             const int i = b0 - kPlocRadius + k;
-            if (i >= 0 && i < nc) sNN[k] = plocNearest(sLo, sHi, first, i, nc);
+            if (i >= 0 && i < nc) sNN[k] = plocNearest(sLo, sHi, first, i, nc, pairs);
         }
         __syncthreads();
         const int i = b0 + threadIdx.x;
@@ -361,7 +386,7 @@ __global__ void __launch_bounds__(kPlocBlock) k_plocMerge(const int* __restrict_
     }
 }
 
-// The tiles' survivors next to each other; the next round's count.
+// The tiles' survivors next to each other; the next round's count and manner.
 __global__ void __launch_bounds__(kPlocBlock) k_plocCompact(const int* __restrict__ clusters, const int* __restrict__ in,
                                                             const int* __restrict__ tileCount, PlocState* state, int parity,
                                                             int* out) {
@@ -384,7 +409,10 @@ __global__ void __launch_bounds__(kPlocBlock) k_plocCompact(const int* __restric
         summed = tile;
         const int cnt = tileCount[tile];
         if ((int)threadIdx.x < cnt) out[offset + threadIdx.x] = in[tile * kPlocBlock + threadIdx.x];
-        if (tile == tiles - 1 && threadIdx.x == 0) state->count[parity ^ 1] = offset + cnt;
+        if (tile == tiles - 1 && threadIdx.x == 0) {
+            state->count[parity ^ 1] = offset + cnt;
+            state->pairs = plocStalled(nc, nc - (offset + cnt));
+        }
         __syncthreads();
     }
 }
@@ -401,7 +429,7 @@ __global__ void __launch_bounds__(kPlocFinishThreads) k_plocFinish(const int* __
     int* sNN = sId + kPlocFinish;
     __shared__ int sWarp[kPlocFinishThreads / 32], sNew[kPlocFinishThreads / 32];
     int nc = state->count[parity];
-    int nodes = state->nodes;
+    int nodes = state->nodes, pairs = state->pairs;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     if (nc > kPlocFinish) return;
     for (int i = tid; i < nc; i += kPlocFinishThreads) {
@@ -411,12 +439,8 @@ __global__ void __launch_bounds__(kPlocFinishThreads) k_plocFinish(const int* __
         sHi[i] = t.hi[id];
     }
     __syncthreads();
-    for (int round = 0; nc > 1; ++round) {
-        if (round >= kPlocMaxRounds) {  // cannot happen: every round joins at least one pair
-            if (tid == 0) state->error = 1;
-            return;
-        }
-        for (int i = tid; i < nc; i += kPlocFinishThreads) sNN[i] = plocNearest(sLo, sHi, 0, i, nc);
+    while (nc > 1) {  // of two rounds at least one joins clusters
+        for (int i = tid; i < nc; i += kPlocFinishThreads) sNN[i] = plocNearest(sLo, sHi, 0, i, nc, pairs);
         __syncthreads();
         constexpr int kPer = kPlocFinish / kPlocFinishThreads;
         int id[kPer], rank[kPer];  // this thread's survivors and their new positions (-1: none)
@@ -469,6 +493,7 @@ __global__ void __launch_bounds__(kPlocFinishThreads) k_plocFinish(const int* __
                 sLo[rank[h]] = lo[h];
                 sHi[rank[h]] = hi[h];
             }
+        pairs = plocStalled(nc, nc - kept);
         nc = kept;
         __syncthreads();  // also: this round's node counts are visible to the next's joins
     }
@@ -754,7 +779,7 @@ cudaError_t buildBlas(const BlasBuildInput& in, BlasBuildOutput* out, cudaStream
     int* start = (int*)(base + oStart);
     TriV* trisBin = wide ? (TriV*)(base + oTrisBin) : out->tris;  // the binary layout gathers in place
     Node2* nodes2 = out->nodes2;
-    int hostCount[4] = {0, 0, 0, 0}, plocFailed = 0;
+    int hostCount[4] = {0, 0, 0, 0};
 
     unsigned int initBounds[12];
     for (int k = 0; k < 12; ++k) initBounds[k] = (k % 6) < 3 ? 0xFFFFFFFFu : 0u;
@@ -785,7 +810,7 @@ cudaError_t buildBlas(const BlasBuildInput& in, BlasBuildOutput* out, cudaStream
         const int grid = std::min((n + kPlocBlock - 1) / kPlocBlock, kPlocGrid);
         int parity = 0, rounds = 0;
         for (int nc = n; nc > kPlocFinish; rounds += kPlocGroup) {
-            if (rounds > kPlocMaxRounds) return cudaErrorUnknown;  // cannot happen: every round merges at least one pair
+            if (rounds > kPlocMaxRounds) return cudaErrorUnknown;  // cannot happen, see kPlocMaxRounds
             for (int k = 0; k < kPlocGroup; ++k) {
                 k_plocMerge<<<grid, kPlocBlock, 0, stream>>>(clA, tree, state, parity, survivors, tileCount);
                 k_plocCompact<<<grid, kPlocBlock, 0, stream>>>(clA, survivors, tileCount, state, parity, clB);
@@ -797,7 +822,6 @@ cudaError_t buildBlas(const BlasBuildInput& in, BlasBuildOutput* out, cudaStream
             nc = *hostCount;
         }
         k_plocFinish<<<1, kPlocFinishThreads, kPlocFinishSmem, stream>>>(clA, tree, state, parity);
-        if ((e = cudaMemcpyAsync(&plocFailed, &state->error, 4, cudaMemcpyDeviceToHost, stream)) != cudaSuccess) return e;
         const int nAll = 2 * n - 1;
         k_dfsOffset<<<(nAll + B - 1) / B, B, 0, stream>>>(nAll, n, parent, left, right, count, start);
         if (!wide && n >= 2)
@@ -863,7 +887,6 @@ cudaError_t buildBlas(const BlasBuildInput& in, BlasBuildOutput* out, cudaStream
     if ((e = cudaMemcpyAsync(hb, bounds, sizeof(hb), cudaMemcpyDeviceToHost, stream)) != cudaSuccess) return e;
     if ((e = cudaStreamSynchronize(stream)) != cudaSuccess) return e;
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    if (plocFailed) return cudaErrorUnknown;
     for (int k = 0; k < 3; ++k) {
         out->boundsLo[k] = orderedFloat(hb[6 + k]);
         out->boundsHi[k] = orderedFloat(hb[9 + k]);
