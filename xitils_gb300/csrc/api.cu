@@ -77,8 +77,8 @@ void dfree(const void* p) {
 }
 
 // Memory of a context's pool back to it. Every call that reads or writes such memory has
-// waited for its work when it returns, so nothing on the device uses it any more; the
-// free goes through the thread's own stream, so that a batch being captured elsewhere is
+// waited for its work when it returns, also when it fails (WaitOnFailure), and a failing
+// call waits before it frees, so nothing on the device uses it any more; the free goes through the thread's own stream, so that a batch being captured elsewhere is
 // not disturbed.
 void poolFree(std::initializer_list<const void*> ps) {
     for (const void* p : ps) {
@@ -396,6 +396,7 @@ xgb_status xgb_texture_create(xgb_ctx* ctx, int width, int height, int channels,
     if (raw) cudaFreeAsync(raw, ctx->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
     if (e != cudaSuccess) {
+        cudaStreamSynchronize(ctx->stream);
         poolFree({tex->d});
         delete tex;
         return cudaFail(ctx, e, "xgb_texture_create");
@@ -496,6 +497,7 @@ static xgb_status createMesh(xgb_ctx* ctx, int vertex_count, const float* positi
         m->rootLeaf = o.rootLeaf;
     }
     if (e != cudaSuccess) {
+        cudaStreamSynchronize(s);
         freeMesh(m);
         delete m;
         return e == cudaErrorMemoryAllocation ? fail(ctx, XGB_OOM, "xgb_mesh_create: out of device memory")
@@ -727,6 +729,7 @@ xgb_status xgb_svndf_create(xgb_ctx* ctx, const xgb_texture* displacement, float
     }
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) {
+        cudaStreamSynchronize(st);
         poolFree({sv->lobes, tex->d});
         delete sv;
         delete tex;
@@ -1043,6 +1046,7 @@ xgb_status xgb_scene_build(xgb_scene* s, void* stream) {
     cudaStream_t st = pick(ctx, stream);
     XGB_CUDA(ctx, cudaStreamSynchronize(st));
     freeSceneDevice(s);
+    WaitOnFailure wait{st};
 
     // tables of meshes, materials and textures referenced by the objects
     std::map<const xgb_mesh*, int> meshIds;
@@ -1290,6 +1294,7 @@ xgb_status xgb_scene_build(xgb_scene* s, void* stream) {
     sd.skyTex = skyTex;
     sd.skyColor = make_float3(s->skyRGB[0], s->skyRGB[1], s->skyRGB[2]);
     XGB_CUDA(ctx, cudaStreamSynchronize(st));
+    wait.done = true;
     s->built = true;
     return XGB_OK;
 }
@@ -1451,6 +1456,7 @@ xgb_status xgb_render(xgb_scene* s, const xgb_integrator_params* params, xgb_fil
     unsigned int cap = P.queue_capacity > 0 ? (unsigned int)P.queue_capacity : (1u << 23);
     if ((unsigned long long)cap > total) cap = (unsigned int)std::max<unsigned long long>(total, 1024ull);
     cap = (cap + 255u) & ~255u;
+    WaitOnFailure wait{st};
     xgb_status bs = ensureBuffers(s, cap, st);
     if (bs) return bs;
     cap = s->rb.capacity;
@@ -1654,6 +1660,7 @@ xgb_status xgb_render(xgb_scene* s, const xgb_integrator_params* params, xgb_fil
             trainMs = ms;
         }
     }
+    wait.done = true;
     const Ctrl& c = *s->ctrlHost;
     if (c.pathsDone > 0) s->vertsPerPath = (double)c.extensionRays / (double)c.pathsDone;
     s->last.paths = c.pathsDone;
@@ -1707,7 +1714,8 @@ static xgb_status sceneQuery(xgb_scene* s, int n, const float* rays, int any, fl
                                   : cudaMemcpyAsync(hits, dOut, 20 * (size_t)n, cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess) e = cudaMemcpyAsync(&ctrl, dCtrl, sizeof(Ctrl), cudaMemcpyDeviceToHost, st);
     cudaFreeAsync(dev, st);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+    const cudaError_t waited = cudaStreamSynchronize(st);
+    if (e == cudaSuccess) e = waited;
     if (e != cudaSuccess) return cudaFail(ctx, e, "xgb_scene_intersect");
     if (ctrl.errors & ERR_STACK) return fail(ctx, XGB_QUEUE_OVERFLOW, "xgb_scene_intersect: traversal stack overflow");
     if (ctrl.errors & ERR_LOOP) return fail(ctx, XGB_DEVICE_TIMEOUT, "xgb_scene_intersect: traversal iteration bound exceeded");

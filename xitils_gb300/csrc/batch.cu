@@ -219,6 +219,7 @@ xgb_status runBatch(xgb_ctx* ctx, BatchState* b, const xgb_batch_job* jobs, int 
     std::memset(&init, 0, sizeof(init));
     init.totalPaths = total;
     *b->ctrlHost = init;
+    WaitOnFailure wait{st};
     cudaError_t e = cudaMemcpyAsync(b->dScenes, b->hScenes, sizeof(SceneDev) * n, cudaMemcpyHostToDevice, st);
     if (e == cudaSuccess) e = cudaMemcpyAsync(b->dParams, b->hParams, sizeof(RenderParams) * n, cudaMemcpyHostToDevice, st);
     if (e == cudaSuccess) e = cudaMemcpyAsync(b->dStart, b->hStart, sizeof(unsigned long long) * (n + 1), cudaMemcpyHostToDevice, st);
@@ -260,6 +261,7 @@ xgb_status runBatch(xgb_ctx* ctx, BatchState* b, const xgb_batch_job* jobs, int 
         if (c.nextPath >= c.totalPaths && c.nOut == 0) break;
         if (block > (1 << 22)) return contextFail(ctx, XGB_DEVICE_TIMEOUT, "xgb_render_batch: wavefront did not drain");
     }
+    wait.done = true;
     if (seconds) *seconds = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
     const Ctrl& c = *b->ctrlHost;
     b->last = xgb_render_stats{};

@@ -142,6 +142,7 @@ extern "C" xgb_status xgb_render_noalloc(xgb_scene* scene, const xgb_integrator_
     rp.film = filmPtr;
     rp.dropNonFinite = (sd.fixes & XGB_FIX_DROP_NONFINITE) ? 1 : 0;
 
+    WaitOnFailure wait{st};
     // The counters keep the previous call's values: start from zero.
     Ctrl host;
     std::memset(&host, 0, sizeof(host));
@@ -168,6 +169,7 @@ extern "C" xgb_status xgb_render_noalloc(xgb_scene* scene, const xgb_integrator_
         if (host.nextPath >= host.totalPaths && host.nOut == 0) break;
         if (guard > (1 << 24)) return XGB_DEVICE_TIMEOUT;
     }
+    wait.done = true;
     if (host.errors & ERR_STACK) return XGB_QUEUE_OVERFLOW;
     if (host.errors & ERR_LOOP) return XGB_DEVICE_TIMEOUT;
     return XGB_OK;

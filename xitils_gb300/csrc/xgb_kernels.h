@@ -187,6 +187,13 @@ void launchShadowBatch(const BatchView& b, ShadowQueue sq, PathQueue out, Ctrl* 
 // A wavefront iteration also hands the shadow rays of the last shade launch to launchShadow;
 // kPlanShadow does only that.
 enum PlanMode : int { kPlanWave = 0, kPlanTail = 1, kPlanTailIfFew = 2, kPlanShadow = 3 };
+// A call that fails after it has put work on its stream waits for that work all the same:
+// the caller frees or reuses next what it reads and writes.
+struct WaitOnFailure {
+    cudaStream_t stream;
+    bool done = false;
+    ~WaitOnFailure() { if (!done) cudaStreamSynchronize(stream); }
+};
 // A second stream for the launches that run beside others, with its two events.
 struct SideLane {
     cudaStream_t stream = nullptr;
