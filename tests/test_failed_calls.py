@@ -1,5 +1,5 @@
 """Calls that fail part-way leave nothing behind: the work they had put on their stream is
-over when they return.
+over when they return, and the next call is not told of their error.
 """
 import ctypes as C
 
@@ -50,3 +50,18 @@ def test_refused_mesh_leaves_no_copies_behind(api_mod):
     for f in films[1:]:
         # the order of a pixel's float sums alone (see test_tail.py)
         np.testing.assert_allclose(f, films[0], rtol=1e-4, atol=1e-6 * float(films[0].mean()))
+
+
+def test_refused_allocation_is_reported_once(api_mod):
+    """A texture of 640 GB does not fit; the calls after it succeed."""
+    api = api_mod
+    ctx = api.Context(0)
+    texel = (C.c_float * 3)(0.5, 0.5, 0.5)
+    tex = C.c_void_p()
+    assert ctx.lib.xgb_texture_create(ctx.h, 200_000, 200_000, 3, texel, 0, 0, C.byref(tex)) != 0 and not tex
+    api.Texture(ctx, np.full((4, 4, 3), 0.25, np.float32))
+    desc = scenes.terrain(grid=33, width=24, height=20, spp=1, env_size=(16, 8))
+    b = api.load_scene(ctx, desc)
+    rt = api.RenderTarget(ctx, desc.width, desc.height)
+    rt.render(b.scene, desc.spp, desc.params)
+    assert np.isfinite(rt.download()).all() and b.scene.stats()["paths"] == desc.n_paths

@@ -270,6 +270,8 @@ struct xgb_scene {
 
 static xgb_status fail(xgb_ctx* ctx, xgb_status st, const std::string& msg) {
     if (ctx) ctx->err = msg;
+    // reported with this status: not once more by the next call's check of its launches
+    if (st == XGB_OOM || st == XGB_CUDA_ERROR) cudaGetLastError();
     return st;
 }
 static xgb_status cudaFail(xgb_ctx* ctx, cudaError_t e, const char* what) {
