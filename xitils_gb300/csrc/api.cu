@@ -153,6 +153,18 @@ static cudaError_t poolAlloc(xgb_ctx* ctx, void** p, size_t bytes, cudaStream_t 
     return cudaMallocFromPoolAsync(p, bytes, ctx->pool, s);
 }
 
+// Memory that a call of this context could still get: the device's free bytes and those its
+// pool holds unused.
+static size_t freeBytes(xgb_ctx* ctx) {
+    size_t room = 0, total = 0;
+    uint64_t reserved = 0, used = 0;
+    if (cudaMemGetInfo(&room, &total) != cudaSuccess) return 0;
+    if (cudaMemPoolGetAttribute(ctx->pool, cudaMemPoolAttrReservedMemCurrent, &reserved) != cudaSuccess ||
+        cudaMemPoolGetAttribute(ctx->pool, cudaMemPoolAttrUsedMemCurrent, &used) != cudaSuccess)
+        return room;
+    return room + (size_t)(reserved - used);
+}
+
 struct xgb_texture {
     xgb_ctx* ctx;
     int w = 0, h = 0, clamp = 1, filter = 1;
@@ -816,6 +828,23 @@ static void freeSceneDevice(xgb_scene* s) {
     s->tables = s->worldBlock = nullptr;
     s->built = false;
 }
+// The world BVH's copies of a scene of several instances, back when a render has no room
+// for its buffers: the kernels that walk the instances need none. Whether there were any.
+static bool dropWorld(xgb_scene* s) {
+    if (!s->worldBlock) return false;
+    poolFree({s->worldBlock});
+    s->worldBlock = nullptr;
+    s->sd.world = WorldDev{};
+    cudaStreamSynchronize(cudaStreamPerThread);
+    cudaMemPoolTrimTo(s->ctx->pool, 0);
+    cudaGetLastError();
+    return true;
+}
+static cudaError_t allocForRender(xgb_scene* s, const std::function<cudaError_t()>& alloc) {
+    cudaError_t e = alloc();
+    if (e != cudaSuccess && dropWorld(s)) e = alloc();
+    return e;
+}
 static void freeBuffers(xgb_scene* s) {
     poolFree({s->rb.block});
     s->rb = RenderBuffers();
@@ -1265,9 +1294,13 @@ xgb_status xgb_scene_build(xgb_scene* s, void* stream) {
             if (tris >= (1ll << 27)) break;
             codes[i] = m->rootIsLeaf ? leafEncode(triBase[i], m->nTris) : nodeBase[i];
         }
-        // without room for the copies the scene keeps the kernels that walk its instances
+        // The copies (112 bytes per triangle) are made where they leave room for what a program
+        // needs next: queues, films, its own memory. Otherwise the scene keeps the kernels that
+        // walk its instances.
         const size_t nodeBytes = sizeof(Node2) * (size_t)nodes, triBytes = sizeof(TriV) * (size_t)tris;
-        if (tris < (1ll << 27) && poolAlloc(ctx, &s->worldBlock, nodeBytes + triBytes, st) == cudaSuccess) {
+        constexpr size_t kWorldSmall = 32ull << 20;  // below, the question (10 us) is not worth asking
+        const bool room = nodeBytes + triBytes <= kWorldSmall || nodeBytes + triBytes <= freeBytes(ctx) / 8;
+        if (tris < (1ll << 27) && room && poolAlloc(ctx, &s->worldBlock, nodeBytes + triBytes, st) == cudaSuccess) {
             Node2* wn = (Node2*)s->worldBlock;
             TriV* wt = (TriV*)((char*)s->worldBlock + nodeBytes);
             std::vector<Node2> top;
@@ -1408,7 +1441,7 @@ static xgb_status ensureBuffers(xgb_scene* s, unsigned int cap, cudaStream_t st)
     size_t shadowBytes = (size_t)cap * (16 * 3 + 8 + 4);
     size_t total = 2 * pathBytes + hitBytes + shadowBytes + 64 * 256;
     void* block = nullptr;
-    cudaError_t e = poolAlloc(s->ctx, &block, total, st);
+    const cudaError_t e = allocForRender(s, [&] { return poolAlloc(s->ctx, &block, total, st); });
     if (e != cudaSuccess) return fail(s->ctx, XGB_OOM, "render: cannot allocate path queues");
     char* p = (char*)block;
     auto take = [&](size_t bytes) { char* r = p; p += (bytes + 255) & ~(size_t)255; return r; };
@@ -1491,7 +1524,7 @@ xgb_status xgb_render(xgb_scene* s, const xgb_integrator_params* params, xgb_fil
             dfree(s->mix);
             s->mix = nullptr;
             s->mixCapacity = 0;
-            if (cudaMalloc((void**)&s->mix, sizeof(float4) * 10 * (size_t)cap) != cudaSuccess)
+            if (allocForRender(s, [&] { return cudaMalloc((void**)&s->mix, sizeof(float4) * 10 * (size_t)cap); }) != cudaSuccess)
                 return fail(ctx, XGB_OOM, "xgb_render: cannot allocate guiding mixtures");
             s->mixCapacity = cap;
         }
@@ -1505,7 +1538,7 @@ xgb_status xgb_render(xgb_scene* s, const xgb_integrator_params* params, xgb_fil
                 dfree(s->pathAcc);
                 s->pathAcc = nullptr;
                 s->pathAccCapacity = 0;
-                if (cudaMalloc((void**)&s->pathAcc, sizeof(float4) * (size_t)total) != cudaSuccess)
+                if (allocForRender(s, [&] { return cudaMalloc((void**)&s->pathAcc, sizeof(float4) * (size_t)total); }) != cudaSuccess)
                     return fail(ctx, XGB_OOM, "xgb_render: cannot allocate guide training accumulators");
                 s->pathAccCapacity = total;
             }
@@ -1778,6 +1811,7 @@ bool sceneView(xgb_scene* s, SceneDev* sd, int* device, int* numSMs, cudaStream_
     *built = s->built ? 1 : 0;
     return true;
 }
+bool sceneDropWorld(xgb_scene* s) { return dropWorld(s); }
 bool filmView(xgb_film* f, const xgb_scene* s, void** d, int* w, int* h, int* fp64) {
     if (!f || !s || f->ctx != s->ctx) return false;
     *d = f->d;

@@ -29,6 +29,7 @@
 
 namespace xgb {
 bool sceneView(xgb_scene* s, SceneDev* sd, int* device, int* numSMs, cudaStream_t* stream, int* built);
+bool sceneDropWorld(xgb_scene* s);
 bool filmPlane(xgb_film* f, void** d, int* w, int* h, int* fp64, int* device, cudaStream_t* ctxStream);
 xgb_ctx* sceneContext(xgb_scene* s);
 int sampleGrouping(const xgb_ctx* ctx);
@@ -214,7 +215,17 @@ xgb_status runBatch(xgb_ctx* ctx, BatchState* b, const xgb_batch_job* jobs, int 
                                                                         std::max<unsigned long long>(total, 1024ull));
     const unsigned int capR = (cap + 255u) & ~255u;
     for (int i = 0; i < n; ++i) b->hParams[i].capacity = capR;
-    if (ensureQueues(b, capR) != cudaSuccess) return contextFail(ctx, XGB_OOM, "xgb_render_batch: cannot allocate queues");
+    cudaError_t room = ensureQueues(b, capR);
+    if (room != cudaSuccess) {  // as xgb_render: the scenes' world BVHs go first
+        bool dropped = false;
+        for (int i = 0; i < n; ++i) dropped = sceneDropWorld(jobs[i].scene) || dropped;
+        for (int i = 0; i < n && dropped; ++i) {
+            int dev, sms, built; cudaStream_t cs;
+            sceneView(jobs[i].scene, &b->hScenes[i], &dev, &sms, &cs, &built);
+        }
+        if (dropped) room = ensureQueues(b, capR);
+    }
+    if (room != cudaSuccess) return contextFail(ctx, XGB_OOM, "xgb_render_batch: cannot allocate queues");
     Ctrl init;
     std::memset(&init, 0, sizeof(init));
     init.totalPaths = total;
