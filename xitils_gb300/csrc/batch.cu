@@ -236,8 +236,10 @@ xgb_status runBatch(xgb_ctx* ctx, BatchState* b, const xgb_batch_job* jobs, int 
     if (e == cudaSuccess) e = cudaMemcpyAsync(b->dStart, b->hStart, sizeof(unsigned long long) * (n + 1), cudaMemcpyHostToDevice, st);
     if (e == cudaSuccess) e = cudaMemcpyAsync(b->ctrl, b->ctrlHost, sizeof(Ctrl), cudaMemcpyHostToDevice, st);
     if (e != cudaSuccess) return contextFail(ctx, XGB_CUDA_ERROR, std::string("xgb_render_batch: ") + cudaGetErrorString(e));
-    const BatchView v{b->dScenes, b->dParams, b->dStart, n, batchKernels(b->hScenes, n), nested, batchTeams(b->hScenes, n)};
-    const int kernels = v.kernels | (nested << 4) | (v.teams << 5);  // which kernels a captured graph holds
+    const BatchView v{b->dScenes, b->dParams, b->dStart, n, batchKernels(b->hScenes, n), nested, batchTeams(b->hScenes, n),
+                      batchCounted(b->hScenes, n)};
+    // which kernels a captured graph holds, and how they run
+    const int kernels = v.kernels | (nested << 4) | (v.teams << 5) | (v.counted << 6);
     const int iters = std::max(2, (o.iterations_per_sync + 1) & ~1);
     const auto t0 = std::chrono::steady_clock::now();
     uint64_t launches = 0;

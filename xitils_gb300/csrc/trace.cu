@@ -106,6 +106,7 @@ struct OneScene {
     __device__ __forceinline__ int jobOf(unsigned int) const { return 0; }
     __device__ __forceinline__ int pixelOf(unsigned int packed) const { return (int)packed; }
     __device__ __forceinline__ bool teams() const { return sc.teams != 0; }
+    __device__ __forceinline__ bool counted() const { return sc.maxSteps != kDefaultMaxSteps; }
     __device__ __forceinline__ const SceneDev& scene(int) const { return sc; }
     __device__ __forceinline__ const RenderParams& params(int) const { return rp; }
 };
@@ -114,6 +115,7 @@ struct BatchScenes {
     __device__ __forceinline__ int jobOf(unsigned int packed) const { return (int)(packed >> 24); }
     __device__ __forceinline__ int pixelOf(unsigned int packed) const { return (int)(packed & 0xFFFFFFu); }
     __device__ __forceinline__ bool teams() const { return b.teams != 0; }
+    __device__ __forceinline__ bool counted() const { return b.counted != 0; }
     __device__ __forceinline__ const SceneDev& scene(int j) const { return b.scenes[j]; }
     __device__ __forceinline__ const RenderParams& params(int j) const { return b.params[j]; }
 };
@@ -137,6 +139,7 @@ struct QueryRays {
     int* occluded;
     __device__ __forceinline__ int jobOf(unsigned int) const { return 0; }
     __device__ __forceinline__ bool teams() const { return false; }
+    __device__ __forceinline__ bool counted() const { return false; }
     __device__ __forceinline__ const SceneDev& scene(int) const { return sc; }
 };
 
@@ -342,19 +345,23 @@ constexpr unsigned int kFetchLanes = 16, kFetchLanesMore = 24;
 // Every lane of the warp makes the same calls. (Claiming chunks of 32 / 64 / 128 rays ahead,
 // to save atomics, left some warps with work when the others had none: the batch took
 // 12.1 / 13.2 / 16.6 ms instead of 11.3.)
+// counted: the caller has set a bound on the steps of a ray (xgb_scene_set_traversal_limits).
+// A step of the loop takes a ray as far as the warp's lanes go on together, so that full
+// warps, filled up at once, that test triangles when no lane is looking any more need the
+// fewest steps: they keep a ray inside a bound that it met on such a warp.
 struct RayClaims {
     unsigned int* head;
     unsigned int n, lanes, next, fetch;
     // few rays: a warp works with its share of lanes only, so that they wait for fewer others
-    __device__ __forceinline__ RayClaims(unsigned int* h, unsigned int count, unsigned int fetchLanes)
+    __device__ __forceinline__ RayClaims(unsigned int* h, unsigned int count, unsigned int fetchLanes, bool counted)
         : head(h), n(count), next(0), fetch(fetchLanes) {
         const unsigned int warps = gridDim.x * (kTraceBlock / 32);
-        lanes = min(32u, (n + warps - 1u) / warps);
+        lanes = counted ? 32u : min(32u, (n + warps - 1u) / warps);
     }
     // The lanes that want a ray (0: none, or not yet worth the trip).
-    __device__ __forceinline__ unsigned int wanted(bool idle) const {
+    __device__ __forceinline__ unsigned int wanted(bool idle, bool counted) const {
         const unsigned int m = __ballot_sync(kWarp, idle && (threadIdx.x & 31) < lanes && next < n);
-        return (unsigned int)__popc(m) >= min(fetch, lanes) ? m : 0u;
+        return counted || (unsigned int)__popc(m) >= min(fetch, lanes) ? m : 0u;
     }
     // The next rays for the lanes of `want`; returns whether this lane got one.
     __device__ __forceinline__ bool take(unsigned int want, unsigned int* ray) {
@@ -404,8 +411,8 @@ __global__ void __launch_bounds__(kTraceBlock, SHELL ? 7 : 8) k_trace_flat2(S sc
     int rayMaxSteps = 0, rayStack = 0;  // a batch: the current ray's job's bounds
     int job = 0;
     const int lane = threadIdx.x & 31;
-    RayClaims claims(head, n, kBatch || scenes.scene(0).large ? kFetchLanes : kFetchLanesMore);
-    const int looking = claims.lanes == 32u ? kLookingLanes<SHELL> : 1;
+    RayClaims claims(head, n, kBatch || scenes.scene(0).large ? kFetchLanes : kFetchLanesMore, scenes.counted());
+    const int looking = claims.lanes == 32u && !scenes.counted() ? kLookingLanes<SHELL> : 1;
     int stack[kStackDepth];
     int sp = 0;
     int nodeAddr = kSentinel, leafAddr = 0;
@@ -429,7 +436,7 @@ __global__ void __launch_bounds__(kTraceBlock, SHELL ? 7 : 8) k_trace_flat2(S sc
     WorkCount wc;
     for (int guard = 0;; ++guard) {
         // every lane of the warp comes here; those without a ray take the next ones together
-        const unsigned int want = claims.wanted(fetch);
+        const unsigned int want = claims.wanted(fetch, scenes.counted());
         if (want && claims.take(want, &ray)) {
             float4 o4, d4;
             if (ANY) { o4 = __ldcs(&s.o[ray]); d4 = __ldcs(&s.d[ray]); tMax = o4.w; }
@@ -609,8 +616,8 @@ __global__ void __launch_bounds__(kTraceBlock, (WorldTraits<S, ENTER>::kMinBlock
     const unsigned int n = ANY ? ctrl->nShadowDue : ctrl->nActive;
     if (n <= kTeamQueue && scenes.teams()) return;  // k_trace_team's
     unsigned int* head = ANY ? &ctrl->shadowHead : &ctrl->extendHead;
-    RayClaims claims(head, n, ANY ? kFetchLanes : kFetchLanesMore);
-    const int looking = claims.lanes == 32u ? kLookingLanes<SHELL> : 1;
+    RayClaims claims(head, n, ANY ? kFetchLanes : kFetchLanesMore, scenes.counted());
+    const int looking = claims.lanes == 32u && !scenes.counted() ? kLookingLanes<SHELL> : 1;
     bool holds = false;  // the lane has a ray
     // one scene: its BVH for every ray; a batch: the current ray's
     const Node2* nodes = kBatch ? nullptr : scenes.scene(0).world.nodes;
@@ -630,7 +637,7 @@ __global__ void __launch_bounds__(kTraceBlock, (WorldTraits<S, ENTER>::kMinBlock
     WorkCount wc;
     for (int guard = 0;; ++guard) {
         // every lane of the warp comes here; those without a ray take the next ones together
-        const unsigned int want = claims.wanted(!holds);
+        const unsigned int want = claims.wanted(!holds, scenes.counted());
         if (want && claims.take(want, &ray)) {
             holds = true;
             float4 o4, d4;
@@ -1019,6 +1026,11 @@ static SceneDev withTeams(const SceneDev& sc, bool any, bool teams) {
     r.teams = sc.teams && teams && sc.maxSteps == kDefaultMaxSteps && sc.stackLimit == kMaxStackLimit &&
               (sc.nInstances <= kFlatInstances || useWorld(sc, any));
     return r;
+}
+int batchCounted(const SceneDev* scenes, int n) {
+    for (int j = 0; j < n; ++j)
+        if (scenes[j].maxSteps != kDefaultMaxSteps) return 1;
+    return 0;
 }
 int batchTeams(const SceneDev* scenes, int n) {
     bool teams = true;

@@ -168,9 +168,11 @@ struct BatchView {
     const unsigned long long* start;  // nJobs + 1 prefix sums of the jobs' path counts
     int nJobs;
     int kernels; // BatchKernels
-    int nested;
-    int teams;  // small queues go to teams of lanes  // some scene has a material that evaluates another (the shade kernel with that code)
+    int nested;   // some scene has a material that evaluates another (the shade kernel with that code)
+    int teams;    // small queues go to teams of lanes
+    int counted;  // some scene bounds the steps of a ray
 };
+int batchCounted(const SceneDev* scenes, int n);
 int batchTeams(const SceneDev* scenes, int n);
 int batchKernels(const SceneDev* scenes, int n);
 void launchGenerateBatch(const BatchView& b, PathQueue q, Ctrl* ctrl, int grid, cudaStream_t s);
