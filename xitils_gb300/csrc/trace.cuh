@@ -441,9 +441,9 @@ constexpr int kFlatInstances = 16;
 
 // Scene::intersect (any = false) or Scene::intersectAny as one function, for a kernel that
 // traces both kinds of rays next to other code: one copy of the traversal keeps the
-// kernel inside the instruction cache. A scene of at most kFlatInstances instances is
-// walked as a list, as the flat kernels of trace.cu do, any other over its top-level
-// BVH, as traceScene does, so that equal distances go to the same triangle as there.
+// kernel inside the instruction cache. A scene that launchExtend gives to the flat kernels
+// is walked as a list, as they do, any other over its top-level BVH, as traceScene does, so
+// that equal distances go to the same triangle as there.
 static __device__ __noinline__ bool traverseWideCall(const MeshDev& m, const WRay& r, float& tMax, TraceHit& hit, int inst,
                                                      unsigned int* errors, Limits lim, bool any) {
     WorkCount wc;
@@ -455,7 +455,7 @@ static __device__ __noinline__ bool traceCall(const SceneDev& sc, V3 o, V3 d, fl
     hit.inst = -1;
     hit.t = tMax;
     const Limits lim = limitsOf(sc);
-    const bool flat = sc.nInstances <= kFlatInstances && sc.blasLayout != 2;
+    const bool flat = sc.nInstances <= kFlatInstances && (sc.blasLayout == 0 || (sc.blasLayout == 1 && !sc.shell));
     const BoxRay br{o.x, o.y, o.z, 1.0f / d.x, 1.0f / d.y, 1.0f / d.z};
     const WRay wr = makeWRay(o, d);
     const int stackCap = lim.stack < kTlasStack ? lim.stack : kTlasStack;
