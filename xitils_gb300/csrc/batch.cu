@@ -146,8 +146,10 @@ cudaError_t ensureJobs(BatchState* b, int n) {
     return e;
 }
 
-// One block of `iters` wavefront iterations (an even count: the queues come back to parity 0).
-void enqueueBlock(BatchState* b, const BatchView& v, unsigned int cap, int iters, int numSMs, cudaStream_t st) {
+// One block of `iters` wavefront iterations (an even count: the queues come back to parity 0);
+// returns the number of kernels launched.
+uint64_t enqueueBlock(BatchState* b, const BatchView& v, unsigned int cap, int iters, int numSMs, cudaStream_t st) {
+    uint64_t launches = 1 + 3 * (uint64_t)iters;  // plan, generate, shade; plan for the last shadow rays
     for (int k = 0; k < iters; ++k) {
         PathQueue& X = b->q[k & 1];
         PathQueue& Y = b->q[(k & 1) ^ 1];
@@ -156,15 +158,15 @@ void enqueueBlock(BatchState* b, const BatchView& v, unsigned int cap, int iters
         // the last vertex's shadow rays beside the rays to the next (see xgb_render)
         if (k > 0) {
             if (b->side.stream) b->side.begin(st);
-            launchShadowBatch(v, b->shadow, X, b->ctrl, numSMs, b->side.stream ? b->side.stream : st);
+            launches += launchShadowBatch(v, b->shadow, X, b->ctrl, numSMs, b->side.stream ? b->side.stream : st);
             if (b->side.stream) b->side.end();
         }
-        launchExtendBatch(v, X, b->hits, (unsigned int*)Y.o, b->ctrl, numSMs, st);
+        launches += launchExtendBatch(v, X, b->hits, (unsigned int*)Y.o, b->ctrl, numSMs, st);
         if (k > 0 && b->side.stream) b->side.wait(st);
         launchShadeBatch(v, X, b->hits, Y, b->shadow, b->ctrl, numSMs, st);
     }
     launchPlan(b->ctrl, cap, st, kPlanShadow);
-    launchShadowBatch(v, b->shadow, b->q[0], b->ctrl, numSMs, st);
+    return launches + launchShadowBatch(v, b->shadow, b->q[0], b->ctrl, numSMs, st);
 }
 
 std::string shapeKey(const xgb_batch_job* jobs, int n) {
@@ -242,7 +244,7 @@ xgb_status runBatch(xgb_ctx* ctx, BatchState* b, const xgb_batch_job* jobs, int 
     const int kernels = v.kernels | (nested << 4) | (v.teams << 5) | (v.counted << 6);
     const int iters = std::max(2, (o.iterations_per_sync + 1) & ~1);
     const auto t0 = std::chrono::steady_clock::now();
-    uint64_t launches = 0;
+    uint64_t launches = 0, perBlock = 0;
     for (int block = 0;; ++block) {
         const bool replay = o.use_graph && block > 0;  // the first block runs direct (and primes the occupancy cache)
         if (replay && !(b->graph && b->graphCap == capR && b->graphIters == iters && b->graphJobs == n &&
@@ -263,8 +265,8 @@ xgb_status runBatch(xgb_ctx* ctx, BatchState* b, const xgb_batch_job* jobs, int 
             b->graphCap = capR; b->graphIters = iters; b->graphJobs = n; b->graphKernels = kernels;
         }
         if (replay) e = cudaGraphLaunch(b->graph, st);
-        else { enqueueBlock(b, v, capR, iters, numSMs, st); e = cudaGetLastError(); }
-        launches += (5 + (v.teams ? 2 : 0)) * (uint64_t)iters + 1;  // k_plan once more for the last shadow rays
+        else { perBlock = enqueueBlock(b, v, capR, iters, numSMs, st); e = cudaGetLastError(); }
+        launches += perBlock;  // the first block is never a replay
         if (e == cudaSuccess) e = cudaMemcpyAsync(b->ctrlHost, b->ctrl, sizeof(Ctrl), cudaMemcpyDeviceToHost, st);
         if (e == cudaSuccess) e = cudaStreamSynchronize(st);
         if (e != cudaSuccess) return contextFail(ctx, XGB_CUDA_ERROR, std::string("xgb_render_batch: ") + cudaGetErrorString(e));

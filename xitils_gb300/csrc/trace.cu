@@ -1112,48 +1112,55 @@ int launchShadow(const SceneDev& scene, const RenderParams& rp, ShadowQueue sq, 
 }
 
 int batchKernels(const SceneDev* scenes, int n) {
-    bool world = true, worldShadow = true, enters = false, flat = true;
+    bool world = true, enters = false, flat = true, single = true;
     for (int j = 0; j < n; ++j) {
         const SceneDev& sc = scenes[j];
-        const bool all = !sc.shell && useWorld(sc, true);
-        worldShadow = worldShadow && all;
-        // scenes of few instances take it only where others in the batch need it
-        world = world && all;
+        world = world && !sc.shell && useWorld(sc, true);
         enters = enters || sc.world.enters;
         flat = flat && sc.nInstances <= kFlatInstances && sc.blasLayout == 0 && !sc.shell;
+        single = single && sc.nInstances == 1;
     }
-    bool single = true;
-    for (int j = 0; j < n; ++j) single = single && scenes[j].nInstances == 1;
-    if (flat && !(single && world)) return worldShadow && !enters ? kBatchFlatWorldShadow : kBatchFlat;
+    if (world && single) return kBatchWorldSingle;
+    // scenes of few instances take the world BVH for their shadow rays, and for the others
+    // only beside scenes of many
+    if (flat) return world && !enters ? kBatchFlatWorldShadow : kBatchFlat;
     return world ? (enters ? kBatchWorldEnter : kBatchWorld) : kBatchGeneral;
 }
-void launchExtendBatch(const BatchView& b, PathQueue q, HitQueue h, unsigned int* retrace, Ctrl* ctrl, int numSMs,
-                       cudaStream_t s) {
+int launchExtendBatch(const BatchView& b, PathQueue q, HitQueue h, unsigned int* retrace, Ctrl* ctrl, int numSMs,
+                      cudaStream_t s) {
     const BatchScenes sc{b};
     if (b.teams) XGB_LAUNCH((k_trace_team<false, BatchScenes>))(sc, q, h, ShadowQueue{}, PathQueue{}, ctrl);
+    int launches = b.teams ? 2 : 1;
     switch (b.kernels) {
+    case kBatchWorldSingle:
     case kBatchWorld:
+        XGB_LAUNCH((k_trace_world<false, false, BatchScenes, false, false>))(sc, q, h, retrace, ShadowQueue{}, PathQueue{}, ctrl);
+        break;
     case kBatchWorldEnter:
-        if (b.kernels == kBatchWorld)
-            XGB_LAUNCH((k_trace_world<false, false, BatchScenes, false, false>))(sc, q, h, retrace, ShadowQueue{}, PathQueue{}, ctrl);
-        else XGB_LAUNCH((k_trace_world<false, false, BatchScenes, true, false>))(sc, q, h, retrace, ShadowQueue{}, PathQueue{}, ctrl);
-        k_retrace<BatchScenes><<<kRetraceBlocks, kTraceBlock, 0, s>>>(sc, q, h, retrace, ctrl);
+        XGB_LAUNCH((k_trace_world<false, false, BatchScenes, true, false>))(sc, q, h, retrace, ShadowQueue{}, PathQueue{}, ctrl);
         break;
     case kBatchFlat:
     case kBatchFlatWorldShadow: XGB_LAUNCH((k_trace_flat2<false, false, BatchScenes>))(sc, q, h, ShadowQueue{}, PathQueue{}, ctrl); break;
     default: XGB_LAUNCH(k_extend_batch)(b, q, h, ctrl);
     }
+    if (b.kernels == kBatchWorld || b.kernels == kBatchWorldEnter) {
+        k_retrace<BatchScenes><<<kRetraceBlocks, kTraceBlock, 0, s>>>(sc, q, h, retrace, ctrl);
+        ++launches;
+    }
+    return launches;
 }
-void launchShadowBatch(const BatchView& b, ShadowQueue sq, PathQueue out, Ctrl* ctrl, int numSMs, cudaStream_t s) {
+int launchShadowBatch(const BatchView& b, ShadowQueue sq, PathQueue out, Ctrl* ctrl, int numSMs, cudaStream_t s) {
     const BatchScenes sc{b};
     if (b.teams) XGB_LAUNCH((k_trace_team<true, BatchScenes>))(sc, PathQueue{}, HitQueue{}, sq, out, ctrl);
     switch (b.kernels) {
+    case kBatchWorldSingle:
     case kBatchWorld:
     case kBatchFlatWorldShadow: XGB_LAUNCH((k_trace_world<true, false, BatchScenes, false, false>))(sc, PathQueue{}, HitQueue{}, nullptr, sq, out, ctrl); break;
     case kBatchWorldEnter: XGB_LAUNCH((k_trace_world<true, false, BatchScenes, true, false>))(sc, PathQueue{}, HitQueue{}, nullptr, sq, out, ctrl); break;
     case kBatchFlat: XGB_LAUNCH((k_trace_flat2<true, false, BatchScenes>))(sc, PathQueue{}, HitQueue{}, sq, out, ctrl); break;
     default: XGB_LAUNCH(k_shadow_batch)(b, sq, out, ctrl);
     }
+    return b.teams ? 2 : 1;
 }
 
 // One instance takes the persistent per-lane kernel: 300,000 closest hits on a terrain of

@@ -160,8 +160,17 @@ struct RenderParams {
 // Device arrays of a batch of render jobs sharing one wavefront (xgb_render_batch):
 // a path of job j carries j << 24 | pixel in its pixel field.
 // Which traversal kernels a batch takes: every scene has a world BVH (without / with
-// instances to enter); every scene has <= 16 instances and binary mesh BVHs; any other.
-enum BatchKernels : int { kBatchGeneral = 0, kBatchFlat = 1, kBatchWorld = 2, kBatchWorldEnter = 3, kBatchFlatWorldShadow = 4 };
+// instances to enter, or all of one instance, where no hit is marked to be traced again);
+// every scene has <= 16 instances and binary mesh BVHs (and a world BVH for the shadow
+// rays); any other.
+enum BatchKernels : int {
+    kBatchGeneral = 0,
+    kBatchFlat = 1,
+    kBatchWorld = 2,
+    kBatchWorldEnter = 3,
+    kBatchFlatWorldShadow = 4,
+    kBatchWorldSingle = 5
+};
 struct BatchView {
     const SceneDev* scenes;
     const RenderParams* params;
@@ -178,9 +187,10 @@ int batchKernels(const SceneDev* scenes, int n);
 void launchGenerateBatch(const BatchView& b, PathQueue q, Ctrl* ctrl, int grid, cudaStream_t s);
 void launchShadeBatch(const BatchView& b, PathQueue in, HitQueue h, PathQueue out, ShadowQueue sq, Ctrl* ctrl,
                       int numSMs, cudaStream_t s);
-void launchExtendBatch(const BatchView& b, PathQueue q, HitQueue h, unsigned int* retrace, Ctrl* ctrl, int numSMs,
-                       cudaStream_t s);
-void launchShadowBatch(const BatchView& b, ShadowQueue sq, PathQueue out, Ctrl* ctrl, int numSMs, cudaStream_t s);
+// Both return the number of kernels launched.
+int launchExtendBatch(const BatchView& b, PathQueue q, HitQueue h, unsigned int* retrace, Ctrl* ctrl, int numSMs,
+                      cudaStream_t s);
+int launchShadowBatch(const BatchView& b, ShadowQueue sq, PathQueue out, Ctrl* ctrl, int numSMs, cudaStream_t s);
 
 // Queue bookkeeping of an iteration. mode kPlanWave: a wavefront iteration; kPlanTail: the
 // new camera paths go to a tail launch; kPlanTailIfFew: nothing happens (and the tail launch
