@@ -171,6 +171,27 @@ struct xgb_texture {
     float4* d = nullptr;
 };
 
+// A mesh's triangles on the host, for the sampling constants of an emitter.
+struct HostTriangles {
+    std::vector<H3> pos;
+    std::vector<int> idx;
+    std::vector<float> triArea;  // TriangleIndexed::surfaceArea (TriangleIndexed.h:56-62)
+    float area = 0;              // TriangleMesh::calcSurfaceArea (TriangleMesh.h:253-258)
+    void measure() {
+        triArea.resize(idx.size() / 3);
+        for (size_t t = 0; t < triArea.size(); ++t) {
+            H3 a = pos[idx[3 * t]], b = pos[idx[3 * t + 1]], c = pos[idx[3 * t + 2]];
+            triArea[t] = lengthH(crossH(sub(b, a), sub(c, a))) / 2.0f;
+            area += triArea[t];
+        }
+    }
+};
+// Meshes of up to this many triangles keep them on the host from the start, others once a scene
+// has them as an emitter (two copies and a wait, 19 us: with those in every build and for every
+// emissive object, 1,000 quads made a scene's build take 18.9 ms instead of 0.2; copying all meshes
+// when they are made would cost a rebuilt frame of 180,000 triangles a fifth of its time).
+constexpr int kHostTriangles = 4096;
+
 struct xgb_mesh {
     xgb_ctx* ctx;
     int nV = 0, nTris = 0;
@@ -186,6 +207,8 @@ struct xgb_mesh {
     TriV* dTris = nullptr;
     int rootIsLeaf = 1, rootLeaf = 0;
     Box bound;                   // TriangleMesh::bound over all vertices
+    mutable std::mutex hostMutex;
+    mutable std::shared_ptr<HostTriangles> host;  // nullptr until it is needed (hostTriangles)
     // shell mapping (xgb_mesh_create_shell): layers of shellFaces triangles each
     const xgb_texture* shellTex = nullptr;
     float shellScale = 0.0f;
@@ -454,6 +477,15 @@ static xgb_status createMesh(xgb_ctx* ctx, int vertex_count, const float* positi
     for (int i = 0; i < vertex_count; ++i) {
         const float* p = positions + (size_t)vs * i;
         m->bound.add(h3(p[0], p[1], p[2]));
+    }
+    if (m->nTris <= kHostTriangles && vertex_count <= 3 * kHostTriangles) {
+        m->host = std::make_shared<HostTriangles>();
+        m->host->idx.assign(indices, indices + index_count);
+        m->host->pos.resize(vertex_count);
+        for (int i = 0; i < vertex_count; ++i) {
+            const float* p = positions + (size_t)vs * i;
+            m->host->pos[i] = h3(p[0], p[1], p[2]);
+        }
     }
     // one allocation: vertex arrays, indices, per-triangle arrays, binary nodes; and a second,
     // for this call, through which the caller's arrays reach the device as they are
@@ -999,32 +1031,25 @@ static int buildTlas(std::vector<Node2>& nodes, std::vector<int>& items, const s
     return me;
 }
 
-// An emitter's triangles on the host, for its sampling constants.
-struct HostTriangles {
-    int nTris = 0;
-    std::vector<H3> pos;
-    std::vector<int> idx;
-    std::vector<float> triArea;  // TriangleIndexed::surfaceArea (TriangleIndexed.h:56-62)
-    float area = 0;              // TriangleMesh::calcSurfaceArea (TriangleMesh.h:253-258)
-    cudaError_t fetch(const xgb_mesh& m, cudaStream_t st) {
-        nTris = m.nTris;
-        std::vector<float4> p(m.nV);
-        idx.resize(3 * (size_t)nTris);
-        cudaError_t e = cudaMemcpyAsync(p.data(), m.dPos, sizeof(float4) * p.size(), cudaMemcpyDeviceToHost, st);
-        if (e == cudaSuccess) e = cudaMemcpyAsync(idx.data(), m.dIdx, 4 * idx.size(), cudaMemcpyDeviceToHost, st);
+// The triangles of an emissive mesh on the host.
+static cudaError_t hostTriangles(const xgb_mesh* mesh, cudaStream_t st, std::shared_ptr<const HostTriangles>* out) {
+    std::lock_guard<std::mutex> lock(mesh->hostMutex);
+    if (!mesh->host) {
+        auto h = std::make_shared<HostTriangles>();
+        std::vector<float4> p(mesh->nV);
+        h->idx.resize(3 * (size_t)mesh->nTris);
+        cudaError_t e = cudaMemcpyAsync(p.data(), mesh->dPos, sizeof(float4) * p.size(), cudaMemcpyDeviceToHost, st);
+        if (e == cudaSuccess) e = cudaMemcpyAsync(h->idx.data(), mesh->dIdx, 4 * h->idx.size(), cudaMemcpyDeviceToHost, st);
         if (e == cudaSuccess) e = cudaStreamSynchronize(st);
         if (e != cudaSuccess) return e;
-        pos.resize(m.nV);
-        for (int i = 0; i < m.nV; ++i) pos[i] = h3(p[i].x, p[i].y, p[i].z);
-        triArea.resize(nTris);
-        for (int t = 0; t < nTris; ++t) {
-            H3 a = pos[idx[3 * t]], b = pos[idx[3 * t + 1]], c = pos[idx[3 * t + 2]];
-            triArea[t] = lengthH(crossH(sub(b, a), sub(c, a))) / 2.0f;
-            area += triArea[t];
-        }
-        return cudaSuccess;
+        h->pos.resize(mesh->nV);
+        for (int i = 0; i < mesh->nV; ++i) h->pos[i] = h3(p[i].x, p[i].y, p[i].z);
+        mesh->host = h;
     }
-};
+    if (mesh->host->triArea.empty()) mesh->host->measure();
+    *out = mesh->host;
+    return cudaSuccess;
+}
 
 // Top level of a world BVH over up to 65,536 boxes, node 0 its root; leaves carry codes[i].
 // A few boxes are merged two by two, the pair with the smallest common box first (the
@@ -1171,24 +1196,23 @@ xgb_status xgb_scene_build(xgb_scene* s, void* stream) {
         }
     for (auto& L : lights) {
         const SceneObject& o = s->objects[L.instance];
-        const xgb_mesh* mesh = o.mesh;
-        HostTriangles tri;
-        XGB_CUDA(ctx, tri.fetch(*mesh, st));
-        const HostTriangles* m = &tri;
+        std::shared_ptr<const HostTriangles> m;
+        XGB_CUDA(ctx, hostTriangles(o.mesh, st, &m));
+        const int nTris = o.mesh->nTris;
         L.triOffset = (int)lightPdf.size();
         // TriangleMesh::surfaceAreaScaling (TriangleMesh.h:193-200, TriangleIndexed.h:64-72)
         float scaled = 0.0f;
-        for (int t = 0; t < m->nTris; ++t) {
+        for (int t = 0; t < nTris; ++t) {
             H3 a = pointH(o.mat, m->pos[m->idx[3 * t]]), b = pointH(o.mat, m->pos[m->idx[3 * t + 1]]),
                c = pointH(o.mat, m->pos[m->idx[3 * t + 2]]);
             float sc = lengthH(crossH(sub(b, a), sub(c, a))) / 2.0f / m->triArea[t];
             scaled += m->triArea[t] * sc;
         }
         float scaling = scaled / m->area;
-        for (int t = 0; t < m->nTris; ++t) {
+        for (int t = 0; t < nTris; ++t) {
             // pdf: TriangleIndexed.h:189 / TriangleMesh.h:221 / Object.h:96 / Scene.h:45
             float pdf = 1.0f / m->triArea[t];
-            pdf /= m->nTris;
+            pdf /= nTris;
             pdf /= scaling;
             pdf /= lights.size();
             lightPdf.push_back(pdf);
