@@ -1291,6 +1291,7 @@ xgb_status xgb_scene_build(xgb_scene* s, void* stream) {
     const float diag = (sceneBox.hi[0] - sceneBox.lo[0]) + (sceneBox.hi[1] - sceneBox.lo[1]) + (sceneBox.hi[2] - sceneBox.lo[2]);
     sd.tieAbs = std::isfinite(diag) ? diag * 0x1p-22f : 0.0f;
     sd.large = totalTris >= kTeamMinTris;
+    sd.listed = inst.size() <= (size_t)kFlatInstances && (blasLayout == 0 || (blasLayout == 1 && !anyShell));
     sd.teams = blasLayout == 0 && std::isfinite(diag) && sd.large;
     sd.world = WorldDev{};
     constexpr long long kWorldMinTris = 4096;  // of few instances, only large scenes gain (trace.cu::useWorld)
@@ -1298,7 +1299,7 @@ xgb_status xgb_scene_build(xgb_scene* s, void* stream) {
         const xgb_mesh* m = s->objects[0].mesh;
         sd.world = WorldDev{m->dNodes2, m->dTris, m->rootIsLeaf ? m->rootLeaf : 0, 0, 1.0f, 0.0f};
     } else if (blasLayout == 0 && inst.size() <= 65536 &&
-               (inst.size() > 16 || (!anyShell && totalTris >= kWorldMinTris))) {
+               (inst.size() > (size_t)kFlatInstances || (!anyShell && totalTris >= kWorldMinTris))) {
         // triangle and node numbers: leaf codes hold 27 bits, the traversal's hit marker 30
         std::vector<int> codes(inst.size());
         std::vector<int> nodeBase(inst.size(), 0), triBase(inst.size(), 0);

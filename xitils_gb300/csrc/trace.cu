@@ -1059,27 +1059,18 @@ int launchExtend(const SceneDev& scene, PathQueue q, HitQueue h, unsigned int* r
     if (sc.teams) XGB_LAUNCH((k_trace_team<false, OneScene>))(OneScene{sc, RenderParams{}}, q, h, ShadowQueue{}, PathQueue{}, ctrl);
     const int before = sc.teams ? 1 : 0;
     RenderParams none{};
-    const bool flat = sc.nInstances <= kFlatInstances;
     if (useWorld(sc, false)) {
         const int n = count ? launchWorld<false, true>(sc, none, q, h, retrace, ShadowQueue{}, PathQueue{}, ctrl, numSMs, s)
                             : launchWorld<false, false>(sc, none, q, h, retrace, ShadowQueue{}, PathQueue{}, ctrl, numSMs, s);
         return n + before;
     }
-    if (sc.shell) {
-        if (flat && sc.blasLayout == 0) {
-            if (count) XGB_LAUNCH((k_trace_flat2<false, true, OneScene, true>))(OneScene{sc, none}, q, h, ShadowQueue{}, PathQueue{}, ctrl);
-            else XGB_LAUNCH((k_trace_flat2<false, false, OneScene, true>))(OneScene{sc, none}, q, h, ShadowQueue{}, PathQueue{}, ctrl);
-        } else if (count) {
-            XGB_LAUNCH((k_extend<true>))(sc, q, h, ctrl);
-        } else {
-            XGB_LAUNCH((k_extend<false>))(sc, q, h, ctrl);
-        }
-        return 1 + before;
-    }
-    if (flat && sc.blasLayout == 1) {
+    if (sc.listed && sc.blasLayout == 1) {
         if (count) XGB_LAUNCH((k_trace_wide<false, true>))(sc, none, q, h, ShadowQueue{}, PathQueue{}, ctrl);
         else XGB_LAUNCH((k_trace_wide<false, false>))(sc, none, q, h, ShadowQueue{}, PathQueue{}, ctrl);
-    } else if (flat && sc.blasLayout == 0) {
+    } else if (sc.listed && sc.shell) {
+        if (count) XGB_LAUNCH((k_trace_flat2<false, true, OneScene, true>))(OneScene{sc, none}, q, h, ShadowQueue{}, PathQueue{}, ctrl);
+        else XGB_LAUNCH((k_trace_flat2<false, false, OneScene, true>))(OneScene{sc, none}, q, h, ShadowQueue{}, PathQueue{}, ctrl);
+    } else if (sc.listed) {
         if (count) XGB_LAUNCH((k_trace_flat2<false, true, OneScene>))(OneScene{sc, none}, q, h, ShadowQueue{}, PathQueue{}, ctrl);
         else XGB_LAUNCH((k_trace_flat2<false, false, OneScene>))(OneScene{sc, none}, q, h, ShadowQueue{}, PathQueue{}, ctrl);
     } else if (count) {
@@ -1094,18 +1085,13 @@ int launchShadow(const SceneDev& scene, const RenderParams& rp, ShadowQueue sq, 
     const SceneDev sc = withTeams(scene, true, teams);
     if (sc.teams) XGB_LAUNCH((k_trace_team<true, OneScene>))(OneScene{sc, rp}, PathQueue{}, HitQueue{}, sq, out, ctrl);
     const int before = sc.teams ? 1 : 0;
-    const bool flat = sc.nInstances <= kFlatInstances;
     if (useWorld(sc, true)) {
         return before + launchWorld<true, false>(sc, rp, PathQueue{}, HitQueue{}, nullptr, sq, out, ctrl, numSMs, s);
     }
-    if (sc.shell) {
-        if (flat && sc.blasLayout == 0)
-            XGB_LAUNCH((k_trace_flat2<true, false, OneScene, true>))(OneScene{sc, rp}, PathQueue{}, HitQueue{}, sq, out, ctrl);
-        else XGB_LAUNCH(k_shadow)(sc, rp, sq, out, ctrl);
-        return 1 + before;
-    }
-    if (flat && sc.blasLayout == 1) XGB_LAUNCH((k_trace_wide<true, false>))(sc, rp, PathQueue{}, HitQueue{}, sq, out, ctrl);
-    else if (flat && sc.blasLayout == 0)
+    if (sc.listed && sc.blasLayout == 1) XGB_LAUNCH((k_trace_wide<true, false>))(sc, rp, PathQueue{}, HitQueue{}, sq, out, ctrl);
+    else if (sc.listed && sc.shell)
+        XGB_LAUNCH((k_trace_flat2<true, false, OneScene, true>))(OneScene{sc, rp}, PathQueue{}, HitQueue{}, sq, out, ctrl);
+    else if (sc.listed)
         XGB_LAUNCH((k_trace_flat2<true, false, OneScene>))(OneScene{sc, rp}, PathQueue{}, HitQueue{}, sq, out, ctrl);
     else XGB_LAUNCH(k_shadow)(sc, rp, sq, out, ctrl);
     return 1 + before;

@@ -436,13 +436,11 @@ __device__ __forceinline__ bool instBoxHit(const BoxRay& b, const float4* boxes,
     return tn <= tf * 1.00000095367431640625f;
 }
 
-// Most instances that the flat kernels and traceFlat walk as a list.
-constexpr int kFlatInstances = 16;
 
 // Scene::intersect (any = false) or Scene::intersectAny as one function, for a kernel that
 // traces both kinds of rays next to other code: one copy of the traversal keeps the
 // kernel inside the instruction cache. A scene that launchExtend gives to the flat kernels
-// is walked as a list, as they do, any other over its top-level BVH, as traceScene does, so
+// (SceneDev::listed) is walked as a list, as they do, any other over its top-level BVH, as traceScene does, so
 // that equal distances go to the same triangle as there.
 static __device__ __noinline__ bool traverseWideCall(const MeshDev& m, const WRay& r, float& tMax, TraceHit& hit, int inst,
                                                      unsigned int* errors, Limits lim, bool any) {
@@ -455,7 +453,7 @@ static __device__ __noinline__ bool traceCall(const SceneDev& sc, V3 o, V3 d, fl
     hit.inst = -1;
     hit.t = tMax;
     const Limits lim = limitsOf(sc);
-    const bool flat = sc.nInstances <= kFlatInstances && (sc.blasLayout == 0 || (sc.blasLayout == 1 && !sc.shell));
+    const bool flat = sc.listed != 0;
     const BoxRay br{o.x, o.y, o.z, 1.0f / d.x, 1.0f / d.y, 1.0f / d.z};
     const WRay wr = makeWRay(o, d);
     const int stackCap = lim.stack < kTlasStack ? lim.stack : kTlasStack;

@@ -181,6 +181,8 @@ constexpr unsigned int kTeamQueue = 16384;
 // Rays of a small scene take few steps: rooms of 742 / 3,022 / 6,022 / 18,022 triangles with the
 // proposal, 120 x 100 x 4, per-lane kernels 2.53 / 2.46 / 2.85 / 3.45 ms, teams 2.83 / 2.60 / 2.82 / 3.10.
 constexpr long long kTeamMinTris = 6000;
+// Most instances that are walked as a list.
+constexpr int kFlatInstances = 16;
 constexpr int kDefaultMaxSteps = 1 << 22;
 constexpr int kMaxStackLimit = 64;
 
@@ -207,6 +209,10 @@ struct SceneDev {
     int teams;
     float tieAbs;
     int large;  // 1: at least kTeamMinTris triangles over all instances
+    // 1: the instances are walked as a list, in their order (the flat kernels of trace.cu and
+    // traceCall): at most kFlatInstances with binary meshes, or 8-wide ones none of which is
+    // shell-mapped; 0: over the top-level BVH (traceScene).
+    int listed;
     WorldDev world;
     const Material* materials;
     const TextureDev* textures;
