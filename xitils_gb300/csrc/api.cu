@@ -1053,15 +1053,13 @@ static cudaError_t hostTriangles(const xgb_mesh* mesh, cudaStream_t st, std::sha
 
 // Top level of a world BVH over up to 65,536 boxes, node 0 its root; leaves carry codes[i].
 // A few boxes are merged two by two, the pair with the smallest common box first (the
-// walls, lights and meshes of a room); many take buildTlas' median splits, whose depth
-// the traversal's stack has room for.
-static void buildWorldTop(std::vector<Node2>& nodes, const std::vector<Box>& boxes, const std::vector<int>& codes) {
+// walls, lights and meshes of a room); many take buildTlas' median splits, `tlas`, whose
+// depth the traversal's stack has room for.
+static void buildWorldTop(std::vector<Node2>& nodes, const std::vector<Node2>& tlas, const std::vector<Box>& boxes,
+                          const std::vector<int>& codes) {
     const int n = (int)boxes.size();
     if (n > 16) {
-        std::vector<int> items(n);
-        for (int i = 0; i < n; ++i) items[i] = i;
-        Box root;
-        buildTlas(nodes, items, boxes, 0, n, &root);
+        nodes = tlas;
         for (Node2& nd : nodes) {
             if (nd.d.x < 0) nd.d.x = codes[leafFirst(nd.d.x)];
             if (nd.d.y < 0) nd.d.y = codes[leafFirst(nd.d.y)];
@@ -1302,7 +1300,7 @@ xgb_status xgb_scene_build(xgb_scene* s, void* stream) {
                (inst.size() > (size_t)kFlatInstances || (!anyShell && totalTris >= kWorldMinTris))) {
         // triangle and node numbers: leaf codes hold 27 bits, the traversal's hit marker 30
         std::vector<int> codes(inst.size());
-        std::vector<int> nodeBase(inst.size(), 0), triBase(inst.size(), 0);
+        std::vector<WorldPart> parts;
         long long nodes = (long long)inst.size() - 1, tris = 0;
         int enters = 0;
         for (size_t i = 0; i < inst.size(); ++i) {
@@ -1312,32 +1310,33 @@ xgb_status xgb_scene_build(xgb_scene* s, void* stream) {
                 enters = 1;
                 continue;
             }
-            nodeBase[i] = (int)std::min<long long>(nodes, INT32_MAX);
-            triBase[i] = (int)std::min<long long>(tris, INT32_MAX);
+            const WorldPart part{m->dNodes2, m->dTris, (int)nodes, (int)tris, (int)i};
             tris += m->nTris;
             if (!m->rootIsLeaf) nodes += m->nTris - 1;
             if (tris >= (1ll << 27)) break;
-            codes[i] = m->rootIsLeaf ? leafEncode(triBase[i], m->nTris) : nodeBase[i];
+            codes[i] = m->rootIsLeaf ? leafEncode(part.triBase, m->nTris) : part.nodeBase;
+            parts.push_back(part);
         }
         // The copies (112 bytes per triangle) are made where they leave room for what a program
         // needs next: queues, films, its own memory. Otherwise the scene keeps the kernels that
         // walk its instances.
         const size_t nodeBytes = sizeof(Node2) * (size_t)nodes, triBytes = sizeof(TriV) * (size_t)tris;
+        const size_t partBytes = sizeof(WorldPart) * parts.size();
         constexpr size_t kWorldSmall = 32ull << 20;  // below, the question (10 us) is not worth asking
         const bool room = nodeBytes + triBytes <= kWorldSmall || nodeBytes + triBytes <= freeBytes(ctx) / 8;
-        if (tris < (1ll << 27) && room && poolAlloc(ctx, &s->worldBlock, nodeBytes + triBytes, st) == cudaSuccess) {
+        if (tris < (1ll << 27) && room && poolAlloc(ctx, &s->worldBlock, nodeBytes + triBytes + partBytes, st) == cudaSuccess) {
             Node2* wn = (Node2*)s->worldBlock;
             TriV* wt = (TriV*)((char*)s->worldBlock + nodeBytes);
             std::vector<Node2> top;
-            buildWorldTop(top, boxes, codes);
+            buildWorldTop(top, tlas, boxes, codes);
             XGB_CUDA(ctx, cudaMemcpyAsync(wn, top.data(), sizeof(Node2) * top.size(), cudaMemcpyHostToDevice, st));
-            for (size_t i = 0; i < inst.size(); ++i) {
-                const xgb_mesh* m = s->objects[i].mesh;
-                if (inst[i].identity)
-                    worldCopy(m->dNodes2, m->dTris, m->nTris, m->rootIsLeaf != 0, (int)i, nodeBase[i], triBase[i], wn, wt, st);
+            if (!parts.empty()) {
+                WorldPart* dParts = (WorldPart*)((char*)wt + triBytes);
+                XGB_CUDA(ctx, cudaMemcpyAsync(dParts, parts.data(), partBytes, cudaMemcpyHostToDevice, st));
+                worldCopy(dParts, (int)parts.size(), (int)top.size(), (int)nodes, (int)tris, wn, wt, st);
+                XGB_CUDA(ctx, cudaGetLastError());
             }
-            XGB_CUDA(ctx, cudaGetLastError());
-            XGB_CUDA(ctx, cudaStreamSynchronize(st));  // `top` is read by the copy
+            XGB_CUDA(ctx, cudaStreamSynchronize(st));  // `top` and `parts` are read by the copies
             sd.world = WorldDev{wn, wt, 0, enters, 1.0f + 0x1p-19f, sd.tieAbs};
         } else {
             cudaGetLastError();

@@ -920,28 +920,41 @@ void expandUv(const float* src, int stride, size_t n, float2* dst, cudaStream_t 
 }
 
 namespace {
-__global__ void k_worldNodes(const Node2* __restrict__ src, int n, int nodeBase, int triBase, Node2* dst) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    Node2 nd = src[i];
-    auto moved = [&](int c) { return c >= 0 ? c + nodeBase : leafEncode(leafFirst(c) + triBase, leafCount(c)); };
-    nd.d.x = moved(nd.d.x);
-    nd.d.y = moved(nd.d.y);
-    dst[nodeBase + i] = nd;
-}
-__global__ void k_worldTris(const TriV* __restrict__ src, int n, int inst, int triBase, TriV* dst) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    TriV t = src[i];
-    t.p1.w = __int_as_float(inst);
-    dst[triBase + i] = t;
+// Every part's nodes and triangles in one launch; a thread looks its part up by the bases (16
+// steps for 65,536 parts). With launches per instance a build of 1,000 small instances took
+// 3.3 ms, of 60,000 201.
+__global__ void k_worldCopy(const WorldPart* __restrict__ parts, int nParts, int firstNode, int nNodes, int nTris, Node2* nodes,
+                            TriV* tris) {
+    auto partOf = [&](int at, bool node) {  // the last part that starts at or before `at`
+        int lo = 0, hi = nParts - 1;
+        while (lo < hi) {
+            const int mid = (lo + hi + 1) >> 1;
+            if ((node ? parts[mid].nodeBase : parts[mid].triBase) <= at) lo = mid;
+            else hi = mid - 1;
+        }
+        return parts[lo];
+    };
+    const int stride = gridDim.x * blockDim.x, first = blockIdx.x * blockDim.x + threadIdx.x;
+    for (int i = first; i < nTris; i += stride) {
+        const WorldPart p = partOf(i, false);
+        TriV t = p.tris[i - p.triBase];
+        t.p1.w = __int_as_float(p.inst);
+        tris[i] = t;
+    }
+    for (int i = firstNode + first; i < nNodes; i += stride) {
+        const WorldPart p = partOf(i, true);
+        Node2 nd = p.nodes[i - p.nodeBase];
+        auto moved = [&](int c) { return c >= 0 ? c + p.nodeBase : leafEncode(leafFirst(c) + p.triBase, leafCount(c)); };
+        nd.d.x = moved(nd.d.x);
+        nd.d.y = moved(nd.d.y);
+        nodes[i] = nd;
+    }
 }
 }  // namespace
 
-void worldCopy(const Node2* nodes, const TriV* tris, int n, bool rootIsLeaf, int inst, int nodeBase, int triBase,
-               Node2* worldNodes, TriV* worldTris, cudaStream_t s) {
-    if (!rootIsLeaf) k_worldNodes<<<(n - 1 + 255) / 256, 256, 0, s>>>(nodes, n - 1, nodeBase, triBase, worldNodes);
-    k_worldTris<<<(n + 255) / 256, 256, 0, s>>>(tris, n, inst, triBase, worldTris);
+void worldCopy(const WorldPart* parts, int nParts, int firstNode, int nNodes, int nTris, Node2* worldNodes, TriV* worldTris,
+               cudaStream_t s) {
+    k_worldCopy<<<rowGrid((size_t)nTris), 256, 0, s>>>(parts, nParts, firstNode, nNodes, nTris, worldNodes, worldTris);
 }
 
 }  // namespace xgb

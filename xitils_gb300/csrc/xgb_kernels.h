@@ -43,10 +43,17 @@ cudaError_t buildBlas(const BlasBuildInput& in, BlasBuildOutput* out, cudaStream
 void expandVec3(const float* src, int stride, size_t n, float4* dst, cudaStream_t s);
 void expandUv(const float* src, int stride, size_t n, float2* dst, cudaStream_t s);
 
-// An instance's share of a world BVH (WorldDev): the mesh's n - 1 nodes renumbered to start
-// at nodeBase, its n triangles at triBase with the instance's number.
-void worldCopy(const Node2* nodes, const TriV* tris, int n, bool rootIsLeaf, int inst, int nodeBase, int triBase,
-               Node2* worldNodes, TriV* worldTris, cudaStream_t s);
+// An instance's share of a world BVH (WorldDev): the mesh's nodes (none when its root is a
+// leaf) renumbered to start at nodeBase, its triangles at triBase with the instance's number.
+struct WorldPart {
+    const Node2* nodes;
+    const TriV* tris;
+    int nodeBase, triBase, inst;
+};
+// Parts on the device, in ascending order of both bases: the world's nodes [firstNode, nNodes)
+// and triangles [0, nTris).
+void worldCopy(const WorldPart* parts, int nParts, int firstNode, int nNodes, int nTris, Node2* worldNodes, TriV* worldTris,
+               cudaStream_t s);
 
 // SVNDF fit of a displacement map (svndf.cu): lobes [resV][resU][5] float4, low
 // heights [resV][resU] float4 (red channel). rate in [1, 16].
