@@ -351,17 +351,18 @@ constexpr unsigned int kFetchLanes = 16, kFetchLanesMore = 24;
 // fewest steps: they keep a ray inside a bound that it met on such a warp.
 struct RayClaims {
     unsigned int* head;
-    unsigned int n, lanes, next, fetch;
+    unsigned int n, lanes, next, enough;
     // few rays: a warp works with its share of lanes only, so that they wait for fewer others
     __device__ __forceinline__ RayClaims(unsigned int* h, unsigned int count, unsigned int fetchLanes, bool counted)
-        : head(h), n(count), next(0), fetch(fetchLanes) {
+        : head(h), n(count), next(0) {
         const unsigned int warps = gridDim.x * (kTraceBlock / 32);
         lanes = counted ? 32u : min(32u, (n + warps - 1u) / warps);
+        enough = counted ? 1u : min(fetchLanes, lanes);
     }
     // The lanes that want a ray (0: none, or not yet worth the trip).
-    __device__ __forceinline__ unsigned int wanted(bool idle, bool counted) const {
+    __device__ __forceinline__ unsigned int wanted(bool idle) const {
         const unsigned int m = __ballot_sync(kWarp, idle && (threadIdx.x & 31) < lanes && next < n);
-        return counted || (unsigned int)__popc(m) >= min(fetch, lanes) ? m : 0u;
+        return (unsigned int)__popc(m) >= enough ? m : 0u;
     }
     // The next rays for the lanes of `want`; returns whether this lane got one.
     __device__ __forceinline__ bool take(unsigned int want, unsigned int* ray) {
@@ -436,7 +437,7 @@ __global__ void __launch_bounds__(kTraceBlock, SHELL ? 7 : 8) k_trace_flat2(S sc
     WorkCount wc;
     for (int guard = 0;; ++guard) {
         // every lane of the warp comes here; those without a ray take the next ones together
-        const unsigned int want = claims.wanted(fetch, scenes.counted());
+        const unsigned int want = claims.wanted(fetch);
         if (want && claims.take(want, &ray)) {
             float4 o4, d4;
             if (ANY) { o4 = __ldcs(&s.o[ray]); d4 = __ldcs(&s.d[ray]); tMax = o4.w; }
@@ -637,7 +638,7 @@ __global__ void __launch_bounds__(kTraceBlock, (WorldTraits<S, ENTER>::kMinBlock
     WorkCount wc;
     for (int guard = 0;; ++guard) {
         // every lane of the warp comes here; those without a ray take the next ones together
-        const unsigned int want = claims.wanted(!holds, scenes.counted());
+        const unsigned int want = claims.wanted(!holds);
         if (want && claims.take(want, &ray)) {
             holds = true;
             float4 o4, d4;
