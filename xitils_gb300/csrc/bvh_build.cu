@@ -920,11 +920,11 @@ void expandUv(const float* src, int stride, size_t n, float2* dst, cudaStream_t 
 }
 
 namespace {
-// Every part's nodes and triangles in one launch; a thread looks its part up by the bases (16
-// steps for 65,536 parts). With launches per instance a build of 1,000 small instances took
-// 3.3 ms, of 60,000 201.
-__global__ void k_worldCopy(const WorldPart* __restrict__ parts, int nParts, int firstNode, int nNodes, int nTris, Node2* nodes,
-                            TriV* tris) {
+// Every part's nodes and triangles, and the top level, in one launch; a thread looks its part
+// up by the bases (16 steps for 65,536 parts). With launches per instance a build of 1,000
+// small instances took 3.3 ms, of 60,000 201.
+__global__ void k_worldCopy(const WorldPart* __restrict__ parts, int nParts, const Node2* __restrict__ top,
+                            const int* __restrict__ codes, int nTop, int nNodes, int nTris, Node2* nodes, TriV* tris) {
     auto partOf = [&](int at, bool node) {  // the last part that starts at or before `at`
         int lo = 0, hi = nParts - 1;
         while (lo < hi) {
@@ -941,7 +941,13 @@ __global__ void k_worldCopy(const WorldPart* __restrict__ parts, int nParts, int
         t.p1.w = __int_as_float(p.inst);
         tris[i] = t;
     }
-    for (int i = firstNode + first; i < nNodes; i += stride) {
+    for (int i = first; codes && i < nTop; i += stride) {
+        Node2 nd = top[i];
+        if (nd.d.x < 0) nd.d.x = codes[leafFirst(nd.d.x)];
+        if (nd.d.y < 0) nd.d.y = codes[leafFirst(nd.d.y)];
+        nodes[i] = nd;
+    }
+    for (int i = nTop + first; i < nNodes; i += stride) {
         const WorldPart p = partOf(i, true);
         Node2 nd = p.nodes[i - p.nodeBase];
         auto moved = [&](int c) { return c >= 0 ? c + p.nodeBase : leafEncode(leafFirst(c) + p.triBase, leafCount(c)); };
@@ -952,9 +958,10 @@ __global__ void k_worldCopy(const WorldPart* __restrict__ parts, int nParts, int
 }
 }  // namespace
 
-void worldCopy(const WorldPart* parts, int nParts, int firstNode, int nNodes, int nTris, Node2* worldNodes, TriV* worldTris,
-               cudaStream_t s) {
-    k_worldCopy<<<rowGrid((size_t)nTris), 256, 0, s>>>(parts, nParts, firstNode, nNodes, nTris, worldNodes, worldTris);
+void worldCopy(const WorldPart* parts, int nParts, const Node2* top, const int* codes, int nTop, int nNodes, int nTris,
+               Node2* worldNodes, TriV* worldTris, cudaStream_t s) {
+    k_worldCopy<<<rowGrid((size_t)std::max(nTop, nTris)), 256, 0, s>>>(parts, nParts, top, codes, nTop, nNodes, nTris,
+                                                                       worldNodes, worldTris);
 }
 
 }  // namespace xgb

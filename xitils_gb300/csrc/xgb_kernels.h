@@ -50,10 +50,11 @@ struct WorldPart {
     const TriV* tris;
     int nodeBase, triBase, inst;
 };
-// Parts on the device, in ascending order of both bases: the world's nodes [firstNode, nNodes)
-// and triangles [0, nTris).
-void worldCopy(const WorldPart* parts, int nParts, int firstNode, int nNodes, int nTris, Node2* worldNodes, TriV* worldTris,
-               cudaStream_t s);
+// Parts on the device, in ascending order of both bases: the world's nodes [nTop, nNodes) and
+// triangles [0, nTris). codes: the world's nodes [0, nTop) are those of `top`, its leaf i
+// with codes[i] in its place (nullptr: they are there already).
+void worldCopy(const WorldPart* parts, int nParts, const Node2* top, const int* codes, int nTop, int nNodes, int nTris,
+               Node2* worldNodes, TriV* worldTris, cudaStream_t s);
 
 // SVNDF fit of a displacement map (svndf.cu): lobes [resV][resU][5] float4, low
 // heights [resV][resU] float4 (red channel). rate in [1, 16].
