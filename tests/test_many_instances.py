@@ -1,0 +1,61 @@
+"""Scenes of many instances take no longer with a world BVH and tail launches than without:
+traversal limits other than the defaults keep a scene on the kernels that walk the instances, so the
+same render is timed both ways in turn, the fastest of a few, and compared with it (films
+as in test_tail.py).
+"""
+import time
+
+import numpy as np
+import pytest
+
+from xitils_gb300 import scenes
+from xitils_gb300.transform import scale, translate
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def api_mod():
+    import __graft_entry__ as g
+    g.build()
+    from xitils_gb300 import api
+    return api
+
+
+def _boxes(n, width, height, level):
+    """A terrain under its sky with n boxes, moved there, many of which overlap; level: with
+    their tops in one plane."""
+    d = scenes.terrain(grid=129, width=width, height=height, spp=1, env_size=(128, 64))
+    cpos, cidx = scenes.unit_cube_mesh()
+    cube = d.add_mesh(cpos, cidx)
+    grey = d.diffuse([0.6, 0.6, 0.6])
+    rng = np.random.default_rng(3)
+    for _ in range(n):
+        x, z = rng.uniform(0.1, 0.9, 2)
+        y = 0.2 if level else rng.uniform(0.15, 0.25)
+        d.add_object(cube, grey, translate(float(x), float(y), float(z)) * scale(0.04, 0.04, 0.04))
+    return d
+
+
+def _both_ways(api, d):
+    ctx = api.Context(0)
+    b = api.load_scene(ctx, d)
+    best, films = [np.inf, np.inf], [None, None]
+    for _ in range(6):
+        for k, stack in enumerate((0, 63)):
+            b.scene.set_traversal_limits(0, stack)
+            rt = api.RenderTarget(ctx, d.width, d.height)
+            t = time.perf_counter()
+            rt.render(b.scene, d.spp, d.params)
+            best[k] = min(best[k], time.perf_counter() - t)
+            films[k] = rt.download()
+    np.testing.assert_allclose(films[0], films[1], rtol=1e-4, atol=1e-6 * float(films[1].mean()))
+    return best
+
+
+def test_many_marked_rays(api_mod):
+    """Level boxes that overlap: most rays hit two instances in the same place, and are traced
+    again in the instance order. A world traversal and a second one of as much work as the other
+    way's cost at most twice the time."""
+    world, walked = _both_ways(api_mod, _boxes(2000, 2048, 2048, True))
+    assert world < 2 * walked, (world, walked)

@@ -36,6 +36,7 @@ __global__ void k_plan(Ctrl* c, unsigned int capacity, int mode, unsigned int ta
     c->nOut = 0;
     c->extendHead = 0;
     c->nRetrace = 0;
+    c->retraceHead = 0;
     if (c->nActive) c->iterations += 1;
     if (mode == kPlanTail || mode == kPlanTailIfFew) c->nTail = c->nActive;
 }

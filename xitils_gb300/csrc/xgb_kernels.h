@@ -76,6 +76,7 @@ struct Ctrl {
     unsigned int nRetrace;         // rays whose hits the instance order decides (k_trace_world)
     unsigned int nShadowDue;       // shadow rays of the previous shade launch, traced beside the next rays
     unsigned int nTail;            // paths the next tail launch finishes (0: it does nothing)
+    unsigned int retraceHead;      // rays of nRetrace that k_retrace has taken
     unsigned long long extensionRays;
     unsigned long long shadowRays;
     unsigned long long iterations;
