@@ -59,3 +59,11 @@ def test_many_marked_rays(api_mod):
     way's cost at most twice the time."""
     world, walked = _both_ways(api_mod, _boxes(2000, 2048, 2048, True))
     assert world < 2 * walked, (world, walked)
+
+
+@pytest.mark.parametrize("n", [17, 300])
+def test_no_large_tail_over_the_top_level(api_mod, n):
+    """Without lights, 500,000 camera paths: many instances stay on the wavefront until 65,536
+    paths are left."""
+    world, walked = _both_ways(api_mod, _boxes(n, 724, 700, False))
+    assert world < 1.25 * walked, (world, walked)

@@ -237,9 +237,13 @@ void launchPlan(Ctrl* ctrl, unsigned int capacity, cudaStream_t s, int mode = kP
 // ones: with 65,536 / 262,144 / 524,288 / 1,048,576 paths the terrain took at 134,000 camera paths 0.585 /
 // 0.450 / 0.436 / 0.440, 524,000 1.62 / 1.17 / 1.14 / 1.14, 700,000 1.70 / 1.45 / 1.31 / 1.53, 2.1
 // million 2.35 / 2.36 / 2.06 / 2.00, 67 million 30.5 / 30.4 / 30.4 / 30.4; the Cornell box at 262,000 paths
-// 0.58 / 1.30 / 1.29 with its light, so scenes with lights keep 65,536.
+// 0.58 / 1.30 / 1.29 with its light, so scenes with lights keep 65,536. Interiors lit by their sky
+// through a window, eleven to fourteen vertices per path, gain too (65,536 / 524,288: an empty
+// room at 262,144 camera paths 1.37 / 0.97, with 200,000 triangles 7.3 / 5.0, 524,000 10.3 / 8.5).
+// Not so scenes that are walked over their top-level BVH, one thread per path, where the wavefront
+// has the world BVH: 30 boxes on the terrain, 507,000 paths, 0.91 / 2.15, 300 boxes 1.73 / 7.2.
 inline unsigned int tailMaxPaths(const SceneDev& sc) {
-    return (sc.nested & 1) ? 4096u : sc.nLights == 0 && !sc.nested ? 524288u : 65536u;
+    return (sc.nested & 1) ? 4096u : sc.nLights == 0 && !sc.nested && sc.listed ? 524288u : 65536u;
 }
 // Finishes the ctrl->nTail paths of `in`; those that outlive the launch's bound go to `out` (tail.cuh).
 void launchTail(const SceneDev& sc, const RenderParams& rp, PathQueue in, PathQueue out, Ctrl* ctrl, int numSMs,
