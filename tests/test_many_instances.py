@@ -1,4 +1,4 @@
-"""Scenes of many instances take no longer with a world BVH and tail launches than without:
+"""Renders take no longer with a world BVH and tail launches than without:
 traversal limits other than the defaults keep a scene on the kernels that walk the instances, so the
 same render is timed both ways in turn, the fastest of a few, and compared with it (films
 as in test_tail.py).
@@ -9,6 +9,7 @@ import numpy as np
 import pytest
 
 from xitils_gb300 import scenes
+from xitils_gb300.scene import SKY_UNIFORM, IntegratorParams, SceneDesc
 from xitils_gb300.transform import scale, translate
 
 pytestmark = pytest.mark.gpu
@@ -37,8 +38,9 @@ def _boxes(n, width, height, level):
     return d
 
 
-def _both_ways(api, d):
+def _both_ways(api, d, layout="binary"):
     ctx = api.Context(0)
+    ctx.set_bvh_layout(layout)
     b = api.load_scene(ctx, d)
     best, films = [np.inf, np.inf], [None, None]
     for _ in range(6):
@@ -66,4 +68,34 @@ def test_no_large_tail_over_the_top_level(api_mod, n):
     """Without lights, 500,000 camera paths: many instances stay on the wavefront until 65,536
     paths are left."""
     world, walked = _both_ways(api_mod, _boxes(n, 724, 700, False))
+    assert world < 1.25 * walked, (world, walked)
+
+
+def _closed_room(width, height, max_depth):
+    """A room lit by its sky through a gap in a wall, with clouds of triangles in it."""
+    d = SceneDesc(name="closed_room", width=width, height=height, spp=1,
+                  params=IntegratorParams(max_depth=max_depth, rr_start=5, rr_prob=0.9, seed=3))
+    grey = d.diffuse([0.7, 0.7, 0.7])
+    for q in ([[0, 0, 0], [0, 0, 1], [1, 0, 1], [1, 0, 0]], [[0, 1, 0], [1, 1, 0], [1, 1, 1], [0, 1, 1]],
+              [[0, 0, 0], [0, 1, 0], [0, 1, 1], [0, 0, 1]], [[0, 0, 0], [1, 0, 0], [1, 1, 0], [0, 1, 0]],
+              [[0, 0, 1], [0, 1, 1], [1, 1, 1], [1, 0, 1]], [[1, 0, 0], [1, 0, 1], [1, 0.5, 1], [1, 0.5, 0]],
+              [[1, 0.8, 0], [1, 0.8, 1], [1, 1, 1], [1, 1, 0]]):
+        d.add_object(d.add_mesh(*scenes.quad(*q)), grey)
+    rng = np.random.default_rng(5)
+    for k in range(5):
+        c = rng.uniform(0.3, 0.7, 3) + rng.normal(scale=0.15, size=(6000, 1, 3))
+        pos = (c + rng.normal(scale=0.02, size=(6000, 3, 3))).reshape(-1, 3).astype(np.float32)
+        m = d.add_mesh(pos, np.arange(18000, dtype=np.int32))
+        d.add_object(m, grey, translate(0.01 * k, 0, 0) if k % 2 else None)
+    d.set_sky(SKY_UNIFORM, (0.8, 0.9, 1.0))
+    d.set_camera(scenes.look_at((0.15, 0.6, 0.1), (0.6, 0.3, 0.8), (0, 1, 0)), 1.1, height / width)
+    return d
+
+
+@pytest.mark.parametrize("layout", ["binary", "wide8"])
+@pytest.mark.parametrize("max_depth", [4, 10])
+def test_no_large_tail_while_paths_stay(api_mod, max_depth, layout):
+    """No lights either, but most paths live through a vertex: they stay on the wavefront until
+    65,536 are left."""
+    world, walked = _both_ways(api_mod, _closed_room(640, 420, max_depth), layout)
     assert world < 1.25 * walked, (world, walked)

@@ -1619,7 +1619,8 @@ xgb_status xgb_render(xgb_scene* s, const xgb_integrator_params* params, xgb_fil
     // nor while profiling, which attributes every stage; traversal limits other than the
     // defaults count the steps of the wavefront's kernels.
     const bool tail = !gd && !prof && s->maxSteps == kDefaultMaxSteps && s->stackLimit == kMaxStackLimit;
-    const unsigned int tailMax = tailMaxPaths(s->sd);
+    const unsigned int tailMax = tailMaxPaths(s->sd, ctx->numSMs), tailOpen = tailOpenPaths(s->sd, ctx->numSMs);
+    bool open = true;  // fewer than half of the paths lived through the last vertex (or none has been)
     // Once every camera path has started, the fewer paths are left the sooner the counters
     // are read again, so that the tail starts in time (a read costs 20 us).
     bool ending = total <= cap;
@@ -1639,7 +1640,9 @@ xgb_status xgb_render(xgb_scene* s, const xgb_integrator_params* params, xgb_fil
             launchGenerate(s->sd, rp, s->rb.q[parity], s->ctrl, gShade, st);
             launches += 2;
         }
-        const int nIter = direct ? 0 : !tail || !ending || left > 4ull * tailMax ? kIterPerCheck : left > 2ull * tailMax ? 4 : 2;
+        const unsigned int few = open ? tailOpen : tailMax;
+        const int nIter = direct ? 0 : !tail || !ending || left > 4ull * few ? kIterPerCheck : left > 2ull * few ? 4
+                        : guard == 0 && left <= few ? 1 : 2;
         for (int k = 0; k < nIter; ++k) {
             PathQueue& X = s->rb.q[parity];
             PathQueue& Y = s->rb.q[parity ^ 1];
@@ -1676,7 +1679,7 @@ xgb_status xgb_render(xgb_scene* s, const xgb_integrator_params* params, xgb_fil
             parity ^= 1;
         }
         if (tail) {
-            if (!direct) { launchPlan(s->ctrl, cap, st, kPlanTailIfFew, tailMax); ++launches; }
+            if (!direct) { launchPlan(s->ctrl, cap, st, kPlanTailIfFew, tailMax, tailOpen); ++launches; }
             launchTail(s->sd, rp, s->rb.q[parity], s->rb.q[parity ^ 1], s->ctrl, ctx->numSMs, st);
             ++launches;
         }
@@ -1686,6 +1689,7 @@ xgb_status xgb_render(xgb_scene* s, const xgb_integrator_params* params, xgb_fil
         if (tail && s->ctrlHost->nTail) parity ^= 1;
         ending = s->ctrlHost->nextPath >= s->ctrlHost->totalPaths;
         left = s->ctrlHost->nOut;
+        open = 2ull * left < s->ctrlHost->nActive;
         if (prof) {
             // stages: plan, generate, extend, [guide inference], shade, shadow
             for (int k = 0; k < kIterPerCheck; ++k) {

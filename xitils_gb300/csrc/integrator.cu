@@ -16,7 +16,7 @@
 
 namespace xgb {
 
-__global__ void k_plan(Ctrl* c, unsigned int capacity, int mode, unsigned int tailMax) {
+__global__ void k_plan(Ctrl* c, unsigned int capacity, int mode, unsigned int tailMax, unsigned int tailOpen) {
     if (mode == kPlanShadow || mode == kPlanWave) {
         c->nShadowDue = c->nShadow;
         c->nShadow = 0;
@@ -26,7 +26,9 @@ __global__ void k_plan(Ctrl* c, unsigned int capacity, int mode, unsigned int ta
     unsigned int nCont = c->nOut;
     unsigned long long remain = c->totalPaths - c->nextPath;
     c->nTail = 0;
-    if (mode == kPlanTailIfFew && (remain != 0 || nCont == 0 || nCont > tailMax)) return;
+    // nActive: the paths before the last vertex
+    const bool few = nCont <= tailMax || (nCont <= tailOpen && 2u * nCont < c->nActive);
+    if (mode == kPlanTailIfFew && (remain != 0 || nCont == 0 || !few)) return;
     unsigned long long room = capacity - nCont;
     unsigned int nNew = (unsigned int)(remain < room ? remain : room);
     c->firstNew = c->nextPath;
@@ -155,8 +157,8 @@ void SideLane::destroy() {
     *this = SideLane{};
 }
 
-void launchPlan(Ctrl* ctrl, unsigned int capacity, cudaStream_t s, int mode, unsigned int tailMax) {
-    k_plan<<<1, 1, 0, s>>>(ctrl, capacity, mode, tailMax);
+void launchPlan(Ctrl* ctrl, unsigned int capacity, cudaStream_t s, int mode, unsigned int tailMax, unsigned int tailOpen) {
+    k_plan<<<1, 1, 0, s>>>(ctrl, capacity, mode, tailMax, tailOpen);
 }
 
 void launchGenerate(const SceneDev& sc, const RenderParams& rp, PathQueue q, Ctrl* ctrl, int grid, cudaStream_t s) {

@@ -23,6 +23,7 @@ namespace xgb {
 constexpr int kTailBlock = 128;
 constexpr int kTailBlocksPerSM = 4;  // 128 registers
 constexpr int kTailVertices = 1024;
+static_assert(kTailBlocksPerSM * kTailBlock == (int)kTailThreadsPerSM, "threads of a full grid");
 
 template <class J, int NESTED>
 __global__ void __launch_bounds__(kTailBlock, kTailBlocksPerSM) k_tail(J jobs, PathQueue in, PathQueue out, Ctrl* ctrl) {

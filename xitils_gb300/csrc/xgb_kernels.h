@@ -204,7 +204,8 @@ int launchShadowBatch(const BatchView& b, ShadowQueue sq, PathQueue out, Ctrl* c
 // Queue bookkeeping of an iteration. mode kPlanWave: a wavefront iteration; kPlanTail: the
 // new camera paths go to a tail launch; kPlanTailIfFew: nothing happens (and the tail launch
 // that follows does nothing) unless every camera path has started and at most tailMax paths
-// are left, which then go to the tail launch.
+// are left, or at most tailOpen and fewer than half of those before the last vertex; they then
+// go to the tail launch.
 // A wavefront iteration also hands the shadow rays of the last shade launch to launchShadow;
 // kPlanShadow does only that.
 enum PlanMode : int { kPlanWave = 0, kPlanTail = 1, kPlanTailIfFew = 2, kPlanShadow = 3 };
@@ -226,24 +227,34 @@ struct SideLane {
     void end() const { cudaEventRecord(join, stream); }
     void wait(cudaStream_t s) const { cudaStreamWaitEvent(s, join, 0); }
 };
-void launchPlan(Ctrl* ctrl, unsigned int capacity, cudaStream_t s, int mode = kPlanWave, unsigned int tailMax = 0);
+void launchPlan(Ctrl* ctrl, unsigned int capacity, cudaStream_t s, int mode = kPlanWave, unsigned int tailMax = 0,
+                unsigned int tailOpen = 0);
 // Paths up to which a tail launch beats the remaining wavefront iterations. Measured with
 // 4,096 / 16,384 / 65,536 / 131,072 paths (none: no tail launches), ms per call: occluded
 // room 384^2 x 8 55.6 / 51.1 / 46.6 / 45.9 (73.8), shell-mapped cloth 320^2 x 4 27.3 / 23.8 /
 // 21.5 / 22.6 (40.9), its SVBRDF variant 26.7 / 24.4 / 23.0 / 25.7 (33.4); microfacet normal
 // mapping, whose walks of up to 100 facets per BSDF call make a warp's lanes wait for one
 // another and its code overflow the instruction cache, 400^2 x 4 6.4 / 7.3 / 10.3 / 10.3 (6.5).
-// Scenes without lights, whose paths leave for the sky after a vertex or two, gain from larger
-// ones: with 65,536 / 262,144 / 524,288 / 1,048,576 paths the terrain took at 134,000 camera paths 0.585 /
-// 0.450 / 0.436 / 0.440, 524,000 1.62 / 1.17 / 1.14 / 1.14, 700,000 1.70 / 1.45 / 1.31 / 1.53, 2.1
-// million 2.35 / 2.36 / 2.06 / 2.00, 67 million 30.5 / 30.4 / 30.4 / 30.4; the Cornell box at 262,000 paths
-// 0.58 / 1.30 / 1.29 with its light, so scenes with lights keep 65,536. Interiors lit by their sky
-// through a window, eleven to fourteen vertices per path, gain too (65,536 / 524,288: an empty
-// room at 262,144 camera paths 1.37 / 0.97, with 200,000 triangles 7.3 / 5.0, 524,000 10.3 / 8.5).
-// Not so scenes that are walked over their top-level BVH, one thread per path, where the wavefront
-// has the world BVH: 30 boxes on the terrain, 507,000 paths, 0.91 / 2.15, 300 boxes 1.73 / 7.2.
-inline unsigned int tailMaxPaths(const SceneDev& sc) {
-    return (sc.nested & 1) ? 4096u : sc.nLights == 0 && !sc.nested && sc.listed ? 524288u : 65536u;
+// Scenes without lights whose instances are walked as a list take larger ones, up to
+// tailOpen, where paths leave fast: fewer than half of them lived through the last vertex
+// (under an open sky 10 to 25 %). With 65,536 / 262,144 / 524,288 / 1,048,576 paths the terrain took
+// at 700,000 camera paths 1.70 / 1.45 / 1.31 / 1.53, 2.1 million 2.35 / 2.36 / 2.06 / 2.00, 67 million
+// 30.5 / 30.4 / 30.4 / 30.4. In closed rooms most paths stay, and the wavefront is faster: with five
+// clouds of triangles, 204,000 camera paths, 3.2 with 65,536, 5.8 with 524,288, 3.6 without tail
+// launches. So is it where a tail thread would walk a top-level BVH and the wavefront has the world
+// BVH (30 boxes on the terrain, 507,000 paths: 0.91 / 2.15; 300 boxes 1.73 / 7.2), and in scenes
+// with lights (Cornell box, 262,000 paths: 0.58 / 1.30). A scene of one instance takes two paths
+// per thread of a full grid (155,648) whether they stay or not: the terrain at 134,000 camera paths
+// 0.51 -> 0.31, closed rooms as one mesh 0.17 to 0.86 of the time without tail launches, but
+// up to 1.34 of it at 320,000. Over 380 random scenes without lights, 66,000 to 2 million paths, the worst call
+// takes 0.96 of the time without tail launches, the mean 0.44.
+constexpr unsigned int kTailThreadsPerSM = 512;
+inline unsigned int tailMaxPaths(const SceneDev& sc, int numSMs) {
+    if (sc.nested & 1) return 4096u;
+    return sc.nLights == 0 && !sc.nested && sc.listed && sc.nInstances == 1 ? 2u * kTailThreadsPerSM * (unsigned int)numSMs : 65536u;
+}
+inline unsigned int tailOpenPaths(const SceneDev& sc, int numSMs) {
+    return sc.nLights == 0 && !sc.nested && sc.listed ? 524288u : tailMaxPaths(sc, numSMs);
 }
 // Finishes the ctrl->nTail paths of `in`; those that outlive the launch's bound go to `out` (tail.cuh).
 void launchTail(const SceneDev& sc, const RenderParams& rp, PathQueue in, PathQueue out, Ctrl* ctrl, int numSMs,
