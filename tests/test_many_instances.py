@@ -99,3 +99,29 @@ def test_no_large_tail_while_paths_stay(api_mod, max_depth, layout):
     65,536 are left."""
     world, walked = _both_ways(api_mod, _closed_room(640, 420, max_depth), layout)
     assert world < 1.25 * walked, (world, walked)
+
+
+def _metal_room(boxes):
+    """A closed room with a ceiling light, of metal, so that paths are long."""
+    d = _closed_room(128, 127, 10)
+    d.spp = 4
+    d.meshes, d.objects = d.meshes[:7], d.objects[:7]
+    metal = d.metal(0.3, [0.8, 0.7, 0.6])
+    for o in d.objects:
+        o.material = metal
+    cpos, cidx = scenes.unit_cube_mesh()
+    cube = d.add_mesh(cpos, cidx)
+    rng = np.random.default_rng(4)
+    for _ in range(boxes):
+        c = rng.uniform(0.1, 0.9, 3)
+        d.add_object(cube, metal, translate(*c) * scale(0.25, 0.25, 0.25))
+    d.add_object(d.add_mesh(*scenes.quad([0.4, 0.99, 0.4], [0.6, 0.99, 0.4], [0.6, 0.99, 0.6], [0.4, 0.99, 0.6])), d.emission([8.0, 8.0, 8.0]))
+    return d
+
+
+@pytest.mark.parametrize("boxes,layout", [(9, "binary"), (16, "binary"), (2, "wide8"), (4, "wide8")])
+def test_no_tail_of_65536_over_the_top_level_or_wide_nodes(api_mod, boxes, layout):
+    """65,024 paths that stay: walked over a top-level BVH, or through 8-wide nodes, by one thread
+    each, they are slower than on the wavefront until 16,384 are left."""
+    world, walked = _both_ways(api_mod, _metal_room(boxes), layout)
+    assert world < 1.25 * walked, (world, walked)

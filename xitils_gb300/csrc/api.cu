@@ -1619,7 +1619,7 @@ xgb_status xgb_render(xgb_scene* s, const xgb_integrator_params* params, xgb_fil
     // nor while profiling, which attributes every stage; traversal limits other than the
     // defaults count the steps of the wavefront's kernels.
     const bool tail = !gd && !prof && s->maxSteps == kDefaultMaxSteps && s->stackLimit == kMaxStackLimit;
-    const unsigned int tailMax = tailMaxPaths(s->sd, ctx->numSMs), tailOpen = tailOpenPaths(s->sd, ctx->numSMs);
+    const unsigned int tailMax = tailMaxPaths(s->sd, ctx->numSMs), tailOpen = tailOpenPaths(s->sd);
     bool open = true;  // fewer than half of the paths lived through the last vertex (or none has been)
     // Once every camera path has started, the fewer paths are left the sooner the counters
     // are read again, so that the tail starts in time (a read costs 20 us).

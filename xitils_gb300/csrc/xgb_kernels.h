@@ -235,26 +235,36 @@ void launchPlan(Ctrl* ctrl, unsigned int capacity, cudaStream_t s, int mode = kP
 // 21.5 / 22.6 (40.9), its SVBRDF variant 26.7 / 24.4 / 23.0 / 25.7 (33.4); microfacet normal
 // mapping, whose walks of up to 100 facets per BSDF call make a warp's lanes wait for one
 // another and its code overflow the instruction cache, 400^2 x 4 6.4 / 7.3 / 10.3 / 10.3 (6.5).
-// Scenes without lights whose instances are walked as a list take larger ones, up to
-// tailOpen, where paths leave fast: fewer than half of them lived through the last vertex
-// (under an open sky 10 to 25 %). With 65,536 / 262,144 / 524,288 / 1,048,576 paths the terrain took
+// A tail thread walks a top-level BVH, or 8-wide nodes, by itself and slowly: those scenes take
+// 16,384 where paths stay (metal rooms of 18 and 11 instances, 65,024 camera paths: 3.1 and 1.4 ms
+// per call with 65,536, 1.0 and 0.7 without tail launches). Over 130 random scenes of each kind,
+// 6,000 to 200,000 paths, the time of that without tail launches is 0.25 / 0.38 in the mean, at
+// worst 0.86 / 0.91 (with 65,536 for all 0.28 / 0.36, at worst 1.04 / 1.47); of 2 to 16 instances
+// and binary meshes, with 65,536, 0.34, above 1 in two of 675.
+//
+// Up to tailOpen where paths leave fast, fewer than half of them having lived through the last
+// vertex (under an open sky 10 to 25 % do): 65,536, and 524,288 in scenes without lights whose
+// instances are walked as a list. With 65,536 / 262,144 / 524,288 / 1,048,576 paths the terrain took
 // at 700,000 camera paths 1.70 / 1.45 / 1.31 / 1.53, 2.1 million 2.35 / 2.36 / 2.06 / 2.00, 67 million
 // 30.5 / 30.4 / 30.4 / 30.4. In closed rooms most paths stay, and the wavefront is faster: with five
 // clouds of triangles, 204,000 camera paths, 3.2 with 65,536, 5.8 with 524,288, 3.6 without tail
-// launches. So is it where a tail thread would walk a top-level BVH and the wavefront has the world
-// BVH (30 boxes on the terrain, 507,000 paths: 0.91 / 2.15; 300 boxes 1.73 / 7.2), and in scenes
-// with lights (Cornell box, 262,000 paths: 0.58 / 1.30). A scene of one instance takes two paths
-// per thread of a full grid (155,648) whether they stay or not: the terrain at 134,000 camera paths
-// 0.51 -> 0.31, closed rooms as one mesh 0.17 to 0.86 of the time without tail launches, but
-// up to 1.34 of it at 320,000. Over 380 random scenes without lights, 66,000 to 2 million paths, the worst call
-// takes 0.96 of the time without tail launches, the mean 0.44.
+// launches. So is it over a top-level BVH (30 boxes on the terrain, 507,000 paths: 0.91 / 2.15;
+// 300 boxes 1.73 / 7.2), and with lights (Cornell box, 262,000 paths: 0.58 / 1.30).
+//
+// A scene of one instance without lights takes two paths per thread of a full grid (155,648)
+// whether they stay or not: the terrain at 134,000 camera paths 0.51 -> 0.31, closed rooms as one
+// mesh 0.17 to 0.86 of the time without tail launches, but up to 1.34 of it at 320,000. Over 380
+// random scenes without lights, 66,000 to 2 million paths, a call takes 0.44 of the time without tail
+// launches in the mean and 0.99 at worst.
 constexpr unsigned int kTailThreadsPerSM = 512;
 inline unsigned int tailMaxPaths(const SceneDev& sc, int numSMs) {
     if (sc.nested & 1) return 4096u;
-    return sc.nLights == 0 && !sc.nested && sc.listed && sc.nInstances == 1 ? 2u * kTailThreadsPerSM * (unsigned int)numSMs : 65536u;
+    if (!sc.listed || sc.blasLayout != 0) return 16384u;
+    return sc.nLights == 0 && !sc.nested && sc.nInstances == 1 ? 2u * kTailThreadsPerSM * (unsigned int)numSMs : 65536u;
 }
-inline unsigned int tailOpenPaths(const SceneDev& sc, int numSMs) {
-    return sc.nLights == 0 && !sc.nested && sc.listed ? 524288u : tailMaxPaths(sc, numSMs);
+inline unsigned int tailOpenPaths(const SceneDev& sc) {
+    if (sc.nested & 1) return 4096u;
+    return sc.nLights == 0 && !sc.nested && sc.listed ? 524288u : 65536u;
 }
 // Finishes the ctrl->nTail paths of `in`; those that outlive the launch's bound go to `out` (tail.cuh).
 void launchTail(const SceneDev& sc, const RenderParams& rp, PathQueue in, PathQueue out, Ctrl* ctrl, int numSMs,
