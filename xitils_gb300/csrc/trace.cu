@@ -349,6 +349,7 @@ constexpr unsigned int kFetchLanes = 16, kFetchLanesMore = 24;
 // A step of the loop takes a ray as far as the warp's lanes go on together, so that full
 // warps, filled up at once, that test triangles when no lane is looking any more need the
 // fewest steps: they keep a ray inside a bound that it met on such a warp.
+constexpr unsigned int kCountedLanes = 64;  // all, and none waits for another
 struct RayClaims {
     unsigned int* head;
     unsigned int n, lanes, next, enough;
@@ -356,7 +357,7 @@ struct RayClaims {
     __device__ __forceinline__ RayClaims(unsigned int* h, unsigned int count, unsigned int fetchLanes, bool counted)
         : head(h), n(count), next(0) {
         const unsigned int warps = gridDim.x * (kTraceBlock / 32);
-        lanes = counted ? 32u : min(32u, (n + warps - 1u) / warps);
+        lanes = counted ? kCountedLanes : min(32u, (n + warps - 1u) / warps);
         enough = counted ? 1u : min(fetchLanes, lanes);
     }
     // The lanes that want a ray (0: none, or not yet worth the trip).
@@ -413,7 +414,7 @@ __global__ void __launch_bounds__(kTraceBlock, SHELL ? 7 : 8) k_trace_flat2(S sc
     int job = 0;
     const int lane = threadIdx.x & 31;
     RayClaims claims(head, n, kBatch || scenes.scene(0).large ? kFetchLanes : kFetchLanesMore, scenes.counted());
-    const int looking = claims.lanes == 32u && !scenes.counted() ? kLookingLanes<SHELL> : 1;
+    const int looking = claims.lanes == 32u ? kLookingLanes<SHELL> : 1;
     int stack[kStackDepth];
     int sp = 0;
     int nodeAddr = kSentinel, leafAddr = 0;
@@ -618,7 +619,7 @@ __global__ void __launch_bounds__(kTraceBlock, (WorldTraits<S, ENTER>::kMinBlock
     if (n <= kTeamQueue && scenes.teams()) return;  // k_trace_team's
     unsigned int* head = ANY ? &ctrl->shadowHead : &ctrl->extendHead;
     RayClaims claims(head, n, ANY ? kFetchLanes : kFetchLanesMore, scenes.counted());
-    const int looking = claims.lanes == 32u && !scenes.counted() ? kLookingLanes<SHELL> : 1;
+    const int looking = claims.lanes == 32u ? kLookingLanes<SHELL> : 1;
     bool holds = false;  // the lane has a ray
     // one scene: its BVH for every ray; a batch: the current ray's
     const Node2* nodes = kBatch ? nullptr : scenes.scene(0).world.nodes;
