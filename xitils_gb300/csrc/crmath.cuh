@@ -304,7 +304,9 @@ XGB_CR_NOINLINE static __host__ __device__ float expDouble(float x) { return (fl
 XGB_CR_NOINLINE static __host__ __device__ float logDouble(float x) { return (float)log((double)x); }
 
 // a b - c d as the FP64 expression rounds it, (float)((double)a * b - (double)c * d): both
-// products and their difference as exact sums of floats, then one rounding. Measured
+// products and their difference as exact sums of floats, then one rounding. That holds
+// while the products neither overflow nor fall under 2^-102, where the low half of an
+// exact product is lost: the callers pass unit vectors. Measured
 // where it matters: the cross products of the samplers' frames, 31 FP64-pipe
 // instructions per path of the terrain's shading at a sixteenth of an SM's issue
 // rate each (61 % FP64 pipe; see k_shade in shade.cuh).

@@ -1,8 +1,9 @@
 // Extension (closest-hit) and shadow (any-hit) kernels of the wavefront.
 //
-// Both are persistent: a grid of (SMs x resident blocks) threads where each
-// warp claims 32 queue entries at a time with one atomicAdd, so the grid drains
-// queues of any length without a relaunch per batch.
+// Both are persistent: a grid of (SMs x resident blocks) whose warps claim queue entries
+// with one atomicAdd for all their lanes that want one -- 32 at a time in the general
+// kernels, as many as are free in the per-lane ones (RayClaims) -- so the grid drains queues
+// of any length without a relaunch per batch.
 #include <map>
 #include <mutex>
 
@@ -594,9 +595,9 @@ __global__ void __launch_bounds__(kTraceBlock, SHELL ? 7 : 8) k_trace_flat2(S sc
 // accepted or refused within that margin marks the ray, and a marked ray is traced again in the
 // instance order (k_retrace).
 //
-// Ten blocks per SM (48 registers, no spills) rather than the nine that 55 registers
-// allow: the terrain's traversal ran 2.5 % faster; twelve (40 registers) spill and
-// ran 7 % slower. A batch (S = BatchScenes) reads its ray's BVH when it fetches the ray.
+// Ten blocks per SM (48 registers, 28 bytes of spills outside the node loop) rather than the
+// nine that 55 registers allow: the terrain's traversal ran 2.5 % faster; twelve (40
+// registers) spill more and ran 7 % slower. A batch (S = BatchScenes) reads its ray's BVH when it fetches the ray.
 constexpr int kReturn = kSentinel - 1;
 constexpr int kWorldDepth = kStackDepth + kTlasStack;  // a mesh's entries and the top level's
 constexpr int kWorldStack = kWorldDepth + 2;           // and a return
