@@ -101,10 +101,10 @@ def test_no_large_tail_while_paths_stay(api_mod, max_depth, layout):
     assert world < 1.25 * walked, (world, walked)
 
 
-def _metal_room(boxes):
+def _metal_room(boxes, spp):
     """A closed room with a ceiling light, of metal, so that paths are long."""
     d = _closed_room(128, 127, 10)
-    d.spp = 4
+    d.spp = spp
     d.meshes, d.objects = d.meshes[:7], d.objects[:7]
     metal = d.metal(0.3, [0.8, 0.7, 0.6])
     for o in d.objects:
@@ -119,9 +119,9 @@ def _metal_room(boxes):
     return d
 
 
-@pytest.mark.parametrize("boxes,layout", [(9, "binary"), (16, "binary"), (2, "wide8"), (4, "wide8")])
-def test_no_tail_of_65536_over_the_top_level_or_wide_nodes(api_mod, boxes, layout):
-    """65,024 paths that stay: walked over a top-level BVH, or through 8-wide nodes, by one thread
-    each, they are slower than on the wavefront until 16,384 are left."""
-    world, walked = _both_ways(api_mod, _metal_room(boxes), layout)
+@pytest.mark.parametrize("boxes,layout,spp", [(9, "binary", 4), (16, "binary", 4), (16, "binary", 1), (30, "binary", 1), (2, "wide8", 4), (4, "wide8", 4)])
+def test_no_large_tail_over_the_top_level_or_wide_nodes(api_mod, boxes, layout, spp):
+    """16,256 and 65,024 paths that stay: walked over a top-level BVH, or through 8-wide nodes, by one
+    thread each, they are slower than on the wavefront until 8,192 are left."""
+    world, walked = _both_ways(api_mod, _metal_room(boxes, spp), layout)
     assert world < 1.25 * walked, (world, walked)

@@ -236,11 +236,12 @@ void launchPlan(Ctrl* ctrl, unsigned int capacity, cudaStream_t s, int mode = kP
 // mapping, whose walks of up to 100 facets per BSDF call make a warp's lanes wait for one
 // another and its code overflow the instruction cache, 400^2 x 4 6.4 / 7.3 / 10.3 / 10.3 (6.5).
 // A tail thread walks a top-level BVH, or 8-wide nodes, by itself and slowly: those scenes take
-// 16,384 where paths stay (metal rooms of 18 and 11 instances, 65,024 camera paths: 3.1 and 1.4 ms
-// per call with 65,536, 1.0 and 0.7 without tail launches). Over 130 random scenes of each kind,
-// 6,000 to 200,000 paths, the time of that without tail launches is 0.25 / 0.38 in the mean, at
-// worst 0.86 / 0.91 (with 65,536 for all 0.28 / 0.36, at worst 1.04 / 1.47); of 2 to 16 instances
-// and binary meshes, with 65,536, 0.34, above 1 in two of 675.
+// 8,192 where paths stay (metal rooms of 18 and 11 instances, 65,024 camera paths: 3.1 and 1.4 ms
+// per call with 65,536, 1.0 and 0.7 without tail launches; of 18 and 25 instances, 16,256 camera
+// paths: 1.57 and 1.77 with 16,384, 0.80 and 0.87 with 8,192, 1.20 and 1.39 without). Over 130
+// random scenes of each kind, 6,000 to 200,000 paths, a call takes 0.25 / 0.41 of the time without
+// tail launches in the mean, at worst 0.84 / 0.96 (with 65,536 for all 0.28 / 0.36, at worst 1.04 /
+// 1.47); of 2 to 16 instances and binary meshes, with 65,536, 0.34, above 1 in two of 675.
 //
 // Up to tailOpen where paths leave fast, fewer than half of them having lived through the last
 // vertex (under an open sky 10 to 25 % do): 65,536, and 524,288 in scenes without lights whose
@@ -259,7 +260,7 @@ void launchPlan(Ctrl* ctrl, unsigned int capacity, cudaStream_t s, int mode = kP
 constexpr unsigned int kTailThreadsPerSM = 512;
 inline unsigned int tailMaxPaths(const SceneDev& sc, int numSMs) {
     if (sc.nested & 1) return 4096u;
-    if (!sc.listed || sc.blasLayout != 0) return 16384u;
+    if (!sc.listed || sc.blasLayout != 0) return 8192u;
     return sc.nLights == 0 && !sc.nested && sc.nInstances == 1 ? 2u * kTailThreadsPerSM * (unsigned int)numSMs : 65536u;
 }
 inline unsigned int tailOpenPaths(const SceneDev& sc) {
