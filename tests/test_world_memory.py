@@ -1,7 +1,7 @@
 """The world BVH of a scene of several instances is a copy that may be left out: it leaves
 the memory that a program had before for its queues, films and tensors.
 
-The device is filled up to a known rest (one allocation, of the size that the driver says is
+The device is filled up to a known rest (one allocation, of the size that CUDA reports as
 free less that rest). Two meshes of 1.2 million triangles have copies of 269 MB: with 1.6 GB
 left they are not made; with 2.5 GB left they are, and a render or a batch whose queues
 need 2.44 GB gives them back. Films equal those of the same calls with room for everything (the order
