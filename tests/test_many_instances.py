@@ -125,3 +125,24 @@ def test_no_large_tail_over_the_top_level_or_wide_nodes(api_mod, boxes, layout, 
     thread each, they are slower than on the wavefront until 8,192 are left."""
     world, walked = _both_ways(api_mod, _metal_room(boxes, spp), layout)
     assert world < 1.25 * walked, (world, walked)
+
+
+@pytest.mark.parametrize("make,first_is_open", [(lambda: _boxes(0, 600, 500, False), True), (lambda: _closed_room(600, 500, 6), False)])
+def test_calls_of_an_open_scene_are_alike(api_mod, make, first_is_open):
+    """A scene's first call asks after a vertex whether its paths leave, a later one may know: the same
+    paths and rays, and films as in test_tail.py."""
+    api = api_mod
+    ctx = api.Context(0)
+    d = make()
+    b = api.load_scene(ctx, d)
+    films, counts = [], []
+    for _ in range(3):
+        rt = api.RenderTarget(ctx, d.width, d.height)
+        rt.render(b.scene, d.spp, d.params)
+        films.append(rt.download())
+        s = b.scene.stats()
+        counts.append((s["paths"], s["extension_rays"], s["shadow_rays"]))
+    assert (counts[0][1] < 2 * counts[0][0]) == first_is_open
+    assert counts[1] == counts[0] and counts[2] == counts[0]
+    for f in films[1:]:
+        np.testing.assert_allclose(f, films[0], rtol=1e-4, atol=1e-6 * float(films[0].mean()))
