@@ -129,20 +129,24 @@ def test_no_large_tail_over_the_top_level_or_wide_nodes(api_mod, boxes, layout, 
 
 @pytest.mark.parametrize("make,first_is_open", [(lambda: _boxes(0, 600, 500, False), True), (lambda: _closed_room(600, 500, 6), False)])
 def test_calls_of_an_open_scene_are_alike(api_mod, make, first_is_open):
-    """A scene's first call asks after a vertex whether its paths leave, a later one may know: the same
-    paths and rays, and films as in test_tail.py."""
+    """A scene's first call asks after a vertex whether its paths leave, a later one, or one into a film
+    of such a scene, may know: the same paths and rays, and films as in test_tail.py."""
     api = api_mod
     ctx = api.Context(0)
     d = make()
+    kept = api.RenderTarget(ctx, d.width, d.height)
     b = api.load_scene(ctx, d)
     films, counts = [], []
-    for _ in range(3):
-        rt = api.RenderTarget(ctx, d.width, d.height)
+    for k in range(4):
+        rt = kept if k in (1, 2) else api.RenderTarget(ctx, d.width, d.height)
+        if k == 2:
+            b = api.load_scene(ctx, d)  # a new scene into a film that knows
+        rt.clear()
         rt.render(b.scene, d.spp, d.params)
         films.append(rt.download())
         s = b.scene.stats()
         counts.append((s["paths"], s["extension_rays"], s["shadow_rays"]))
     assert (counts[0][1] < 2 * counts[0][0]) == first_is_open
-    assert counts[1] == counts[0] and counts[2] == counts[0]
+    assert all(c == counts[0] for c in counts)
     for f in films[1:]:
         np.testing.assert_allclose(f, films[0], rtol=1e-4, atol=1e-6 * float(films[0].mean()))

@@ -236,6 +236,7 @@ struct xgb_film {
     void* d = nullptr;
     void* aov = nullptr;  // albedo plane then normal plane, same element type as d
     float* stage = nullptr;  // packed float RGB(A) of one plane for downloads (allocated at the first one)
+    double vertsPerPath = 4.0;  // of the last call into it
 };
 
 struct xgb_guide {
@@ -301,6 +302,7 @@ struct xgb_scene {
     float4* pathAcc = nullptr;  // guide training: per-path contributions of a call
     unsigned long long pathAccCapacity = 0;
     double vertsPerPath = 4.0;  // extension rays per path of the last call (sizes the record rate, tells open scenes)
+    bool rendered = false;      // there was one
 };
 
 static xgb_status fail(xgb_ctx* ctx, xgb_status st, const std::string& msg) {
@@ -1619,11 +1621,17 @@ xgb_status xgb_render(xgb_scene* s, const xgb_integrator_params* params, xgb_fil
     // nor while profiling, which attributes every stage; traversal limits other than the
     // defaults count the steps of the wavefront's kernels.
     const bool tail = !gd && !prof && s->maxSteps == kDefaultMaxSteps && s->stackLimit == kMaxStackLimit;
-    // A scene walked as a list whose paths had fewer than two vertices in its last call is taken
-    // as open from the start; one that has not been rendered is asked after the first vertex
-    // (the terrain at 262,000 / 524,000 camera paths 0.51 / 0.77 ms so, 0.45 / 0.70 once known).
+    // A scene walked as a list whose paths had fewer than 2.4 vertices in its last call is taken
+    // as open from the start; one that has not been rendered, too, where those of the film's
+    // last call had (the frames of an animation, rebuilt one by one); any other is asked after the
+    // first vertex (the terrain at 262,000 / 524,000 camera paths 0.51 / 0.77 ms so, 0.45 / 0.70
+    // once known). Under an open sky 1.0 to 2.1 vertices per path were seen, in closed rooms 2.6 and
+    // more; where a depth limit or Russian roulette ends those sooner, the tail launch loses
+    // nothing (120 random rooms, 66,000 to 520,000 paths, at worst 1.01 of the time without one).
+    // Whichever kernels trace a path, the film is the same.
     const unsigned int tailOpen = tailOpenPaths(s->sd);
-    const unsigned int tailMax = s->sd.listed && s->vertsPerPath < 2.0 ? tailOpen : tailMaxPaths(s->sd, ctx->numSMs);
+    const bool wasOpen = s->sd.listed && (s->rendered ? s->vertsPerPath : film->vertsPerPath) < 2.4;
+    const unsigned int tailMax = wasOpen ? tailOpen : tailMaxPaths(s->sd, ctx->numSMs);
     bool open = true;  // fewer than half of the paths lived through the last vertex (or none has been)
     // Once every camera path has started, the fewer paths are left the sooner the counters
     // are read again, so that the tail starts in time (a read costs 20 us).
@@ -1736,7 +1744,10 @@ xgb_status xgb_render(xgb_scene* s, const xgb_integrator_params* params, xgb_fil
     }
     wait.done = true;
     const Ctrl& c = *s->ctrlHost;
-    if (c.pathsDone > 0) s->vertsPerPath = (double)c.extensionRays / (double)c.pathsDone;
+    if (c.pathsDone > 0) {
+        s->vertsPerPath = film->vertsPerPath = (double)c.extensionRays / (double)c.pathsDone;
+        s->rendered = true;
+    }
     s->last.paths = c.pathsDone;
     s->last.extension_rays = c.extensionRays;
     s->last.shadow_rays = c.shadowRays;
