@@ -7,6 +7,7 @@
 // Scene.h:40-55) instead of per sample. This file is compiled with
 // -ffp-contract=off so the host float arithmetic matches the reference's.
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
@@ -236,7 +237,7 @@ struct xgb_film {
     void* d = nullptr;
     void* aov = nullptr;  // albedo plane then normal plane, same element type as d
     float* stage = nullptr;  // packed float RGB(A) of one plane for downloads (allocated at the first one)
-    double vertsPerPath = 4.0;  // of the last call into it
+    std::atomic<double> vertsPerPath{4.0};  // of the last call into it (renders of several threads may share a film)
 };
 
 struct xgb_guide {
@@ -1630,7 +1631,7 @@ xgb_status xgb_render(xgb_scene* s, const xgb_integrator_params* params, xgb_fil
     // nothing (120 random rooms, 66,000 to 520,000 paths, at worst 1.01 of the time without one).
     // Whichever kernels trace a path, the film is the same.
     const unsigned int tailOpen = tailOpenPaths(s->sd);
-    const bool wasOpen = s->sd.listed && (s->rendered ? s->vertsPerPath : film->vertsPerPath) < 2.4;
+    const bool wasOpen = s->sd.listed && (s->rendered ? s->vertsPerPath : film->vertsPerPath.load()) < 2.4;
     const unsigned int tailMax = wasOpen ? tailOpen : tailMaxPaths(s->sd, ctx->numSMs);
     bool open = true;  // fewer than half of the paths lived through the last vertex (or none has been)
     // Once every camera path has started, the fewer paths are left the sooner the counters
@@ -1745,7 +1746,8 @@ xgb_status xgb_render(xgb_scene* s, const xgb_integrator_params* params, xgb_fil
     wait.done = true;
     const Ctrl& c = *s->ctrlHost;
     if (c.pathsDone > 0) {
-        s->vertsPerPath = film->vertsPerPath = (double)c.extensionRays / (double)c.pathsDone;
+        s->vertsPerPath = (double)c.extensionRays / (double)c.pathsDone;
+        film->vertsPerPath = s->vertsPerPath;
         s->rendered = true;
     }
     s->last.paths = c.pathsDone;
